@@ -37,6 +37,17 @@ __device__ __forceinline__ bool mbar_try_wait(uint64_t *bar, uint32_t parity) {
       : "memory");
   return ok != 0;
 }
+__device__ __forceinline__ bool mbar_try_wait_hint(uint64_t *bar, uint32_t parity, uint32_t hint_ns) {
+  uint32_t ok;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t}"
+      : "=r"(ok)
+      : "r"(smem_addr(bar)), "r"(parity), "r"(hint_ns)
+      : "memory");
+  return ok != 0;
+}
 __device__ __forceinline__ uint64_t global_ns() {
   uint64_t t;
   asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
@@ -52,6 +63,25 @@ __device__ __forceinline__ bool mbar_wait(uint64_t *bar, uint32_t parity, uint64
     if (mbar_try_wait(bar, parity)) return true;
     if ((n & 63u) == 0 && global_ns() - t0 > limit_ns) return false;
   }
+}
+// The same with the limit counted in tries (a few instructions, where the
+// timed loop would bloat an unrolled caller): each try suspends the thread
+// for at most about kSpinHintNs, so the limit is about 2 s.
+constexpr uint32_t kSpinTries = 1u << 20, kSpinHintNs = 2000;
+__device__ __forceinline__ bool mbar_spin(uint64_t *bar, uint32_t parity) {
+  uint32_t n = kSpinTries;
+  while (!mbar_try_wait_hint(bar, parity, kSpinHintNs))
+    if (--n == 0) return false;
+  return true;
+}
+// Moves registers between the warpgroups of a CTA (warpgroup-uniform).
+template <int N>
+__device__ __forceinline__ void setmaxnreg_inc() {
+  asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(N));
+}
+template <int N>
+__device__ __forceinline__ void setmaxnreg_dec() {
+  asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(N));
 }
 // Orders: the values in `v` have been produced (their loads have returned)
 // before any later volatile asm executes.

@@ -57,11 +57,10 @@ struct State {
   ShotDesc desc;                 // the shot (passed by value to every launch)
   ShotMaps maps;                 // its TMA descriptors
   int tile_rows = 12, stages = 5, zchunks = 0;
-  int grid = 0, nitems = 0, ntx = 0, nty = 0, chunk = 0;  // the FP32 launch's items
-  bool spread = false;       // the plan shares out its last round (segment list launch)
+  int ntx = 0, nty = 0;      // tiles in x and y
   int4 *seg = nullptr;       // the plan as work segments {x0, y0, z0, z1}
   int *cta_first = nullptr;  // [seg_grid + 1]: first segment of each CTA
-  int nseg = 0, seg_grid = 0;
+  int nseg = 0, grid = 0;
   long launches = 0;
   size_t dev_bytes = 0;
   int num_sms = 0;
@@ -438,8 +437,6 @@ struct Split {
   std::vector<int4> seg;
   std::vector<int> first;
   long max_cost = 0, total_cost = 0;
-  bool spread = false;  // false: uniform chunks of `len` planes, all round-robin
-  int len = 0;
 };
 
 Split split_work(int ctas, int ntx, int nty, int TY, int zlo, int depth, int nchunk, bool spread = true) {
@@ -483,8 +480,6 @@ Split split_work(int ctas, int ntx, int nty, int TY, int zlo, int depth, int nch
     }
   }
   Split sp;
-  sp.spread = full < items;
-  sp.len = len;
   sp.first.push_back(0);
   for (int b = 0; b < ctas; ++b) {
     sp.seg.insert(sp.seg.end(), per[b].begin(), per[b].end());
@@ -706,25 +701,13 @@ int setup_tiles(int rows, int stages) {
   // CTAs past the last one with work are not launched.
   int grid = ctas;
   while (grid > 1 && sp.first[grid - 1] == sp.first[grid]) --grid;
-  g.seg_grid = grid;
+  g.grid = grid;
   g.nseg = (int)sp.seg.size();
-  g.spread = sp.spread;
-  if (sp.spread) {
-    g.nitems = g.nseg;
-    g.grid = grid;
-    g.chunk = 0;
-  } else {
-    // A round-robin plan: the FP32 kernel decodes its items arithmetically
-    // (tiles x chunks of `len` planes, chunk-major), no list lookups.
-    g.chunk = sp.len;
-    g.nitems = g.ntx * g.nty * ((sz - 2 * bord + sp.len - 1) / sp.len);
-    g.grid = std::min(g.nitems, ctas);
-  }
   memset(&g.desc, 0, sizeof(g.desc));
   g.desc.F[0] = g.F[0];
   g.desc.F[1] = g.F[1];
   g.desc.sx = sx; g.desc.sy = sy; g.desc.sz = sz; g.desc.pitch = g.pitch; g.desc.bord = bord;
-  g.desc.ntx = g.ntx; g.desc.nty = g.nty; g.desc.chunk = g.chunk;
+  g.desc.ntx = g.ntx; g.desc.nty = g.nty;
   g.desc.src_x = g.desc.src_y = g.desc.src_z = -1000;
   g.desc.cor_x = g.desc.cor_y = g.desc.cor_z = -1000;
   return FLETCHER_OK;
@@ -1010,9 +993,9 @@ int step() {
   P.shots = nullptr;
   P.maps = nullptr;
   P.items = nullptr;
-  P.seg = g.spread ? g.seg : nullptr;
+  P.seg = g.seg;
   P.cta_first = g.cta_first;
-  P.nitems = g.nitems;
+  P.nitems = g.nseg;
   P.parity = c;
   P.inv_dx = 1.0f / g.dx;
   P.inv_dy = 1.0f / g.dy;
@@ -1073,8 +1056,6 @@ int step() {
     memset(&HL, 0, sizeof(HL));
     HL.batch = false;
     HL.h.p = P;
-    HL.h.p.seg = g.seg;  // the 16-bit kernel always walks the segment list
-    HL.h.p.nitems = g.nseg;
     HL.h.out_hi = g.Hh[p];
     HL.h.out_lo = g.Hl[p];
     HL.h.e_cur = g.E + g.ecur * sz;
@@ -1084,7 +1065,7 @@ int step() {
     HL.m = g.hm[c];
     HL.tile_rows = g.tile_rows;
     HL.stages = g.stages;
-    HL.grid = g.seg_grid;
+    HL.grid = g.grid;
     CK(propagate_half_launch(HL, g.form == FLETCHER_FORM_FP16X, g_stream));
     g.ecur = enew;
   } else {
@@ -1561,8 +1542,8 @@ struct Batch {
   // Chain schedule (FP32, chains > 0, FLETCHER_BatchSetChains): every step
   // of a shot is a single-shot launch; the shots are dealt over `chains`
   // concurrent streams, each running its shots one after another.  Per
-  // shot: its descriptor with the single-shot plan's chunk, its tensor
-  // maps, and its plan (tile items, or a segment list in d_sseg / d_sfirst).
+  // shot: its descriptor, its tensor maps, and its plan (a segment list in
+  // d_sseg / d_sfirst).
   int chains = -1;  // -1: chosen at the run (batch_auto_chains)
   int last_chains = 0;  // the schedule of the last run
   std::vector<ShotDesc> h_desc;
@@ -1571,7 +1552,7 @@ struct Batch {
   std::vector<HalfShotMaps> h_hmaps;
   std::vector<ShotDesc> s_desc;
   std::vector<int> s_nitems, s_grid;
-  std::vector<long> s_seg_off, s_first_off;  // s_seg_off < 0: tile items
+  std::vector<long> s_seg_off, s_first_off;
   int4 *d_sseg = nullptr;
   int *d_sfirst = nullptr;
   int splan_ctas = 0;
@@ -1766,8 +1747,7 @@ int batch_plan(int ctas) {
 }
 
 // The chain schedule's per-shot plans for `ctas` persistent CTAs: each
-// shot's own single-shot plan, as DRIVER_Initialize would make it (the
-// 16-bit kernel always walks a segment list).
+// shot's own single-shot plan, as DRIVER_Initialize would make it.
 int batch_single_plans(int ctas) {
   if (B.splan_ctas == ctas && !B.s_desc.empty()) return FLETCHER_OK;
   if (B.d_sseg) cudaFree(B.d_sseg);
@@ -1787,21 +1767,15 @@ int batch_single_plans(int ctas) {
     const int depth = s.sz - 2 * B.bord;
     const Split sp = plan_segments(ctas, s.ntx, s.nty, B.sealed_rows, B.bord, depth, 0);
     ShotDesc d = B.h_desc[i];
-    if (sp.spread || batch_half()) {
-      B.s_seg_off[i] = (long)segs.size();
-      B.s_first_off[i] = (long)firsts.size();
-      segs.insert(segs.end(), sp.seg.begin(), sp.seg.end());
-      firsts.insert(firsts.end(), sp.first.begin(), sp.first.end());
-      int grid = ctas;
-      while (grid > 1 && sp.first[grid - 1] == sp.first[grid]) --grid;
-      B.s_grid[i] = grid;
-      B.s_nitems[i] = (int)sp.seg.size();
-      d.chunk = 0;
-    } else {
-      d.chunk = sp.len;
-      B.s_nitems[i] = s.ntx * s.nty * ((depth + sp.len - 1) / sp.len);
-      B.s_grid[i] = std::min(B.s_nitems[i], ctas);
-    }
+    B.s_seg_off[i] = (long)segs.size();
+    B.s_first_off[i] = (long)firsts.size();
+    segs.insert(segs.end(), sp.seg.begin(), sp.seg.end());
+    firsts.insert(firsts.end(), sp.first.begin(), sp.first.end());
+    int grid = ctas;
+    while (grid > 1 && sp.first[grid - 1] == sp.first[grid]) --grid;
+    B.s_grid[i] = grid;
+    B.s_nitems[i] = (int)sp.seg.size();
+    d.chunk = 0;
     B.s_desc[i] = d;
   }
   if (!segs.empty()) {
@@ -1993,8 +1967,8 @@ int batch_issue_chains(int chains, int steps, const float *src) {
       const ShotMaps &m = B.h_maps[i];
       P.one = B.s_desc[i];
       P.nitems = B.s_nitems[i];
-      P.seg = B.s_seg_off[i] < 0 ? nullptr : B.d_sseg + B.s_seg_off[i];
-      P.cta_first = B.s_seg_off[i] < 0 ? nullptr : B.d_sfirst + B.s_first_off[i];
+      P.seg = B.d_sseg + B.s_seg_off[i];
+      P.cta_first = B.d_sfirst + B.s_first_off[i];
       L.grid = B.s_grid[i];
       L.m.arr = m.arr;
       L.m.upd = m.upd;

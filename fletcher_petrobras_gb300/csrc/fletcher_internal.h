@@ -57,18 +57,17 @@ struct ShotMaps {
   CUtensorMap upd;      // coefficients, box (TX, TY, 7, 1)
 };
 
-// One launch: every active shot advances one step.
-//  * batched launches: work items {shot, x0, y0, chunk index}, ordered by
-//    shot; CTA b takes items b, b + grid, ... below nitems;
-//  * single-shot launches with seg: segments {x0, y0, z0, z1} (a z range of
-//    one tile column); CTA b takes segments cta_first[b] .. cta_first[b+1]-1;
-//  * single-shot launches without seg: items = tiles x uniform z-chunks of
-//    one.chunk planes, chunk-major, CTA b takes b, b + grid, ... below nitems.
+// One launch: every active shot advances one step.  The work is a list of
+// segments {x0 + (shot << 16), y0, z0, z1}, each a z range of one tile column
+// of a shot (single-shot launches: shot 0); CTA b takes the segments
+// cta_first[b] .. cta_first[b+1]-1.  (Batched 16-bit launches: work items
+// {shot, x0, y0, chunk index}, ordered by shot; CTA b takes items b,
+// b + grid, ... below nitems.)
 struct PropParams {
   ShotDesc one;                     // single-shot launches: the shot itself
   const ShotDesc *shots;            // batched launches: per-shot descriptors
   const ShotMaps *maps;
-  const int4 *items;                // batched launches
+  const int4 *items;                // batched 16-bit launches
   int nitems;
   int parity;                       // current field = F[parity], previous = F[1 - parity]
   float inv_dx, inv_dy, inv_dz;     // 1/dx, 1/dy, 1/dz
@@ -80,8 +79,8 @@ struct PropParams {
   float src;                        // value added at each shot's source cell (src_z >= 0)
   float cor;                        // value owed at each shot's cor cell (cor_z >= 0)
   unsigned int *err;                // error word (bit 0: bounded wait gave up)
-  const int4 *seg;                  // single-shot launches with a segment list
-  const int *cta_first;             // their [grid + 1] first segments
+  const int4 *seg;                  // the segment list
+  const int *cta_first;             // its [grid + 1] first segments
   const float *media;               // media-table layout: angle terms [kAngleCoef][kMediaMax]
   unsigned long long wait_ns;       // limit of the step's waits (ns)
   int stall_step;                   // test hook: CTA 0 skips the loads of its stall_step-th step (-1: none)
@@ -112,6 +111,7 @@ int propagate_fp32_threads(int tile_rows);
 int propagate_fp32_ctas_per_sm(int tile_rows);
 cudaError_t propagate_fp32_prepare(int tile_rows, int stages);
 cudaError_t propagate_fp32_launch(const PropLaunch &L, cudaStream_t s);
+cudaError_t propagate_d1d1_launch(const PropLaunch &L, cudaStream_t s);
 // Tile shape of the Der1-Der1 numerics (the only one built for it).
 constexpr int kD1D1Rows = 16, kD1D1Stages = 4;
 // Most concurrent chains of the batched shots' chain schedule, and the
@@ -213,5 +213,7 @@ void snapshot_release();             // driver.cu calls it when the state goes a
 
 // Time limit of every device-side wait (ns).
 constexpr uint64_t kWaitLimitNs = 2000000000ull;
+// Limit of an aborting producer's wait for each stage's loads.
+constexpr uint64_t kDrainNs = 200000000ull;
 
 }  // namespace flt

@@ -5,24 +5,47 @@
 // weighted by the ch1d** and v2** coefficients of original/precomp.h), with
 // the source of original/OpenMP/openmp_insertsource.c:7-13 fused in.
 //
-// Structure (one CTA per SM, persistent):
-//  * a work item is a 32 x TY column tile of one z-chunk; the CTA streams
-//    its planes k = z0-4 .. z1+3 in z;
-//  * thread 0 issues TMA loads S-1 planes ahead into a ring of shared-memory
-//    stages: the (p,q) halo tile of plane k (box 40 x (TY+8)), the three
-//    in-plane coefficients of plane k, and the seven other coefficients and
-//    the previous (p,q) of plane k-4, which is updated at this step;
-//  * each thread owns one (x, y) column.  When plane k arrives it reads its
-//    9-point x and y neighbourhoods from shared memory and forms Der2x,
-//    Der2y and the first derivatives D1x, D1y; DerCross xy is D1x applied to
-//    D1y (exchanged through shared memory, including the 4-column x halo);
+// Structure (one CTA per SM, persistent, warp-specialised):
+//  * a work item is a 32 x TY column tile of one z range; the CTA streams its
+//    planes k = z0-4 .. z1+3 in z through a ring of S shared-memory stages;
+//  * the producer (one thread of the helper warps) issues a stage's TMA
+//    loads as soon as every reader has released it: the (p,q) halo tile of
+//    plane k (box 40 x (TY+8)), the three in-plane coefficients of plane k,
+//    and the seven other coefficients and the previous (p,q) of plane k-4,
+//    which is updated at this step;
+//  * the halo warps (three helper warps) evaluate D1y in the tile's 8 halo
+//    columns, ahead of the compute warps, and add the step's source to the
+//    tile of the plane that holds it;
+//  * TY compute warps: each thread owns one (x, y) column.  When plane k
+//    arrives it reads its 9-point x and y neighbourhoods from shared memory
+//    and forms Der2x, Der2y and the first derivatives D1x, D1y; DerCross xy
+//    is D1x applied to D1y, whose row of the tile only this warp and the
+//    halo columns write (so compute warps never wait for one another);
 //    DerCross xz and yz are the z first derivative of the D1x / D1y values,
 //    which each thread keeps for 9 planes in registers, as it keeps p and q
-//    for Der2z;
+//    for Der2z; the in-plane terms A and B wait in shared memory;
 //  * both fields travel as one 64-bit (p, q) pair and are updated with the
 //    packed .f32x2 add/mul/fma instructions;
 //  * plane k-4 is completed at step k and written with coalesced 64-bit
 //    stores into the previous-field buffer (in place).
+//
+// What bounds it: HBM.  At 504^3 (183 M updated cells, 64 B each) a step
+// takes 1.86 ms, 93% of the measured copy bandwidth, against 2.22 ms (78%)
+// for the kernel before it, whose 16 warps exchanged D1y, and refilled the
+// stages, in one CTA-wide exchange a plane; 128^3 + shell 81.8 against 92.8
+// us, 56^3 + shell 14.4 against 18.5 us.  Two causes:
+//  * the loop is unrolled over the 9 ring slots, and with the producer, the
+//    source and the timed waits in it the code was 102 KB (the instruction
+//    fetch was the stall of 1.1 of 8.4 cycles an issue); moved to the helper
+//    warps and counted waits, it is 39 KB;
+//  * a stage is refilled the moment its last reader releases it, whichever
+//    warp that is, and the warps may run up to S planes apart.  (Groups of 4
+//    warps that exchange among themselves, with the refill still issued by
+//    a compute warp, took 2.48 ms: warps that run ahead of the producing
+//    warp find their loads not yet issued.)
+// 16 rows: 16 compute warps at 112 registers hold the 27 ring values and a
+// plane's neighbourhood without a spill; 12 rows took 322 and 8 rows (two
+// CTAs an SM) 377 us where 16 rows take 309 (312^3 updated cells).
 //
 // Media-table layout (template parameter MT): instead of the ten coefficient
 // planes a stage holds the one-byte medium ids of planes k and k-4 and the
@@ -42,279 +65,285 @@
 
 namespace flt {
 
-// D1D1: the Der1-Der1 numerics.  HOOK: the fault-injection variant (waits
-// limited to P.wait_ns, CTA 0 skipping the loads of step P.stall_step),
-// launched only when a test injects a stall.  MT: the media-table layout of
-// the coefficients.
-template <int TY, int S, bool ISO, int MODE, int MINB, bool D1D1 = false, bool HOOK = false, bool MT = false>
-__global__ void __launch_bounds__(kTileX *TY, MINB)
+constexpr int kHelperWarps = 4;  // producer warp + 3 halo warps: one warpgroup (setmaxnreg works on warpgroups)
+constexpr int kHaloWarps = kHelperWarps - 1;
+
+// Shared memory of a CTA.  Rows: the D1y exchange buffers, one per stage
+// (two for the 8 x 5 shape, whose two CTAs share an SM's memory).
+template <int TY, int S, bool MT>
+struct Layout {
+  using G = Geo<TY, false, MT>;
+  static constexpr int NB = (TY <= 8 && S > 4) ? 2 : S;
+  static constexpr int OFF_ROWS = S * G::STAGE_B;
+  static constexpr int OFF_AB = OFF_ROWS + NB * G::ROW_B;
+  static constexpr int OFF_TAB = OFF_AB + G::AB_B;
+  static constexpr int OFF_HDR = OFF_TAB + G::TAB_B;  // the item that starts in stage s
+  static constexpr int OFF_BAR = OFF_HDR + S * 16;    // full[S], halo[S], empty[S]
+  static constexpr size_t BYTES = size_t(OFF_BAR) + 3 * S * 8 + 128;
+};
+
+// Register split (setmaxnreg): the compute warps take what the helper warps
+// give back.  Per SM sub-partition, TY/4 compute warps and one helper warp
+// share (TY/4 + 1) x the launch's registers a thread (96 at 16 rows, 128 at
+// 12, 80 at 8): 4 x 112 + 32 = 5 x 96, 3 x 160 + 32 = 4 x 128, 2 x 104 + 32 = 3 x 80.
+constexpr int kHelperRegs = 32;
+template <int TY>
+struct Regs {
+  static constexpr int kCompute = TY == 16 ? 112 : TY == 12 ? 160 : 104;
+  static constexpr int kLaunch = TY == 16 ? 96 : TY == 12 ? 128 : 80;
+  static_assert((TY / 4) * kCompute + kHelperRegs <= (TY / 4 + 1) * kLaunch, "the split exceeds the launch's registers");
+};
+
+// HOOK: the fault-injection variant (waits limited to P.wait_ns, CTA 0
+// skipping the loads of step P.stall_step), launched only when a test
+// injects a stall.  MT: the media-table layout of the coefficients.
+template <int TY, int S, bool ISO, bool BATCH, int MINB, bool HOOK = false, bool MT = false>
+__global__ void __launch_bounds__(kTileX *(TY + kHelperWarps), MINB)
     k_propagate_fp32(const __grid_constant__ SingleMaps SM, const __grid_constant__ PropParams P) {
-  constexpr bool BATCH = MODE == kItemsBatch;
-  static_assert(!D1D1 || (!ISO && !BATCH), "the Der1-Der1 numerics scale every derivative, single shot only");
-  static_assert(!MT || (!BATCH && !HOOK && !D1D1), "the media-table layout runs single-shot plain steps");
-  using G = Geo<TY, D1D1, MT>;
+  static_assert(!MT || (!BATCH && !HOOK), "the media-table layout runs single-shot plain steps");
+  using G = Geo<TY, false, MT>;
+  using L = Layout<TY, S, MT>;
   extern __shared__ unsigned char smem_dyn[];
   // Align in the shared window (pointer arithmetic on the shared array keeps
   // every access below a shared-memory access).
   unsigned char *smem = smem_dyn + ((128u - (smem_addr(smem_dyn) & 127u)) & 127u);
-  f2 *dbuf = reinterpret_cast<f2 *>(smem + S * G::STAGE_B);
-  float4 *ABs = reinterpret_cast<float4 *>(smem + S * G::STAGE_B + G::DBUF_B);  // [5][NT] (AB_SMEM)
-  f2 *Cs = reinterpret_cast<f2 *>(ABs + kABSlots * G::NT);  // [kABSlots][NT] (Der1-Der1 numerics: ch1dxy * pxy)
-  float *s_med = reinterpret_cast<float *>(smem + S * G::STAGE_B + G::DBUF_B + G::AB_B);  // [6][256] (MT)
-  uint64_t *full = reinterpret_cast<uint64_t *>(smem + S * G::STAGE_B + G::DBUF_B + G::AB_B + G::TAB_B);
-  uint64_t *xchg = full + S;  // D1y rows written (one arrival per warp)
-  int *s_abort = reinterpret_cast<int *>(xchg + 1);
+  f2 *rows = reinterpret_cast<f2 *>(smem + L::OFF_ROWS);         // [NB][TY][HX]
+  float4 *ABs = reinterpret_cast<float4 *>(smem + L::OFF_AB);    // [kABSlots][NT]
+  float *s_med = reinterpret_cast<float *>(smem + L::OFF_TAB);   // [6][256] (MT)
+  int4 *hdr = reinterpret_cast<int4 *>(smem + L::OFF_HDR);
+  uint64_t *full = reinterpret_cast<uint64_t *>(smem + L::OFF_BAR);
+  uint64_t *halo = full + S;   // halo columns (and source) of the stage's plane written
+  uint64_t *empty = halo + S;  // stage released by every reader
 
   const int tid = threadIdx.x;
   const int lx = tid & 31;
-  const int ly = tid >> 5;
-
-  // This CTA's items.  A segment run's end lives in shared memory (read once
-  // per item), so the loop keeps no register for it.
-  const ItemRange R = item_range<MODE>(P);
-  if (R.first >= R.end) return;
-  volatile int *s_end = s_abort + 1;
-  int *s_issued = s_abort + 2;  // fault-injection variant: steps this CTA has issued
-  auto item_end = [&]() { return MODE != kItemsTiles ? *s_end : P.nitems; };
-  auto item_step = [&]() { return MODE != kItemsTiles ? 1 : (int)gridDim.x; };
-  // The producer is lane 0 of the last warp (warps 0 .. TY/4-1 carry the
-  // halo-column work).  Its cursor, in shared memory, is the next step to load.
-  const bool producer = tid == (TY - 1) * 32;
-  auto maps_of = [&](const Item &it) {
-    StepMaps m;
-    if constexpr (BATCH) {
-      const ShotMaps *sm = P.maps + it.shot;
-      m.cur = &sm->halo[P.parity];
-      m.prev = &sm->pt[P.parity ^ 1];
-      m.arr = &sm->arr;
-      m.upd = &sm->upd;
-    } else {
-      m.cur = &SM.cur_halo;
-      m.prev = &SM.prev_pt;
-      m.arr = &SM.arr;
-      m.upd = &SM.upd;
+  const int wid = __shfl_sync(0xffffffffu, tid >> 5, 0);  // warp-uniform
+  const int first = P.cta_first[blockIdx.x], nitems = P.cta_first[blockIdx.x + 1] - first;
+  if (nitems <= 0) return;
+  constexpr int kHalo = TY / 4 < kHaloWarps ? TY / 4 : kHaloWarps;  // halo warps with work
+  if (tid == 0) {
+    for (int s = 0; s < S; ++s) {
+      mbar_init(&full[s], 1);
+      mbar_init(&halo[s], kHalo);
+      mbar_init(&empty[s], TY + kHalo);
     }
-    m.ids = &SM.ids;
-    m.vel = &SM.vel;
-    return m;
+    mbar_fence_init();
+  }
+  if constexpr (MT) {
+    for (int i = tid; i < kAngleCoef * kMediaMax; i += kTileX * (TY + kHelperWarps)) s_med[i] = P.media[i];
+  }
+  __syncthreads();
+  // Every wait is bounded; the fault-injection variant's by P.wait_ns.
+  auto wait = [&](uint64_t *bar, uint32_t parity) {
+    if constexpr (HOOK) return mbar_wait(bar, parity, P.wait_ns);
+    else return mbar_spin(bar, parity);
   };
-  Cursor *cur = reinterpret_cast<Cursor *>(s_abort + 4);
-  // Issues the cursor's step into its stage and advances the cursor.  (Test
-  // hook: CTA 0 skips the loads of its P.stall_step-th step, so that the
-  // waits for that stage give up and the launch reports a timeout.)
-  auto produce = [&]() {
-    Cursor c = *cur;
-    if constexpr (HOOK) {
-      if (*s_issued != P.stall_step || blockIdx.x != 0)
-        issue_step<TY, MT>(smem + c.stage * G::STAGE_B, &full[c.stage], c.it, c.k, maps_of(c.it));
-      ++*s_issued;
-    } else {
-      issue_step<TY, MT>(smem + c.stage * G::STAGE_B, &full[c.stage], c.it, c.k, maps_of(c.it));
-    }
-    if (++c.stage == S) c.stage = 0;
-    if (++c.k >= c.it.z1 + kLag) {
-      c.item += item_step();
-      if (c.item < item_end()) {
-        c.it = decode_item<TY, MODE>(c.item, P);
-        c.k = c.it.z0 - kRadius;
+
+  if (wid >= TY) {
+    setmaxnreg_dec<kHelperRegs>();
+    const int4 *seg = P.seg + first;
+    int stage = 0;
+    uint32_t phase = 0;
+    if (wid == TY) {
+      // ---- producer ----
+      if (lx != 0) return;
+      auto maps_of = [&](int shot) {
+        StepMaps m;
         if constexpr (BATCH) {
-          // Batched shots keep their tensor maps in global memory: fetch
-          // those of the item after this one into the descriptor cache now,
-          // an item ahead of their first use.
-          if (c.item + 1 < item_end()) {
-            const StepMaps m = maps_of(decode_item<TY, MODE>(c.item + 1, P));
-            tma_prefetch_desc(m.cur);
-            tma_prefetch_desc(m.prev);
-            tma_prefetch_desc(m.arr);
-            tma_prefetch_desc(m.upd);
+          const ShotMaps *sm = P.maps + shot;
+          m.cur = &sm->halo[P.parity];
+          m.prev = &sm->pt[P.parity ^ 1];
+          m.arr = &sm->arr;
+          m.upd = &sm->upd;
+        } else {
+          m.cur = &SM.cur_halo;
+          m.prev = &SM.prev_pt;
+          m.arr = &SM.arr;
+          m.upd = &SM.upd;
+        }
+        m.ids = &SM.ids;
+        m.vel = &SM.vel;
+        return m;
+      };
+      auto prefetch = [&](int shot) {
+        const StepMaps m = maps_of(shot);
+        tma_prefetch_desc(m.cur);
+        tma_prefetch_desc(m.prev);
+        tma_prefetch_desc(MT ? m.ids : m.arr);
+        tma_prefetch_desc(MT ? m.vel : m.upd);
+      };
+      int4 next = seg[0];
+      prefetch(decode_item<BATCH>(next).shot);
+      int issued = 0;
+      bool ok = true;
+      for (int i = 0; i < nitems && ok; ++i) {
+        const int4 w = next;
+        const Item it = decode_item<BATCH>(w);
+        if (i + 1 < nitems) {
+          next = seg[i + 1];
+          // Batched shots keep their tensor maps in global memory: fetch the
+          // next item's into the descriptor cache an item ahead.
+          if constexpr (BATCH) prefetch(decode_item<BATCH>(next).shot);
+        }
+        const StepMaps m = maps_of(it.shot);
+        for (int k = it.z0 - kRadius; k < it.z1 + kLag; ++k) {
+          // (The first S waits pass at once: the stage was never filled.)
+          if (!wait(&empty[stage], phase ^ 1u)) {
+            ok = false;
+            break;
+          }
+          fence_proxy_async_smem();
+          if (k == it.z0 - kRadius) hdr[stage] = w;
+          // Test hook: CTA 0 skips the loads of its P.stall_step-th step, so
+          // that the waits for that stage give up.
+          if (!HOOK || issued != P.stall_step || blockIdx.x != 0)
+            issue_step<TY, MT>(smem + stage * G::STAGE_B, &full[stage], it, k, m);
+          ++issued;
+          if (++stage == S) {
+            stage = 0;
+            phase ^= 1u;
           }
         }
       }
-    }
-    *cur = c;
-  };
-  if (tid == 0) {
-    for (int s = 0; s < S; ++s) mbar_init(&full[s], 1);
-    mbar_init(xchg, TY);
-    mbar_fence_init();
-    *s_abort = 0;
-    *s_issued = 0;
-    if constexpr (MODE != kItemsTiles) *s_end = R.end;
-  }
-  if constexpr (MT) {
-    for (int i = tid; i < kAngleCoef * kMediaMax; i += kTileX * TY) s_med[i] = P.media[i];
-  }
-  if (producer) {
-    Cursor c;
-    c.it = decode_item<TY, MODE>(R.first, P);
-    c.item = R.first;
-    c.k = c.it.z0 - kRadius;
-    c.stage = 0;
-    *cur = c;
-  }
-  __syncthreads();
-  if (producer) {
-    {
-      const StepMaps m = maps_of(cur->it);
-      tma_prefetch_desc(m.cur);
-      tma_prefetch_desc(m.prev);
-      if constexpr (MT) {
-        tma_prefetch_desc(m.ids);
-        tma_prefetch_desc(m.vel);
-      } else {
-        tma_prefetch_desc(m.arr);
-        tma_prefetch_desc(m.upd);
+      if (!ok) {
+        // A bounded wait gave up: wait, bounded, for the loads still in
+        // flight into this CTA's stages, then leave (every other thread
+        // gives up on its own bounded waits).
+        atomicOr(P.err, 2u);
+        for (int a = 1; a <= S && a <= issued; ++a) {
+          const int s2 = stage >= a ? stage - a : stage + S - a;
+          (void)mbar_wait(&full[s2], stage >= a ? phase : phase ^ 1u, kDrainNs);
+        }
       }
-      if (BATCH && cur->item + 1 < item_end()) {
-        const StepMaps m2 = maps_of(decode_item<TY, MODE>(cur->item + 1, P));
-        tma_prefetch_desc(m2.cur);
-        tma_prefetch_desc(m2.prev);
-        tma_prefetch_desc(m2.arr);
-        tma_prefetch_desc(m2.upd);
+      return;
+    }
+    // ---- halo warps ----
+    const int hw = wid - TY - 1;
+    if (hw >= kHalo) return;
+    const int hxc = (lx & 7) < 4 ? (lx & 7) : G::TX + (lx & 7);  // lane -> halo column, row lane / 8 of a group of 4
+    int rb = 0;
+    for (int i = 0; i < nitems; ++i) {
+      const Item it = decode_item<BATCH>(seg[i]);
+      const ShotDesc &sd = BATCH ? P.shots[it.shot] : P.one;
+      const int src_z = sd.src_z;
+      for (int k = it.z0 - kRadius; k < it.z1 + kLag; ++k) {
+        bool ok = wait(&full[stage], phase);
+        if constexpr (L::NB < S) {
+          // The row buffer's last readers: the step NB back.
+          const int es = stage >= L::NB ? stage - L::NB : stage + S - L::NB;
+          ok = ok && wait(&empty[es], stage >= L::NB ? phase : phase ^ 1u);
+        }
+        if (!ok) {
+          atomicOr(P.err, 1u);
+          return;
+        }
+        f2 *H = reinterpret_cast<f2 *>(smem + stage * G::STAGE_B);
+        if (k == src_z) {
+          // Fused source (original/OpenMP/openmp_insertsource.c:7-13): the
+          // current p and q gain `src` at the source cell before the update
+          // reads them.  (On this plane the compute warps wait for the halo
+          // warps before they read the tile.)
+          const int rx = sd.src_x - (it.x0 - kRadius), ry = sd.src_y - (it.y0 - kRadius);
+          if (hw == 0 && lx == 0 && rx >= 0 && rx < G::HX && ry >= 0 && ry < G::HY) {
+            H[ry * G::HX + rx] = add2(H[ry * G::HX + rx], splat(P.src));
+            fence_proxy_async_smem();
+          }
+          asm volatile("bar.sync 1, %0;" ::"n"(32 * kHalo) : "memory");
+        }
+        if (k >= it.z0 && k < it.z1) {
+          f2 *db = rows + (L::NB < S ? rb : stage) * (TY * G::HX);
+          for (int r = hw * 4 + (lx >> 3); r < TY; r += 4 * kHalo) {
+            const f2 *h = H + (r + kRadius) * G::HX + hxc;
+            f2 d = mul2(splat(cL1), sub2(h[G::HX], h[-G::HX]));
+            d = fma2(splat(cL2), sub2(h[2 * G::HX], h[-2 * G::HX]), d);
+            d = fma2(splat(cL3), sub2(h[3 * G::HX], h[-3 * G::HX]), d);
+            d = fma2(splat(cL4), sub2(h[4 * G::HX], h[-4 * G::HX]), d);
+            db[r * G::HX + hxc] = d;
+          }
+        }
+        __syncwarp();
+        if (lx == 0) {
+          mbar_arrive(&halo[stage]);
+          mbar_arrive(&empty[stage]);
+        }
+        if (L::NB < S && ++rb == L::NB) rb = 0;
+        if (++stage == S) {
+          stage = 0;
+          phase ^= 1u;
+        }
       }
     }
-    // Prologue: the first S-2 steps of this CTA.
-    for (int a = 0; a < S - 2 && cur->item < item_end(); ++a) produce();
+    return;
   }
 
-  const uint64_t wait_ns = HOOK ? P.wait_ns : kWaitLimitNs;
+  // ---- compute warps ----
+  setmaxnreg_inc<Regs<TY>::kCompute>();
+  const int ly = wid;
   // Spacing factors (unused on isotropic grids).
   const float sxy = P.inv_dxy, sxz = P.inv_dxz, syz = P.inv_dyz;
   const float sxx = P.inv_dxx, syy = P.inv_dyy, szz = P.inv_dzz;
-  // Halo-column duty: warps 0 .. TY/4-1 evaluate D1y in the 4 columns left
-  // and right of the tile for all TY rows (lane -> row 4*warp + lane/8).
-  const bool halo_warp = ly < TY / 4;
-  const int hr = ly * 4 + (lx >> 3);
-  const int hxc = (lx & 7) < 4 ? (lx & 7) : G::TX + (lx & 7);
-  const int hh = (hr + kRadius) * G::HX + hxc;
-
+  const int ci = ly * G::TX + lx;
+  const int hc = (ly + kRadius) * G::HX + (lx + kRadius);
   int stage = 0;
-  uint32_t phase = 0, xphase = 0;
-  int dsel = 0;
+  uint32_t phase = 0;
+  int rb = 0;
   int abw = 0;  // shared A/B ring slot of the arriving plane (the plane kLag back is at abw + 1)
-  for (int item = R.first; item < item_end(); item += item_step()) {
-    const Item it = decode_item<TY, MODE>(item, P);
+  for (int item = 0; item < nitems; ++item) {
+    if (!wait(&full[stage], phase)) {
+      if (lx == 0) atomicOr(P.err, 1u);
+      return;
+    }
+    const Item it = decode_item<BATCH>(hdr[stage]);
     const ShotDesc &sd = BATCH ? P.shots[it.shot] : P.one;
-    const int kbeg = it.z0 - kRadius;
     const int kend = it.z1 + kLag;
     const int gx = it.x0 + lx;
     const int gy = it.y0 + ly;
     const int bord = sd.bord, sxs = sd.sx, sys = sd.sy;
     const bool valid = (gx >= bord) && (gx < sxs - bord) && (gy >= bord) && (gy < sys - bord);
     const long plane = (long)sd.pitch * sys;
-    unsigned long long *out = reinterpret_cast<unsigned long long *>(sd.F[P.parity ^ 1]) + ((long)gy * sd.pitch + gx);
-    const int src_z = sd.src_z, cor_z = sd.cor_z;  // cells are read from `sd` on the (rare) planes
-    const int ci = ly * G::TX + lx;
-    const int hc = (ly + kRadius) * G::HX + (lx + kRadius);
+    unsigned long long *out =
+        reinterpret_cast<unsigned long long *>(sd.F[P.parity ^ 1]) + (it.z0 * plane + (long)gy * sd.pitch + gx);
+    const int src_z = sd.src_z;
+    // The cell that lacks the last step's source, if it is this thread's.
+    const int cor_k = (gx == sd.cor_x && gy == sd.cor_y) ? sd.cor_z + kLag : -1000;
 
-    f2 Pr[kRing], Dx[kRing], Dy[kRing], A[kRing], B[kRing];
+    f2 Pr[kRing], Dx[kRing], Dy[kRing];
 
-    for (int kb = kbeg; kb < kend; kb += kRing) {
+    for (int kb = it.z0 - kRadius; kb < kend; kb += kRing) {
 #pragma unroll
       for (int j = 0; j < kRing; ++j) {
         const int k = kb + j;
         if (k >= kend) break;
         unsigned char *st = smem + stage * G::STAGE_B;
-        if (!mbar_wait(&full[stage], phase, wait_ns)) {
-          *s_abort = 1;
-          atomicOr(P.err, 1u);
-          goto aborted;
+        if (!wait(&full[stage], phase) || (k == src_z && !wait(&halo[stage], phase))) {
+          if (lx == 0) atomicOr(P.err, 1u);
+          return;
         }
         const bool center = (k >= it.z0) && (k < it.z1);
         const bool upd = (k - kLag >= it.z0);
-        const bool src_plane = (k == src_z);
-        const f2 *H = reinterpret_cast<const f2 *>(st);
-
-        f2 c = H[hc];
+        const f2 *H = reinterpret_cast<const f2 *>(st) + hc;
+        const f2 c = H[0];
         f2 xa[4], xb[4], ya[4], yb[4];
 #pragma unroll
         for (int o = 1; o <= 4; ++o) {
-          xa[o - 1] = H[hc + o];
-          xb[o - 1] = H[hc - o];
-          ya[o - 1] = H[hc + o * G::HX];
-          yb[o - 1] = H[hc - o * G::HX];
+          xa[o - 1] = H[o];
+          xb[o - 1] = H[-o];
+          ya[o - 1] = H[o * G::HX];
+          yb[o - 1] = H[-o * G::HX];
         }
-        // Fused source (original/OpenMP/openmp_insertsource.c:7-13): the
-        // current p and q gain `src` at the source cell before the update
-        // reads them; added to this thread's copies of the plane.
-        if (src_plane) {
-          const int src_x = sd.src_x, src_y = sd.src_y;
-          const f2 sv = splat(P.src);
-          f2 dummy;
-          if (gy == src_y && abs(src_x - gx) <= kRadius) add_at(c, xa, xb, src_x - gx, sv);
-          if (gx == src_x && src_y != gy && abs(src_y - gy) <= kRadius) add_at(dummy, ya, yb, src_y - gy, sv);
-        }
-        f2 d1x, d1y;
-        if constexpr (D1D1) {
-          // der1der1/sample.h:35-49: pDx = Der1_x(p) / dx and pDy = Der1_y(p) / dy.
-          d1x = d1_ref(xa[0], xb[0], xa[1], xb[1], xa[2], xb[2], xa[3], xb[3], P.inv_dx);
-          d1y = d1_ref(ya[0], yb[0], ya[1], yb[1], ya[2], yb[2], ya[3], yb[3], P.inv_dy);
-        } else {
-          d1x = d1(xa[0], xb[0], xa[1], xb[1], xa[2], xb[2], xa[3], xb[3]);
-          d1y = d1(ya[0], yb[0], ya[1], yb[1], ya[2], yb[2], ya[3], yb[3]);
-        }
+        const f2 d1x = d1(xa[0], xb[0], xa[1], xb[1], xa[2], xb[2], xa[3], xb[3]);
+        const f2 d1y = d1(ya[0], yb[0], ya[1], yb[1], ya[2], yb[2], ya[3], yb[3]);
         Pr[j] = c;
         Dx[j] = d1x;
         Dy[j] = d1y;
         f2 d2x, d2y;
-        constexpr int DB_N = D1D1 ? G::HY * G::TX : TY * G::HX;
-        f2 *db = dbuf + dsel * DB_N;
-        if constexpr (D1D1) {
-          if (center) {
-            d2x = d2_ref(c, xa[0], xb[0], xa[1], xb[1], xa[2], xb[2], xa[3], xb[3], sxx);
-            d2y = d2_ref(c, ya[0], yb[0], ya[1], yb[1], ya[2], yb[2], ya[3], yb[3], syy);
-            // pDx of the tile column and of its 4-row y halo: the row's own
-            // value, and warps 0..7 one halo row each (halo-tile rows 0..3 and
-            // TY+4..TY+7).
-            db[(ly + kRadius) * G::TX + lx] = d1x;
-            if (ly < 2 * kRadius) {
-              const int hrow = ly < kRadius ? ly : TY + ly;
-              const int hb0 = hrow * G::HX + lx + kRadius;
-              f2 ha[4], hb[4], dummy;
-#pragma unroll
-              for (int o = 1; o <= 4; ++o) {
-                ha[o - 1] = H[hb0 + o];
-                hb[o - 1] = H[hb0 - o];
-              }
-              if (src_plane && it.y0 - kRadius + hrow == sd.src_y && abs(sd.src_x - gx) <= kRadius)
-                add_at(dummy, ha, hb, sd.src_x - gx, splat(P.src));
-              db[hrow * G::TX + lx] = d1_ref(ha[0], hb[0], ha[1], hb[1], ha[2], hb[2], ha[3], hb[3], P.inv_dx);
-            }
-          }
-        } else if (center) {
+        f2 *dr = rows + (L::NB < S ? rb : stage) * (TY * G::HX) + ly * G::HX + lx + kRadius;
+        if (center) {
           d2x = scale<ISO>(d2(c, xa[0], xb[0], xa[1], xb[1], xa[2], xb[2], xa[3], xb[3]), sxx);
           d2y = scale<ISO>(d2(c, ya[0], yb[0], ya[1], yb[1], ya[2], yb[2], ya[3], yb[3]), syy);
-          db[ly * G::HX + lx + kRadius] = d1y;
-          if (halo_warp) {
-            f2 ha[4], hb[4];
-#pragma unroll
-            for (int o = 1; o <= 4; ++o) {
-              ha[o - 1] = H[hh + o * G::HX];
-              hb[o - 1] = H[hh - o * G::HX];
-            }
-            if (src_plane) {
-              const int src_x = sd.src_x, src_y = sd.src_y;
-              const int hgy = it.y0 + hr;
-              if (hxc == src_x - (it.x0 - kRadius) && src_y != hgy && abs(src_y - hgy) <= kRadius) {
-                f2 dummy;
-                add_at(dummy, ha, hb, src_y - hgy, splat(P.src));
-              }
-            }
-            db[hr * G::HX + hxc] = d1(ha[0], hb[0], ha[1], hb[1], ha[2], hb[2], ha[3], hb[3]);
-          }
+          dr[0] = d1y;
         }
-        // Split-phase exchange: announce this warp's D1y (and, by program
-        // order, that it has finished the previous step), update plane k-4,
-        // which needs no exchanged data, then wait for the other warps.
         __syncwarp();
-        if (lx == 0) mbar_arrive(xchg);
-        // The producer has passed the exchange of the previous step, so every
-        // thread is past the step before it: refill that step's stage with
-        // the next step due (S-2 steps ahead of this one).
-        if (producer && cur->item < item_end()) {
-          fence_proxy_async_smem();
-          produce();
-        }
         if (upd) {
           const int cs = (j + kRing - kLag) % kRing;  // ring slot of plane k-kLag
           // RP(o): plane k-kLag+o for o = 0..4, k-kLag-(kRing-o) for o > 4.
@@ -322,111 +351,53 @@ __global__ void __launch_bounds__(kTileX *TY, MINB)
 #define RX(o) Dx[(cs + (o)) % kRing]
 #define RY(o) Dy[(cs + (o)) % kRing]
           constexpr int M1 = kRing - 1, M2 = kRing - 2, M3 = kRing - 3, M4 = kRing - 4;
-          f2 d2z, dxz, dyz;
-          if constexpr (D1D1) {
-            // der1der1/sample.h:58-66: pzz, pxz = Der1_z(pDx) / dz, pyz = Der1_z(pDy) / dz.
-            d2z = d2_ref(RP(0), RP(1), RP(M1), RP(2), RP(M2), RP(3), RP(M3), RP(4), RP(M4), szz);
-            dxz = d1_ref(RX(1), RX(M1), RX(2), RX(M2), RX(3), RX(M3), RX(4), RX(M4), P.inv_dz);
-            dyz = d1_ref(RY(1), RY(M1), RY(2), RY(M2), RY(3), RY(M3), RY(4), RY(M4), P.inv_dz);
-          } else {
-            d2z = scale<ISO>(d2(RP(0), RP(1), RP(M1), RP(2), RP(M2), RP(3), RP(M3), RP(4), RP(M4)), szz);
-            dxz = scale<ISO>(d1(RX(1), RX(M1), RX(2), RX(M2), RX(3), RX(M3), RX(4), RX(M4)), sxz);
-            dyz = scale<ISO>(d1(RY(1), RY(M1), RY(2), RY(M2), RY(3), RY(M3), RY(4), RY(M4)), syz);
-          }
+          const f2 d2z = scale<ISO>(d2(RP(0), RP(1), RP(M1), RP(2), RP(M2), RP(3), RP(M3), RP(4), RP(M4)), szz);
+          const f2 dxz = scale<ISO>(d1(RX(1), RX(M1), RX(2), RX(M2), RX(3), RX(M3), RX(4), RX(M4)), sxz);
+          const f2 dyz = scale<ISO>(d1(RY(1), RY(M1), RY(2), RY(M2), RY(3), RY(M3), RY(4), RY(M4)), syz);
 #undef RP
 #undef RX
 #undef RY
-          const float *cu = reinterpret_cast<const float *>(st + G::OFF_UPD);
+          const float *cu = reinterpret_cast<const float *>(st + G::OFF_UPD) + ci;
           float czz, cxz, cyz, v2px, v2pz, v2sz, v2pn;
           if constexpr (MT) {
             const int md = st[G::OFF_IDU + ci];
             czz = s_med[(DC_ZZ * kMediaMax) + md];
             cxz = s_med[(DC_XZ * kMediaMax) + md];
             cyz = s_med[(DC_YZ * kMediaMax) + md];
-            v2px = cu[ci];
-            v2pz = cu[G::NT + ci];
-            v2sz = cu[2 * G::NT + ci];
-            v2pn = cu[3 * G::NT + ci];
+            v2px = cu[0];
+            v2pz = cu[G::NT];
+            v2sz = cu[2 * G::NT];
+            v2pn = cu[3 * G::NT];
           } else {
-            czz = cu[ci];
-            cxz = cu[G::NT + ci];
-            cyz = cu[2 * G::NT + ci];
-            v2px = cu[3 * G::NT + ci];
-            v2pz = cu[4 * G::NT + ci];
-            v2sz = cu[5 * G::NT + ci];
-            v2pn = cu[6 * G::NT + ci];
+            czz = cu[0];
+            cxz = cu[G::NT];
+            cyz = cu[2 * G::NT];
+            v2px = cu[3 * G::NT];
+            v2pz = cu[4 * G::NT];
+            v2sz = cu[5 * G::NT];
+            v2pn = cu[6 * G::NT];
           }
-          f2 Ak, Bk;
-          if constexpr (G::AB_SMEM) {
-            const float4 ab = ABs[(abw == kLag ? 0 : abw + 1) * G::NT + ci];
-            Ak = mk2(ab.x, ab.y);
-            Bk = mk2(ab.z, ab.w);
-          } else {
-            Ak = A[cs];
-            Bk = B[cs];
-          }
-          f2 h1, h2;
-          float rhsp, rhsq;
-          if constexpr (D1D1) {
-            // der1der1/sample.h:70-117 in its order, each operation rounded:
-            // h1 = cpxx + cpyy + cpzz + cpxy + cpxz + cpyz (A = cpxx + cpyy,
-            // C = cpxy from the plane's arrival), h2 = pxx + pyy + pzz - h1.
-            const f2 Ck = Cs[(abw == kLag ? 0 : abw + 1) * G::NT + ci];
-            h1 = add_rn(add_rn(add_rn(add_rn(Ak, mul_rn(czz, d2z)), Ck), mul_rn(cxz, dxz)), mul_rn(cyz, dyz));
-            h2 = sub_rn(add_rn(Bk, d2z), h1);
-            const float h1p = lo(h1), h1q = hi(h1), h2p = lo(h2), h2q = hi(h2);
-            const float t = __fmul_rn(v2pz, h1q);
-            rhsp = __fadd_rn(__fadd_rn(__fmul_rn(v2px, h2p), t), __fmul_rn(v2sz, __fsub_rn(h1p, h1q)));
-            rhsq = __fsub_rn(__fadd_rn(__fmul_rn(v2pn, h2p), t), __fmul_rn(v2sz, __fsub_rn(h2p, h2q)));
-          } else {
-            h1 = fma2(splat(cyz), dyz, fma2(splat(cxz), dxz, fma2(splat(czz), d2z, Ak)));
-            h2 = sub2(add2(Bk, d2z), h1);
-            const float h1p = lo(h1), h1q = hi(h1), h2p = lo(h2), h2q = hi(h2);
-            // Explicit roundings: every unrolled copy computes identical floats.
-            const float t = __fmul_rn(v2pz, h1q);
-            rhsp = __fmaf_rn(v2sz, __fsub_rn(h1p, h1q), __fmaf_rn(v2px, h2p, t));
-            rhsq = __fmaf_rn(-v2sz, __fsub_rn(h2p, h2q), __fmaf_rn(v2pn, h2p, t));
-          }
+          const float4 ab = ABs[(abw == kLag ? 0 : abw + 1) * G::NT + ci];
+          const f2 Ak = mk2(ab.x, ab.y), Bk = mk2(ab.z, ab.w);
+          const f2 h1 = fma2(splat(cyz), dyz, fma2(splat(cxz), dxz, fma2(splat(czz), d2z, Ak)));
+          const f2 h2 = sub2(add2(Bk, d2z), h1);
+          const float h1p = lo(h1), h1q = hi(h1), h2p = lo(h2), h2q = hi(h2);
+          // Explicit roundings: every unrolled copy computes identical floats.
+          const float t = __fmul_rn(v2pz, h1q);
+          const float rhsp = __fmaf_rn(v2sz, __fsub_rn(h1p, h1q), __fmaf_rn(v2px, h2p, t));
+          const float rhsq = __fmaf_rn(-v2sz, __fsub_rn(h2p, h2q), __fmaf_rn(v2pn, h2p, t));
           f2 old = reinterpret_cast<const f2 *>(st + G::OFF_PP)[ci];
-          const int zc = k - kLag;
-          if (zc == cor_z) {
-            if (gx == sd.cor_x && gy == sd.cor_y) old = add2(old, splat(P.cor));
-          }
+          if (k == cor_k) old = add2(old, splat(P.cor));
           const f2 cur = Pr[cs];
-          f2 nw;
-          if constexpr (D1D1) {
-            // pp = 2 pc - pp + rhs * dt * dt (der1der1/sample.h:119-120).
-            nw = add_rn(sub_rn(add_rn(cur, cur), old), mul_rn(P.dt, mul_rn(P.dt, mk2(rhsp, rhsq))));
-          } else {
-            nw = fma2(mk2(rhsp, rhsq), splat(P.dt2), sub2(add2(cur, cur), old));
-          }
-          if (valid) out[(long)zc * plane] = nw.v;
+          const f2 nw = fma2(mk2(rhsp, rhsq), splat(P.dt2), sub2(add2(cur, cur), old));
+          if (valid) *out = nw.v;
+          out += plane;
         }
-        if (!mbar_wait(xchg, xphase, wait_ns)) {
-          // A warp of this CTA stopped arriving (it gave up a wait itself):
-          // leave too, so that no thread keeps waiting step after step.
-          *s_abort = 1;
-          atomicOr(P.err, 2u);
-          goto aborted;
-        }
-        xphase ^= 1u;
-        if constexpr (D1D1) {
-          if (center) {
-            // pxy = Der1_y(pDx) / dy (der1der1/sample.h:55); A = cpxx + cpyy,
-            // B = pxx + pyy, C = cpxy.
-            const f2 *dc = db + (ly + kRadius) * G::TX + lx;
-            constexpr int W = G::TX;
-            const f2 pxy = d1_ref(dc[W], dc[-W], dc[2 * W], dc[-2 * W], dc[3 * W], dc[-3 * W], dc[4 * W], dc[-4 * W],
-                                  P.inv_dy);
-            const float *ca = reinterpret_cast<const float *>(st + G::OFF_ARR);
-            const float cxx = ca[ci], cyy = ca[G::NT + ci], cxy = ca[2 * G::NT + ci];
-            const f2 av = add_rn(mul_rn(cxx, d2x), mul_rn(cyy, d2y));
-            const f2 bv = add_rn(d2x, d2y);
-            ABs[abw * G::NT + ci] = make_float4(lo(av), hi(av), lo(bv), hi(bv));
-            Cs[abw * G::NT + ci] = mul_rn(cxy, pxy);
+        if (center) {
+          if (!wait(&halo[stage], phase)) {
+            if (lx == 0) atomicOr(P.err, 2u);
+            return;
           }
-        } else if (center) {
-          const f2 *dr = db + ly * G::HX + lx + kRadius;
           const f2 dxy = scale<ISO>(d1(dr[1], dr[-1], dr[2], dr[-2], dr[3], dr[-3], dr[4], dr[-4]), sxy);
           float cxx, cyy, cxy;
           if constexpr (MT) {
@@ -435,22 +406,20 @@ __global__ void __launch_bounds__(kTileX *TY, MINB)
             cyy = s_med[(DC_YY * kMediaMax) + md];
             cxy = s_med[(DC_XY * kMediaMax) + md];
           } else {
-            const float *ca = reinterpret_cast<const float *>(st + G::OFF_ARR);
-            cxx = ca[ci];
-            cyy = ca[G::NT + ci];
-            cxy = ca[2 * G::NT + ci];
+            const float *ca = reinterpret_cast<const float *>(st + G::OFF_ARR) + ci;
+            cxx = ca[0];
+            cyy = ca[G::NT];
+            cxy = ca[2 * G::NT];
           }
           const f2 av = fma2(splat(cxy), dxy, fma2(splat(cyy), d2y, mul2(splat(cxx), d2x)));
           const f2 bv = add2(d2x, d2y);
-          if constexpr (G::AB_SMEM) {
-            ABs[abw * G::NT + ci] = make_float4(lo(av), hi(av), lo(bv), hi(bv));
-          } else {
-            A[j] = av;
-            B[j] = bv;
-          }
+          ABs[abw * G::NT + ci] = make_float4(lo(av), hi(av), lo(bv), hi(bv));
         }
-        dsel ^= 1;
+        // This warp is done with the stage.
+        __syncwarp();
+        if (lx == 0) mbar_arrive(&empty[stage]);
         abw = abw == kLag ? 0 : abw + 1;
+        if (L::NB < S && ++rb == L::NB) rb = 0;
         if (++stage == S) {
           stage = 0;
           phase ^= 1u;
@@ -458,31 +427,28 @@ __global__ void __launch_bounds__(kTileX *TY, MINB)
       }
     }
   }
-  return;
-aborted:
-  // A bounded wait gave up.  Every thread leaves (the others give up on
-  // their own bounded waits or see the flag); thread 0 first waits, bounded,
-  // for the loads that may still be in flight into this CTA's stages.
-  *s_abort = 1;
-  if (tid == 0) {
-    for (int a = 0; a < S - 2; ++a) {
-      const int s2 = (stage + a) % S;
-      (void)mbar_wait(&full[s2], phase ^ uint32_t(stage + a >= S), kWaitLimitNs);
-    }
-  }
 }
 
 // ---- host side ---------------------------------------------------------------
 
+template <int TY, int S, bool MT = false>
+constexpr size_t smem_bytes() {
+  return Layout<TY, S, MT>::BYTES;
+}
+
+template <class K>
+static cudaError_t set_smem(K kern, size_t smem) {
+  return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+}
+
 template <int TY, int S, int MINB>
 static cudaError_t prepare_t() {
   constexpr size_t smem = smem_bytes<TY, S>();
+  static_assert(smem * MINB + MINB * 1024 <= 228 * 1024, "tile shape exceeds the shared memory of an SM");
   cudaError_t e = cudaSuccess;
-  for (auto kern : {k_propagate_fp32<TY, S, true, kItemsTiles, MINB>, k_propagate_fp32<TY, S, false, kItemsTiles, MINB>,
-                    k_propagate_fp32<TY, S, true, kItemsBatch, MINB>, k_propagate_fp32<TY, S, false, kItemsBatch, MINB>,
-                    k_propagate_fp32<TY, S, true, kItemsSegments, MINB>,
-                    k_propagate_fp32<TY, S, false, kItemsSegments, MINB>})
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  for (auto kern : {k_propagate_fp32<TY, S, true, false, MINB>, k_propagate_fp32<TY, S, false, false, MINB>,
+                    k_propagate_fp32<TY, S, true, true, MINB>, k_propagate_fp32<TY, S, false, true, MINB>})
+    if (e == cudaSuccess) e = set_smem(kern, smem);
   return e;
 }
 
@@ -496,18 +462,14 @@ static cudaError_t launch_t(const PropLaunch &L, cudaStream_t s) {
     ready = true;
   }
   const bool iso = L.p.iso != 0;
-  auto kern = L.batch      ? (iso ? k_propagate_fp32<TY, S, true, kItemsBatch, MINB>
-                                  : k_propagate_fp32<TY, S, false, kItemsBatch, MINB>)
-              : L.p.seg    ? (iso ? k_propagate_fp32<TY, S, true, kItemsSegments, MINB>
-                                  : k_propagate_fp32<TY, S, false, kItemsSegments, MINB>)
-                           : (iso ? k_propagate_fp32<TY, S, true, kItemsTiles, MINB>
-                                  : k_propagate_fp32<TY, S, false, kItemsTiles, MINB>);
-  kern<<<L.grid, kTileX * TY, smem, s>>>(L.m, L.p);
+  auto kern = L.batch ? (iso ? k_propagate_fp32<TY, S, true, true, MINB> : k_propagate_fp32<TY, S, false, true, MINB>)
+                      : (iso ? k_propagate_fp32<TY, S, true, false, MINB> : k_propagate_fp32<TY, S, false, false, MINB>);
+  kern<<<L.grid, propagate_fp32_threads(TY), smem, s>>>(L.m, L.p);
   return cudaGetLastError();
 }
 
-// Supported shapes: rows per tile x stages.  TY = 16 runs one 512-thread CTA
-// per SM; TY = 8 runs two 256-thread CTAs per SM.
+// Supported shapes: rows per tile x stages.  Tiles of 16 and 12 rows run one
+// CTA per SM, tiles of 8 rows two.
 #define FLT_SHAPES(X) X(12, 4, 1) X(12, 5, 1) X(12, 6, 1) X(16, 4, 1) X(16, 5, 1) X(8, 4, 2) X(8, 5, 2)
 
 size_t propagate_fp32_smem_bytes(int ty, int st) {
@@ -518,7 +480,7 @@ size_t propagate_fp32_smem_bytes(int ty, int st) {
   return 0;
 }
 bool propagate_fp32_supported(int ty, int st) { return propagate_fp32_smem_bytes(ty, st) != 0; }
-int propagate_fp32_threads(int ty) { return kTileX * ty; }
+int propagate_fp32_threads(int ty) { return kTileX * (ty + kHelperWarps); }
 int propagate_fp32_ctas_per_sm(int ty) { return ty == 8 ? 2 : 1; }
 
 cudaError_t propagate_fp32_prepare(int ty, int st) {
@@ -529,48 +491,17 @@ cudaError_t propagate_fp32_prepare(int ty, int st) {
   return cudaErrorInvalidValue;
 }
 
-// The Der1-Der1 numerics: one shape (kD1D1Rows x kD1D1Stages), single shot.
-static cudaError_t launch_d1d1(const PropLaunch &L, cudaStream_t s) {
-  constexpr int TY = kD1D1Rows, S = kD1D1Stages;
-  constexpr size_t smem = smem_bytes<TY, S, true>();
-  static_assert(smem <= 227 * 1024, "Der1-Der1 shape exceeds the shared memory of a CTA");
-  auto tiles = k_propagate_fp32<TY, S, false, kItemsTiles, 1, true>;
-  auto segs = k_propagate_fp32<TY, S, false, kItemsSegments, 1, true>;
-  static bool ready = false;
-  if (!ready) {
-    for (auto kern : {tiles, segs}) {
-      const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-      if (e != cudaSuccess) return e;
-    }
-    ready = true;
-  }
-  if (L.batch || L.tile_rows != TY || L.stages != S) return cudaErrorInvalidValue;
-  (L.p.seg ? segs : tiles)<<<L.grid, kTileX * TY, smem, s>>>(L.m, L.p);
-  return cudaGetLastError();
-}
-
 // The fault-injection variant: the default shape, single shot.
 static cudaError_t launch_hook(const PropLaunch &L, cudaStream_t s) {
   constexpr int TY = 16, S = 5;
   constexpr size_t smem = smem_bytes<TY, S>();
-  auto tiles_i = k_propagate_fp32<TY, S, true, kItemsTiles, 1, false, true>;
-  auto tiles_a = k_propagate_fp32<TY, S, false, kItemsTiles, 1, false, true>;
-  auto segs_i = k_propagate_fp32<TY, S, true, kItemsSegments, 1, false, true>;
-  auto segs_a = k_propagate_fp32<TY, S, false, kItemsSegments, 1, false, true>;
-  static bool ready = false;
-  if (!ready) {
-    for (auto kern : {tiles_i, tiles_a, segs_i, segs_a}) {
-      const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-      if (e != cudaSuccess) return e;
-    }
-    ready = true;
-  }
   // Any pipeline depth of the step's own shape: the plan depends on the rows
   // only.  (The coefficient planes are present in either layout.)
   if (L.batch || L.d1d1 || L.tile_rows != TY) return cudaErrorInvalidValue;
-  const bool iso = L.p.iso != 0;
-  auto kern = L.p.seg ? (iso ? segs_i : segs_a) : (iso ? tiles_i : tiles_a);
-  kern<<<L.grid, kTileX * TY, smem, s>>>(L.m, L.p);
+  auto kern = L.p.iso ? k_propagate_fp32<TY, S, true, false, 1, true> : k_propagate_fp32<TY, S, false, false, 1, true>;
+  const cudaError_t e = set_smem(kern, smem);
+  if (e != cudaSuccess) return e;
+  kern<<<L.grid, propagate_fp32_threads(TY), smem, s>>>(L.m, L.p);
   return cudaGetLastError();
 }
 
@@ -579,23 +510,19 @@ static cudaError_t launch_hook(const PropLaunch &L, cudaStream_t s) {
 
 template <int TY, int S>
 static cudaError_t launch_media_t(const PropLaunch &L, cudaStream_t s) {
-  constexpr size_t smem = smem_bytes<TY, S, false, true>();
+  constexpr size_t smem = smem_bytes<TY, S, true>();
   static_assert(smem <= 227 * 1024, "media-table shape exceeds the shared memory of a CTA");
-  auto tiles_i = k_propagate_fp32<TY, S, true, kItemsTiles, 1, false, false, true>;
-  auto tiles_a = k_propagate_fp32<TY, S, false, kItemsTiles, 1, false, false, true>;
-  auto segs_i = k_propagate_fp32<TY, S, true, kItemsSegments, 1, false, false, true>;
-  auto segs_a = k_propagate_fp32<TY, S, false, kItemsSegments, 1, false, false, true>;
+  auto kern_i = k_propagate_fp32<TY, S, true, false, 1, false, true>;
+  auto kern_a = k_propagate_fp32<TY, S, false, false, 1, false, true>;
   static bool ready = false;
   if (!ready) {
-    for (auto kern : {tiles_i, tiles_a, segs_i, segs_a}) {
-      const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    for (auto kern : {kern_i, kern_a}) {
+      const cudaError_t e = set_smem(kern, smem);
       if (e != cudaSuccess) return e;
     }
     ready = true;
   }
-  const bool iso = L.p.iso != 0;
-  auto kern = L.p.seg ? (iso ? segs_i : segs_a) : (iso ? tiles_i : tiles_a);
-  kern<<<L.grid, kTileX * TY, smem, s>>>(L.m, L.p);
+  (L.p.iso ? kern_i : kern_a)<<<L.grid, propagate_fp32_threads(TY), smem, s>>>(L.m, L.p);
   return cudaGetLastError();
 }
 
@@ -609,7 +536,7 @@ bool propagate_fp32_media_supported(int ty, int st) {
 
 cudaError_t propagate_fp32_launch(const PropLaunch &L, cudaStream_t s) {
   if (L.p.stall_step >= 0) return launch_hook(L, s);
-  if (L.d1d1) return launch_d1d1(L, s);
+  if (L.d1d1) return propagate_d1d1_launch(L, s);
   if (L.media) {
     if (L.batch || !L.p.media) return cudaErrorInvalidValue;
 #define X(a, b) \

@@ -1,6 +1,6 @@
-// Pipeline pieces of the FP32 step kernel (propagate_fp32.cu): the
-// shared-memory stage layout, the work items of a launch, and the
-// producer's TMA issue of one step.
+// Pipeline pieces of the FP32 step kernels (propagate_fp32.cu,
+// propagate_d1d1.cu): the shared-memory stage layout, the work items of a
+// launch, and the producer's TMA issue of one step.
 #pragma once
 #include "device_util.cuh"
 #include "fletcher_internal.h"
@@ -10,10 +10,6 @@ namespace flt {
 // Plane k arrives at step k; plane k - kLag is updated at that step.  Its
 // z stencil (planes k-kLag-4 .. k-kLag+4) lives in per-thread rings of
 // kRing planes, and its in-plane terms in kABSlots shared-memory slots.
-// kLag = 4 uses the arriving plane at once.  kLag = 5 makes the update
-// independent of the same step's arrival work, at one more ring plane (124
-// instead of 121 registers) and one more 8 KB slot: bit-identical, and 3%
-// slower at 504^3 (2.287 against 2.217 ms per step).
 constexpr int kLag = 4;
 constexpr int kRing = kLag + 5;
 constexpr int kABSlots = kLag + 1;
@@ -36,98 +32,40 @@ struct Geo {
   static constexpr int OFF_IDU = OFF_IDC + ID_B;  // ids of plane k-4
   static constexpr int STAGE_B = (OFF_IDU + ID_B + 127) / 128 * 128;
   static constexpr int TAB_B = MT ? kAngleCoef * kMediaMax * 4 : 0;
-  // Exchange buffer, double-buffered: D1y of the tile rows with their 4-column
-  // x halo, or (Der1-Der1 numerics) D1x of the tile columns with their 4-row
-  // y halo.
-  static constexpr int DBUF_B = D1D1 ? 2 * HY * TX * 8 : 2 * TY * HX * 8;
-  // Tiles of 16 rows (512 threads, at most 128 registers a thread), and of 8
-  // rows (two CTAs per SM), keep the per-cell in-plane terms (A, B; and C
-  // for the Der1-Der1 numerics) of the last 5 planes in shared memory
-  // instead of a 9-plane register ring.
-  static constexpr bool AB_SMEM = TY >= 16 || TY <= 8;  // 8 rows run two CTAs per SM (128 registers)
-  static constexpr int AB_B = AB_SMEM ? kABSlots * NT * (D1D1 ? 24 : 16) : 0;
+  // One exchange buffer: D1y of the tile rows with their 4-column x halo, or
+  // (Der1-Der1 numerics) D1x of the tile columns with their 4-row y halo.
+  static constexpr int ROW_B = D1D1 ? HY * TX * 8 : TY * HX * 8;
+  // The per-cell in-plane terms (A, B; and C for the Der1-Der1 numerics) of
+  // the last 5 planes.
+  static constexpr int AB_B = kABSlots * NT * (D1D1 ? 24 : 16);
   static_assert(TY % 4 == 0, "tile rows must be a multiple of 4");
-  static_assert(!D1D1 || (AB_SMEM && TY >= 8), "the Der1-Der1 numerics keep their in-plane terms in shared memory");
   static_assert(HALO_B % 128 == 0 && ARR_B % 128 == 0 && UPD_B % 128 == 0 && ID_B % 128 == 0,
                 "stage regions 128-B aligned");
   static_assert(!(MT && D1D1), "the Der1-Der1 numerics read the coefficient planes");
 };
 
-template <int TY, int S, bool D1D1 = false, bool MT = false>
-constexpr size_t smem_bytes() {
-  using G = Geo<TY, D1D1, MT>;
-  return size_t(S) * G::STAGE_B + G::DBUF_B + G::AB_B + G::TAB_B + 8 * S + 8 + 16 + 64 + 128;
-}
-
-// A work item resolved against its shot: tile origin, z range, and (batched
-// launches) the shot's descriptors.
+// A work item: a z range [z0, z1) of the tile column at (x0, y0) of a shot,
+// stored as a segment {x0 + (shot << 16), y0, z0, z1}.  CTA b of a launch
+// takes the segments P.cta_first[b] .. P.cta_first[b + 1] - 1 of P.seg.
 struct Item {
   int x0, y0, z0, z1;
   int shot;
 };
 
-// Work-item kinds of a launch (template parameter MODE):
-//  * kItemsTiles: single shot, items = tiles x uniform z-chunks, chunk-major,
-//    CTA b takes b, b + grid, ... (decoded arithmetically, no lookups);
-//  * kItemsBatch: batched shots, P.seg {x0 + (shot << 16), y0, z0, z1}, CTA
-//    b takes its run cta_first[b] .. cta_first[b + 1] - 1 (each running
-//    shot's own single-shot plan, stacked);
-//  * kItemsSegments: single shot, P.seg {x0, y0, z0, z1}, CTA b takes its run
-//    cta_first[b] .. cta_first[b + 1] - 1.
-constexpr int kItemsTiles = 0, kItemsBatch = 1, kItemsSegments = 2;
-
-template <int TY, int MODE>
-__device__ __forceinline__ Item decode_item(int item, const PropParams &P) {
+template <bool BATCH>
+__device__ __forceinline__ Item decode_item(int4 w) {
   Item it;
-  if constexpr (MODE == kItemsBatch) {
-    const int4 w = P.seg[item];  // {x0 + (shot << 16), y0, z0, z1}
-    it.x0 = w.x & 0xffff;
-    it.y0 = w.y;
-    it.z0 = w.z;
-    it.z1 = w.w;
-    it.shot = w.x >> 16;
-  } else if constexpr (MODE == kItemsSegments) {
-    const int4 w = P.seg[item];  // {x0, y0, z0, z1}
-    it.x0 = w.x;
-    it.y0 = w.y;
-    it.z0 = w.z;
-    it.z1 = w.w;
-    it.shot = 0;
-  } else {
-    const ShotDesc &d = P.one;
-    const int tx = item % d.ntx;
-    const int r = item / d.ntx;
-    const int ty = r % d.nty;
-    const int ch = r / d.nty;
-    it.x0 = kRadius + tx * kTileX;
-    it.y0 = kRadius + ty * TY;
-    it.z0 = d.bord + ch * d.chunk;
-    it.z1 = min(it.z0 + d.chunk, d.sz - d.bord);
-    it.shot = 0;
-  }
+  it.x0 = BATCH ? w.x & 0xffff : w.x;
+  it.y0 = w.y;
+  it.z0 = w.z;
+  it.z1 = w.w;
+  it.shot = BATCH ? w.x >> 16 : 0;
   return it;
-}
-
-// The items of this CTA: first, end and stride.
-struct ItemRange {
-  int first, end, step;
-};
-template <int MODE>
-__device__ __forceinline__ ItemRange item_range(const PropParams &P) {
-  if constexpr (MODE != kItemsTiles) return {P.cta_first[blockIdx.x], P.cta_first[blockIdx.x + 1], 1};
-  else return {(int)blockIdx.x, P.nitems, (int)gridDim.x};
 }
 
 // Descriptors used for one step of item `it` (ids, vel: media-table layout).
 struct StepMaps {
   const CUtensorMap *cur, *prev, *arr, *upd, *ids, *vel;
-};
-
-// The producer's position (next step to load), kept in shared memory so it
-// costs no registers in the other threads.
-struct Cursor {
-  Item it;
-  int item, k, stage;
 };
 
 // Issues the TMA loads of one step (plane k of item `it`) into `stage`.

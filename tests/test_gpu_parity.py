@@ -360,3 +360,18 @@ def test_pitch_padding_is_never_read(kw):
     for a, b in zip(*out):
         assert np.isfinite(b).all()
         assert np.array_equal(a, b)
+
+
+@pytest.mark.parametrize("tile", [(16, 5, -16), (16, 4, -11), (12, 6, -16), (8, 5, -16), (8, 4, -7)])
+def test_many_short_items_per_cta(tile, orc):
+    """Several work items per CTA, each shorter than the stage ring and the
+    z stencil (3 planes and up), so that stages, exchange buffers and the
+    items' headers turn over across item ends; the source on a plane that is
+    the halo of one item and the first plane of the next."""
+    prob = Problem("short", 170, 130, 30, absorb=5, dt=0.0006, steps=9, fcut=45.0, kind="layered", layers=4, seed=12)
+    prob = prob.with_(source=(4 + 64, 4 + 48, 4 + 9))
+    m = prob.model()
+    got = gpu_run(prob, m, tile=tile, use_run=True)
+    ref = orc.run_f32(prob, m)
+    for a, b in zip(got, ref):
+        assert rel_l2(a, b) < TOL_SHORT
