@@ -12,6 +12,13 @@ __device__ __forceinline__ uint32_t smem_addr(const void *p) {
   return static_cast<uint32_t>(__cvta_generic_to_shared(p));
 }
 
+// A warp-uniform value, as the compiler can see: it and what derives from it
+// may then live in uniform registers.
+__device__ __forceinline__ int uniform(int v) { return __shfl_sync(0xffffffffu, v, 0); }
+__device__ __forceinline__ int4 uniform4(int4 v) {
+  return make_int4(uniform(v.x), uniform(v.y), uniform(v.z), uniform(v.w));
+}
+
 // ---- mbarrier ---------------------------------------------------------------
 __device__ __forceinline__ void mbar_init(uint64_t *bar, uint32_t count) {
   asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_addr(bar)), "r"(count) : "memory");

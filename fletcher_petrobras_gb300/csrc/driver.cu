@@ -648,15 +648,6 @@ int build_half_maps(HalfMaps hm[2], unsigned *const Hh[2], unsigned short *const
   return FLETCHER_OK;
 }
 
-// Work items of one shot, chunk-major then rows then columns, so CTAs that
-// run at the same time work on neighbouring tiles of the same z range.
-void fill_items(int4 *items, int shot, int ntx, int nty, int nchunk, int TY) {
-  int n = 0;
-  for (int c = 0; c < nchunk; ++c)
-    for (int ty = 0; ty < nty; ++ty)
-      for (int tx = 0; tx < ntx; ++tx) items[n++] = make_int4(shot, kRadius + tx * kTileX, kRadius + ty * TY, c);
-}
-
 }  // namespace flt
 
 namespace {
@@ -685,10 +676,7 @@ int setup_tiles(int rows, int stages) {
   g.stages = stages;
   g.ntx = (sx - bord - kRadius + kTileX - 1) / kTileX;
   g.nty = (sy - bord - kRadius + TY - 1) / TY;
-  const int per_sm = half_form() ? propagate_half_ctas_per_sm(TY, stages, g.form == FLETCHER_FORM_FP16X, false)
-                                  : propagate_fp32_ctas_per_sm(TY);
-  if (per_sm < 1) return fail(FLETCHER_ERR_CUDA, "tile shape (%d rows, %d stages) fits no CTA on an SM", TY, stages);
-  const int ctas = g.num_sms * per_sm;
+  const int ctas = g.num_sms * (half_form() ? 1 : propagate_fp32_ctas_per_sm(TY));
   const Split sp = plan_segments(ctas, g.ntx, g.nty, TY, bord, sz - 2 * bord, g.zchunks);
   if (g.seg) cudaFree(g.seg);
   if (g.cta_first) cudaFree(g.cta_first);
@@ -707,7 +695,6 @@ int setup_tiles(int rows, int stages) {
   g.desc.F[0] = g.F[0];
   g.desc.F[1] = g.F[1];
   g.desc.sx = sx; g.desc.sy = sy; g.desc.sz = sz; g.desc.pitch = g.pitch; g.desc.bord = bord;
-  g.desc.ntx = g.ntx; g.desc.nty = g.nty;
   g.desc.src_x = g.desc.src_y = g.desc.src_z = -1000;
   g.desc.cor_x = g.desc.cor_y = g.desc.cor_z = -1000;
   return FLETCHER_OK;
@@ -992,10 +979,8 @@ int step() {
   P.media = g.mtab;
   P.shots = nullptr;
   P.maps = nullptr;
-  P.items = nullptr;
   P.seg = g.seg;
   P.cta_first = g.cta_first;
-  P.nitems = g.nseg;
   P.parity = c;
   P.inv_dx = 1.0f / g.dx;
   P.inv_dy = 1.0f / g.dy;
@@ -1504,7 +1489,7 @@ struct BatchShot {
   int *E = nullptr;
   unsigned *Mx = nullptr;
   float *coef = nullptr;
-  int ntx = 0, nty = 0, chunk = 0, nchunk = 0;
+  int ntx = 0, nty = 0;
 };
 
 struct Batch {
@@ -1514,14 +1499,12 @@ struct Batch {
   float dx = 0, dy = 0, dz = 0, dt = 0;
   std::vector<BatchShot> shots;
   std::vector<int> order;      // shot indices, longest run first
-  std::vector<int> items_upto; // items of order[0..i]
   int sealed_rows = 0;
   ShotDesc *d_desc = nullptr;
   ShotMaps *d_maps = nullptr;
-  int4 *d_items = nullptr;          // 16-bit forms: {shot, x0, y0, chunk} items
-  // FP32: for r running shots (the first r of `order`), their single-shot
-  // plans stacked per CTA at d_plan + plan_off[r-1] ({x0 + (shot << 16), y0,
-  // z0, z1}), each CTA's first segment at d_first + (r-1) * (plan_ctas + 1).
+  // For r running shots (the first r of `order`), their single-shot plans
+  // stacked per CTA at d_plan + plan_off[r-1] ({tile x index + (shot << 16),
+  // y0, z0, z1}), each CTA's first segment at d_first + (r-1) * (plan_ctas + 1).
   int4 *d_plan = nullptr;
   int *d_first = nullptr;
   std::vector<long> plan_off;
@@ -1551,7 +1534,7 @@ struct Batch {
   std::vector<HalfShot> h_hshots;   // 16-bit forms
   std::vector<HalfShotMaps> h_hmaps;
   std::vector<ShotDesc> s_desc;
-  std::vector<int> s_nitems, s_grid;
+  std::vector<int> s_grid;
   std::vector<long> s_seg_off, s_first_off;
   int4 *d_sseg = nullptr;
   int *d_sfirst = nullptr;
@@ -1574,13 +1557,11 @@ void batch_free_tables() {
   B.splan_ctas = 0;
   if (B.d_desc) cudaFree(B.d_desc);
   if (B.d_maps) cudaFree(B.d_maps);
-  if (B.d_items) cudaFree(B.d_items);
   if (B.d_hshots) cudaFree(B.d_hshots);
   if (B.d_hmaps) cudaFree(B.d_hmaps);
   if (B.d_order) cudaFree(B.d_order);
   B.d_desc = nullptr;
   B.d_maps = nullptr;
-  B.d_items = nullptr;
   B.d_hshots = nullptr;
   B.d_hmaps = nullptr;
   B.d_order = nullptr;
@@ -1629,21 +1610,15 @@ int batch_seal(int rows, int stages) {
   std::vector<ShotMaps> maps(ns);
   std::vector<HalfShot> hshots(ns);
   std::vector<HalfShotMaps> hmaps(ns);
-  std::vector<int4> items;
   B.order.resize(ns);
   for (int i = 0; i < ns; ++i) B.order[i] = i;
   std::stable_sort(B.order.begin(), B.order.end(),
                    [](int a, int b) { return B.shots[a].nsteps > B.shots[b].nsteps; });
-  B.items_upto.assign(ns, 0);
   for (int oi = 0; oi < ns; ++oi) {
     const int i = B.order[oi];
     BatchShot &s = B.shots[i];
-    const int depth = s.sz - 2 * B.bord;
     s.ntx = (s.sx - B.bord - kRadius + kTileX - 1) / kTileX;
     s.nty = (s.sy - B.bord - kRadius + rows - 1) / rows;
-    s.nchunk = (depth + 127) / 128;
-    s.chunk = (depth + s.nchunk - 1) / s.nchunk;
-    s.nchunk = (depth + s.chunk - 1) / s.chunk;
     if (build_maps(&maps[i], s.F, s.coef, s.sx, s.sy, s.sz, s.pitch, rows)) return g_last_err;
     if (batch_half()) {
       if (build_half_maps(hmaps[i].m, s.Hh, s.Hl, maps[i], s.sx, s.sy, s.sz, s.pitch, rows)) return g_last_err;
@@ -1660,22 +1635,15 @@ int batch_seal(int rows, int stages) {
     d.F[0] = s.F[0];
     d.F[1] = s.F[1];
     d.sx = s.sx; d.sy = s.sy; d.sz = s.sz; d.pitch = s.pitch; d.bord = B.bord;
-    d.ntx = s.ntx; d.nty = s.nty; d.chunk = s.chunk;
     d.src_x = (int)(s.isrc % s.sx);
     d.src_y = (int)((s.isrc / s.sx) % s.sy);
     d.src_z = (int)(s.isrc / ((long)s.sx * s.sy));
     d.cor_x = d.src_x; d.cor_y = d.src_y; d.cor_z = d.src_z;
-    const size_t base = items.size();
-    items.resize(base + (size_t)s.ntx * s.nty * s.nchunk);
-    fill_items(items.data() + base, i, s.ntx, s.nty, s.nchunk, rows);
-    B.items_upto[oi] = (int)items.size();
   }
   CK(dev_malloc(&B.d_desc, sizeof(ShotDesc) * ns));
   CK(dev_malloc(&B.d_maps, sizeof(ShotMaps) * ns));
-  CK(dev_malloc(&B.d_items, sizeof(int4) * items.size()));
   CK(cudaMemcpy(B.d_desc, desc.data(), sizeof(ShotDesc) * ns, cudaMemcpyHostToDevice));
   CK(cudaMemcpy(B.d_maps, maps.data(), sizeof(ShotMaps) * ns, cudaMemcpyHostToDevice));
-  CK(cudaMemcpy(B.d_items, items.data(), sizeof(int4) * items.size(), cudaMemcpyHostToDevice));
   B.h_desc = desc;
   B.h_maps = maps;
   B.h_hshots = hshots;
@@ -1693,7 +1661,7 @@ int batch_seal(int rows, int stages) {
   return FLETCHER_OK;
 }
 
-// The FP32 batch's work split for `ctas` persistent CTAs: each shot's own
+// The persistent launch's work split for `ctas` persistent CTAs: each shot's own
 // single-shot plan (plan_segments, the balanced split the shot would get
 // alone), and for every number r of running shots those of the first r
 // shots of `order` stacked per CTA -- CTA b runs its segments of
@@ -1707,11 +1675,11 @@ int batch_plan(int ctas) {
   B.d_plan = nullptr;
   B.d_first = nullptr;
   const int ns = (int)B.shots.size();
-  if (ns >= 32768) return fail(FLETCHER_ERR_ARGS, "a batch holds at most 32767 shots");
+  if (!batch_half() && ns >= 32768) return fail(FLETCHER_ERR_ARGS, "a batch holds at most 32767 shots");
   std::vector<Split> per(ns);
   for (int oi = 0; oi < ns; ++oi) {
     const BatchShot &s = B.shots[B.order[oi]];
-    if (s.sx >= 65536) return fail(FLETCHER_ERR_ARGS, "batched shots need sx < 65536");
+    if (!batch_half() && s.sx >= 65536) return fail(FLETCHER_ERR_ARGS, "batched shots need sx < 65536");
     per[oi] = plan_segments(ctas, s.ntx, s.nty, B.sealed_rows, B.bord, s.sz - 2 * B.bord, 0);
   }
   std::vector<int4> plan;
@@ -1729,7 +1697,7 @@ int batch_plan(int ctas) {
         const int shot = B.order[oi];
         for (int k = sp.first[b]; k < sp.first[b + 1]; ++k) {
           const int4 w = sp.seg[k];
-          plan.push_back(make_int4(w.x | (shot << 16), w.y, w.z, w.w));
+          plan.push_back(make_int4((w.x - kRadius) / kTileX | (shot << 16), w.y, w.z, w.w));
         }
       }
     }
@@ -1746,6 +1714,14 @@ int batch_plan(int ctas) {
   return FLETCHER_OK;
 }
 
+// Whether the batch fits the segments' packing (16 bits of shot and of tile
+// column).
+bool batch_packs() {
+  for (const BatchShot &s : B.shots)
+    if (s.ntx > 65535) return false;
+  return B.shots.size() <= 65536;
+}
+
 // The chain schedule's per-shot plans for `ctas` persistent CTAs: each
 // shot's own single-shot plan, as DRIVER_Initialize would make it.
 int batch_single_plans(int ctas) {
@@ -1756,7 +1732,6 @@ int batch_single_plans(int ctas) {
   B.d_sfirst = nullptr;
   const int ns = (int)B.shots.size();
   B.s_desc.assign(ns, ShotDesc());
-  B.s_nitems.assign(ns, 0);
   B.s_grid.assign(ns, 1);
   B.s_seg_off.assign(ns, -1);
   B.s_first_off.assign(ns, -1);
@@ -1766,7 +1741,6 @@ int batch_single_plans(int ctas) {
     const BatchShot &s = B.shots[i];
     const int depth = s.sz - 2 * B.bord;
     const Split sp = plan_segments(ctas, s.ntx, s.nty, B.sealed_rows, B.bord, depth, 0);
-    ShotDesc d = B.h_desc[i];
     B.s_seg_off[i] = (long)segs.size();
     B.s_first_off[i] = (long)firsts.size();
     segs.insert(segs.end(), sp.seg.begin(), sp.seg.end());
@@ -1774,9 +1748,7 @@ int batch_single_plans(int ctas) {
     int grid = ctas;
     while (grid > 1 && sp.first[grid - 1] == sp.first[grid]) --grid;
     B.s_grid[i] = grid;
-    B.s_nitems[i] = (int)sp.seg.size();
-    d.chunk = 0;
-    B.s_desc[i] = d;
+    B.s_desc[i] = B.h_desc[i];
   }
   if (!segs.empty()) {
     CK(dev_malloc(&B.d_sseg, sizeof(int4) * segs.size()));
@@ -1821,7 +1793,6 @@ int batch_issue(int it0, int it1, const float *src) {
   PropParams &P = L.p;
   P.shots = B.d_desc;
   P.maps = B.d_maps;
-  P.items = B.d_items;
   P.inv_dx = 1.0f / B.dx;
   P.inv_dy = 1.0f / B.dy;
   P.inv_dz = 1.0f / B.dz;
@@ -1835,16 +1806,16 @@ int batch_issue(int it0, int it1, const float *src) {
   P.dt2 = P.iso ? (B.dt * B.dt) * P.inv_dxx : B.dt * B.dt;
   P.dt = B.dt;
   P.err = B.err_dev;
-  const int ctas = B.ctas;
   int active = ns;  // shots still running, a prefix of B.order
   for (int it = it0; it < it1; ++it) {
     while (active > 0 && B.shots[B.order[active - 1]].nsteps <= it) --active;
     if (active == 0) break;
-    P.nitems = B.items_upto[active - 1];
     P.parity = it & 1;
     P.src = src[it];
     P.cor = it > 0 ? src[it - 1] : 0.0f;
-    L.grid = P.nitems < ctas ? P.nitems : ctas;
+    P.seg = B.d_plan + B.plan_off[active - 1];
+    P.cta_first = B.d_first + (size_t)(active - 1) * (B.plan_ctas + 1);
+    L.grid = B.plan_grid[active - 1];
     if (batch_half()) {
       // The new field's plane exponents (every running shot, one launch),
       // then the step; the current field uses exponent slot it % 3.
@@ -1865,9 +1836,6 @@ int batch_issue(int it0, int it1, const float *src) {
       B.launches += 2;
       continue;
     }
-    P.seg = B.d_plan + B.plan_off[active - 1];
-    P.cta_first = B.d_first + (size_t)(active - 1) * (B.plan_ctas + 1);
-    L.grid = B.plan_grid[active - 1];
     CK(propagate_fp32_launch(L, g_stream));
     ++B.launches;
   }
@@ -1937,7 +1905,6 @@ int batch_issue_chains(int chains, int steps, const float *src) {
         HL.batch = false;
         HL.h.p = P;
         HL.h.p.one = B.s_desc[i];
-        HL.h.p.nitems = B.s_nitems[i];
         HL.h.p.seg = B.d_sseg + B.s_seg_off[i];
         HL.h.p.cta_first = B.d_sfirst + B.s_first_off[i];
         HL.tile_rows = B.sealed_rows;
@@ -1966,7 +1933,6 @@ int batch_issue_chains(int chains, int steps, const float *src) {
       }
       const ShotMaps &m = B.h_maps[i];
       P.one = B.s_desc[i];
-      P.nitems = B.s_nitems[i];
       P.seg = B.d_sseg + B.s_seg_off[i];
       P.cta_first = B.d_sfirst + B.s_first_off[i];
       L.grid = B.s_grid[i];
@@ -2147,25 +2113,18 @@ extern "C" int FLETCHER_BatchRun(const float *src, int max_steps, int use_graph,
                             ? propagate_half_prepare(B.sealed_rows, B.stages, B.form == FLETCHER_FORM_FP16X, true)
                             : propagate_fp32_prepare(B.sealed_rows, B.stages);
   if (pe != cudaSuccess) return fail(FLETCHER_ERR_CUDA, "kernel attribute set-up failed");
-  const int per_sm = batch_half() ? propagate_half_ctas_per_sm(B.sealed_rows, B.stages,
-                                                               B.form == FLETCHER_FORM_FP16X, true)
-                                  : propagate_fp32_ctas_per_sm(B.sealed_rows);
-  if (per_sm < 1)
-    return fail(FLETCHER_ERR_CUDA, "tile shape (%d rows, %d stages) fits no CTA on an SM", B.sealed_rows, B.stages);
-  B.ctas = B.num_sms * per_sm;
-  const int nchains = B.chains < 0 ? batch_auto_chains(steps) : B.chains;
+  B.ctas = B.num_sms * (batch_half() ? 1 : propagate_fp32_ctas_per_sm(B.sealed_rows));
+  int nchains = B.chains < 0 ? batch_auto_chains(steps) : B.chains;
+  // The persistent launch's segments hold 16 bits of shot and of tile column:
+  // a 16-bit batch beyond that runs as one chain (the same fields).
+  if (nchains == 0 && batch_half() && !batch_packs()) nchains = 1;
   B.last_chains = nchains;
   const bool chains = nchains > 0;
-  int plan_ctas = B.ctas;
-  if (chains && batch_half()) {
-    // The single-shot 16-bit kernel: its own attributes and residency.
-    const bool ext = B.form == FLETCHER_FORM_FP16X;
-    if (propagate_half_prepare(B.sealed_rows, B.stages, ext, false) != cudaSuccess)
-      return fail(FLETCHER_ERR_CUDA, "kernel attribute set-up failed");
-    plan_ctas = B.num_sms * propagate_half_ctas_per_sm(B.sealed_rows, B.stages, ext, false);
-    if (plan_ctas < 1) return fail(FLETCHER_ERR_CUDA, "tile shape fits no single-shot CTA on an SM");
-  }
-  if (chains ? batch_single_plans(plan_ctas) : (!batch_half() && batch_plan(B.ctas))) return g_last_err;
+  // The chain schedule's 16-bit kernel is another instantiation.
+  if (chains && batch_half() &&
+      propagate_half_prepare(B.sealed_rows, B.stages, B.form == FLETCHER_FORM_FP16X, false) != cudaSuccess)
+    return fail(FLETCHER_ERR_CUDA, "kernel attribute set-up failed");
+  if (chains ? batch_single_plans(B.ctas) : batch_plan(B.ctas)) return g_last_err;
   auto issue = [&]() { return chains ? batch_issue_chains(nchains, steps, src) : batch_issue(0, steps, src); };
   cudaEvent_t e0, e1;
   CK(cudaEventCreate(&e0));

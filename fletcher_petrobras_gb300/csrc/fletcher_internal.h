@@ -41,7 +41,6 @@ static_assert(DC_V2PX == kAngleCoef && DC_V2PN == kNumCoef - 1, "velocity terms 
 struct ShotDesc {
   float2 *F[2];                  // the two field buffers
   int sx, sy, sz, pitch, bord;
-  int ntx, nty, chunk;           // tiles in x and y, z-chunk length
   int src_x, src_y, src_z;       // cell that gains the step's source (src_z < 0: none)
   int cor_x, cor_y, cor_z;       // cell whose previous-field value lacks the last step's
                                  //   source (added on read; cor_z < 0: none)
@@ -58,17 +57,13 @@ struct ShotMaps {
 };
 
 // One launch: every active shot advances one step.  The work is a list of
-// segments {x0 + (shot << 16), y0, z0, z1}, each a z range of one tile column
-// of a shot (single-shot launches: shot 0); CTA b takes the segments
-// cta_first[b] .. cta_first[b+1]-1.  (Batched 16-bit launches: work items
-// {shot, x0, y0, chunk index}, ordered by shot; CTA b takes items b,
-// b + grid, ... below nitems.)
+// segments, each a z range of one tile column of a shot: {x0, y0, z0, z1}, in
+// batched launches {tile x index + (shot << 16), y0, z0, z1}.  CTA b takes
+// the segments cta_first[b] .. cta_first[b+1]-1.
 struct PropParams {
   ShotDesc one;                     // single-shot launches: the shot itself
   const ShotDesc *shots;            // batched launches: per-shot descriptors
   const ShotMaps *maps;
-  const int4 *items;                // batched 16-bit launches
-  int nitems;
   int parity;                       // current field = F[parity], previous = F[1 - parity]
   float inv_dx, inv_dy, inv_dz;     // 1/dx, 1/dy, 1/dz
   float inv_dxx, inv_dyy, inv_dzz;  // 1/(dx*dx), 1/(dy*dy), 1/(dz*dz) as the reference forms them
@@ -95,7 +90,7 @@ struct SingleMaps {
 struct PropLaunch {
   PropParams p;
   SingleMaps m;           // single-shot launches
-  bool batch;             // true: p.shots / p.maps / p.items describe the work
+  bool batch;             // true: p.shots / p.maps describe the shots
   bool d1d1;              // Der1-Der1 numerics (single shot, 16 x 4 tiles)
   bool media;             // media-table coefficient layout (single shot)
   int tile_rows;          // TY
@@ -151,7 +146,7 @@ struct HalfParams {
   unsigned short *out_lo;             // new field: residual bytes (extended form)
   const int *e_cur, *e_prev, *e_new;  // per-plane exponents of the current, previous and new field
   unsigned *m_new;                    // per-plane max |value| of the new field (float bits), atomicMax
-  // Batched launches (p.items, p.shots): per-shot buffers and maps, and the
+  // Batched launches (p.shots): per-shot buffers and maps, and the
   // exponent slot of the current field (step % 3).
   const HalfShot *hshots;
   const HalfShotMaps *hmaps;
@@ -162,13 +157,12 @@ struct HalfLaunch {
   HalfParams h;
   HalfMaps m;
   int tile_rows, stages, grid;
-  bool batch;  // h.p.items / h.p.shots / h.hshots / h.hmaps describe the work
+  bool batch;  // h.p.shots / h.hshots / h.hmaps describe the shots
 };
 
 bool propagate_half_supported(int tile_rows, int stages);
 cudaError_t propagate_half_launch(const HalfLaunch &L, bool ext, cudaStream_t s);
 cudaError_t propagate_half_prepare(int tile_rows, int stages, bool ext, bool batch);
-int propagate_half_ctas_per_sm(int tile_rows, int stages, bool ext, bool batch);
 cudaError_t half_scales(const unsigned *m_cur, unsigned *m_prev, int *e_new, int sz, int src_z, float src_abs,
                         cudaStream_t s);
 // Before a batched 16-bit step: the new field's plane exponents and the

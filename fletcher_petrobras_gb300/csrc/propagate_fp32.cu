@@ -80,6 +80,8 @@ struct Layout {
   static constexpr int OFF_HDR = OFF_TAB + G::TAB_B;  // the item that starts in stage s
   static constexpr int OFF_BAR = OFF_HDR + S * 16;    // full[S], halo[S], empty[S]
   static constexpr size_t BYTES = size_t(OFF_BAR) + 3 * S * 8 + 128;
+  static_assert(OFF_ROWS % 16 == 0 && OFF_AB % 16 == 0 && OFF_TAB % 4 == 0 && OFF_HDR % 16 == 0 && OFF_BAR % 8 == 0,
+                "shared-memory alignment");
 };
 
 // Register split (setmaxnreg): the compute warps take what the helper warps
@@ -117,7 +119,7 @@ __global__ void __launch_bounds__(kTileX *(TY + kHelperWarps), MINB)
 
   const int tid = threadIdx.x;
   const int lx = tid & 31;
-  const int wid = __shfl_sync(0xffffffffu, tid >> 5, 0);  // warp-uniform
+  const int wid = uniform(tid >> 5);
   const int first = P.cta_first[blockIdx.x], nitems = P.cta_first[blockIdx.x + 1] - first;
   if (nitems <= 0) return;
   constexpr int kHalo = TY / 4 < kHaloWarps ? TY / 4 : kHaloWarps;  // halo warps with work
@@ -293,7 +295,7 @@ __global__ void __launch_bounds__(kTileX *(TY + kHelperWarps), MINB)
       if (lx == 0) atomicOr(P.err, 1u);
       return;
     }
-    const Item it = decode_item<BATCH>(hdr[stage]);
+    const Item it = decode_item<BATCH>(uniform4(hdr[stage]));
     const ShotDesc &sd = BATCH ? P.shots[it.shot] : P.one;
     const int kend = it.z1 + kLag;
     const int gx = it.x0 + lx;

@@ -45,8 +45,9 @@ struct Geo {
 };
 
 // A work item: a z range [z0, z1) of the tile column at (x0, y0) of a shot,
-// stored as a segment {x0 + (shot << 16), y0, z0, z1}.  CTA b of a launch
-// takes the segments P.cta_first[b] .. P.cta_first[b + 1] - 1 of P.seg.
+// stored as a segment {x0, y0, z0, z1}, in batched launches {tile x index +
+// (shot << 16), y0, z0, z1}.  CTA b of a launch takes the segments
+// P.cta_first[b] .. P.cta_first[b + 1] - 1 of P.seg.
 struct Item {
   int x0, y0, z0, z1;
   int shot;
@@ -55,11 +56,11 @@ struct Item {
 template <bool BATCH>
 __device__ __forceinline__ Item decode_item(int4 w) {
   Item it;
-  it.x0 = BATCH ? w.x & 0xffff : w.x;
+  it.x0 = BATCH ? kRadius + (w.x & 0xffff) * kTileX : w.x;
   it.y0 = w.y;
   it.z0 = w.z;
   it.z1 = w.w;
-  it.shot = BATCH ? w.x >> 16 : 0;
+  it.shot = BATCH ? int((unsigned)w.x >> 16) : 0;
   return it;
 }
 

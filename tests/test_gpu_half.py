@@ -143,6 +143,24 @@ def test_launch_shapes_bit_identical(form, tile):
         assert np.array_equal(a, b)
 
 
+@pytest.mark.parametrize("tile", [(16, 5, -16), (16, 4, -11), (12, 6, -16), (8, 6, -16)])
+@pytest.mark.parametrize("form", ["fp16x", "fp16"])
+def test_many_short_items_per_cta(form, tile):
+    """Several work items per CTA, each shorter than the stage ring, the
+    decoded-tile ring and the z stencil: the same floats as whole columns,
+    within the form's short-run bound of the FP32 form."""
+    prob = Problem("hshort", 170, 130, 30, absorb=5, dt=0.0006, steps=9, fcut=45.0, kind="layered", layers=4, seed=12)
+    prob = prob.with_(source=(4 + 64, 4 + 48, 4 + 9))
+    m = prob.model()
+    base, _ = run(prob, m, form, tile=(16, 5, -1))
+    got, _ = run(prob, m, form, tile=tile)
+    for a, b in zip(base, got):
+        assert np.array_equal(a, b)
+    ref, _ = run(prob, m, "fp32")
+    for a, b in zip(base, ref):
+        assert rel_l2(a, b) < TOL[form]["short"]
+
+
 @pytest.mark.parametrize("form", ["fp16x", "fp16"])
 def test_initial_fields_round_trip(form):
     """Encoding of initial fields: every value within the form's significand
