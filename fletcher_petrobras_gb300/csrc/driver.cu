@@ -788,8 +788,6 @@ int initialize(int sx, int sy, int sz, int bord, float dx, float dy, float dz, f
   } else {
     CK(dev_malloc(&g.F[0], g.npitch * sizeof(float2)));
     CK(dev_malloc(&g.F[1], g.npitch * sizeof(float2)));
-    CK(cudaMemsetAsync(g.F[0], 0, g.npitch * sizeof(float2), s));
-    CK(cudaMemsetAsync(g.F[1], 0, g.npitch * sizeof(float2), s));
     g.dev_bytes = 2 * g.npitch * sizeof(float2);
   }
   CK(dev_malloc(&g.coef, g.npitch * kNumCoef * sizeof(float)));
@@ -798,7 +796,6 @@ int initialize(int sx, int sy, int sz, int bord, float dx, float dy, float dz, f
   *g.err_host = 0;
   CK(cudaHostGetDevicePointer((void **)&g.err_dev, g.err_host, 0));
   g.dev_bytes += g.npitch * kNumCoef * sizeof(float) + g.n * sizeof(float);
-  CK(cudaMemsetAsync(g.coef, 0, g.npitch * kNumCoef * sizeof(float), s));
   g_init_mark[1] = now_s();
 
   // Raw model arrays -> coefficients.  On systems whose GPU reads pageable
@@ -864,11 +861,18 @@ int initialize(int sx, int sy, int sz, int bord, float dx, float dy, float dz, f
     }
     if (half) {
       // Buffer 0 holds the current field (exponent slot 0), buffer 1 the
-      // previous one (slot 2).
-      CK(half_encode(p, q, g.Hh[b], g.Hl[b], g.E + (b ? 2 : 0) * sz, g.Mx + b * sz, sx, sy, sz, g.pitch, ext, s));
-    } else {
+      // previous one (slot 2).  Zero fields: the cleared buffers, exponents
+      // and maxima are their stored form.
+      if (p || q)
+        CK(half_encode(p, q, g.Hh[b], g.Hl[b], g.E + (b ? 2 : 0) * sz, g.Mx + b * sz, sx, sy, sz, g.pitch, ext,
+                       s));
+    } else if (p || q) {
+      // (No kernel reads the pitch padding, of the fields or of the
+      // coefficients: only the grid's cells are written.)
       k_pack<<<grid_for(g.n), 256, 0, s>>>(p, q, g.F[b], sx, sy, sz, g.pitch);
       CK(cudaGetLastError());
+    } else {
+      CK(cudaMemsetAsync(g.F[b], 0, g.npitch * sizeof(float2), s));
     }
   }
   CK(cudaStreamSynchronize(s));

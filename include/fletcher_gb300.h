@@ -24,7 +24,8 @@ extern "C" {
 /* ===== Part 1: the reference back-end interface ========================= */
 
 /* Replaces original/driver.h:8-12.  Copies the six raw model arrays and the
- * four initial fields (sx*sy*sz floats each, x fastest) to the GPU, computes
+ * four initial fields (sx*sy*sz floats each, x fastest; a NULL field starts
+ * at zero) to the GPU, computes
  * the ten coefficient fields there in FP64 (original/precomp.h:14-58) and
  * keeps everything resident.  Requires bord >= 4 (the stencil radius).  A
  * model value that is not finite (NaN or infinity) is rejected with
