@@ -200,10 +200,8 @@ __device__ __forceinline__ long ghost_index(const Ghost &G, long i, int sy, int 
 // vpz, epsilon, delta of a cell from its coefficients (v2pz = vpz^2,
 // v2px = vpz^2 (1 + 2 eps), v2pn = vpz^2 (1 + 2 delta): original/precomp.h).
 __device__ __forceinline__ float4 medium_of(const float *coef, int x, int y, int z, int sy, int pitch) {
-  const size_t plane = (size_t)sy * pitch, row = (size_t)y * pitch + x;
-  const size_t base = (size_t)z * kNumCoef * plane + row;
-  const float v2px = coef[base + DC_V2PX * plane], v2pz = coef[base + DC_V2PZ * plane];
-  const float v2pn = coef[base + DC_V2PN * plane];
+  const float *c = coef + coef_index(x, y, z, sy, pitch);
+  const float v2px = c[DC_V2PX * kTileX], v2pz = c[DC_V2PZ * kTileX], v2pn = c[DC_V2PN * kTileX];
   float4 m;
   m.x = sqrtf(v2pz);
   m.y = v2pz > 0.f ? 0.5f * (v2px / v2pz - 1.0f) : 0.f;
@@ -292,8 +290,8 @@ __device__ float2 outer_update(const float2 *F, const float *coef, int x, int y,
   const float qxx = d2[0].y * sx2, qyy = d2[1].y * sy2, qzz = d2[2].y * sz2;
   const float pxy = dc[0].x * sxy, pyz = dc[1].x * syz, pxz = dc[2].x * sxz;
   const float qxy = dc[0].y * sxy, qyz = dc[1].y * syz, qxz = dc[2].y * sxz;
-  const size_t plane = (size_t)sy * pitch, base = (size_t)z * kNumCoef * plane + (size_t)y * pitch + x;
-  auto C = [&](int k) { return coef[base + k * plane]; };
+  const float *c0 = coef + coef_index(x, y, z, sy, pitch);
+  auto C = [&](int k) { return c0[k * kTileX]; };
   const float cxx = C(DC_XX), cyy = C(DC_YY), czz = C(DC_ZZ), cxy = C(DC_XY), cyz = C(DC_YZ), cxz = C(DC_XZ);
   const float h1p = cxx * pxx + cyy * pyy + czz * pzz + cxy * pxy + cyz * pyz + cxz * pxz;
   const float h1q = cxx * qxx + cyy * qyy + czz * qzz + cxy * qxy + cyz * qyz + cxz * qxz;

@@ -6,14 +6,15 @@
 //   F[0], F[1]  (p, q) pairs of float, [sz][sy][pitch], pitch = sx rounded
 //               up to 32; one buffer holds the current field, the other the
 //               previous field, and they swap after every step;
-//   coef        ten FP32 coefficient fields, [sz][10][sy][pitch], computed on
-//               the GPU in FP64 from the raw model arrays;
+//   coef        ten FP32 coefficient fields, by row and tile column
+//               ([sz][sy][tile][10][32], coef_index), computed on the GPU in
+//               FP64 from the raw model arrays;
 //   scratch     one unpitched sx*sy*sz float volume for host transfers;
 //   ids, media  media-table layout (FP32 form, when the model has at most 256
 //               distinct (phi, theta) pairs): one byte per cell naming its
 //               pair, [sz][sy][ipitch] with cell x at byte x + 12, and the six
 //               angle coefficients of each pair, [6][256]; the steps then
-//               read only the four velocity planes of coef.
+//               read only the four velocity terms of coef.
 // The 16-bit forms replace F by Hh[b] (half2 per cell) and, for FP16X, Hl[b]
 // (residual bytes), with per-plane exponents E (three fields: current,
 // previous, next) and per-plane maxima Mx (one per buffer).
@@ -259,9 +260,9 @@ __global__ void k_precompute(Raw6 raw, float *__restrict__ coef, int sx, int sy,
     c[DC_V2PZ] = v2pz;
     c[DC_V2SZ] = v2sz;
     c[DC_V2PN] = v2pn;
-    const size_t x = i % sx, y = (i / sx) % sy, z = i / ((size_t)sx * sy);
+    float *out = coef + coef_index((int)(i % sx), (int)((i / sx) % sy), (int)(i / ((size_t)sx * sy)), sy, pitch);
 #pragma unroll
-    for (int k = 0; k < kNumCoef; ++k) coef[((z * kNumCoef + k) * sy + y) * pitch + x] = c[k];
+    for (int k = 0; k < kNumCoef; ++k) out[k * kTileX] = c[k];
   }
 }
 
@@ -321,9 +322,8 @@ __global__ void k_media_table(const unsigned long long *keys, const unsigned lon
   const int slot = threadIdx.x;
   const bool used = keys[slot] != kEmptyKey;
   const size_t i = used ? rep[slot] : 0;
-  const size_t x = i % sx, y = (i / sx) % sy, z = i / ((size_t)sx * sy);
-  for (int k = 0; k < kAngleCoef; ++k)
-    tab[k * kMediaMax + slot] = used ? coef[((z * kNumCoef + k) * sy + y) * pitch + x] : 0.f;
+  const float *c = coef + coef_index((int)(i % sx), (int)((i / sx) % sy), (int)(i / ((size_t)sx * sy)), sy, pitch);
+  for (int k = 0; k < kAngleCoef; ++k) tab[k * kMediaMax + slot] = used ? c[k * kTileX] : 0.f;
 }
 
 // (p, q) volumes -> pitched pair buffer.  Null p or q gives zeros.
@@ -352,8 +352,8 @@ __global__ void k_unpack_coef(const float *__restrict__ coef, float *__restrict_
                               int pitch) {
   const size_t n = (size_t)sx * sy * sz;
   for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
-    const size_t x = i % sx, y = (i / sx) % sy, z = i / ((size_t)sx * sy);
-    out[i] = coef[((z * kNumCoef + k) * sy + y) * pitch + x];
+    out[i] = coef[coef_index((int)(i % sx), (int)((i / sx) % sy), (int)(i / ((size_t)sx * sy)), sy, pitch) +
+                  k * kTileX];
   }
 }
 
@@ -365,6 +365,19 @@ __global__ void k_poison_pad(float *buf, int width, int sx, int pitch, long rows
   for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < n; i += (long)gridDim.x * blockDim.x) {
     const long r = i / pad, c = i % pad;
     buf[r * (long)pitch * width + (long)sx * width + c] = v;
+  }
+}
+
+// The same for the coefficient block: the columns of its tiles that hold no
+// grid cell.
+__global__ void k_poison_coef(float *coef, int sx, int pitch, long rows, float v) {
+  const int nt = coef_tiles(pitch), width = nt * kTileX;
+  const long n = rows * width;
+  for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < n; i += (long)gridDim.x * blockDim.x) {
+    const int xs = (int)(i % width), x = xs - kCoefShift;
+    if (x >= 0 && x < sx) continue;
+    float *c = coef + (i / width * nt + xs / kTileX) * (kNumCoef * kTileX) + xs % kTileX;
+    for (int k = 0; k < kNumCoef; ++k) c[k * kTileX] = v;
   }
 }
 
@@ -599,6 +612,15 @@ int ensure_stream() {
 
 namespace flt {
 
+// A box of `n` coefficients of a tile's rows.
+int encode_coef(CUtensorMap *m, float *coef, int sy, int sz, int pitch, int n, int TY) {
+  const cuuint64_t row = (cuuint64_t)kNumCoef * kTileX, nt = (cuuint64_t)coef_tiles(pitch);
+  const cuuint64_t dims[4] = {row, nt, (cuuint64_t)sy, (cuuint64_t)sz};
+  const cuuint64_t str[3] = {row * 4, row * nt * 4, row * nt * sy * 4};
+  const cuuint32_t box[4] = {(cuuint32_t)(kTileX * n), 1, (cuuint32_t)TY, 1};
+  return encode(m, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, coef, dims, str, box);
+}
+
 // The six TMA descriptors of one shot: both field buffers with the halo box
 // and the point box, and the coefficient block with the 3- and 7-coefficient
 // boxes.
@@ -611,14 +633,8 @@ int build_maps(ShotMaps *m, float2 *const F[2], float *coef, int sx, int sy, int
     if (encode(&m->halo[b], CU_TENSOR_MAP_DATA_TYPE_INT64, 3, F[b], dims, str, hbox)) return g_last_err;
     if (encode(&m->pt[b], CU_TENSOR_MAP_DATA_TYPE_INT64, 3, F[b], dims, str, pbox)) return g_last_err;
   }
-  const cuuint64_t cdims[4] = {(cuuint64_t)sx, (cuuint64_t)sy, (cuuint64_t)kNumCoef, (cuuint64_t)sz};
-  const cuuint64_t cstr[3] = {(cuuint64_t)pitch * 4, (cuuint64_t)pitch * sy * 4,
-                              (cuuint64_t)pitch * sy * kNumCoef * 4};
-  const cuuint32_t abox[4] = {(cuuint32_t)kTileX, (cuuint32_t)TY, (cuuint32_t)kArrivalCoef, 1};
-  const cuuint32_t ubox[4] = {(cuuint32_t)kTileX, (cuuint32_t)TY, (cuuint32_t)kUpdateCoef, 1};
-  if (encode(&m->arr, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, coef, cdims, cstr, abox)) return g_last_err;
-  if (encode(&m->upd, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, coef, cdims, cstr, ubox)) return g_last_err;
-  return FLETCHER_OK;
+  if (encode_coef(&m->arr, coef, sy, sz, pitch, kArrivalCoef, TY)) return g_last_err;
+  return encode_coef(&m->upd, coef, sy, sz, pitch, kUpdateCoef, TY);
 }
 
 // TMA descriptors of the 16-bit forms: for each choice of current buffer c,
@@ -665,11 +681,7 @@ int setup_tiles(int rows, int stages) {
     const cuuint64_t istr[2] = {(cuuint64_t)g.ipitch, (cuuint64_t)g.ipitch * sy};
     const cuuint32_t ibox[3] = {(cuuint32_t)kTileX, (cuuint32_t)TY, 1};
     if (encode(&g.mids, CU_TENSOR_MAP_DATA_TYPE_UINT8, 3, g.ids, idims, istr, ibox)) return g_last_err;
-    const cuuint64_t cdims[4] = {(cuuint64_t)sx, (cuuint64_t)sy, (cuuint64_t)kNumCoef, (cuuint64_t)sz};
-    const cuuint64_t cstr[3] = {(cuuint64_t)g.pitch * 4, (cuuint64_t)g.pitch * sy * 4,
-                                (cuuint64_t)g.pitch * sy * kNumCoef * 4};
-    const cuuint32_t vbox[4] = {(cuuint32_t)kTileX, (cuuint32_t)TY, (cuuint32_t)kVelCoef, 1};
-    if (encode(&g.mvel, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, g.coef, cdims, cstr, vbox)) return g_last_err;
+    if (encode_coef(&g.mvel, g.coef, sy, sz, g.pitch, kVelCoef, TY)) return g_last_err;
   }
   if (half_form() && build_half_maps(g.hm, g.Hh, g.Hl, g.maps, sx, sy, sz, g.pitch, TY)) return g_last_err;
   g.tile_rows = rows;
@@ -790,12 +802,12 @@ int initialize(int sx, int sy, int sz, int bord, float dx, float dy, float dz, f
     CK(dev_malloc(&g.F[1], g.npitch * sizeof(float2)));
     g.dev_bytes = 2 * g.npitch * sizeof(float2);
   }
-  CK(dev_malloc(&g.coef, g.npitch * kNumCoef * sizeof(float)));
+  CK(dev_malloc(&g.coef, coef_floats(sy, sz, g.pitch) * sizeof(float)));
   CK(dev_malloc(&g.scratch, g.n * sizeof(float)));
   CK(cudaHostAlloc(&g.err_host, sizeof(unsigned), cudaHostAllocMapped));
   *g.err_host = 0;
   CK(cudaHostGetDevicePointer((void **)&g.err_dev, g.err_host, 0));
-  g.dev_bytes += g.npitch * kNumCoef * sizeof(float) + g.n * sizeof(float);
+  g.dev_bytes += coef_floats(sy, sz, g.pitch) * sizeof(float) + g.n * sizeof(float);
   g_init_mark[1] = now_s();
 
   // Raw model arrays -> coefficients.  On systems whose GPU reads pageable
@@ -1246,15 +1258,14 @@ extern "C" int FLETCHER_SetForm(int form) {
 extern "C" int FLETCHER_DebugPoisonPadding(float v) {
   if (!g.init) return fail(FLETCHER_ERR_ARGS, "FLETCHER_DebugPoisonPadding before DRIVER_Initialize");
   if (half_form()) return fail(FLETCHER_ERR_ARGS, "FLETCHER_DebugPoisonPadding: FP32 form only");
-  if (g.pitch == g.sx) return FLETCHER_OK;  // no padding
   const long rows = (long)g.sy * g.sz;
-  for (int b = 0; b < 2; ++b) {
+  for (int b = 0; b < 2 && g.pitch > g.sx; ++b) {
     k_poison_pad<<<grid_for((size_t)rows * (g.pitch - g.sx) * 2), 256, 0, g_stream>>>(
         reinterpret_cast<float *>(g.F[b]), 2, g.sx, g.pitch, rows, v);
     CK(cudaGetLastError());
   }
-  k_poison_pad<<<grid_for((size_t)rows * kNumCoef * (g.pitch - g.sx)), 256, 0, g_stream>>>(
-      g.coef, 1, g.sx, g.pitch, rows * kNumCoef, v);
+  k_poison_coef<<<grid_for((size_t)rows * coef_tiles(g.pitch) * kTileX), 256, 0, g_stream>>>(g.coef, g.sx, g.pitch,
+                                                                                              rows, v);
   CK(cudaGetLastError());
   CK(cudaStreamSynchronize(g_stream));
   return FLETCHER_OK;
@@ -2021,7 +2032,7 @@ extern "C" int FLETCHER_BatchAddShot(int sx, int sy, int sz, const float *model,
     ok = ok && dev_malloc(&s.E, 3 * sz * sizeof(int)) == cudaSuccess;
     ok = ok && dev_malloc(&s.Mx, 2 * sz * sizeof(unsigned)) == cudaSuccess;
   }
-  ok = ok && dev_malloc(&s.coef, s.npitch * kNumCoef * sizeof(float)) == cudaSuccess;
+  ok = ok && dev_malloc(&s.coef, coef_floats(sy, sz, s.pitch) * sizeof(float)) == cudaSuccess;
   float *raw = nullptr;
   ok = ok && dev_malloc(&raw, 6 * s.n * sizeof(float)) == cudaSuccess;
   auto release = [&]() {
@@ -2043,7 +2054,6 @@ extern "C" int FLETCHER_BatchAddShot(int sx, int sy, int sz, const float *model,
   HostPins pin;
   pin.add(model, 6 * s.n * sizeof(float));
   cudaError_t e = cudaMemcpyAsync(raw, model, 6 * s.n * sizeof(float), cudaMemcpyHostToDevice, st);
-  if (e == cudaSuccess) e = cudaMemsetAsync(s.coef, 0, s.npitch * kNumCoef * sizeof(float), st);
   const unsigned long long all_finite = ~0ull;
   if (e == cudaSuccess)
     e = cudaMemcpyToSymbolAsync(g_bad_model, &all_finite, sizeof(all_finite), 0, cudaMemcpyHostToDevice, st);
@@ -2074,7 +2084,7 @@ extern "C" int FLETCHER_BatchAddShot(int sx, int sy, int sz, const float *model,
     return -fail(FLETCHER_ERR_ARGS, "shot %zu: model array %s holds a value that is not finite at cell %llu",
                  B.shots.size(), kModelNames[bad % 8], bad / 8);
   }
-  B.dev_bytes += 2 * fbytes + s.npitch * kNumCoef * sizeof(float);
+  B.dev_bytes += 2 * fbytes + coef_floats(sy, sz, s.pitch) * sizeof(float);
   if (half) B.dev_bytes += (ext ? 2 * s.npitch * sizeof(unsigned short) : 0) + 5 * sz * sizeof(int);
   if (s.n > B.max_n) {
     if (B.scratch) cudaFree(B.scratch);

@@ -10,13 +10,29 @@ constexpr int kRadius = 4;   // stencil half-width of Der2 / DerCross
 constexpr int kTileX = 32;   // tile width in x: one warp per tile row
 constexpr int kNumCoef = 10;
 
-// Device coefficient block layout: [z][c][y][pitch] with c in this order.
-// The first three are read when a plane arrives (in-plane terms), the other
-// seven when the plane is updated four planes later.
+// Device coefficient block layout: [z][y][t][c][32], c in this order and t the
+// tile column of cell x (32 cells, the tiles of the step kernels: t =
+// (x + kCoefShift) / 32), so that the coefficients a tile row needs together
+// are contiguous: 384 bytes of the first three, read when a plane arrives
+// (in-plane terms), and 896 of the other seven, read when the plane is updated
+// four planes later.  Against ten separate planes ([z][c][y][x], 128 bytes at
+// a time): 504^3 1.865 -> 1.792 ms a step (and up to 2.03 ms before on other
+// boxes), 128^3 + shell 82.0 -> 76.4 us.
 enum DevCoef {
   DC_XX = 0, DC_YY, DC_XY,                    // arrival: ch1dxx ch1dyy ch1dxy
   DC_ZZ, DC_XZ, DC_YZ, DC_V2PX, DC_V2PZ, DC_V2SZ, DC_V2PN  // update
 };
+constexpr int kCoefShift = kTileX - kRadius;  // tiles start at x = kRadius + 32 t
+__host__ __device__ inline int coef_tiles(int pitch) { return pitch / kTileX + 1; }
+// Floats of the block; index of coefficient 0 of cell (x, y, z), that of
+// coefficient c being kTileX * c further.
+__host__ __device__ inline size_t coef_floats(int sy, int sz, int pitch) {
+  return (size_t)sz * sy * coef_tiles(pitch) * (kNumCoef * kTileX);
+}
+__host__ __device__ inline size_t coef_index(int x, int y, int z, int sy, int pitch) {
+  const int xs = x + kCoefShift;
+  return (((size_t)z * sy + y) * coef_tiles(pitch) + xs / kTileX) * (kNumCoef * kTileX) + xs % kTileX;
+}
 constexpr int kArrivalCoef = 3;
 constexpr int kUpdateCoef = 7;
 
@@ -52,8 +68,8 @@ struct ShotDesc {
 struct ShotMaps {
   CUtensorMap halo[2];  // field buffer b, box (TX+8, TY+8, 1)
   CUtensorMap pt[2];    // field buffer b, box (TX, TY, 1)
-  CUtensorMap arr;      // coefficients, box (TX, TY, 3, 1)
-  CUtensorMap upd;      // coefficients, box (TX, TY, 7, 1)
+  CUtensorMap arr;      // coefficients, box (TX * 3, 1, TY, 1) of (coefficients, tile, y, z)
+  CUtensorMap upd;      // coefficients, box (TX * 7, 1, TY, 1)
 };
 
 // One launch: every active shot advances one step.  The work is a list of
@@ -84,7 +100,7 @@ struct PropParams {
 // The four descriptors a single-shot launch passes as kernel parameters.
 struct SingleMaps {
   CUtensorMap cur_halo, prev_pt, arr, upd;
-  CUtensorMap ids, vel;  // media-table layout: id volume, box (TX, TY, 1); velocity terms, box (TX, TY, 4, 1)
+  CUtensorMap ids, vel;  // media-table layout: id volume, box (TX, TY, 1); velocity terms, box (TX * 4, 1, TY, 1)
 };
 
 struct PropLaunch {
@@ -184,7 +200,7 @@ struct ResidentView {
   float dx = 0, dy = 0, dz = 0, dt = 0;
   const float2 *cur = nullptr, *prev = nullptr;  // current and previous (p, q) fields (FP32 form)
   float2 *next = nullptr;                        // the buffer the step writes
-  const float *coef = nullptr;                   // [z][10][y][pitch] (DevCoef order)
+  const float *coef = nullptr;                   // coefficient block (DevCoef order)
   cudaStream_t stream = nullptr;
   int num_sms = 0;
   unsigned *err = nullptr;                       // the error word (bit 0: a bounded wait gave up)

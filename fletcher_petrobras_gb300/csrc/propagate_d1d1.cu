@@ -203,10 +203,10 @@ __global__ void __launch_bounds__(kTileX *TY, 1)
 #undef RP
 #undef RX
 #undef RY
-          const float *cu = reinterpret_cast<const float *>(st + G::OFF_UPD);
-          const float czz = cu[ci], cxz = cu[G::NT + ci], cyz = cu[2 * G::NT + ci];
-          const float v2px = cu[3 * G::NT + ci], v2pz = cu[4 * G::NT + ci];
-          const float v2sz = cu[5 * G::NT + ci], v2pn = cu[6 * G::NT + ci];
+          const float *cu = reinterpret_cast<const float *>(st + G::OFF_UPD) + (ly * (kUpdateCoef * G::TX) + lx);
+          const float czz = cu[0], cxz = cu[G::TX], cyz = cu[2 * G::TX];
+          const float v2px = cu[3 * G::TX], v2pz = cu[4 * G::TX];
+          const float v2sz = cu[5 * G::TX], v2pn = cu[6 * G::TX];
           const int slot = abw == kLag ? 0 : abw + 1;
           const float4 ab = ABs[slot * G::NT + ci];
           const f2 Ak = mk2(ab.x, ab.y), Bk = mk2(ab.z, ab.w);
@@ -244,8 +244,8 @@ __global__ void __launch_bounds__(kTileX *TY, 1)
           constexpr int W = G::TX;
           const f2 pxy = d1_ref(dc[W], dc[-W], dc[2 * W], dc[-2 * W], dc[3 * W], dc[-3 * W], dc[4 * W], dc[-4 * W],
                                 P.inv_dy);
-          const float *ca = reinterpret_cast<const float *>(st + G::OFF_ARR);
-          const float cxx = ca[ci], cyy = ca[G::NT + ci], cxy = ca[2 * G::NT + ci];
+          const float *ca = reinterpret_cast<const float *>(st + G::OFF_ARR) + (ly * (kArrivalCoef * G::TX) + lx);
+          const float cxx = ca[0], cyy = ca[G::TX], cxy = ca[2 * G::TX];
           const f2 av = add_rn(mul_rn(cxx, d2x), mul_rn(cyy, d2y));
           const f2 bv = add_rn(d2x, d2y);
           ABs[abw * G::NT + ci] = make_float4(lo(av), hi(av), lo(bv), hi(bv));

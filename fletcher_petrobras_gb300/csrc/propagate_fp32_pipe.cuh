@@ -80,19 +80,20 @@ __device__ __forceinline__ void issue_step(unsigned char *stage, uint64_t *bar, 
   const bool upd = (k - kLag >= it.z0);
   const uint32_t bytes =
       G::HALO_B + (center ? G::ARR_B + G::ID_B : 0) + (upd ? G::UPD_B + G::PP_B + G::ID_B : 0);
+  const int ct = (it.x0 + kCoefShift) / kTileX;  // tile column in the coefficient block
   mbar_arrive_expect_tx(bar, bytes);
   tma_load_3d(stage, m.cur, bar, it.x0 - kRadius, it.y0 - kRadius, k);
   if constexpr (MT) {
     if (center) tma_load_3d(stage + G::OFF_IDC, m.ids, bar, it.x0 + kIdShift, it.y0, k);
     if (upd) {
-      tma_load_4d(stage + G::OFF_UPD, m.vel, bar, it.x0, it.y0, DC_V2PX, k - kLag);
+      tma_load_4d(stage + G::OFF_UPD, m.vel, bar, DC_V2PX * kTileX, ct, it.y0, k - kLag);
       tma_load_3d(stage + G::OFF_IDU, m.ids, bar, it.x0 + kIdShift, it.y0, k - kLag);
       tma_load_3d(stage + G::OFF_PP, m.prev, bar, it.x0, it.y0, k - kLag);
     }
   } else {
-    if (center) tma_load_4d(stage + G::OFF_ARR, m.arr, bar, it.x0, it.y0, 0, k);
+    if (center) tma_load_4d(stage + G::OFF_ARR, m.arr, bar, 0, ct, it.y0, k);
     if (upd) {
-      tma_load_4d(stage + G::OFF_UPD, m.upd, bar, it.x0, it.y0, kArrivalCoef, k - kLag);
+      tma_load_4d(stage + G::OFF_UPD, m.upd, bar, kArrivalCoef * kTileX, ct, it.y0, k - kLag);
       tma_load_3d(stage + G::OFF_PP, m.prev, bar, it.x0, it.y0, k - kLag);
     }
   }
