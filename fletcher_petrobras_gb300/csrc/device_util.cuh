@@ -110,6 +110,14 @@ __device__ __forceinline__ unsigned atom_add_acq_rel_cta(unsigned *p, unsigned v
   return old;
 }
 
+// ---- dependent launches ----------------------------------------------------
+// A step's launch may start while the launch before it still runs
+// (launch_step): its CTAs set themselves up, then wait here until that launch
+// has completed and its writes are visible.
+__device__ __forceinline__ void wait_previous_launch() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+// Lets the next launch start as CTAs of this one leave.
+__device__ __forceinline__ void allow_next_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
 // ---- TMA -----------------------------------------------------------------
 __device__ __forceinline__ void fence_proxy_async_smem() {
   asm volatile("fence.proxy.async.shared::cta;" ::: "memory");

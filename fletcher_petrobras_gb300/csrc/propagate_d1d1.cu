@@ -83,6 +83,8 @@ __global__ void __launch_bounds__(kTileX *TY, 1)
     *cur = c;
   }
   __syncthreads();
+  allow_next_launch();
+  wait_previous_launch();
   if (producer) {
     tma_prefetch_desc(maps.cur);
     tma_prefetch_desc(maps.prev);
@@ -288,8 +290,7 @@ cudaError_t propagate_d1d1_launch(const PropLaunch &L, cudaStream_t s) {
     ready = true;
   }
   if (L.batch || L.tile_rows != TY || L.stages != S) return cudaErrorInvalidValue;
-  k_propagate_d1d1<TY, S><<<L.grid, kTileX * TY, smem, s>>>(L.m, L.p);
-  return cudaGetLastError();
+  return launch_step(k_propagate_d1d1<TY, S>, L.grid, kTileX * TY, smem, s, L.m, L.p);
 }
 
 }  // namespace flt

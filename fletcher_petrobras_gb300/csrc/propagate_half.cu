@@ -237,6 +237,8 @@ __global__ void __launch_bounds__(kTileX *(TY + kHelperWarps), 1)
     mbar_fence_init();
   }
   __syncthreads();
+  allow_next_launch();
+  wait_previous_launch();
 
   if (wid >= TY) {
     setmaxnreg_dec<RegsH<TY>::kHelper>();
@@ -562,6 +564,8 @@ __global__ void __launch_bounds__(kTileX *(TY + kHelperWarps), 1)
 __global__ void k_half_scales(const unsigned *__restrict__ m_cur, unsigned *__restrict__ m_prev, int *__restrict__ e_new,
                               int sz, int src_z, float src_abs) {
   const int z = blockIdx.x * blockDim.x + threadIdx.x;
+  allow_next_launch();
+  wait_previous_launch();
   if (z >= sz) return;
   float b = 0.0f;
   for (int dz = -kRadius; dz <= kRadius; ++dz)
@@ -662,8 +666,7 @@ static cudaError_t launch_half_t(const HalfLaunch &L, cudaStream_t s) {
   const cudaError_t e = prepare_half_t<TY, S, EXT, BATCH>();
   if (e != cudaSuccess) return e;
   auto kern = L.h.p.iso ? k_propagate_half<TY, S, true, EXT, BATCH> : k_propagate_half<TY, S, false, EXT, BATCH>;
-  kern<<<L.grid, kTileX * (TY + kHelperWarps), LayoutH<TY, S, EXT>::BYTES, s>>>(L.m, L.h);
-  return cudaGetLastError();
+  return launch_step(kern, L.grid, kTileX * (TY + kHelperWarps), LayoutH<TY, S, EXT>::BYTES, s, L.m, L.h);
 }
 
 bool propagate_half_supported(int tile_rows, int stages) {
@@ -700,14 +703,15 @@ cudaError_t propagate_half_prepare(int tile_rows, int stages, bool ext, bool bat
 
 cudaError_t half_scales(const unsigned *m_cur, unsigned *m_prev, int *e_new, int sz, int src_z, float src_abs,
                         cudaStream_t s) {
-  k_half_scales<<<(sz + 127) / 128, 128, 0, s>>>(m_cur, m_prev, e_new, sz, src_z, src_abs);
-  return cudaGetLastError();
+  return launch_step(k_half_scales, (sz + 127) / 128, 128, 0, s, m_cur, m_prev, e_new, sz, src_z, src_abs);
 }
 
 // The same for every running shot of a batch (block i: shot order[i]); the
 // current field is in buffer c and uses exponent slot ecur.
 __global__ void k_half_scales_batch(const HalfShot *__restrict__ hs, const ShotDesc *__restrict__ sd,
                                     const int *__restrict__ order, int c, int ecur, float src_abs) {
+  allow_next_launch();
+  wait_previous_launch();
   const int shot = order[blockIdx.x];
   const int sz = sd[shot].sz, src_z = sd[shot].src_z;
   const unsigned *m_cur = hs[shot].Mx + c * sz;
@@ -732,8 +736,7 @@ __global__ void k_half_scales_batch(const HalfShot *__restrict__ hs, const ShotD
 
 cudaError_t half_scales_batch(const HalfShot *hs, const ShotDesc *sd, const int *order, int active, int c, int ecur,
                               float src_abs, cudaStream_t s) {
-  k_half_scales_batch<<<active, 256, 0, s>>>(hs, sd, order, c, ecur, src_abs);
-  return cudaGetLastError();
+  return launch_step(k_half_scales_batch, active, 256, 0, s, hs, sd, order, c, ecur, src_abs);
 }
 
 cudaError_t half_encode(const float *p, const float *q, unsigned *hv, unsigned short *rv, int *e, unsigned *m, int sx,
