@@ -29,23 +29,28 @@
 //  * plane k-4 is completed at step k and written with coalesced 64-bit
 //    stores into the previous-field buffer (in place).
 //
-// What bounds it: HBM.  At 504^3 (183 M updated cells, 64 B each) a step
-// takes 1.86 ms, 93% of the measured copy bandwidth, against 2.22 ms (78%)
-// for the kernel before it, whose 16 warps exchanged D1y, and refilled the
-// stages, in one CTA-wide exchange a plane; 128^3 + shell 81.8 against 92.8
-// us, 56^3 + shell 14.4 against 18.5 us.  Two causes:
+// What bounds it: HBM and the shared-memory pipe, about equally.  At 504^3
+// (183 M updated cells, 64 B each) a step takes 1.79 to 1.81 ms, 96% of the
+// measured copy bandwidth; a plane of a tile costs an SM about 1500 cycles of
+// shared-memory wavefronts (38 loads and stores a warp, the TMA writes), 0.73
+// us, which is what it takes there.  Before the warps were specialised, 16
+// warps that exchanged D1y, and refilled the stages, in one CTA-wide exchange
+// a plane took 2.22 ms.  What made the difference:
 //  * the loop is unrolled over the 9 ring slots, and with the producer, the
 //    source and the timed waits in it the code was 102 KB (the instruction
 //    fetch was the stall of 1.1 of 8.4 cycles an issue); moved to the helper
-//    warps and counted waits, it is 39 KB;
+//    warps and counted waits, it is 34 KB;
 //  * a stage is refilled the moment its last reader releases it, whichever
 //    warp that is, and the warps may run up to S planes apart.  (Groups of 4
 //    warps that exchange among themselves, with the refill still issued by
 //    a compute warp, took 2.48 ms: warps that run ahead of the producing
 //    warp find their loads not yet issued.)
+//  * one wait a step (for the halo warps, which wait for the loads) and one
+//    base address for all that a stage holds: 14% fewer instructions, 272^3
+//    updated cells 205.1 -> 203.5 us.
 // 16 rows: 16 compute warps at 112 registers hold the 27 ring values and a
-// plane's neighbourhood without a spill; 12 rows took 322 and 8 rows (two
-// CTAs an SM) 377 us where 16 rows take 309 (312^3 updated cells).
+// plane's neighbourhood without a spill; 12 rows take 225 and 8 rows (two
+// CTAs an SM) 214 us where 16 rows take 203.5 (272^3 updated cells).
 //
 // Media-table layout (template parameter MT): instead of the ten coefficient
 // planes a stage holds the one-byte medium ids of planes k and k-4 and the
@@ -68,19 +73,30 @@ namespace flt {
 constexpr int kHelperWarps = 4;  // producer warp + 3 halo warps: one warpgroup (setmaxnreg works on warpgroups)
 constexpr int kHaloWarps = kHelperWarps - 1;
 
-// Shared memory of a CTA.  Rows: the D1y exchange buffers, one per stage
-// (two for the 8 x 5 shape, whose two CTAs share an SM's memory).
+// Shared memory of a CTA: S stages, then what is not per stage.  A stage
+// holds its TMA tiles (Geo), the D1y exchange rows of its plane, the in-plane
+// terms (A, B) of its plane when five stages match their five slots, and a
+// control block: everything a step addresses is one base away.  (The 8 x 5
+// shape, whose two CTAs share an SM's memory, has two exchange buffers.)
 template <int TY, int S, bool MT>
 struct Layout {
   using G = Geo<TY, false, MT>;
   static constexpr int NB = (TY <= 8 && S > 4) ? 2 : S;
-  static constexpr int OFF_ROWS = S * G::STAGE_B;
-  static constexpr int OFF_AB = OFF_ROWS + NB * G::ROW_B;
-  static constexpr int OFF_TAB = OFF_AB + G::AB_B;
-  static constexpr int OFF_HDR = OFF_TAB + G::TAB_B;  // the item that starts in stage s
-  static constexpr int OFF_BAR = OFF_HDR + S * 16;    // full[S], halo[S], empty[S]
-  static constexpr size_t BYTES = size_t(OFF_BAR) + 3 * S * 8 + 128;
-  static_assert(OFF_ROWS % 16 == 0 && OFF_AB % 16 == 0 && OFF_TAB % 4 == 0 && OFF_HDR % 16 == 0 && OFF_BAR % 8 == 0,
+  static constexpr bool ROWS_IN = NB == S, AB_IN = S == kABSlots;
+  static constexpr int AB_SLOT = G::NT * 16;
+  static constexpr int OFF_SROWS = G::STAGE_B;
+  static constexpr int OFF_SAB = OFF_SROWS + (ROWS_IN ? G::ROW_B : 0);
+  static constexpr int OFF_CTL = OFF_SAB + (AB_IN ? AB_SLOT : 0);
+  static constexpr int OFF_HDR = OFF_CTL;         // the item that starts in the stage
+  static constexpr int OFF_FULL = OFF_CTL + 16;   // barriers: loads landed,
+  static constexpr int OFF_READY = OFF_CTL + 24;  //   halo columns and source written too,
+  static constexpr int OFF_EMPTY = OFF_CTL + 32;  //   released by every reader
+  static constexpr int SB = OFF_CTL + 128;
+  static constexpr int OFF_ROWS = S * SB;  // [NB] exchange buffers, when not in the stages
+  static constexpr int OFF_AB = OFF_ROWS + (ROWS_IN ? 0 : NB * G::ROW_B);
+  static constexpr int OFF_TAB = OFF_AB + (AB_IN ? 0 : kABSlots * AB_SLOT);
+  static constexpr size_t BYTES = size_t(OFF_TAB) + G::TAB_B + 128;
+  static_assert(OFF_CTL % 128 == 0 && OFF_ROWS % 128 == 0 && OFF_AB % 128 == 0 && OFF_TAB % 128 == 0,
                 "shared-memory alignment");
 };
 
@@ -109,13 +125,8 @@ __global__ void __launch_bounds__(kTileX *(TY + kHelperWarps), MINB)
   // Align in the shared window (pointer arithmetic on the shared array keeps
   // every access below a shared-memory access).
   unsigned char *smem = smem_dyn + ((128u - (smem_addr(smem_dyn) & 127u)) & 127u);
-  f2 *rows = reinterpret_cast<f2 *>(smem + L::OFF_ROWS);         // [NB][TY][HX]
-  float4 *ABs = reinterpret_cast<float4 *>(smem + L::OFF_AB);    // [kABSlots][NT]
-  float *s_med = reinterpret_cast<float *>(smem + L::OFF_TAB);   // [6][256] (MT)
-  int4 *hdr = reinterpret_cast<int4 *>(smem + L::OFF_HDR);
-  uint64_t *full = reinterpret_cast<uint64_t *>(smem + L::OFF_BAR);
-  uint64_t *halo = full + S;   // halo columns (and source) of the stage's plane written
-  uint64_t *empty = halo + S;  // stage released by every reader
+  float *s_med = reinterpret_cast<float *>(smem + L::OFF_TAB);  // [6][256] (MT)
+  auto bar = [&](unsigned char *st, int off) { return reinterpret_cast<uint64_t *>(st + off); };
 
   const int tid = threadIdx.x;
   const int lx = tid & 31;
@@ -125,9 +136,10 @@ __global__ void __launch_bounds__(kTileX *(TY + kHelperWarps), MINB)
   constexpr int kHalo = TY / 4 < kHaloWarps ? TY / 4 : kHaloWarps;  // halo warps with work
   if (tid == 0) {
     for (int s = 0; s < S; ++s) {
-      mbar_init(&full[s], 1);
-      mbar_init(&halo[s], kHalo);
-      mbar_init(&empty[s], TY + kHalo);
+      unsigned char *st = smem + s * L::SB;
+      mbar_init(bar(st, L::OFF_FULL), 1);
+      mbar_init(bar(st, L::OFF_READY), kHalo);
+      mbar_init(bar(st, L::OFF_EMPTY), TY + kHalo);
     }
     mbar_fence_init();
   }
@@ -138,9 +150,9 @@ __global__ void __launch_bounds__(kTileX *(TY + kHelperWarps), MINB)
   allow_next_launch();
   wait_previous_launch();
   // Every wait is bounded; the fault-injection variant's by P.wait_ns.
-  auto wait = [&](uint64_t *bar, uint32_t parity) {
-    if constexpr (HOOK) return mbar_wait(bar, parity, P.wait_ns);
-    else return mbar_spin(bar, parity);
+  auto wait = [&](uint64_t *b, uint32_t parity) {
+    if constexpr (HOOK) return mbar_wait(b, parity, P.wait_ns);
+    else return mbar_spin(b, parity);
   };
 
   if (wid >= TY) {
@@ -192,16 +204,17 @@ __global__ void __launch_bounds__(kTileX *(TY + kHelperWarps), MINB)
         const StepMaps m = maps_of(it.shot);
         for (int k = it.z0 - kRadius; k < it.z1 + kLag; ++k) {
           // (The first S waits pass at once: the stage was never filled.)
-          if (!wait(&empty[stage], phase ^ 1u)) {
+          unsigned char *st = smem + stage * L::SB;
+          if (!wait(bar(st, L::OFF_EMPTY), phase ^ 1u)) {
             ok = false;
             break;
           }
           fence_proxy_async_smem();
-          if (k == it.z0 - kRadius) hdr[stage] = w;
+          if (k == it.z0 - kRadius) *reinterpret_cast<int4 *>(st + L::OFF_HDR) = w;
           // Test hook: CTA 0 skips the loads of its P.stall_step-th step, so
           // that the waits for that stage give up.
           if (!HOOK || issued != P.stall_step || blockIdx.x != 0)
-            issue_step<TY, MT>(smem + stage * G::STAGE_B, &full[stage], it, k, m);
+            issue_step<TY, MT>(st, bar(st, L::OFF_FULL), it, k, m);
           ++issued;
           if (++stage == S) {
             stage = 0;
@@ -216,7 +229,7 @@ __global__ void __launch_bounds__(kTileX *(TY + kHelperWarps), MINB)
         atomicOr(P.err, 2u);
         for (int a = 1; a <= S && a <= issued; ++a) {
           const int s2 = stage >= a ? stage - a : stage + S - a;
-          (void)mbar_wait(&full[s2], stage >= a ? phase : phase ^ 1u, kDrainNs);
+          (void)mbar_wait(bar(smem + s2 * L::SB, L::OFF_FULL), stage >= a ? phase : phase ^ 1u, kDrainNs);
         }
       }
       return;
@@ -231,22 +244,22 @@ __global__ void __launch_bounds__(kTileX *(TY + kHelperWarps), MINB)
       const ShotDesc &sd = BATCH ? P.shots[it.shot] : P.one;
       const int src_z = sd.src_z;
       for (int k = it.z0 - kRadius; k < it.z1 + kLag; ++k) {
-        bool ok = wait(&full[stage], phase);
+        unsigned char *st = smem + stage * L::SB;
+        bool ok = wait(bar(st, L::OFF_FULL), phase);
         if constexpr (L::NB < S) {
           // The row buffer's last readers: the step NB back.
           const int es = stage >= L::NB ? stage - L::NB : stage + S - L::NB;
-          ok = ok && wait(&empty[es], stage >= L::NB ? phase : phase ^ 1u);
+          ok = ok && wait(bar(smem + es * L::SB, L::OFF_EMPTY), stage >= L::NB ? phase : phase ^ 1u);
         }
         if (!ok) {
           atomicOr(P.err, 1u);
           return;
         }
-        f2 *H = reinterpret_cast<f2 *>(smem + stage * G::STAGE_B);
+        f2 *H = reinterpret_cast<f2 *>(st);
         if (k == src_z) {
           // Fused source (original/OpenMP/openmp_insertsource.c:7-13): the
           // current p and q gain `src` at the source cell before the update
-          // reads them.  (On this plane the compute warps wait for the halo
-          // warps before they read the tile.)
+          // reads them.
           const int rx = sd.src_x - (it.x0 - kRadius), ry = sd.src_y - (it.y0 - kRadius);
           if (hw == 0 && lx == 0 && rx >= 0 && rx < G::HX && ry >= 0 && ry < G::HY) {
             H[ry * G::HX + rx] = add2(H[ry * G::HX + rx], splat(P.src));
@@ -255,7 +268,7 @@ __global__ void __launch_bounds__(kTileX *(TY + kHelperWarps), MINB)
           asm volatile("bar.sync 1, %0;" ::"n"(32 * kHalo) : "memory");
         }
         if (k >= it.z0 && k < it.z1) {
-          f2 *db = rows + (L::NB < S ? rb : stage) * (TY * G::HX);
+          f2 *db = reinterpret_cast<f2 *>(L::ROWS_IN ? st + L::OFF_SROWS : smem + L::OFF_ROWS + rb * G::ROW_B);
           for (int r = hw * 4 + (lx >> 3); r < TY; r += 4 * kHalo) {
             const f2 *h = H + (r + kRadius) * G::HX + hxc;
             f2 d = mul2(splat(cL1), sub2(h[G::HX], h[-G::HX]));
@@ -267,10 +280,10 @@ __global__ void __launch_bounds__(kTileX *(TY + kHelperWarps), MINB)
         }
         __syncwarp();
         if (lx == 0) {
-          mbar_arrive(&halo[stage]);
-          mbar_arrive(&empty[stage]);
+          mbar_arrive(bar(st, L::OFF_READY));
+          mbar_arrive(bar(st, L::OFF_EMPTY));
         }
-        if (L::NB < S && ++rb == L::NB) rb = 0;
+        if (!L::ROWS_IN && ++rb == L::NB) rb = 0;
         if (++stage == S) {
           stage = 0;
           phase ^= 1u;
@@ -290,16 +303,17 @@ __global__ void __launch_bounds__(kTileX *(TY + kHelperWarps), MINB)
   const int hc = (ly + kRadius) * G::HX + (lx + kRadius);
   int stage = 0;
   uint32_t phase = 0;
-  int rb = 0;
+  int rb = 0;   // exchange buffer (when not in the stages)
   int abw = 0;  // shared A/B ring slot of the arriving plane (the plane kLag back is at abw + 1)
+  unsigned char *st = smem;
   for (int item = 0; item < nitems; ++item) {
-    if (!wait(&full[stage], phase)) {
+    if (!wait(bar(st, L::OFF_READY), phase)) {
       if (lx == 0) atomicOr(P.err, 1u);
       return;
     }
-    const Item it = decode_item<BATCH>(uniform4(hdr[stage]));
+    const Item it = decode_item<BATCH>(uniform4(*reinterpret_cast<const int4 *>(st + L::OFF_HDR)));
     const ShotDesc &sd = BATCH ? P.shots[it.shot] : P.one;
-    const int kend = it.z1 + kLag;
+    const int depth = it.z1 - it.z0;
     const int gx = it.x0 + lx;
     const int gy = it.y0 + ly;
     const int bord = sd.bord, sxs = sd.sx, sys = sd.sy;
@@ -307,24 +321,23 @@ __global__ void __launch_bounds__(kTileX *(TY + kHelperWarps), MINB)
     const long plane = (long)sd.pitch * sys;
     unsigned long long *out =
         reinterpret_cast<unsigned long long *>(sd.F[P.parity ^ 1]) + (it.z0 * plane + (long)gy * sd.pitch + gx);
-    const int src_z = sd.src_z;
     // The cell that lacks the last step's source, if it is this thread's.
-    const int cor_k = (gx == sd.cor_x && gy == sd.cor_y) ? sd.cor_z + kLag : -1000;
+    const int cor_k = (gx == sd.cor_x && gy == sd.cor_y) ? sd.cor_z + kLag - it.z0 : -1000;
 
     f2 Pr[kRing], Dx[kRing], Dy[kRing];
 
-    for (int kb = it.z0 - kRadius; kb < kend; kb += kRing) {
+    for (int kb = -kRadius; kb < depth + kLag; kb += kRing) {
 #pragma unroll
       for (int j = 0; j < kRing; ++j) {
-        const int k = kb + j;
-        if (k >= kend) break;
-        unsigned char *st = smem + stage * G::STAGE_B;
-        if (!wait(&full[stage], phase) || (k == src_z && !wait(&halo[stage], phase))) {
+        const int k = kb + j;  // plane, counted from the item's first
+        if (k >= depth + kLag) break;
+        if (!wait(bar(st, L::OFF_READY), phase)) {
           if (lx == 0) atomicOr(P.err, 1u);
           return;
         }
-        const bool center = (k >= it.z0) && (k < it.z1);
-        const bool upd = (k - kLag >= it.z0);
+        unsigned char *const st_next = stage == S - 1 ? smem : st + L::SB;
+        const bool center = (unsigned)k < (unsigned)depth;
+        const bool upd = k >= kLag;
         const f2 *H = reinterpret_cast<const f2 *>(st) + hc;
         const f2 c = H[0];
         f2 xa[4], xb[4], ya[4], yb[4];
@@ -341,7 +354,8 @@ __global__ void __launch_bounds__(kTileX *(TY + kHelperWarps), MINB)
         Dx[j] = d1x;
         Dy[j] = d1y;
         f2 d2x, d2y;
-        f2 *dr = rows + (L::NB < S ? rb : stage) * (TY * G::HX) + ly * G::HX + lx + kRadius;
+        f2 *dr = reinterpret_cast<f2 *>(L::ROWS_IN ? st + L::OFF_SROWS : smem + L::OFF_ROWS + rb * G::ROW_B) +
+                 (ly * G::HX + lx + kRadius);
         if (center) {
           d2x = scale<ISO>(d2(c, xa[0], xb[0], xa[1], xb[1], xa[2], xb[2], xa[3], xb[3]), sxx);
           d2y = scale<ISO>(d2(c, ya[0], yb[0], ya[1], yb[1], ya[2], yb[2], ya[3], yb[3]), syy);
@@ -382,7 +396,9 @@ __global__ void __launch_bounds__(kTileX *(TY + kHelperWarps), MINB)
             v2sz = cu[5 * G::TX];
             v2pn = cu[6 * G::TX];
           }
-          const float4 ab = ABs[(abw == kLag ? 0 : abw + 1) * G::NT + ci];
+          // (With five slots the plane kLag back is the next one round.)
+          const float4 ab = reinterpret_cast<const float4 *>(
+              L::AB_IN ? st_next + L::OFF_SAB : smem + L::OFF_AB + (abw == kLag ? 0 : abw + 1) * L::AB_SLOT)[ci];
           const f2 Ak = mk2(ab.x, ab.y), Bk = mk2(ab.z, ab.w);
           const f2 h1 = fma2(splat(cyz), dyz, fma2(splat(cxz), dxz, fma2(splat(czz), d2z, Ak)));
           const f2 h2 = sub2(add2(Bk, d2z), h1);
@@ -399,10 +415,6 @@ __global__ void __launch_bounds__(kTileX *(TY + kHelperWarps), MINB)
           out += plane;
         }
         if (center) {
-          if (!wait(&halo[stage], phase)) {
-            if (lx == 0) atomicOr(P.err, 2u);
-            return;
-          }
           const f2 dxy = scale<ISO>(d1(dr[1], dr[-1], dr[2], dr[-2], dr[3], dr[-3], dr[4], dr[-4]), sxy);
           float cxx, cyy, cxy;
           if constexpr (MT) {
@@ -418,13 +430,15 @@ __global__ void __launch_bounds__(kTileX *(TY + kHelperWarps), MINB)
           }
           const f2 av = fma2(splat(cxy), dxy, fma2(splat(cyy), d2y, mul2(splat(cxx), d2x)));
           const f2 bv = add2(d2x, d2y);
-          ABs[abw * G::NT + ci] = make_float4(lo(av), hi(av), lo(bv), hi(bv));
+          reinterpret_cast<float4 *>(L::AB_IN ? st + L::OFF_SAB : smem + L::OFF_AB + abw * L::AB_SLOT)[ci] =
+              make_float4(lo(av), hi(av), lo(bv), hi(bv));
         }
         // This warp is done with the stage.
         __syncwarp();
-        if (lx == 0) mbar_arrive(&empty[stage]);
-        abw = abw == kLag ? 0 : abw + 1;
-        if (L::NB < S && ++rb == L::NB) rb = 0;
+        if (lx == 0) mbar_arrive(bar(st, L::OFF_EMPTY));
+        if (!L::AB_IN) abw = abw == kLag ? 0 : abw + 1;
+        if (!L::ROWS_IN && ++rb == L::NB) rb = 0;
+        st = st_next;
         if (++stage == S) {
           stage = 0;
           phase ^= 1u;

@@ -23,10 +23,13 @@
 //
 // What bounds it: FP16 the shared-memory pipe (80% busy) and issue (68%),
 // with the FP32 stencil's reads plus the decode; FP16X issue (its decode and
-// encode).  272^3 updated cells: FP16 244 us a step, FP16X 298, against 337
+// encode).  272^3 updated cells: FP16 232 us a step, FP16X 290, against 337
 // and 377 us when all 16 warps decoded each plane between two CTA-wide
 // barriers.  The residual bytes take no conversion instruction (decode,
-// encode): 310 -> 298 us.
+// encode): 12 of 310 us.  Four decoded tiles instead of three: FP16 244 ->
+// 232 us.  Not kept: one barrier for tile and halo columns (FP16 239, FP16X
+// 315 us: the compute warps start later), and the halo columns on the
+// producer's warp (323 and 372 us: they then wait for the slowest warp).
 #include <cuda_fp16.h>
 
 #include "device_util.cuh"
@@ -65,34 +68,49 @@ struct GeoH {
 
 constexpr int kHelperWarps = 4;  // producer warp + 3 decode warps: one warpgroup (setmaxnreg works on warpgroups)
 constexpr int kDecodeWarps = kHelperWarps - 1;
-constexpr int kDecoded = 3;      // decoded tiles and exchange buffers: the decode warps run at most that far ahead
 
-// Shared memory of a CTA.
+// Shared memory of a CTA: S stages (TMA tiles, the in-plane terms A, B of the
+// stage's plane when five stages match their five slots, and a control
+// block), then the decoded tiles with their exchange rows.
 template <int TY, int S, bool EXT>
 struct LayoutH {
   using G = GeoH<TY, EXT>;
-  static constexpr int OFF_H32 = S * G::STAGE_B;
-  static constexpr int OFF_ROWS = OFF_H32 + kDecoded * G::H32_B;
-  static constexpr int OFF_AB = OFF_ROWS + kDecoded * G::ROW_B;
-  static constexpr int OFF_HDR = OFF_AB + G::AB_B;    // the item that starts in stage s
-  static constexpr int OFF_SCALE = OFF_HDR + S * 16;  // 2^-e of the previous and 2^e of the new plane of the step
-  static constexpr int OFF_PLANE = OFF_SCALE + S * 8;  // the new plane (-1: none) and its shot (producer only)
-  static constexpr int OFF_BAR = OFF_PLANE + S * 8;   // full[S], decoded[S], halo[S], empty[S]
-  static constexpr int OFF_MAX = OFF_BAR + 4 * S * 8;  // the CTA's largest magnitude on the new plane
-  static constexpr size_t BYTES = size_t(OFF_MAX) + 4 * S + 128;
-  static_assert(G::STAGE_B % 128 == 0 && OFF_H32 % 16 == 0 && OFF_ROWS % 16 == 0 && OFF_AB % 16 == 0 &&
-                    OFF_HDR % 16 == 0 && OFF_SCALE % 8 == 0 && OFF_PLANE % 8 == 0 && OFF_BAR % 8 == 0 &&
-                    OFF_MAX % 4 == 0,
-                "shared-memory alignment");
+  static constexpr bool AB_IN = S == 5;
+  static constexpr int AB_SLOT = G::NT * 16;
+  static constexpr int OFF_SAB = G::STAGE_B;
+  static constexpr int OFF_CTL = OFF_SAB + (AB_IN ? AB_SLOT : 0);
+  static constexpr int OFF_HDR = OFF_CTL;         // the item that starts in the stage
+  static constexpr int OFF_SCALE = OFF_CTL + 16;  // 2^-e of the previous and 2^e of the new plane of the step
+  static constexpr int OFF_FULL = OFF_CTL + 24;   // barriers: loads landed,
+  static constexpr int OFF_READY = OFF_CTL + 32;  //   FP32 tile and scales written,
+  static constexpr int OFF_HALO = OFF_CTL + 40;   //   halo columns written,
+  static constexpr int OFF_EMPTY = OFF_CTL + 48;  //   released by every reader
+  static constexpr int OFF_PLANE = OFF_CTL + 56;  // the new plane (-1: none) and its shot (producer only)
+  static constexpr int OFF_MAX = OFF_CTL + 64;    // the CTA's largest magnitude on the new plane
+  static constexpr int SB = OFF_CTL + 128;
+  static constexpr int TILE_B = G::H32_B + G::ROW_B;  // decoded tile, exchange rows
+  static constexpr int OFF_TILES = S * SB;
+  // Decoded tiles: the decode warps run at most that far ahead.
+  static constexpr int REST = S * SB + (AB_IN ? 0 : 5 * AB_SLOT) + 128;
+  static constexpr int ND = REST + 4 * TILE_B <= 227 * 1024 ? 4 : 3;
+  static constexpr int OFF_AB = OFF_TILES + ND * TILE_B;
+  static constexpr size_t BYTES = size_t(REST) + ND * TILE_B;
   static_assert(BYTES <= 227 * 1024, "tile shape exceeds the shared memory of a CTA");
+  static_assert(OFF_CTL % 128 == 0 && OFF_TILES % 128 == 0 && TILE_B % 128 == 0 && G::H32_B % 16 == 0 &&
+                    OFF_AB % 128 == 0,
+                "shared-memory alignment");
 };
 
 // Register split (setmaxnreg), as in propagate_fp32.cu: TY/4 compute warps
 // and one helper warp per SM sub-partition share what the launch gives them.
-template <int TY>
+// FP16X at 16 rows: its decode needs the registers to keep several cells in
+// flight (272^3 updated cells: 311 us a step with 32 for the decode warps, 290
+// with 64, although the compute warps then spill 60 bytes); FP16 does not
+// (232 us with 32, 246 with 64).
+template <int TY, bool EXT>
 struct RegsH {
-  static constexpr int kCompute = TY == 16 ? 112 : TY == 12 ? 152 : 216;
-  static constexpr int kHelper = TY == 16 ? 32 : TY == 12 ? 56 : 72;
+  static constexpr int kCompute = TY == 16 ? (EXT ? 104 : 112) : TY == 12 ? 152 : 216;
+  static constexpr int kHelper = TY == 16 ? (EXT ? 64 : 32) : TY == 12 ? 56 : 72;
   static constexpr int kLaunch = TY == 16 ? 96 : TY == 12 ? 128 : 168;
   static_assert((TY / 4) * kCompute + kHelper <= (TY / 4 + 1) * kLaunch, "the split exceeds the launch's registers");
 };
@@ -209,17 +227,10 @@ __global__ void __launch_bounds__(kTileX *(TY + kHelperWarps), 1)
   const PropParams &P = H.p;
   extern __shared__ unsigned char smem_dyn[];
   unsigned char *smem = smem_dyn + ((128u - (smem_addr(smem_dyn) & 127u)) & 127u);
-  f2 *H32 = reinterpret_cast<f2 *>(smem + L::OFF_H32);         // [kDecoded][HY][HX]
-  f2 *rows = reinterpret_cast<f2 *>(smem + L::OFF_ROWS);       // [kDecoded][TY][HX]
-  float4 *ABs = reinterpret_cast<float4 *>(smem + L::OFF_AB);  // [5][NT]
-  int4 *hdr = reinterpret_cast<int4 *>(smem + L::OFF_HDR);
-  float2 *scl = reinterpret_cast<float2 *>(smem + L::OFF_SCALE);
-  unsigned *smax = reinterpret_cast<unsigned *>(smem + L::OFF_MAX);
-  int2 *plane_of = reinterpret_cast<int2 *>(smem + L::OFF_PLANE);
-  uint64_t *full = reinterpret_cast<uint64_t *>(smem + L::OFF_BAR);
-  uint64_t *decoded = full + S;   // FP32 tile of the stage's plane written (and the step's scales)
-  uint64_t *halo = decoded + S;   // halo columns of D1y written
-  uint64_t *empty = halo + S;     // stage (and decoded tile) released by every reader
+  auto bar = [&](unsigned char *st, int off) { return reinterpret_cast<uint64_t *>(st + off); };
+  auto scale_of = [&](unsigned char *st) { return reinterpret_cast<float2 *>(st + L::OFF_SCALE); };
+  auto max_of = [&](unsigned char *st) { return reinterpret_cast<unsigned *>(st + L::OFF_MAX); };
+  auto plane_of = [&](unsigned char *st) { return reinterpret_cast<int2 *>(st + L::OFF_PLANE); };
 
   const int tid = threadIdx.x;
   const int lx = tid & 31;
@@ -228,11 +239,12 @@ __global__ void __launch_bounds__(kTileX *(TY + kHelperWarps), 1)
   if (nitems <= 0) return;
   if (tid == 0) {
     for (int s = 0; s < S; ++s) {
-      mbar_init(&full[s], 1);
-      mbar_init(&decoded[s], kDecodeWarps);
-      mbar_init(&halo[s], kDecodeWarps);
-      mbar_init(&empty[s], TY + kDecodeWarps);
-      smax[s] = 0u;
+      unsigned char *st = smem + s * L::SB;
+      mbar_init(bar(st, L::OFF_FULL), 1);
+      mbar_init(bar(st, L::OFF_READY), kDecodeWarps);
+      mbar_init(bar(st, L::OFF_HALO), kDecodeWarps);
+      mbar_init(bar(st, L::OFF_EMPTY), TY + kDecodeWarps);
+      *max_of(st) = 0u;
     }
     mbar_fence_init();
   }
@@ -241,7 +253,7 @@ __global__ void __launch_bounds__(kTileX *(TY + kHelperWarps), 1)
   wait_previous_launch();
 
   if (wid >= TY) {
-    setmaxnreg_dec<RegsH<TY>::kHelper>();
+    setmaxnreg_dec<RegsH<TY, EXT>::kHelper>();
     const int4 *seg = P.seg + first;
     int stage = 0;
     uint32_t phase = 0;
@@ -256,9 +268,9 @@ __global__ void __launch_bounds__(kTileX *(TY + kHelperWarps), 1)
       bool ok = true;
       // The CTA's maximum on the plane whose step held stage s (every warp
       // has released it) goes to the plane's global maximum.
-      auto take_max = [&](int s) {
-        const unsigned v = smax[s];
-        smax[s] = 0u;
+      auto take_max = [&](unsigned char *st) {
+        const unsigned v = *max_of(st);
+        *max_of(st) = 0u;
         return v;
       };
       auto fold_max = [&](int2 pl, float sc, unsigned v) {
@@ -281,17 +293,18 @@ __global__ void __launch_bounds__(kTileX *(TY + kHelperWarps), 1)
         }
         for (int k = it.z0 - kRadius; k < it.z1 + kRadius; ++k) {
           // (The first S waits pass at once: the stage was never filled.)
-          if (!mbar_spin(&empty[stage], phase ^ 1u)) {
+          unsigned char *st = smem + stage * L::SB;
+          if (!mbar_spin(bar(st, L::OFF_EMPTY), phase ^ 1u)) {
             ok = false;
             break;
           }
-          const int2 pl = issued >= S ? plane_of[stage] : make_int2(-1, 0);
-          const float sc = scl[stage].y;
-          const unsigned v = take_max(stage);
+          const int2 pl = issued >= S ? *plane_of(st) : make_int2(-1, 0);
+          const float sc = scale_of(st)->y;
+          const unsigned v = take_max(st);
           fence_proxy_async_smem();
-          if (k == it.z0 - kRadius) hdr[stage] = w;
-          plane_of[stage] = make_int2(k - kRadius >= it.z0 ? k - kRadius : -1, it.shot);
-          issue_half<TY, EXT>(smem + stage * G::STAGE_B, &full[stage], it, k, maps_of(it.shot));
+          if (k == it.z0 - kRadius) *reinterpret_cast<int4 *>(st + L::OFF_HDR) = w;
+          *plane_of(st) = make_int2(k - kRadius >= it.z0 ? k - kRadius : -1, it.shot);
+          issue_half<TY, EXT>(st, bar(st, L::OFF_FULL), it, k, maps_of(it.shot));
           ++issued;
           if (++stage == S) {
             stage = 0;
@@ -303,8 +316,9 @@ __global__ void __launch_bounds__(kTileX *(TY + kHelperWarps), 1)
       // The maxima of the last steps, in order.
       for (int a = issued < S ? issued : S; a >= 1 && ok; --a) {
         const int s2 = stage >= a ? stage - a : stage + S - a;
-        if (!mbar_spin(&empty[s2], stage >= a ? phase : phase ^ 1u)) ok = false;
-        else fold_max(plane_of[s2], scl[s2].y, take_max(s2));
+        unsigned char *st = smem + s2 * L::SB;
+        if (!mbar_spin(bar(st, L::OFF_EMPTY), stage >= a ? phase : phase ^ 1u)) ok = false;
+        else fold_max(*plane_of(st), scale_of(st)->y, take_max(st));
       }
       if (!ok) {
         // A bounded wait gave up: wait, bounded, for the loads still in
@@ -313,7 +327,7 @@ __global__ void __launch_bounds__(kTileX *(TY + kHelperWarps), 1)
         atomicOr(P.err, 2u);
         for (int a = 1; a <= S && a <= issued; ++a) {
           const int s2 = stage >= a ? stage - a : stage + S - a;
-          (void)mbar_wait(&full[s2], stage >= a ? phase : phase ^ 1u, kDrainNs);
+          (void)mbar_wait(bar(smem + s2 * L::SB, L::OFF_FULL), stage >= a ? phase : phase ^ 1u, kDrainNs);
         }
       }
       return;
@@ -351,14 +365,16 @@ __global__ void __launch_bounds__(kTileX *(TY + kHelperWarps), 1)
             en = e_new[k + 1 - kRadius];
           }
         }
-        // The decoded tile's last readers: the step kDecoded back.
-        const int es = stage >= kDecoded ? stage - kDecoded : stage + S - kDecoded;
-        if (!mbar_spin(&empty[es], stage >= kDecoded ? phase : phase ^ 1u) || !mbar_spin(&full[stage], phase)) {
+        // The decoded tile's last readers: the step L::ND back.
+        // (With ND = S that is the step whose stage was refilled.)
+        const int es = stage >= L::ND ? stage - L::ND : stage + S - L::ND;
+        unsigned char *st = smem + stage * L::SB;
+        if ((L::ND < S && !mbar_spin(bar(smem + es * L::SB, L::OFF_EMPTY), stage >= L::ND ? phase : phase ^ 1u)) ||
+            !mbar_spin(bar(st, L::OFF_FULL), phase)) {
           atomicOr(P.err, 1u);
           return;
         }
-        const unsigned char *st = smem + stage * G::STAGE_B;
-        f2 *Hs = H32 + ds * G::HXY;
+        f2 *Hs = reinterpret_cast<f2 *>(smem + L::OFF_TILES + ds * L::TILE_B);
         // Decode once per cell, two cells per thread (one 64-bit load of two
         // half2 cells, one 128-bit store of their FP32 pairs).  The source
         // cell then gains the step's source
@@ -385,14 +401,14 @@ __global__ void __launch_bounds__(kTileX *(TY + kHelperWarps), 1)
             if (dt == (src_c >> 1) % NDT) Hs[src_c] = add2(Hs[src_c], splat(P.src));
           }
         }
-        if (dt == 0) scl[stage] = ps;
+        if (dt == 0) *scale_of(st) = ps;
         __syncwarp();
-        if (lx == 0) mbar_arrive(&decoded[stage]);
+        if (lx == 0) mbar_arrive(bar(st, L::OFF_READY));
         if (k >= it.z0 && k < it.z1) {
           // D1y in the halo columns, from rows that the other decode warps
           // wrote too.
           asm volatile("bar.sync 1, %0;" ::"n"(NDT) : "memory");
-          f2 *db = rows + ds * (TY * G::HX);
+          f2 *db = Hs + G::HXY;
           for (int r = hw * 4 + (lx >> 3); r < TY; r += 4 * kDecodeWarps) {
             const f2 *h = Hs + (r + kRadius) * G::HX + hxc;
             f2 d = mul2(splat(cL1), sub2(h[G::HX], h[-G::HX]));
@@ -404,10 +420,10 @@ __global__ void __launch_bounds__(kTileX *(TY + kHelperWarps), 1)
         }
         __syncwarp();
         if (lx == 0) {
-          mbar_arrive(&halo[stage]);
-          mbar_arrive(&empty[stage]);
+          mbar_arrive(bar(st, L::OFF_HALO));
+          mbar_arrive(bar(st, L::OFF_EMPTY));
         }
-        if (++ds == kDecoded) ds = 0;
+        if (++ds == L::ND) ds = 0;
         if (++stage == S) {
           stage = 0;
           phase ^= 1u;
@@ -418,7 +434,7 @@ __global__ void __launch_bounds__(kTileX *(TY + kHelperWarps), 1)
   }
 
   // ---- compute warps ----
-  setmaxnreg_inc<RegsH<TY>::kCompute>();
+  setmaxnreg_inc<RegsH<TY, EXT>::kCompute>();
   const int ly = wid;
   const float sxy = P.inv_dxy, sxz = P.inv_dxz, syz = P.inv_dyz;
   const float sxx = P.inv_dxx, syy = P.inv_dyy, szz = P.inv_dzz;
@@ -428,14 +444,15 @@ __global__ void __launch_bounds__(kTileX *(TY + kHelperWarps), 1)
   uint32_t phase = 0;
   int ds = 0;   // decoded tile
   int abw = 0;  // shared A/B ring slot of the arriving plane (the plane 4 back is at abw + 1)
+  unsigned char *st = smem;
   for (int item = 0; item < nitems; ++item) {
-    if (!mbar_spin(&full[stage], phase)) {
+    if (!mbar_spin(bar(st, L::OFF_READY), phase)) {
       if (lx == 0) atomicOr(P.err, 1u);
       return;
     }
-    const HItem it = decode_hitem<BATCH>(uniform4(hdr[stage]));
+    const HItem it = decode_hitem<BATCH>(uniform4(*reinterpret_cast<const int4 *>(st + L::OFF_HDR)));
     const ShotDesc &sd = BATCH ? P.shots[it.shot] : P.one;
-    const int kend = it.z1 + kRadius;
+    const int depth = it.z1 - it.z0;
     const int gx = it.x0 + lx;
     const int gy = it.y0 + ly;
     const bool valid = (gx >= sd.bord) && (gx < sd.sx - sd.bord) && (gy >= sd.bord) && (gy < sd.sy - sd.bord);
@@ -444,23 +461,24 @@ __global__ void __launch_bounds__(kTileX *(TY + kHelperWarps), 1)
     unsigned *const out_hi = BATCH ? H.hshots[it.shot].hi[1 - P.parity] : H.out_hi;
     unsigned short *const out_lo = BATCH ? H.hshots[it.shot].lo[1 - P.parity] : H.out_lo;
     // The cell that lacks the last step's source, if it is this thread's.
-    const int cor_k = (gx == sd.cor_x && gy == sd.cor_y) ? sd.cor_z + kRadius : -1000;
+    const int cor_k = (gx == sd.cor_x && gy == sd.cor_y) ? sd.cor_z + kRadius - it.z0 : -1000;
 
     f2 Pr[9], Dx[9], Dy[9];
 
-    for (int kb = it.z0 - kRadius; kb < kend; kb += 9) {
+    for (int kb = -kRadius; kb < depth + kRadius; kb += 9) {
 #pragma unroll
       for (int j = 0; j < 9; ++j) {
-        const int k = kb + j;
-        if (k >= kend) break;
-        const unsigned char *st = smem + stage * G::STAGE_B;
-        if (!mbar_spin(&full[stage], phase) || !mbar_spin(&decoded[stage], phase)) {
+        const int k = kb + j;  // plane, counted from the item's first
+        if (k >= depth + kRadius) break;
+        if (!mbar_spin(bar(st, L::OFF_READY), phase)) {
           if (lx == 0) atomicOr(P.err, 1u);
           return;
         }
-        const bool center = (k >= it.z0) && (k < it.z1);
-        const bool upd = (k - kRadius >= it.z0);
-        const f2 *Hs = H32 + ds * G::HXY + hc;
+        unsigned char *const st_next = stage == S - 1 ? smem : st + L::SB;
+        const bool center = (unsigned)k < (unsigned)depth;
+        const bool upd = k >= kRadius;
+        f2 *const tile = reinterpret_cast<f2 *>(smem + L::OFF_TILES + ds * L::TILE_B);
+        const f2 *Hs = tile + hc;
         const f2 c = Hs[0];
         f2 xa[4], xb[4], ya[4], yb[4];
 #pragma unroll
@@ -476,7 +494,7 @@ __global__ void __launch_bounds__(kTileX *(TY + kHelperWarps), 1)
         Dx[j] = d1x;
         Dy[j] = d1y;
         f2 d2x, d2y;
-        f2 *dr = rows + ds * (TY * G::HX) + ly * G::HX + lx + kRadius;
+        f2 *dr = tile + (G::HXY + ly * G::HX + lx + kRadius);
         if (center) {
           d2x = scale<ISO>(d2(c, xa[0], xb[0], xa[1], xb[1], xa[2], xb[2], xa[3], xb[3]), sxx);
           d2y = scale<ISO>(d2(c, ya[0], yb[0], ya[1], yb[1], ya[2], yb[2], ya[3], yb[3]), syy);
@@ -498,7 +516,9 @@ __global__ void __launch_bounds__(kTileX *(TY + kHelperWarps), 1)
           const float czz = cu[0], cxz = cu[G::TX], cyz = cu[2 * G::TX];
           const float v2px = cu[3 * G::TX], v2pz = cu[4 * G::TX];
           const float v2sz = cu[5 * G::TX], v2pn = cu[6 * G::TX];
-          const float4 ab = ABs[(abw == 4 ? 0 : abw + 1) * G::NT + ci];
+          // (With five slots the plane 4 back is the next one round.)
+          const float4 ab = reinterpret_cast<const float4 *>(
+              L::AB_IN ? st_next + L::OFF_SAB : smem + L::OFF_AB + (abw == 4 ? 0 : abw + 1) * L::AB_SLOT)[ci];
           const f2 Ak = mk2(ab.x, ab.y), Bk = mk2(ab.z, ab.w);
           const f2 h1 = fma2(splat(cyz), dyz, fma2(splat(cxz), dxz, fma2(splat(czz), d2z, Ak)));
           const f2 h2 = sub2(add2(Bk, d2z), h1);
@@ -509,7 +529,7 @@ __global__ void __launch_bounds__(kTileX *(TY + kHelperWarps), 1)
           const unsigned phv = reinterpret_cast<const unsigned *>(st + G::OFF_PHI)[ci];
           unsigned short prv = 0;
           if constexpr (EXT) prv = reinterpret_cast<const unsigned short *>(st + G::OFF_PLO)[ly * G::HX + lx + kRadius];
-          const float2 sc = scl[stage];  // 2^-e of the previous field, 2^e of the new one
+          const float2 sc = *scale_of(st);  // 2^-e of the previous field, 2^e of the new one
           f2 old = decode<EXT>(phv, prv, sc.x);
           if (k == cor_k) old = add2(old, splat(P.cor));
           const f2 curv = Pr[cs];
@@ -528,10 +548,10 @@ __global__ void __launch_bounds__(kTileX *(TY + kHelperWarps), 1)
           unsigned mb = 0u;
           if (valid) mb = max(__float_as_uint(fabsf(lo(nw))), __float_as_uint(fabsf(hi(nw))));
           mb = __reduce_max_sync(0xffffffffu, mb);
-          if (lx == 0 && mb) atomicMax(&smax[stage], mb);
+          if (lx == 0 && mb) atomicMax(max_of(st), mb);
         }
         if (center) {
-          if (!mbar_spin(&halo[stage], phase)) {
+          if (!mbar_spin(bar(st, L::OFF_HALO), phase)) {
             if (lx == 0) atomicOr(P.err, 2u);
             return;
           }
@@ -540,13 +560,15 @@ __global__ void __launch_bounds__(kTileX *(TY + kHelperWarps), 1)
           const float cxx = ca[0], cyy = ca[G::TX], cxy = ca[2 * G::TX];
           const f2 av = fma2(splat(cxy), dxy, fma2(splat(cyy), d2y, mul2(splat(cxx), d2x)));
           const f2 bv = add2(d2x, d2y);
-          ABs[abw * G::NT + ci] = make_float4(lo(av), hi(av), lo(bv), hi(bv));
+          reinterpret_cast<float4 *>(L::AB_IN ? st + L::OFF_SAB : smem + L::OFF_AB + abw * L::AB_SLOT)[ci] =
+              make_float4(lo(av), hi(av), lo(bv), hi(bv));
         }
         // This warp is done with the stage.
         __syncwarp();
-        if (lx == 0) mbar_arrive(&empty[stage]);
-        abw = abw == 4 ? 0 : abw + 1;
-        if (++ds == kDecoded) ds = 0;
+        if (lx == 0) mbar_arrive(bar(st, L::OFF_EMPTY));
+        if (!L::AB_IN) abw = abw == 4 ? 0 : abw + 1;
+        if (++ds == L::ND) ds = 0;
+        st = st_next;
         if (++stage == S) {
           stage = 0;
           phase ^= 1u;
