@@ -20,6 +20,7 @@
 // previous, next) and per-plane maxima Mx (one per buffer).
 #include <cuda.h>
 #include <cuda_runtime.h>
+#include <math.h>
 #include <stdarg.h>
 #include <stdio.h>
 #include <stdlib.h>
@@ -62,6 +63,7 @@ struct State {
   int4 *seg = nullptr;       // the plan as work segments {x0, y0, z0, z1}
   int *cta_first = nullptr;  // [seg_grid + 1]: first segment of each CTA
   int nseg = 0, grid = 0;
+  bool skip_rows = false;
   long launches = 0;
   size_t dev_bytes = 0;
   int num_sms = 0;
@@ -427,98 +429,185 @@ int grid_for(size_t n) {
   return (int)(b < cap ? (b ? b : 1) : cap);
 }
 
-// Chooses the number of z-chunks: balances the persistent CTAs' last round
-// against the 8 warm-up planes each chunk re-reads.
-// Work split of one shot among `ctas` persistent CTAs, as segments {x0, y0,
-// z0, z1} (a z range of one tile column) listed CTA by CTA.  The tiles
-// (x fastest) are cut into z-chunks; the chunk-major items fill whole rounds
-// of `ctas` (CTA b takes items b, b + ctas, ...: CTAs side by side work on
-// neighbouring tiles at the same depth and share their halo rows through
-// L2).  With `spread`, each item of the last, partial round is then cut into
-// equal z pieces of at least kMinPiece planes, as many as lets every CTA
-// take at most one piece; without it the partial round stays round-robin.
-// The plan (chunk count 1..16 or `req`, spread or not) minimises the busiest
-// CTA's cost: its planes plus kHaloCost a segment for the 8 halo planes,
-// shared-out pieces counting 3/2 (measured on GB300 at 280^3, 328^3 and
-// 576^3: the pieces of neighbouring tiles run at different depths and lose
-// their L2 halo sharing); a spread plan must beat the best round-robin one
-// by 3%.
-constexpr int kMinPiece = 8;
+// ---- work split ----------------------------------------------------------------
+//
+// A launch's work is a list of segments {x0, y0, z0, z1} (a z range of one
+// tile column), dealt to `ctas` persistent CTAs.  The step kernels take a
+// CTA's time to be its segments' planes, plus kHaloCost a segment for the 8
+// halo planes, at a fixed time a plane: over nine grids of 0.03 to 20 M cells
+// and 21 splits of each, FP32 took 2 us + 0.67 .. 0.74 us a unit of the
+// busiest CTA's cost, however the planes were dealt.  So the plan makes the
+// busiest CTA's cost small.  Costs count rows: a plane of a tile costs its
+// rows in the updated region (the compute warps of the others skip it), at
+// least kMinRowShare of a full tile's (8 of 16 rows took 0.62 of a plane's
+// time with the GPU to themselves, 0.8 with all CTAs at work).
+//
+//  * Aligned rounds: the full tiles (x fastest) are cut into z-chunks; the
+//    chunk-major items fill whole rounds of `ctas` (CTA b takes items b,
+//    b + ctas, ...), so that CTAs side by side work on neighbouring tiles at
+//    the same depth and share their halo rows through L2.
+//  * The rest (the items of the last, partial round, and the tiles with fewer
+//    rows) is a pool of columns cut into contiguous pieces that fill every
+//    CTA up to the same cost.
+// The chunk count (1..16 or `req`), and what goes to the pool, are those of
+// the lowest cost.  Pool pieces run at other depths than their neighbours:
+// where the step streams from DRAM (`hbm`) that costs up to kPoolPenalty more
+// (everything pooled: 205 x 129 x 173 took 0.82 instead of 0.70 us a unit, 160
+// x 200 x 120 0.83); below kL2Bytes it costs nothing.
 constexpr int kHaloCost = 4;
+constexpr double kMinRowShare = 0.8;
+constexpr double kPoolPenalty = 0.25;
 
 struct Split {
   std::vector<int4> seg;
   std::vector<int> first;
-  long max_cost = 0, total_cost = 0;
+  long max_cost = 0;     // the busiest CTA's, in planes of a full tile
+  double est = 0.0;      // max_cost with the pool's penalty
+  bool apart = false;    // tiles with fewer rows counted as such
 };
 
-Split split_work(int ctas, int ntx, int nty, int TY, int zlo, int depth, int nchunk, bool spread = true) {
-  const int ntiles = ntx * nty;
-  const int len = (depth + nchunk - 1) / nchunk;
-  const int cc = (depth + len - 1) / len;
-  const long items = (long)ntiles * cc;
-  const long full = spread ? items / ctas * ctas : items;
-  auto tile_x0 = [&](long t) { return kRadius + (int)(t % ntx) * kTileX; };
-  auto tile_y0 = [&](long t) { return kRadius + (int)(t / ntx) * TY; };
-  auto item_z = [&](long i, int *z0, int *z1) {
-    const int ch = (int)(i / ntiles);
-    *z0 = ch * len;
-    *z1 = std::min(depth, *z0 + len);
-  };
-  std::vector<std::vector<int4>> per(ctas);
-  std::vector<long> cost(ctas, 0);
-  for (long i = 0; i < full; ++i) {
-    int z0, z1;
-    item_z(i, &z0, &z1);
-    const long t = i % ntiles;
-    per[i % ctas].push_back(make_int4(tile_x0(t), tile_y0(t), zlo + z0, zlo + z1));
-    cost[i % ctas] += 2 * ((z1 - z0) + kHaloCost);  // costs in half planes
-  }
-  // The partial round: each of its items cut into p equal z pieces (at
-  // least kMinPiece planes, p * items <= ctas), one piece per CTA.
-  const long rem = items - full;
-  if (rem > 0) {
-    const long p = std::max(1L, std::min((long)ctas / rem, (long)len / kMinPiece));
-    long b = 0;
-    for (long i = full; i < items; ++i) {
-      int z0, z1;
-      item_z(i, &z0, &z1);
-      const long t = i % ntiles, n = z1 - z0;
-      for (long j = 0; j < p; ++j, ++b) {
-        const int a0 = z0 + (int)(n * j / p), a1 = z0 + (int)(n * (j + 1) / p);
-        if (a1 <= a0) continue;
-        per[b % ctas].push_back(make_int4(tile_x0(t), tile_y0(t), zlo + a0, zlo + a1));
-        cost[b % ctas] += 3 * ((a1 - a0) + kHaloCost);
+// A tile column (or z range of one) to be dealt.  Batched launches: x0 is the
+// tile's x index, `tag` the shot (the segments' upper bits).
+struct Column {
+  int x0, y0, z0, z1, rows, tag;
+};
+
+int row_cost(int rows, int TY) { return std::max(rows, (int)ceil(kMinRowShare * TY)); }
+
+// Deals the columns of `pool` in order to the CTAs, CTA b up to cost `cap`
+// less base[b] (in row planes); returns whether all of it fits, and with
+// `out` appends each CTA's segments.
+bool deal_pool(const std::vector<Column> &pool, int TY, const std::vector<long> &base, long cap,
+               std::vector<std::vector<int4>> *out, std::vector<long> *cost) {
+  size_t c = 0;
+  int z = pool.empty() ? 0 : pool[0].z0;
+  for (size_t b = 0; b < base.size() && c < pool.size(); ++b) {
+    long room = cap - base[b];
+    while (c < pool.size()) {
+      const Column &k = pool[c];
+      const int w = row_cost(k.rows, TY);
+      const long n = std::min<long>(k.z1 - z, room / w - kHaloCost);
+      if (n < 1) break;
+      if (out) {
+        (*out)[b].push_back(make_int4(k.x0 | (k.tag << 16), k.y0, z, z + (int)n));
+        (*cost)[b] += w * (n + kHaloCost);
       }
+      room -= w * (n + kHaloCost);
+      z += (int)n;
+      if (z == k.z1 && ++c < pool.size()) z = pool[c].z0;
     }
   }
+  return c == pool.size();
+}
+
+// The smallest cap that deals the pool.
+long pool_cap(const std::vector<Column> &pool, int TY, const std::vector<long> &base) {
+  long lo = 0, hi = 0, work = 0;
+  for (long v : base) hi = std::max(hi, v);
+  lo = hi;
+  for (const Column &k : pool) work += (long)row_cost(k.rows, TY) * (k.z1 - k.z0 + kHaloCost);
+  if (pool.empty()) return lo;
+  hi += work;
+  while (lo < hi) {
+    const long mid = (lo + hi) / 2;
+    if (deal_pool(pool, TY, base, mid, nullptr, nullptr)) hi = mid;
+    else lo = mid + 1;
+  }
+  return lo;
+}
+
+// The plan with `nchunk` chunks; `pooled`: the partial round goes to the pool
+// (otherwise it stays round-robin).  Without `build` only its cost.
+Split split_work(int ctas, int ntx, int nty, int TY, int last_rows, int zlo, int depth, int nchunk, bool pooled,
+                 bool apart, bool hbm, bool build) {
+  const int len = (depth + nchunk - 1) / nchunk;
+  const int cc = (depth + len - 1) / len;
+  // Tiles in rounds: those of the whole rows, or all of them.
+  const bool last = pooled && apart && last_rows < TY;
+  const int ntiles = ntx * (last ? nty - 1 : nty);
+  const long items = (long)ntiles * cc;
+  const long full = pooled ? items / ctas * ctas : items;
+  auto column = [&](long i) {
+    const int ch = (int)(i / ntiles), t = (int)(i % ntiles);
+    return Column{kRadius + t % ntx * kTileX, kRadius + t / ntx * TY, zlo + ch * len,
+                  zlo + std::min(depth, (ch + 1) * len), TY, 0};
+  };
+  std::vector<long> cost(ctas, 0);
+  std::vector<std::vector<int4>> per(build ? ctas : 0);
+  for (long i = 0; i < full; ++i) {
+    const int ch = (int)(i / ntiles);
+    cost[i % ctas] += (long)TY * (std::min(depth - ch * len, len) + kHaloCost);
+    if (build) {
+      const Column k = column(i);
+      per[i % ctas].push_back(make_int4(k.x0, k.y0, k.z0, k.z1));
+    }
+  }
+  std::vector<Column> pool;
+  for (long i = full; i < items; ++i) {
+    // Chunks of one column that follow each other in the pool join up.
+    pool.push_back(column(i));
+  }
+  if (full == 0 && ntiles > 0) {
+    pool.clear();
+    for (long t = 0; t < ntiles; ++t) {
+      pool.push_back(column(t));
+      pool.back().z1 = zlo + depth;
+    }
+  }
+  if (last)
+    for (int t = 0; t < ntx; ++t)
+      pool.push_back(Column{kRadius + t * kTileX, kRadius + (nty - 1) * TY, zlo, zlo + depth, last_rows, 0});
+  const long cap = pool_cap(pool, TY, cost);
   Split sp;
+  sp.max_cost = (cap + TY - 1) / TY;
+  sp.est = (double)cap / TY;
+  sp.apart = last;
+  if (hbm) {
+    const double planes = (double)ntx * ((nty - 1) + (double)last_rows / TY) * depth;
+    const double in_rounds = std::min(planes, (double)full / std::max(1L, items) * ntiles * depth);
+    if (planes * kTileX * TY * 64.0 > kL2Bytes) sp.est *= 1.0 + kPoolPenalty * (1.0 - in_rounds / planes);
+  }
+  if (!build) return sp;
+  deal_pool(pool, TY, std::vector<long>(cost), cap, &per, &cost);
   sp.first.push_back(0);
   for (int b = 0; b < ctas; ++b) {
     sp.seg.insert(sp.seg.end(), per[b].begin(), per[b].end());
     sp.first.push_back((int)sp.seg.size());
-    sp.max_cost = std::max(sp.max_cost, cost[b] / 2);
-    sp.total_cost += cost[b] / 2;
   }
   return sp;
 }
 
-Split plan_segments(int ctas, int ntx, int nty, int TY, int zlo, int depth, int req) {
-  if (req > 0) return split_work(ctas, ntx, nty, TY, zlo, depth, std::min(req, depth));
-  if (req < 0) return split_work(ctas, ntx, nty, TY, zlo, depth, std::min(-req, depth), false);
-  Split best[2];  // round-robin, spread
+// req > 0: that many chunks, the partial round dealt from the pool; req < 0:
+// -req chunks, all round-robin.  last_rows: rows of the last tile row in the
+// updated region.
+Split plan_segments(int ctas, int ntx, int nty, int TY, int last_rows, int zlo, int depth, int req, bool hbm) {
+  if (req)
+    return split_work(ctas, ntx, nty, TY, last_rows, zlo, depth, std::min(std::abs(req), depth), req > 0, false, hbm,
+                      true);
+  int best = 1, best_mode = 0;
+  double est = 0.0;
   for (int c = 1; c <= 16 && c <= depth; ++c)
-    for (int spread = 0; spread < 2; ++spread) {
-      Split sp = split_work(ctas, ntx, nty, TY, zlo, depth, c, spread != 0);
-      Split &b = best[spread];
-      if (b.first.empty() || sp.max_cost < b.max_cost || (sp.max_cost == b.max_cost && sp.total_cost < b.total_cost))
-        b = std::move(sp);
+    for (int mode = 0; mode < (last_rows < TY ? 3 : 2); ++mode) {
+      const Split sp = split_work(ctas, ntx, nty, TY, last_rows, zlo, depth, c, mode > 0, mode > 1, hbm, false);
+      if (est == 0.0 || sp.est < est) {
+        est = sp.est;
+        best = c;
+        best_mode = mode;
+      }
     }
-  // Round-robin keeps neighbouring tiles in step for L2 and measured faster
-  // at 504^3 than a spread plan the model rates 1% cheaper: spread only when
-  // it saves more than 3%.
-  return best[1].max_cost * 100 < best[0].max_cost * 97 ? best[1] : best[0];
+  return split_work(ctas, ntx, nty, TY, last_rows, zlo, depth, best, best_mode > 0, best_mode > 1, hbm, true);
 }
+
+// Whether a step streams from DRAM about as fast as its CTAs work: FP32 with
+// coefficient planes (0.70 us a plane and CTA, 0.73 us of bytes); the media
+// table and the 16-bit forms read fewer bytes, the Der1-Der1 numerics work
+// longer.
+bool plan_hbm(int form, int numerics, bool media) {
+  return form == FLETCHER_FORM_FP32 && numerics == FLETCHER_NUMERICS_FAST && !media;
+}
+
+// Rows of the last of `nty` tile rows that lie in the updated region.
+int last_tile_rows(int sy, int bord, int nty, int TY) { return sy - bord - kRadius - (nty - 1) * TY; }
 
 int check_dims(int sx, int sy, int sz) {
   if (!g.init) return fail(FLETCHER_ERR_ARGS, "DRIVER_Initialize has not been called");
@@ -689,7 +778,8 @@ int setup_tiles(int rows, int stages) {
   g.ntx = (sx - bord - kRadius + kTileX - 1) / kTileX;
   g.nty = (sy - bord - kRadius + TY - 1) / TY;
   const int ctas = g.num_sms * (half_form() ? 1 : propagate_fp32_ctas_per_sm(TY));
-  const Split sp = plan_segments(ctas, g.ntx, g.nty, TY, bord, sz - 2 * bord, g.zchunks);
+  const Split sp = plan_segments(ctas, g.ntx, g.nty, TY, last_tile_rows(sy, bord, g.nty, TY), bord, sz - 2 * bord,
+                                 g.zchunks, plan_hbm(g.form, g.numerics, g.media));
   if (g.seg) cudaFree(g.seg);
   if (g.cta_first) cudaFree(g.cta_first);
   g.seg = nullptr;
@@ -703,6 +793,7 @@ int setup_tiles(int rows, int stages) {
   while (grid > 1 && sp.first[grid - 1] == sp.first[grid]) --grid;
   g.grid = grid;
   g.nseg = (int)sp.seg.size();
+  g.skip_rows = sp.apart;
   memset(&g.desc, 0, sizeof(g.desc));
   g.desc.F[0] = g.F[0];
   g.desc.F[1] = g.F[1];
@@ -997,6 +1088,7 @@ int step() {
   P.maps = nullptr;
   P.seg = g.seg;
   P.cta_first = g.cta_first;
+  P.skip_rows = g.skip_rows;
   P.parity = c;
   P.inv_dx = 1.0f / g.dx;
   P.inv_dy = 1.0f / g.dy;
@@ -1316,7 +1408,7 @@ extern "C" int FLETCHER_PlanSegments(int ctas, int ntx, int nty, int tile_rows, 
                                      int *seg_out, int cap, int *first_out, long *max_cost) {
   if (ctas < 1 || ntx < 1 || nty < 1 || tile_rows < 1 || depth < 1 || cap < 0 || !first_out)
     return -fail(FLETCHER_ERR_ARGS, "FLETCHER_PlanSegments: bad arguments");
-  const Split sp = plan_segments(ctas, ntx, nty, tile_rows, zlo, depth, zchunks);
+  const Split sp = plan_segments(ctas, ntx, nty, tile_rows, tile_rows, zlo, depth, zchunks, true);
   const int n = (int)sp.seg.size();
   if (seg_out && n <= cap) memcpy(seg_out, sp.seg.data(), sizeof(int4) * n);
   memcpy(first_out, sp.first.data(), sizeof(int) * (ctas + 1));
@@ -1517,9 +1609,9 @@ struct Batch {
   int sealed_rows = 0;
   ShotDesc *d_desc = nullptr;
   ShotMaps *d_maps = nullptr;
-  // For r running shots (the first r of `order`), their single-shot plans
-  // stacked per CTA at d_plan + plan_off[r-1] ({tile x index + (shot << 16),
-  // y0, z0, z1}), each CTA's first segment at d_first + (r-1) * (plan_ctas + 1).
+  // The plan for r running shots (the first r of `order`) at d_plan +
+  // plan_off[r-1] ({tile x index + (shot << 16), y0, z0, z1}), each CTA's first
+  // segment at d_first + (r-1) * (plan_ctas + 1).
   int4 *d_plan = nullptr;
   int *d_first = nullptr;
   std::vector<long> plan_off;
@@ -1550,6 +1642,7 @@ struct Batch {
   std::vector<HalfShotMaps> h_hmaps;
   std::vector<ShotDesc> s_desc;
   std::vector<int> s_grid;
+  std::vector<char> s_skip;
   std::vector<long> s_seg_off, s_first_off;
   int4 *d_sseg = nullptr;
   int *d_sfirst = nullptr;
@@ -1676,47 +1769,73 @@ int batch_seal(int rows, int stages) {
   return FLETCHER_OK;
 }
 
-// The persistent launch's work split for `ctas` persistent CTAs: each shot's own
-// single-shot plan (plan_segments, the balanced split the shot would get
-// alone), and for every number r of running shots those of the first r
-// shots of `order` stacked per CTA -- CTA b runs its segments of
-// order[0], then of order[1], ...  So neighbouring CTAs work on
-// neighbouring tiles of the same shot, and every CTA's load is balanced
-// shot by shot.
+// The persistent launch's work split for `ctas` persistent CTAs, for every
+// number r of running shots that a run passes through (the first r of
+// `order`): the shots that give every CTA kPooledPlanes planes and more keep
+// their own single-shot plans, stacked per CTA; the columns of the others are
+// one pool, cut so that every CTA ends up with the same cost.  A small shot's
+// own plan cuts it into ctas pieces of a few planes, each with its 8 halo
+// planes.  Stacked -> pooled, us a step: 24 shots of 48^3 updated cells 123
+// -> 44, of 64^3 150 -> 104, 16 of 88^3 (10 planes a CTA) 174 -> 165; 12 of
+// 108^3 (20) FP32 211 -> 235, 16-bit 314 -> 265.  So the line lies at 14 planes
+// a CTA for FP32, which streams from DRAM (pool pieces share no halos), and
+// at 64 for the 16-bit forms (6 shots of 158^3, 52 planes: FP16X 429 -> 404).
+constexpr double kPooledPlanes = 64.0, kPooledPlanesHbm = 14.0;
 int batch_plan(int ctas) {
   if (B.d_plan && B.plan_ctas == ctas) return FLETCHER_OK;
   if (B.d_plan) cudaFree(B.d_plan);
   if (B.d_first) cudaFree(B.d_first);
   B.d_plan = nullptr;
   B.d_first = nullptr;
-  const int ns = (int)B.shots.size();
+  const int ns = (int)B.shots.size(), TY = B.sealed_rows;
   if (!batch_half() && ns >= 32768) return fail(FLETCHER_ERR_ARGS, "a batch holds at most 32767 shots");
-  std::vector<Split> per(ns);
+  std::vector<Split> own(ns);
+  std::vector<char> pooled(ns, 0);
   for (int oi = 0; oi < ns; ++oi) {
     const BatchShot &s = B.shots[B.order[oi]];
     if (!batch_half() && s.sx >= 65536) return fail(FLETCHER_ERR_ARGS, "batched shots need sx < 65536");
-    per[oi] = plan_segments(ctas, s.ntx, s.nty, B.sealed_rows, B.bord, s.sz - 2 * B.bord, 0);
+    const int depth = s.sz - 2 * B.bord;
+    pooled[oi] = (double)s.ntx * s.nty * depth < (batch_half() ? kPooledPlanes : kPooledPlanesHbm) * ctas;
+    if (!pooled[oi])
+      own[oi] = plan_segments(ctas, s.ntx, s.nty, TY, last_tile_rows(s.sy, B.bord, s.nty, TY), B.bord, depth, 0,
+                              plan_hbm(B.form, FLETCHER_NUMERICS_FAST, false));
   }
   std::vector<int4> plan;
   std::vector<int> first((size_t)ns * (ctas + 1));
   B.plan_off.assign(ns, 0);
   B.plan_grid.assign(ns, 1);
   for (int r = 1; r <= ns; ++r) {
-    const size_t base = plan.size();
-    B.plan_off[r - 1] = (long)base;
+    if (r < ns && B.shots[B.order[r - 1]].nsteps == B.shots[B.order[r]].nsteps) continue;  // never r running
+    std::vector<std::vector<int4>> per(ctas);
+    std::vector<long> cost(ctas, 0);
+    std::vector<Column> pool;
+    for (int oi = 0; oi < r; ++oi) {
+      const int shot = B.order[oi];
+      const BatchShot &s = B.shots[shot];
+      if (pooled[oi]) {
+        const int last = last_tile_rows(s.sy, B.bord, s.nty, TY);
+        for (int t = 0; t < s.ntx * s.nty; ++t)
+          pool.push_back(Column{t % s.ntx, kRadius + t / s.ntx * TY, B.bord, s.sz - B.bord,
+                                t / s.ntx == s.nty - 1 ? last : TY, shot});
+        continue;
+      }
+      for (int b = 0; b < ctas; ++b)
+        for (int k = own[oi].first[b]; k < own[oi].first[b + 1]; ++k) {
+          const int4 w = own[oi].seg[k];
+          per[b].push_back(make_int4((w.x - kRadius) / kTileX | (shot << 16), w.y, w.z, w.w));
+          cost[b] += (long)TY * (w.w - w.z + kHaloCost);
+        }
+    }
+    const std::vector<long> base(cost);
+    deal_pool(pool, TY, base, pool_cap(pool, TY, base), &per, &cost);
+    const size_t at = plan.size();
+    B.plan_off[r - 1] = (long)at;
     int *f = first.data() + (size_t)(r - 1) * (ctas + 1);
     for (int b = 0; b < ctas; ++b) {
-      f[b] = (int)(plan.size() - base);
-      for (int oi = 0; oi < r; ++oi) {
-        const Split &sp = per[oi];
-        const int shot = B.order[oi];
-        for (int k = sp.first[b]; k < sp.first[b + 1]; ++k) {
-          const int4 w = sp.seg[k];
-          plan.push_back(make_int4((w.x - kRadius) / kTileX | (shot << 16), w.y, w.z, w.w));
-        }
-      }
+      f[b] = (int)(plan.size() - at);
+      plan.insert(plan.end(), per[b].begin(), per[b].end());
     }
-    f[ctas] = (int)(plan.size() - base);
+    f[ctas] = (int)(plan.size() - at);
     int grid = ctas;  // CTAs past the last one with work are not launched
     while (grid > 1 && f[grid - 1] == f[grid]) --grid;
     B.plan_grid[r - 1] = grid;
@@ -1748,6 +1867,7 @@ int batch_single_plans(int ctas) {
   const int ns = (int)B.shots.size();
   B.s_desc.assign(ns, ShotDesc());
   B.s_grid.assign(ns, 1);
+  B.s_skip.assign(ns, 0);
   B.s_seg_off.assign(ns, -1);
   B.s_first_off.assign(ns, -1);
   std::vector<int4> segs;
@@ -1755,7 +1875,9 @@ int batch_single_plans(int ctas) {
   for (int i = 0; i < ns; ++i) {
     const BatchShot &s = B.shots[i];
     const int depth = s.sz - 2 * B.bord;
-    const Split sp = plan_segments(ctas, s.ntx, s.nty, B.sealed_rows, B.bord, depth, 0);
+    const Split sp = plan_segments(ctas, s.ntx, s.nty, B.sealed_rows,
+                                   last_tile_rows(s.sy, B.bord, s.nty, B.sealed_rows), B.bord, depth, 0,
+                                   plan_hbm(B.form, FLETCHER_NUMERICS_FAST, false));
     B.s_seg_off[i] = (long)segs.size();
     B.s_first_off[i] = (long)firsts.size();
     segs.insert(segs.end(), sp.seg.begin(), sp.seg.end());
@@ -1763,6 +1885,7 @@ int batch_single_plans(int ctas) {
     int grid = ctas;
     while (grid > 1 && sp.first[grid - 1] == sp.first[grid]) --grid;
     B.s_grid[i] = grid;
+    B.s_skip[i] = sp.apart;
     B.s_desc[i] = B.h_desc[i];
   }
   if (!segs.empty()) {
@@ -1830,6 +1953,7 @@ int batch_issue(int it0, int it1, const float *src) {
     P.cor = it > 0 ? src[it - 1] : 0.0f;
     P.seg = B.d_plan + B.plan_off[active - 1];
     P.cta_first = B.d_first + (size_t)(active - 1) * (B.plan_ctas + 1);
+    P.skip_rows = 1;
     L.grid = B.plan_grid[active - 1];
     if (batch_half()) {
       // The new field's plane exponents (every running shot, one launch),
@@ -1922,6 +2046,7 @@ int batch_issue_chains(int chains, int steps, const float *src) {
         HL.h.p.one = B.s_desc[i];
         HL.h.p.seg = B.d_sseg + B.s_seg_off[i];
         HL.h.p.cta_first = B.d_sfirst + B.s_first_off[i];
+        HL.h.p.skip_rows = B.s_skip[i];
         HL.tile_rows = B.sealed_rows;
         HL.stages = B.stages;
         HL.grid = B.s_grid[i];
@@ -1950,6 +2075,7 @@ int batch_issue_chains(int chains, int steps, const float *src) {
       P.one = B.s_desc[i];
       P.seg = B.d_sseg + B.s_seg_off[i];
       P.cta_first = B.d_sfirst + B.s_first_off[i];
+      P.skip_rows = B.s_skip[i];
       L.grid = B.s_grid[i];
       L.m.arr = m.arr;
       L.m.upd = m.upd;

@@ -324,6 +324,29 @@ __global__ void __launch_bounds__(kTileX *(TY + kHelperWarps), MINB)
     // The cell that lacks the last step's source, if it is this thread's.
     const int cor_k = (gx == sd.cor_x && gy == sd.cor_y) ? sd.cor_z + kLag - it.z0 : -1000;
 
+    if (P.skip_rows && (gy < bord || gy >= sys - bord)) {
+      // A row outside the updated region: nothing to compute, only the
+      // stages to release in step.  (Not where the plan deals every tile
+      // alike: tiles that run ahead of their neighbours share fewer halo
+      // rows; 312^3 updated cells 304.7 -> 308.5 us.)
+      for (int k = -kRadius; k < depth + kLag; ++k) {
+        if (!wait(bar(st, L::OFF_READY), phase)) {
+          if (lx == 0) atomicOr(P.err, 1u);
+          return;
+        }
+        __syncwarp();
+        if (lx == 0) mbar_arrive(bar(st, L::OFF_EMPTY));
+        if (!L::AB_IN) abw = abw == kLag ? 0 : abw + 1;
+        if (!L::ROWS_IN && ++rb == L::NB) rb = 0;
+        st = stage == S - 1 ? smem : st + L::SB;
+        if (++stage == S) {
+          stage = 0;
+          phase ^= 1u;
+        }
+      }
+      continue;
+    }
+
     f2 Pr[kRing], Dx[kRing], Dy[kRing];
 
     for (int kb = -kRadius; kb < depth + kLag; kb += kRing) {

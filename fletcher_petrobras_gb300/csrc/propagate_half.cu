@@ -463,6 +463,27 @@ __global__ void __launch_bounds__(kTileX *(TY + kHelperWarps), 1)
     // The cell that lacks the last step's source, if it is this thread's.
     const int cor_k = (gx == sd.cor_x && gy == sd.cor_y) ? sd.cor_z + kRadius - it.z0 : -1000;
 
+    if (P.skip_rows && (gy < sd.bord || gy >= sd.sy - sd.bord)) {
+      // A row outside the updated region: nothing to compute, only the
+      // stages to release in step.
+      for (int k = -kRadius; k < depth + kRadius; ++k) {
+        if (!mbar_spin(bar(st, L::OFF_READY), phase)) {
+          if (lx == 0) atomicOr(P.err, 1u);
+          return;
+        }
+        __syncwarp();
+        if (lx == 0) mbar_arrive(bar(st, L::OFF_EMPTY));
+        if (!L::AB_IN) abw = abw == 4 ? 0 : abw + 1;
+        if (++ds == L::ND) ds = 0;
+        st = stage == S - 1 ? smem : st + L::SB;
+        if (++stage == S) {
+          stage = 0;
+          phase ^= 1u;
+        }
+      }
+      continue;
+    }
+
     f2 Pr[9], Dx[9], Dy[9];
 
     for (int kb = -kRadius; kb < depth + kRadius; kb += 9) {

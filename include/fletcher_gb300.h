@@ -188,11 +188,11 @@ int FLETCHER_SetTileConfig(int tile_rows, int stages, int zchunks);
 /* The work split of a single-shot launch (host only): ntx x nty tiles of
  * 32 x tile_rows cells, planes [zlo, zlo + depth), over `ctas` persistent
  * CTAs.  Whole rounds of z-chunks go round-robin (CTAs side by side on
- * neighbouring tiles); the last partial round is shared out in equal
- * pieces of at least 8 planes.  Writes the segments {x0, y0, z0, z1} CTA by
- * CTA into seg_out (when they fit in `cap`), each CTA's first segment into
- * first_out [ctas + 1], and the busiest CTA's cost (its planes plus 4 a
- * segment for the halo, shared-out pieces counting 3/2) into max_cost;
+ * neighbouring tiles); the last partial round is cut into contiguous pieces
+ * that fill every CTA up to the same cost.  Writes the segments {x0, y0, z0,
+ * z1} CTA by CTA into seg_out (when they fit in `cap`), each CTA's first
+ * segment into first_out [ctas + 1], and the busiest CTA's cost (its planes
+ * plus 4 a segment for the halo) into max_cost;
  * returns the segment count (negative on error).  zchunks as in
  * FLETCHER_SetTileConfig (0: the cheapest plan). */
 int FLETCHER_PlanSegments(int ctas, int ntx, int nty, int tile_rows, int zlo, int depth, int zchunks, int *seg_out,

@@ -375,3 +375,17 @@ def test_many_short_items_per_cta(tile, orc):
     ref = orc.run_f32(prob, m)
     for a, b in zip(got, ref):
         assert rel_l2(a, b) < TOL_SHORT
+
+
+@pytest.mark.parametrize("ny", [33, 40, 47, 1, 16])
+def test_last_tile_row_with_few_rows(ny, orc):
+    """The last tile row holds 1, 8, 15, 9 or 8 rows of the updated region (its
+    other warps do not compute, and the plan counts it apart), in a grid small
+    enough to be pooled and with a source in that row."""
+    prob = Problem("rows", 70, ny, 21, absorb=4, dt=0.0006, steps=14, fcut=45.0, kind="layered", layers=3, seed=15)
+    prob = prob.with_(source=(4 + 37, prob.sy - 5, 4 + 11))
+    m = prob.model()
+    got = gpu_run(prob, m, use_run=True)
+    ref = orc.run_f32(prob, m)
+    for a, b in zip(got, ref):
+        assert rel_l2(a, b) < TOL_SHORT
