@@ -23,7 +23,7 @@
 //
 // What bounds it: FP16 the shared-memory pipe (80% busy) and issue (68%),
 // with the FP32 stencil's reads plus the decode; FP16X issue (its decode and
-// encode).  272^3 updated cells: FP16 232 us a step, FP16X 290, against 337
+// encode).  272^3 updated cells: FP16 230 us a step, FP16X 280, against 337
 // and 377 us when all 16 warps decoded each plane between two CTA-wide
 // barriers.  The residual bytes take no conversion instruction (decode,
 // encode): 12 of 310 us.  Four decoded tiles instead of three: FP16 244 ->
@@ -66,8 +66,6 @@ struct GeoH {
   static_assert(ARR_B % 128 == 0 && UPD_B % 128 == 0, "stage regions 128-B aligned");
 };
 
-constexpr int kHelperWarps = 4;  // producer warp + 3 decode warps: one warpgroup (setmaxnreg works on warpgroups)
-constexpr int kDecodeWarps = kHelperWarps - 1;
 
 // Shared memory of a CTA: S stages (TMA tiles, the in-plane terms A, B of the
 // stage's plane when five stages match their five slots, and a control
@@ -101,18 +99,23 @@ struct LayoutH {
                 "shared-memory alignment");
 };
 
-// Register split (setmaxnreg), as in propagate_fp32.cu: TY/4 compute warps
-// and one helper warp per SM sub-partition share what the launch gives them.
-// FP16X at 16 rows: its decode needs the registers to keep several cells in
-// flight (272^3 updated cells: 311 us a step with 32 for the decode warps, 290
-// with 64, although the compute warps then spill 60 bytes); FP16 does not
-// (232 us with 32, 246 with 64).
+// Warps and register split (setmaxnreg, which works on warpgroups), as in
+// propagate_fp32.cu: TY/4 compute warps and kHelpers/4 helper warps per SM
+// sub-partition share what the launch gives them.
+// FP16X at 16 rows decodes with seven warps (272^3 updated cells: 311 us a
+// step with three of 32 registers, 287 with three of 64, which keep more cells
+// in flight, 280 with seven of 32; its compute warps then spill 32 bytes); FP16
+// with three (230 us; 246 with 64 registers, its compute warps at 104).
 template <int TY, bool EXT>
 struct RegsH {
+  static constexpr int kHelpers = TY == 16 && EXT ? 8 : 4;  // producer warp + decode warps
+  static constexpr int kDecode = kHelpers - 1;
+  static constexpr int kThreads = kTileX * (TY + kHelpers);
   static constexpr int kCompute = TY == 16 ? (EXT ? 104 : 112) : TY == 12 ? 152 : 216;
-  static constexpr int kHelper = TY == 16 ? (EXT ? 64 : 32) : TY == 12 ? 56 : 72;
-  static constexpr int kLaunch = TY == 16 ? 96 : TY == 12 ? 128 : 168;
-  static_assert((TY / 4) * kCompute + kHelper <= (TY / 4 + 1) * kLaunch, "the split exceeds the launch's registers");
+  static constexpr int kHelper = TY == 16 ? 32 : TY == 12 ? 56 : 72;
+  static constexpr int kLaunch = TY == 16 ? (EXT ? 80 : 96) : TY == 12 ? 128 : 168;
+  static_assert(TY / 4 * kCompute + kHelpers / 4 * kHelper <= (TY + kHelpers) / 4 * kLaunch,
+                "the split exceeds the launch's registers");
 };
 
 // 2^e as a float (|e| <= 126).
@@ -220,10 +223,11 @@ __device__ __forceinline__ void issue_half(unsigned char *stage, uint64_t *bar, 
 // BATCH: the items belong to the shots of a batch (P.shots, H.hshots,
 // H.hmaps: buffers, exponents and tensor maps by shot).
 template <int TY, int S, bool ISO, bool EXT, bool BATCH>
-__global__ void __launch_bounds__(kTileX *(TY + kHelperWarps), 1)
+__global__ void __launch_bounds__(RegsH<TY, EXT>::kThreads, 1)
     k_propagate_half(const __grid_constant__ HalfMaps M, const __grid_constant__ HalfParams H) {
   using G = GeoH<TY, EXT>;
   using L = LayoutH<TY, S, EXT>;
+  constexpr int kDecodeWarps = RegsH<TY, EXT>::kDecode;
   const PropParams &P = H.p;
   extern __shared__ unsigned char smem_dyn[];
   unsigned char *smem = smem_dyn + ((128u - (smem_addr(smem_dyn) & 127u)) & 127u);
@@ -709,7 +713,7 @@ static cudaError_t launch_half_t(const HalfLaunch &L, cudaStream_t s) {
   const cudaError_t e = prepare_half_t<TY, S, EXT, BATCH>();
   if (e != cudaSuccess) return e;
   auto kern = L.h.p.iso ? k_propagate_half<TY, S, true, EXT, BATCH> : k_propagate_half<TY, S, false, EXT, BATCH>;
-  return launch_step(kern, L.grid, kTileX * (TY + kHelperWarps), LayoutH<TY, S, EXT>::BYTES, s, L.m, L.h);
+  return launch_step(kern, L.grid, RegsH<TY, EXT>::kThreads, LayoutH<TY, S, EXT>::BYTES, s, L.m, L.h);
 }
 
 bool propagate_half_supported(int tile_rows, int stages) {
