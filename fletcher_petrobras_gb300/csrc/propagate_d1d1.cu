@@ -6,10 +6,17 @@
 // every operation is rounded on its own in the reference's order, p and q
 // separately.
 //
-// One CTA per SM, persistent, 16 warps of one tile row each.  As
-// pxy = Der1_y(pDx) needs pDx of the rows above and below, all warps exchange
-// it every plane; lane 0 of the last warp issues the TMA loads (S-2 steps
-// ahead) right after its own arrival at that exchange.
+// The warps are specialised as in propagate_fp32.cu: a producer thread issues
+// the TMA loads, the halo warps add the step's source and evaluate pDx in the
+// tile's 8 halo rows, and 16 compute warps run a tile row each.  As
+// pxy = Der1_y(pDx) needs pDx of the rows above and below, the compute warps
+// exchange it every plane: a warp announces its row, updates plane k-4, which
+// needs no exchanged data, and only then waits for the other rows.
+//
+// What bounds it: issue (scalar p and q, no fused multiply-adds: about 400
+// instructions a warp and plane).  Against the kernel whose compute warps
+// issued the loads and added the source themselves: 128 x 112 x 104 updated
+// cells 30.6 -> 26.3 us a step, 280 x 200 x 150 170 -> 128, 272^3 327 -> 283.
 #include "device_util.cuh"
 #include "fletcher_internal.h"
 #include "propagate_fp32_pipe.cuh"
@@ -19,136 +26,202 @@ namespace flt {
 
 namespace {
 
-template <int TY, int S>
-constexpr size_t smem_bytes_d1d1() {
-  using G = Geo<TY, true>;
-  return size_t(S) * G::STAGE_B + 2 * G::ROW_B + G::AB_B + 8 * S + 8 + 64 + 128;
-}
+constexpr int TY = kD1D1Rows, S = kD1D1Stages;
+using G = Geo<TY, true>;
+constexpr int kHelperWarps = 4, kHaloWarps = kHelperWarps - 1;
+constexpr int kThreads = kTileX * (TY + kHelperWarps);
+// Registers: 4 x 112 + 32 = 5 x 96 a sub-partition, as in propagate_fp32.cu.
+constexpr int kComputeRegs = 112, kHelperRegs = 32;
 
-// The producer's position (next step to load), kept in shared memory so it
-// costs no registers in the other threads.
-struct Cursor {
-  Item it;
-  int item, k, stage;
-};
+// Shared memory: S stages (TMA tiles, pDx of the tile's columns with its
+// 4-row halo, a control block), then the in-plane terms (A, B and C) of the
+// last 5 planes.
+constexpr int OFF_ROWS = G::STAGE_B;
+constexpr int OFF_HDR = OFF_ROWS + G::ROW_B;  // the item that starts in the stage
+constexpr int OFF_FULL = OFF_HDR + 16;        // barriers: loads landed,
+constexpr int OFF_READY = OFF_HDR + 24;       //   source and pDx halo rows written,
+constexpr int OFF_XCHG = OFF_HDR + 32;        //   pDx rows of the compute warps written,
+constexpr int OFF_EMPTY = OFF_HDR + 40;       //   released by every reader
+constexpr int SB = OFF_HDR + 128;
+constexpr int OFF_AB = S * SB;                          // [kABSlots][NT] of 16 bytes
+constexpr int OFF_C = OFF_AB + kABSlots * G::NT * 16;   // [kABSlots][NT] of 8 bytes: ch1dxy * pxy
+constexpr size_t kSmem = size_t(OFF_C) + kABSlots * G::NT * 8 + 128;
+static_assert(kSmem <= 227 * 1024, "Der1-Der1 shape exceeds the shared memory of a CTA");
+static_assert(OFF_HDR % 128 == 0 && SB % 128 == 0 && OFF_AB % 128 == 0 && OFF_C % 128 == 0, "shared-memory alignment");
 
-template <int TY, int S>
-__global__ void __launch_bounds__(kTileX *TY, 1)
+__global__ void __launch_bounds__(kThreads, 1)
     k_propagate_d1d1(const __grid_constant__ SingleMaps SM, const __grid_constant__ PropParams P) {
-  using G = Geo<TY, true>;
   extern __shared__ unsigned char smem_dyn[];
   unsigned char *smem = smem_dyn + ((128u - (smem_addr(smem_dyn) & 127u)) & 127u);
-  f2 *dbuf = reinterpret_cast<f2 *>(smem + S * G::STAGE_B);
-  float4 *ABs = reinterpret_cast<float4 *>(smem + S * G::STAGE_B + 2 * G::ROW_B);  // [kABSlots][NT]
-  f2 *Cs = reinterpret_cast<f2 *>(ABs + kABSlots * G::NT);                         // [kABSlots][NT]: ch1dxy * pxy
-  uint64_t *full = reinterpret_cast<uint64_t *>(smem + S * G::STAGE_B + 2 * G::ROW_B + G::AB_B);
-  uint64_t *xchg = full + S;  // pDx rows written (one arrival per warp)
-  Cursor *cur = reinterpret_cast<Cursor *>(xchg + 1);
+  auto bar = [&](unsigned char *st, int off) { return reinterpret_cast<uint64_t *>(st + off); };
 
   const int tid = threadIdx.x;
   const int lx = tid & 31;
-  const int ly = __shfl_sync(0xffffffffu, tid >> 5, 0);  // warp-uniform
-  const int first = P.cta_first[blockIdx.x], end = P.cta_first[blockIdx.x + 1];
-  if (first >= end) return;
-  const bool producer = tid == (TY - 1) * 32;
-  StepMaps maps;
-  maps.cur = &SM.cur_halo;
-  maps.prev = &SM.prev_pt;
-  maps.arr = &SM.arr;
-  maps.upd = &SM.upd;
-  // Issues the cursor's step into its stage and advances the cursor.
-  auto produce = [&]() {
-    Cursor c = *cur;
-    issue_step<TY>(smem + c.stage * G::STAGE_B, &full[c.stage], c.it, c.k, maps);
-    if (++c.stage == S) c.stage = 0;
-    if (++c.k >= c.it.z1 + kLag) {
-      if (++c.item < end) {
-        c.it = decode_item<false>(P.seg[c.item]);
-        c.k = c.it.z0 - kRadius;
-      }
-    }
-    *cur = c;
-  };
+  const int wid = uniform(tid >> 5);
+  const int first = P.cta_first[blockIdx.x], nitems = P.cta_first[blockIdx.x + 1] - first;
+  if (nitems <= 0) return;
   if (tid == 0) {
-    for (int s = 0; s < S; ++s) mbar_init(&full[s], 1);
-    mbar_init(xchg, TY);
+    for (int s = 0; s < S; ++s) {
+      unsigned char *st = smem + s * SB;
+      mbar_init(bar(st, OFF_FULL), 1);
+      mbar_init(bar(st, OFF_READY), kHaloWarps);
+      mbar_init(bar(st, OFF_XCHG), TY);
+      mbar_init(bar(st, OFF_EMPTY), TY + kHaloWarps);
+    }
     mbar_fence_init();
-  }
-  if (producer) {
-    Cursor c;
-    c.it = decode_item<false>(P.seg[first]);
-    c.item = first;
-    c.k = c.it.z0 - kRadius;
-    c.stage = 0;
-    *cur = c;
   }
   __syncthreads();
   allow_next_launch();
   wait_previous_launch();
-  if (producer) {
-    tma_prefetch_desc(maps.cur);
-    tma_prefetch_desc(maps.prev);
-    tma_prefetch_desc(maps.arr);
-    tma_prefetch_desc(maps.upd);
-    // Prologue: the first S-2 steps of this CTA.
-    for (int a = 0; a < S - 2 && cur->item < end; ++a) produce();
+  const ShotDesc &sd = P.one;
+
+  if (wid >= TY) {
+    setmaxnreg_dec<kHelperRegs>();
+    const int4 *seg = P.seg + first;
+    int stage = 0;
+    uint32_t phase = 0;
+    if (wid == TY) {
+      // ---- producer ----
+      if (lx != 0) return;
+      StepMaps maps;
+      maps.cur = &SM.cur_halo;
+      maps.prev = &SM.prev_pt;
+      maps.arr = &SM.arr;
+      maps.upd = &SM.upd;
+      tma_prefetch_desc(maps.cur);
+      tma_prefetch_desc(maps.prev);
+      tma_prefetch_desc(maps.arr);
+      tma_prefetch_desc(maps.upd);
+      int4 next = seg[0];
+      int issued = 0;
+      bool ok = true;
+      for (int i = 0; i < nitems && ok; ++i) {
+        const int4 w = next;
+        const Item it = decode_item<false>(w);
+        if (i + 1 < nitems) next = seg[i + 1];
+        for (int k = it.z0 - kRadius; k < it.z1 + kLag; ++k) {
+          unsigned char *st = smem + stage * SB;
+          // (The first S waits pass at once: the stage was never filled.)
+          if (!mbar_spin(bar(st, OFF_EMPTY), phase ^ 1u)) {
+            ok = false;
+            break;
+          }
+          fence_proxy_async_smem();
+          if (k == it.z0 - kRadius) *reinterpret_cast<int4 *>(st + OFF_HDR) = w;
+          issue_step<TY>(st, bar(st, OFF_FULL), it, k, maps);
+          ++issued;
+          if (++stage == S) {
+            stage = 0;
+            phase ^= 1u;
+          }
+        }
+      }
+      if (!ok) {
+        // A bounded wait gave up: wait, bounded, for the loads still in
+        // flight, then leave (every other thread gives up on its own waits).
+        atomicOr(P.err, 2u);
+        for (int a = 1; a <= S && a <= issued; ++a) {
+          const int s2 = stage >= a ? stage - a : stage + S - a;
+          (void)mbar_wait(bar(smem + s2 * SB, OFF_FULL), stage >= a ? phase : phase ^ 1u, kDrainNs);
+        }
+      }
+      return;
+    }
+    // ---- halo warps ----
+    const int hw = wid - TY - 1;
+    for (int i = 0; i < nitems; ++i) {
+      const Item it = decode_item<false>(seg[i]);
+      const int src_z = sd.src_z;
+      for (int k = it.z0 - kRadius; k < it.z1 + kLag; ++k) {
+        unsigned char *st = smem + stage * SB;
+        if (!mbar_spin(bar(st, OFF_FULL), phase)) {
+          atomicOr(P.err, 1u);
+          return;
+        }
+        f2 *H = reinterpret_cast<f2 *>(st);
+        if (k == src_z) {
+          // Fused source (original/OpenMP/openmp_insertsource.c:7-13): the
+          // current p and q gain `src` at the source cell before the update
+          // reads them.
+          const int rx = sd.src_x - (it.x0 - kRadius), ry = sd.src_y - (it.y0 - kRadius);
+          if (hw == 0 && lx == 0 && rx >= 0 && rx < G::HX && ry >= 0 && ry < G::HY) {
+            H[ry * G::HX + rx] = add2(H[ry * G::HX + rx], splat(P.src));
+            fence_proxy_async_smem();
+          }
+          asm volatile("bar.sync 1, %0;" ::"n"(32 * kHaloWarps) : "memory");
+        }
+        if (k >= it.z0 && k < it.z1) {
+          // pDx of the tile's 4-row y halo (halo-tile rows 0..3 and TY+4..TY+7).
+          f2 *db = reinterpret_cast<f2 *>(st + OFF_ROWS);
+          for (int r = hw; r < 2 * kRadius; r += kHaloWarps) {
+            const int hrow = r < kRadius ? r : TY + r;
+            const f2 *h = H + hrow * G::HX + lx + kRadius;
+            db[hrow * G::TX + lx] = d1_ref(h[1], h[-1], h[2], h[-2], h[3], h[-3], h[4], h[-4], P.inv_dx);
+          }
+        }
+        __syncwarp();
+        if (lx == 0) {
+          mbar_arrive(bar(st, OFF_READY));
+          mbar_arrive(bar(st, OFF_EMPTY));
+        }
+        if (++stage == S) {
+          stage = 0;
+          phase ^= 1u;
+        }
+      }
+    }
+    return;
   }
 
+  // ---- compute warps ----
+  setmaxnreg_inc<kComputeRegs>();
+  const int ly = wid;
   const float sxx = P.inv_dxx, syy = P.inv_dyy, szz = P.inv_dzz;
-  const ShotDesc &sd = P.one;
+  const int ci = ly * G::TX + lx;
+  const int hc = (ly + kRadius) * G::HX + (lx + kRadius);
   int stage = 0;
-  uint32_t phase = 0, xphase = 0;
-  int dsel = 0;
-  int abw = 0;  // shared A/B ring slot of the arriving plane (the plane kLag back is at abw + 1)
-  for (int item = first; item < end; ++item) {
-    const Item it = decode_item<false>(P.seg[item]);
-    const int kbeg = it.z0 - kRadius;
-    const int kend = it.z1 + kLag;
+  uint32_t phase = 0;
+  int abw = 0;  // shared A/B/C ring slot of the arriving plane (the plane kLag back is at abw + 1)
+  unsigned char *st = smem;
+  for (int item = 0; item < nitems; ++item) {
+    if (!mbar_spin(bar(st, OFF_READY), phase)) {
+      if (lx == 0) atomicOr(P.err, 1u);
+      return;
+    }
+    const Item it = decode_item<false>(uniform4(*reinterpret_cast<const int4 *>(st + OFF_HDR)));
+    const int depth = it.z1 - it.z0;
     const int gx = it.x0 + lx;
     const int gy = it.y0 + ly;
     const int bord = sd.bord, sxs = sd.sx, sys = sd.sy;
     const bool valid = (gx >= bord) && (gx < sxs - bord) && (gy >= bord) && (gy < sys - bord);
     const long plane = (long)sd.pitch * sys;
-    unsigned long long *out = reinterpret_cast<unsigned long long *>(sd.F[P.parity ^ 1]) + ((long)gy * sd.pitch + gx);
-    const int src_z = sd.src_z, cor_z = sd.cor_z;  // cells are read from `sd` on the (rare) planes
-    const int ci = ly * G::TX + lx;
-    const int hc = (ly + kRadius) * G::HX + (lx + kRadius);
+    unsigned long long *out =
+        reinterpret_cast<unsigned long long *>(sd.F[P.parity ^ 1]) + (it.z0 * plane + (long)gy * sd.pitch + gx);
+    // The cell that lacks the last step's source, if it is this thread's.
+    const int cor_k = (gx == sd.cor_x && gy == sd.cor_y) ? sd.cor_z + kLag - it.z0 : -1000;
 
     f2 Pr[kRing], Dx[kRing], Dy[kRing];
 
-    for (int kb = kbeg; kb < kend; kb += kRing) {
+    for (int kb = -kRadius; kb < depth + kLag; kb += kRing) {
 #pragma unroll
       for (int j = 0; j < kRing; ++j) {
-        const int k = kb + j;
-        if (k >= kend) break;
-        unsigned char *st = smem + stage * G::STAGE_B;
-        if (!mbar_wait(&full[stage], phase, kWaitLimitNs)) {
-          atomicOr(P.err, 1u);
-          goto aborted;
+        const int k = kb + j;  // plane, counted from the item's first
+        if (k >= depth + kLag) break;
+        if (!mbar_spin(bar(st, OFF_READY), phase)) {
+          if (lx == 0) atomicOr(P.err, 1u);
+          return;
         }
-        const bool center = (k >= it.z0) && (k < it.z1);
-        const bool upd = (k - kLag >= it.z0);
-        const bool src_plane = (k == src_z);
-        const f2 *H = reinterpret_cast<const f2 *>(st);
-
-        f2 c = H[hc];
+        const bool center = (unsigned)k < (unsigned)depth;
+        const bool upd = k >= kLag;
+        const f2 *H = reinterpret_cast<const f2 *>(st) + hc;
+        const f2 c = H[0];
         f2 xa[4], xb[4], ya[4], yb[4];
 #pragma unroll
         for (int o = 1; o <= 4; ++o) {
-          xa[o - 1] = H[hc + o];
-          xb[o - 1] = H[hc - o];
-          ya[o - 1] = H[hc + o * G::HX];
-          yb[o - 1] = H[hc - o * G::HX];
-        }
-        // Fused source (original/OpenMP/openmp_insertsource.c:7-13): the
-        // current p and q gain `src` at the source cell before the update
-        // reads them; added to this thread's copies of the plane.
-        if (src_plane) {
-          const int src_x = sd.src_x, src_y = sd.src_y;
-          const f2 sv = splat(P.src);
-          f2 dummy;
-          if (gy == src_y && abs(src_x - gx) <= kRadius) add_at(c, xa, xb, src_x - gx, sv);
-          if (gx == src_x && src_y != gy && abs(src_y - gy) <= kRadius) add_at(dummy, ya, yb, src_y - gy, sv);
+          xa[o - 1] = H[o];
+          xb[o - 1] = H[-o];
+          ya[o - 1] = H[o * G::HX];
+          yb[o - 1] = H[-o * G::HX];
         }
         // der1der1/sample.h:35-49: pDx = Der1_x(p) / dx and pDy = Der1_y(p) / dy.
         const f2 d1x = d1_ref(xa[0], xb[0], xa[1], xb[1], xa[2], xb[2], xa[3], xb[3], P.inv_dx);
@@ -157,40 +230,16 @@ __global__ void __launch_bounds__(kTileX *TY, 1)
         Dx[j] = d1x;
         Dy[j] = d1y;
         f2 d2x, d2y;
-        f2 *db = dbuf + dsel * (G::HY * G::TX);
+        f2 *dc = reinterpret_cast<f2 *>(st + OFF_ROWS) + ((ly + kRadius) * G::TX + lx);
         if (center) {
+          dc[0] = d1x;
           d2x = d2_ref(c, xa[0], xb[0], xa[1], xb[1], xa[2], xb[2], xa[3], xb[3], sxx);
           d2y = d2_ref(c, ya[0], yb[0], ya[1], yb[1], ya[2], yb[2], ya[3], yb[3], syy);
-          // pDx of the tile column and of its 4-row y halo: the row's own
-          // value, and warps 0..7 one halo row each (halo-tile rows 0..3 and
-          // TY+4..TY+7).
-          db[(ly + kRadius) * G::TX + lx] = d1x;
-          if (ly < 2 * kRadius) {
-            const int hrow = ly < kRadius ? ly : TY + ly;
-            const int hb0 = hrow * G::HX + lx + kRadius;
-            f2 ha[4], hb[4], dummy;
-#pragma unroll
-            for (int o = 1; o <= 4; ++o) {
-              ha[o - 1] = H[hb0 + o];
-              hb[o - 1] = H[hb0 - o];
-            }
-            if (src_plane && it.y0 - kRadius + hrow == sd.src_y && abs(sd.src_x - gx) <= kRadius)
-              add_at(dummy, ha, hb, sd.src_x - gx, splat(P.src));
-            db[hrow * G::TX + lx] = d1_ref(ha[0], hb[0], ha[1], hb[1], ha[2], hb[2], ha[3], hb[3], P.inv_dx);
-          }
         }
-        // Split-phase exchange: announce this warp's pDx (and, by program
-        // order, that it has finished the previous step), update plane k-4,
-        // which needs no exchanged data, then wait for the other warps.
+        // Split-phase exchange: announce this warp's pDx, update plane k-4,
+        // then wait for the other rows.
         __syncwarp();
-        if (lx == 0) mbar_arrive(xchg);
-        // The producer has passed the exchange of the previous step, so every
-        // thread is past the step before it: refill that step's stage with
-        // the next step due (S-2 steps ahead of this one).
-        if (producer && cur->item < end) {
-          fence_proxy_async_smem();
-          produce();
-        }
+        if (lx == 0) mbar_arrive(bar(st, OFF_XCHG));
         if (upd) {
           const int cs = (j + kRing - kLag) % kRing;  // ring slot of plane k-kLag
           // RP(o): plane k-kLag+o for o = 0..4, k-kLag-(kRing-o) for o > 4.
@@ -210,12 +259,12 @@ __global__ void __launch_bounds__(kTileX *TY, 1)
           const float v2px = cu[3 * G::TX], v2pz = cu[4 * G::TX];
           const float v2sz = cu[5 * G::TX], v2pn = cu[6 * G::TX];
           const int slot = abw == kLag ? 0 : abw + 1;
-          const float4 ab = ABs[slot * G::NT + ci];
+          const float4 ab = reinterpret_cast<const float4 *>(smem + OFF_AB)[slot * G::NT + ci];
           const f2 Ak = mk2(ab.x, ab.y), Bk = mk2(ab.z, ab.w);
           // der1der1/sample.h:70-117 in its order, each operation rounded:
           // h1 = cpxx + cpyy + cpzz + cpxy + cpxz + cpyz (A = cpxx + cpyy,
           // C = cpxy from the plane's arrival), h2 = pxx + pyy + pzz - h1.
-          const f2 Ck = Cs[slot * G::NT + ci];
+          const f2 Ck = reinterpret_cast<const f2 *>(smem + OFF_C)[slot * G::NT + ci];
           const f2 h1 = add_rn(add_rn(add_rn(add_rn(Ak, mul_rn(czz, d2z)), Ck), mul_rn(cxz, dxz)), mul_rn(cyz, dyz));
           const f2 h2 = sub_rn(add_rn(Bk, d2z), h1);
           const float h1p = lo(h1), h1q = hi(h1), h2p = lo(h2), h2q = hi(h2);
@@ -223,26 +272,20 @@ __global__ void __launch_bounds__(kTileX *TY, 1)
           const float rhsp = __fadd_rn(__fadd_rn(__fmul_rn(v2px, h2p), t), __fmul_rn(v2sz, __fsub_rn(h1p, h1q)));
           const float rhsq = __fsub_rn(__fadd_rn(__fmul_rn(v2pn, h2p), t), __fmul_rn(v2sz, __fsub_rn(h2p, h2q)));
           f2 old = reinterpret_cast<const f2 *>(st + G::OFF_PP)[ci];
-          const int zc = k - kLag;
-          if (zc == cor_z) {
-            if (gx == sd.cor_x && gy == sd.cor_y) old = add2(old, splat(P.cor));
-          }
+          if (k == cor_k) old = add2(old, splat(P.cor));
           const f2 now = Pr[cs];
           // pp = 2 pc - pp + rhs * dt * dt (der1der1/sample.h:119-120).
           const f2 nw = add_rn(sub_rn(add_rn(now, now), old), mul_rn(P.dt, mul_rn(P.dt, mk2(rhsp, rhsq))));
-          if (valid) out[(long)zc * plane] = nw.v;
+          if (valid) *out = nw.v;
+          out += plane;
         }
-        if (!mbar_wait(xchg, xphase, kWaitLimitNs)) {
-          // A warp of this CTA stopped arriving (it gave up a wait itself):
-          // leave too, so that no thread keeps waiting step after step.
-          atomicOr(P.err, 2u);
-          goto aborted;
-        }
-        xphase ^= 1u;
         if (center) {
+          if (!mbar_spin(bar(st, OFF_XCHG), phase)) {
+            if (lx == 0) atomicOr(P.err, 2u);
+            return;
+          }
           // pxy = Der1_y(pDx) / dy (der1der1/sample.h:55); A = cpxx + cpyy,
           // B = pxx + pyy, C = cpxy.
-          const f2 *dc = db + (ly + kRadius) * G::TX + lx;
           constexpr int W = G::TX;
           const f2 pxy = d1_ref(dc[W], dc[-W], dc[2 * W], dc[-2 * W], dc[3 * W], dc[-3 * W], dc[4 * W], dc[-4 * W],
                                 P.inv_dy);
@@ -250,27 +293,19 @@ __global__ void __launch_bounds__(kTileX *TY, 1)
           const float cxx = ca[0], cyy = ca[G::TX], cxy = ca[2 * G::TX];
           const f2 av = add_rn(mul_rn(cxx, d2x), mul_rn(cyy, d2y));
           const f2 bv = add_rn(d2x, d2y);
-          ABs[abw * G::NT + ci] = make_float4(lo(av), hi(av), lo(bv), hi(bv));
-          Cs[abw * G::NT + ci] = mul_rn(cxy, pxy);
+          reinterpret_cast<float4 *>(smem + OFF_AB)[abw * G::NT + ci] = make_float4(lo(av), hi(av), lo(bv), hi(bv));
+          reinterpret_cast<f2 *>(smem + OFF_C)[abw * G::NT + ci] = mul_rn(cxy, pxy);
         }
-        dsel ^= 1;
+        // This warp is done with the stage.
+        __syncwarp();
+        if (lx == 0) mbar_arrive(bar(st, OFF_EMPTY));
         abw = abw == kLag ? 0 : abw + 1;
+        st = stage == S - 1 ? smem : st + SB;
         if (++stage == S) {
           stage = 0;
           phase ^= 1u;
         }
       }
-    }
-  }
-  return;
-aborted:
-  // A bounded wait gave up.  Every thread leaves (the others give up on
-  // their own bounded waits); thread 0 first waits, bounded, for the loads
-  // that may still be in flight into this CTA's stages.
-  if (tid == 0) {
-    for (int a = 0; a < S - 2; ++a) {
-      const int s2 = (stage + a) % S;
-      (void)mbar_wait(&full[s2], phase ^ uint32_t(stage + a >= S), kWaitLimitNs);
     }
   }
 }
@@ -279,18 +314,14 @@ aborted:
 
 // One shape (kD1D1Rows x kD1D1Stages), single shot.
 cudaError_t propagate_d1d1_launch(const PropLaunch &L, cudaStream_t s) {
-  constexpr int TY = kD1D1Rows, S = kD1D1Stages;
-  constexpr size_t smem = smem_bytes_d1d1<TY, S>();
-  static_assert(smem <= 227 * 1024, "Der1-Der1 shape exceeds the shared memory of a CTA");
   static bool ready = false;
   if (!ready) {
-    const cudaError_t e =
-        cudaFuncSetAttribute(k_propagate_d1d1<TY, S>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    const cudaError_t e = cudaFuncSetAttribute(k_propagate_d1d1, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmem);
     if (e != cudaSuccess) return e;
     ready = true;
   }
   if (L.batch || L.tile_rows != TY || L.stages != S) return cudaErrorInvalidValue;
-  return launch_step(k_propagate_d1d1<TY, S>, L.grid, kTileX * TY, smem, s, L.m, L.p);
+  return launch_step(k_propagate_d1d1, L.grid, kThreads, kSmem, s, L.m, L.p);
 }
 
 }  // namespace flt

@@ -35,9 +35,6 @@ struct Geo {
   // One exchange buffer: D1y of the tile rows with their 4-column x halo, or
   // (Der1-Der1 numerics) D1x of the tile columns with their 4-row y halo.
   static constexpr int ROW_B = D1D1 ? HY * TX * 8 : TY * HX * 8;
-  // The per-cell in-plane terms (A, B; and C for the Der1-Der1 numerics) of
-  // the last 5 planes.
-  static constexpr int AB_B = kABSlots * NT * (D1D1 ? 24 : 16);
   static_assert(TY % 4 == 0, "tile rows must be a multiple of 4");
   static_assert(HALO_B % 128 == 0 && ARR_B % 128 == 0 && UPD_B % 128 == 0 && ID_B % 128 == 0,
                 "stage regions 128-B aligned");

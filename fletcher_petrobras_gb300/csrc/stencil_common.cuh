@@ -62,15 +62,4 @@ __device__ __forceinline__ f2 scale(f2 v, float s) {
   else return mul2(splat(s), v);
 }
 
-// Adds `s` to the register among {c, a[0..3] (offsets +1..+4), b[0..3]
-// (offsets -1..-4)} at offset d from the centre (|d| <= 4).
-__device__ __forceinline__ void add_at(f2 &c, f2 (&a)[4], f2 (&b)[4], int d, f2 s) {
-  if (d == 0) c = add2(c, s);
-#pragma unroll
-  for (int j = 1; j <= 4; ++j) {
-    if (d == j) a[j - 1] = add2(a[j - 1], s);
-    if (d == -j) b[j - 1] = add2(b[j - 1], s);
-  }
-}
-
 }  // namespace flt

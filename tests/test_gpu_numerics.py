@@ -72,6 +72,19 @@ def test_d1d1_numerics_independent_of_work_split(zchunks):
         assert np.array_equal(a, b)
 
 
+@pytest.mark.parametrize("zchunks", [-16, 11])
+def test_d1d1_many_short_items_per_cta(zchunks):
+    """Several work items per CTA, each shorter than the z stencil, give the
+    floats of whole tile columns."""
+    prob = Problem("d1d1short", 170, 130, 30, absorb=5, dt=0.0006, steps=9, fcut=45.0, kind="layered", layers=4,
+                   seed=12, source=(4 + 64, 4 + 48, 4 + 9))
+    m = prob.model()
+    base = run(prob, m, "d1d1", zchunks=-1)
+    got = run(prob, m, "d1d1", zchunks=zchunks)
+    for a, b in zip(base, got):
+        assert np.array_equal(a, b)
+
+
 def test_d1d1_numerics_rejects_16bit_forms():
     prop = Propagator(form="fp16x", numerics="d1d1")
     prob = Problem("d1d1half", 20, 20, 20, absorb=4, dt=0.0006, steps=2, kind="layered", layers=2, seed=1)
