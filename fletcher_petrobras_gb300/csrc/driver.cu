@@ -17,7 +17,7 @@
 //               read only the four velocity terms of coef.
 // The 16-bit forms replace F by Hh[b] (half2 per cell) and, for FP16X, Hl[b]
 // (residual bytes), with per-plane exponents E (three fields: current,
-// previous, next) and per-plane maxima Mx (one per buffer).
+// previous, next) and per-plane maxima Mx (those and one being cleared).
 #include <cuda.h>
 #include <cuda_runtime.h>
 #include <math.h>
@@ -72,8 +72,8 @@ struct State {
   unsigned *Hh[2] = {nullptr, nullptr};
   unsigned short *Hl[2] = {nullptr, nullptr};
   int *E = nullptr;        // [3][sz] plane exponents, slot of the current field = ecur
-  unsigned *Mx = nullptr;  // [2][sz] plane maxima (float bits) of the field in buffer b
-  int ecur = 0;
+  unsigned *Mx = nullptr;  // [4][sz] plane maxima (float bits), slot of the current field = mcur
+  int ecur = 0, mcur = 0;
   HalfMaps hm[2];          // maps of a step whose current field is in buffer b
   int numerics = FLETCHER_NUMERICS_FAST;
   // Media-table layout (FP32 form).
@@ -886,10 +886,10 @@ int initialize(int sx, int sy, int sz, int bord, float dx, float dy, float dz, f
       }
     }
     CK(dev_malloc(&g.E, 3 * sz * sizeof(int)));
-    CK(dev_malloc(&g.Mx, 2 * sz * sizeof(unsigned)));
+    CK(dev_malloc(&g.Mx, 4 * sz * sizeof(unsigned)));
     CK(cudaMemsetAsync(g.E, 0, 3 * sz * sizeof(int), s));
-    CK(cudaMemsetAsync(g.Mx, 0, 2 * sz * sizeof(unsigned), s));
-    g.dev_bytes = 2 * g.npitch * (sizeof(unsigned) + (ext ? sizeof(unsigned short) : 0)) + 5 * sz * sizeof(int);
+    CK(cudaMemsetAsync(g.Mx, 0, 4 * sz * sizeof(unsigned), s));
+    g.dev_bytes = 2 * g.npitch * (sizeof(unsigned) + (ext ? sizeof(unsigned short) : 0)) + 7 * sz * sizeof(int);
   } else {
     CK(dev_malloc(&g.F[0], g.npitch * sizeof(float2)));
     CK(dev_malloc(&g.F[1], g.npitch * sizeof(float2)));
@@ -953,6 +953,7 @@ int initialize(int sx, int sy, int sz, int bord, float dx, float dy, float dz, f
   // arrays, so their contents are the initial state).
   g.cur = 0;
   g.ecur = 0;
+  g.mcur = 0;
   const float *fp[2][2] = {{pc, qc}, {pp, qp}};
   for (int b = 0; b < 2; ++b) {
     const float *p = fp[b][0], *q = fp[b][1];
@@ -965,11 +966,11 @@ int initialize(int sx, int sy, int sz, int bord, float dx, float dy, float dz, f
       q = q ? raw + g.n : nullptr;
     }
     if (half) {
-      // Buffer 0 holds the current field (exponent slot 0), buffer 1 the
-      // previous one (slot 2).  Zero fields: the cleared buffers, exponents
+      // Buffer 0 holds the current field (slot 0 of the exponents and of the
+      // maxima), buffer 1 the previous one (slots 2 and 3).  Zero fields: the cleared buffers, exponents
       // and maxima are their stored form.
       if (p || q)
-        CK(half_encode(p, q, g.Hh[b], g.Hl[b], g.E + (b ? 2 : 0) * sz, g.Mx + b * sz, sx, sy, sz, g.pitch, ext,
+        CK(half_encode(p, q, g.Hh[b], g.Hl[b], g.E + (b ? 2 : 0) * sz, g.Mx + (b ? 3 : 0) * sz, sx, sy, sz, g.pitch, ext,
                        s));
     } else if (p || q) {
       // (No kernel reads the pitch padding, of the fields or of the
@@ -1142,11 +1143,6 @@ int step() {
   if (half_form()) {
     const int enew = (g.ecur + 1) % 3, eprev = (g.ecur + 2) % 3;
     const int sz = g.sz;
-    int sz_src = -1000;
-    if (fused) sz_src = want.src_z;
-    else if (g.owed.on) sz_src = want.cor_z;
-    const float sabs = fabsf(P.src) + fabsf(P.cor);
-    CK(half_scales(g.Mx + c * sz, g.Mx + p * sz, g.E + enew * sz, sz, sz_src, sabs, g_stream));
     HalfLaunch HL;
     memset(&HL, 0, sizeof(HL));
     HL.batch = false;
@@ -1156,13 +1152,17 @@ int step() {
     HL.h.e_cur = g.E + g.ecur * sz;
     HL.h.e_prev = g.E + eprev * sz;
     HL.h.e_new = g.E + enew * sz;
-    HL.h.m_new = g.Mx + p * sz;
+    HL.h.m_cur = g.Mx + g.mcur * sz;
+    HL.h.m_prev = g.Mx + (g.mcur + 3) % 4 * sz;
+    HL.h.m_new = g.Mx + (g.mcur + 1) % 4 * sz;
+    HL.h.m_clear = g.Mx + (g.mcur + 2) % 4 * sz;
     HL.m = g.hm[c];
     HL.tile_rows = g.tile_rows;
     HL.stages = g.stages;
     HL.grid = g.grid;
     CK(propagate_half_launch(HL, g.form == FLETCHER_FORM_FP16X, g_stream));
     g.ecur = enew;
+    g.mcur = (g.mcur + 1) % 4;
   } else {
     const bool abc = abc_active();
     CK(propagate_fp32_launch(L, g_stream));
@@ -1592,7 +1592,7 @@ struct BatchShot {
   size_t n = 0, npitch = 0;
   float2 *F[2] = {nullptr, nullptr};  // FP32 form
   // 16-bit forms: the two field buffers (half2 per cell, residual bytes),
-  // per-plane exponents [3][sz] and maxima [2][sz].
+  // per-plane exponents [3][sz] and maxima [4][sz].
   unsigned *Hh[2] = {nullptr, nullptr};
   unsigned short *Hl[2] = {nullptr, nullptr};
   int *E = nullptr;
@@ -2036,9 +2036,8 @@ int batch_issue_chains(int chains, int steps, const float *src) {
     CK(cudaStreamWaitEvent(cs, B.fork, 0));
     for (const int i : chain[c]) {
       if (half) {
-        // The single-shot 16-bit step: the new planes' scales, then the
-        // step (buffer it & 1 current, exponent slot it % 3, as the
-        // persistent launch keeps them).
+        // The single-shot 16-bit step (buffer it & 1 current, exponent slot
+        // it % 3, as the persistent launch keeps them).
         const HalfShot &h = B.h_hshots[i];
         const int sz = B.shots[i].sz;
         HalfLaunch HL;
@@ -2059,17 +2058,18 @@ int batch_issue_chains(int chains, int steps, const float *src) {
           HL.h.p.parity = cur;
           HL.h.p.src = src[it];
           HL.h.p.cor = it > 0 ? src[it - 1] : 0.0f;
-          CK(half_scales(h.Mx + cur * sz, h.Mx + prv * sz, h.E + enew * sz, sz, HL.h.p.one.src_z,
-                         fabsf(HL.h.p.src) + fabsf(HL.h.p.cor), cs));
           HL.h.out_hi = h.hi[prv];
           HL.h.out_lo = h.lo[prv];
           HL.h.e_cur = h.E + ecur * sz;
           HL.h.e_prev = h.E + eprev * sz;
           HL.h.e_new = h.E + enew * sz;
-          HL.h.m_new = h.Mx + prv * sz;
+          HL.h.m_cur = h.Mx + it % 4 * sz;
+          HL.h.m_prev = h.Mx + (it + 3) % 4 * sz;
+          HL.h.m_new = h.Mx + (it + 1) % 4 * sz;
+          HL.h.m_clear = h.Mx + (it + 2) % 4 * sz;
           HL.m = B.h_hmaps[i].m[cur];
           CK(propagate_half_launch(HL, ext, cs));
-          B.launches += 2;
+          B.launches += ext ? 1 : 2;
         }
         continue;
       }
@@ -2158,7 +2158,7 @@ extern "C" int FLETCHER_BatchAddShot(int sx, int sy, int sz, const float *model,
   }
   if (half) {
     ok = ok && dev_malloc(&s.E, 3 * sz * sizeof(int)) == cudaSuccess;
-    ok = ok && dev_malloc(&s.Mx, 2 * sz * sizeof(unsigned)) == cudaSuccess;
+    ok = ok && dev_malloc(&s.Mx, 4 * sz * sizeof(unsigned)) == cudaSuccess;
   }
   ok = ok && dev_malloc(&s.coef, coef_floats(sy, sz, s.pitch) * sizeof(float)) == cudaSuccess;
   float *raw = nullptr;
@@ -2196,7 +2196,7 @@ extern "C" int FLETCHER_BatchAddShot(int sx, int sy, int sz, const float *model,
     if (e == cudaSuccess && s.Hl[b]) e = cudaMemsetAsync(s.Hl[b], 0, s.npitch * sizeof(unsigned short), st);
   }
   if (e == cudaSuccess && half) e = cudaMemsetAsync(s.E, 0, 3 * sz * sizeof(int), st);
-  if (e == cudaSuccess && half) e = cudaMemsetAsync(s.Mx, 0, 2 * sz * sizeof(unsigned), st);
+  if (e == cudaSuccess && half) e = cudaMemsetAsync(s.Mx, 0, 4 * sz * sizeof(unsigned), st);
   if (e == cudaSuccess) e = cudaStreamSynchronize(st);
   cudaFree(raw);
   raw = nullptr;
@@ -2213,7 +2213,7 @@ extern "C" int FLETCHER_BatchAddShot(int sx, int sy, int sz, const float *model,
                  B.shots.size(), kModelNames[bad % 8], bad / 8);
   }
   B.dev_bytes += 2 * fbytes + coef_floats(sy, sz, s.pitch) * sizeof(float);
-  if (half) B.dev_bytes += (ext ? 2 * s.npitch * sizeof(unsigned short) : 0) + 5 * sz * sizeof(int);
+  if (half) B.dev_bytes += (ext ? 2 * s.npitch * sizeof(unsigned short) : 0) + 7 * sz * sizeof(int);
   if (s.n > B.max_n) {
     if (B.scratch) cudaFree(B.scratch);
     B.scratch = nullptr;
@@ -2237,7 +2237,7 @@ extern "C" int FLETCHER_BatchReset(void) {
       if (s.Hl[b]) CK(cudaMemsetAsync(s.Hl[b], 0, s.npitch * sizeof(unsigned short), g_stream));
     }
     if (s.E) CK(cudaMemsetAsync(s.E, 0, 3 * s.sz * sizeof(int), g_stream));
-    if (s.Mx) CK(cudaMemsetAsync(s.Mx, 0, 2 * s.sz * sizeof(unsigned), g_stream));
+    if (s.Mx) CK(cudaMemsetAsync(s.Mx, 0, 4 * s.sz * sizeof(unsigned), g_stream));
   }
   CK(cudaStreamSynchronize(g_stream));
   return FLETCHER_OK;

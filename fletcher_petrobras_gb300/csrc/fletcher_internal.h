@@ -172,7 +172,8 @@ struct HalfShot {
   unsigned *hi[2];        // the two field buffers: (p, q) as half2 per cell
   unsigned short *lo[2];  // their residual bytes (extended form; null otherwise)
   int *E;                 // [3][sz] per-plane exponents; the field of step it uses slot it % 3
-  unsigned *Mx;           // [2][sz] per-plane max |value| (float bits) of the field in buffer b
+  unsigned *Mx;           // per-plane max |value| (float bits): persistent steps [2][sz], of the field in
+                          //   buffer b; chained steps [4][sz], of the field of step it in slot it % 4
 };
 
 // A batched shot's tensor maps, by the buffer that holds the current field.
@@ -184,8 +185,13 @@ struct HalfParams {
   PropParams p;                       // geometry (p.one), spacing, source, error word
   unsigned *out_hi;                   // new field: half2 per cell
   unsigned short *out_lo;             // new field: residual bytes (extended form)
-  const int *e_cur, *e_prev, *e_new;  // per-plane exponents of the current, previous and new field
-  unsigned *m_new;                    // per-plane max |value| of the new field (float bits), atomicMax
+  const int *e_cur, *e_prev;          // per-plane exponents of the current and previous field
+  int *e_new;                         // those of the new field (FP16X: set by the step itself)
+  // Per-plane max |value| (float bits) of the current and previous field, of
+  // the new one (atomicMax, cleared by the step before), and the slot this
+  // step clears for the next.
+  const unsigned *m_cur, *m_prev;
+  unsigned *m_new, *m_clear;
   // Batched launches (p.shots): per-shot buffers and maps, and the
   // exponent slot of the current field (step % 3).
   const HalfShot *hshots;
@@ -201,12 +207,12 @@ struct HalfLaunch {
 };
 
 bool propagate_half_supported(int tile_rows, int stages);
+// One 16-bit step; FP16 single shots: preceded by the launch that sets the new
+// planes' exponents (in batches half_scales_batch does).
 cudaError_t propagate_half_launch(const HalfLaunch &L, bool ext, cudaStream_t s);
 cudaError_t propagate_half_prepare(int tile_rows, int stages, bool ext, bool batch);
-cudaError_t half_scales(const unsigned *m_cur, unsigned *m_prev, int *e_new, int sz, int src_z, float src_abs,
-                        cudaStream_t s);
 // Before a batched 16-bit step: the new field's plane exponents and the
-// cleared maxima (as half_scales) of the first `active` shots of `order`,
+// cleared maxima of the first `active` shots of `order`,
 // block i taking shot order[i]; the current field is in buffer c, its
 // exponents in slot ecur.
 cudaError_t half_scales_batch(const HalfShot *hs, const ShotDesc *sd, const int *order, int active, int c, int ecur,

@@ -3,10 +3,11 @@
 //
 // Storage of one field buffer: (p, q) as a half2 per cell, [z][y][pitch],
 // with one power-of-two scale per z-plane: stored = value * 2^e[z].  The
-// scale of every new plane is set before the step (k_half_scales) from the
-// largest magnitudes of the current field within 4 planes and of the
-// previous field at that plane, so the new values stay below 2^14 (2^16 is
-// FP16's limit) and far above its subnormal range.
+// scale of every new plane comes from the largest magnitudes of the current
+// field within 4 planes and of the previous field at that plane, so the new
+// values stay below 2^14 (2^16 is FP16's limit) and far above its subnormal
+// range.  The FP16X single-shot step sets it itself, plane by plane; the others
+// have it set by a small launch before the step.
 //
 // The extended form (EXT) adds one signed byte per value: the rounding error
 // of the half in units of 2^-8 of the half's last place, i.e. a 19-bit
@@ -78,13 +79,14 @@ struct LayoutH {
   static constexpr int OFF_SAB = G::STAGE_B;
   static constexpr int OFF_CTL = OFF_SAB + (AB_IN ? AB_SLOT : 0);
   static constexpr int OFF_HDR = OFF_CTL;         // the item that starts in the stage
-  static constexpr int OFF_SCALE = OFF_CTL + 16;  // 2^-e of the previous and 2^e of the new plane of the step
-  static constexpr int OFF_FULL = OFF_CTL + 24;   // barriers: loads landed,
-  static constexpr int OFF_READY = OFF_CTL + 32;  //   FP32 tile and scales written,
-  static constexpr int OFF_HALO = OFF_CTL + 40;   //   halo columns written,
-  static constexpr int OFF_EMPTY = OFF_CTL + 48;  //   released by every reader
-  static constexpr int OFF_PLANE = OFF_CTL + 56;  // the new plane (-1: none) and its shot (producer only)
-  static constexpr int OFF_MAX = OFF_CTL + 64;    // the CTA's largest magnitude on the new plane
+  static constexpr int OFF_SCALE = OFF_CTL + 16;  // 2^-e of the arriving plane and of the previous field's
+                                                  //   plane of the step, 2^e of the new one
+  static constexpr int OFF_FULL = OFF_CTL + 32;   // barriers: loads landed,
+  static constexpr int OFF_READY = OFF_CTL + 40;  //   FP32 tile written,
+  static constexpr int OFF_HALO = OFF_CTL + 48;   //   halo columns written,
+  static constexpr int OFF_EMPTY = OFF_CTL + 56;  //   released by every reader
+  static constexpr int OFF_PLANE = OFF_CTL + 64;  // the new plane (-1: none) and its shot (producer only)
+  static constexpr int OFF_MAX = OFF_CTL + 72;    // the CTA's largest magnitude on the new plane
   static constexpr int SB = OFF_CTL + 128;
   static constexpr int TILE_B = G::H32_B + G::ROW_B;  // decoded tile, exchange rows
   static constexpr int OFF_TILES = S * SB;
@@ -182,6 +184,19 @@ __device__ __forceinline__ HItem decode_hitem(int4 w) {
   return it;
 }
 
+// The exponent of a plane of the new field from its largest possible
+// magnitude: 4 x the current field's largest magnitude within 4 planes (m_cur,
+// float bits), plus the previous field's at that plane, plus 4 x the sources
+// near the source plane.
+__device__ __forceinline__ int plane_exponent(unsigned m_cur, unsigned m_prev, float src_abs) {
+  float b = 4.0f * __uint_as_float(m_cur) + __uint_as_float(m_prev);
+  b += 4.0f * src_abs;
+  if (!(b > 0.0f)) return 0;
+  int ex;
+  frexpf(b, &ex);  // b < 2^ex
+  return min(max(14 - ex, -100), 100);
+}
+
 // Fetches a step's tensor maps into the descriptor cache (the residual
 // maps exist in the extended form only).
 template <bool EXT>
@@ -220,6 +235,15 @@ __device__ __forceinline__ void issue_half(unsigned char *stage, uint64_t *bar, 
   }
 }
 
+// Whether the step sets the new field's plane exponents itself: the FP16X
+// single-shot step, on the producer's warp, ahead of the loads.  Instead of a
+// launch before each step (k_half_scales): 128^3 + shell 102.1 -> 98.3 us a
+// step, 205 x 129 x 173 82.4 -> 78.5, 56^3 + shell 19.4 -> 18.0, 272^3 279.6 ->
+// 274.3.  In FP16, whose stages turn over faster, the slower producer costs
+// more than the launch (298 x 249 x 215 190 -> 202 us; on a decode warp
+// 236), and in batches the shots' pointers spill (6 shots of 158^3 381 -> 639).
+__host__ __device__ constexpr bool own_scales(bool ext, bool batch) { return ext && !batch; }
+
 // BATCH: the items belong to the shots of a batch (P.shots, H.hshots,
 // H.hmaps: buffers, exponents and tensor maps by shot).
 template <int TY, int S, bool ISO, bool EXT, bool BATCH>
@@ -228,11 +252,12 @@ __global__ void __launch_bounds__(RegsH<TY, EXT>::kThreads, 1)
   using G = GeoH<TY, EXT>;
   using L = LayoutH<TY, S, EXT>;
   constexpr int kDecodeWarps = RegsH<TY, EXT>::kDecode;
+  constexpr bool OWN_SCALES = own_scales(EXT, BATCH);
   const PropParams &P = H.p;
   extern __shared__ unsigned char smem_dyn[];
   unsigned char *smem = smem_dyn + ((128u - (smem_addr(smem_dyn) & 127u)) & 127u);
   auto bar = [&](unsigned char *st, int off) { return reinterpret_cast<uint64_t *>(st + off); };
-  auto scale_of = [&](unsigned char *st) { return reinterpret_cast<float2 *>(st + L::OFF_SCALE); };
+  auto scale_of = [&](unsigned char *st) { return reinterpret_cast<float4 *>(st + L::OFF_SCALE); };
   auto max_of = [&](unsigned char *st) { return reinterpret_cast<unsigned *>(st + L::OFF_MAX); };
   auto plane_of = [&](unsigned char *st) { return reinterpret_cast<int2 *>(st + L::OFF_PLANE); };
 
@@ -263,14 +288,25 @@ __global__ void __launch_bounds__(RegsH<TY, EXT>::kThreads, 1)
     uint32_t phase = 0;
     if (wid == TY) {
       // ---- producer ----
-      if (lx != 0) return;
+      // (One thread, or with OWN_SCALES its warp: lane 0 issues and stores.)
+      if (!OWN_SCALES && lx != 0) return;
       auto maps_of = [&](int shot) -> const HalfMaps & {
         if constexpr (BATCH) return H.hmaps[shot].m[P.parity];
         else return M;
       };
-      int issued = 0;
-      bool ok = true;
-      // The CTA's maximum on the plane whose step held stage s (every warp
+      // What the scales of step k of an item need, by lane, loaded a step ahead:
+      // lanes 0..8 the current field's maxima within 4 planes of the plane
+      // updated, lane 9 the previous field's, lanes 10 and 11 the exponents of
+      // the previous field's plane and of the arriving one.
+      auto load_scales = [&](const HItem &it, int k) -> unsigned {
+        const int zc = k - kRadius;
+        if (lx == 11) return (unsigned)H.e_cur[k];
+        if (zc < it.z0) return 0u;
+        if (lx == 10) return (unsigned)H.e_prev[zc];
+        if (lx == 9) return H.m_prev[zc];
+        return lx < 9 ? H.m_cur[zc - kRadius + lx] : 0u;
+      };
+      // The CTA's maximum on the plane whose step held a stage (every warp
       // has released it) goes to the plane's global maximum.
       auto take_max = [&](unsigned char *st) {
         const unsigned v = *max_of(st);
@@ -284,45 +320,81 @@ __global__ void __launch_bounds__(RegsH<TY, EXT>::kThreads, 1)
         // Beyond FP16's range: the scale bound was exceeded.
         if (!(__fmul_rn(__uint_as_float(v), sc) < 65504.0f)) atomicOr(P.err, 4u);
       };
-      int4 next = seg[0];
-      prefetch_maps<EXT>(maps_of(decode_hitem<BATCH>(next).shot));
-      for (int i = 0; i < nitems && ok; ++i) {
-        const int4 w = next;
-        const HItem it = decode_hitem<BATCH>(w);
-        if (i + 1 < nitems) {
-          next = seg[i + 1];
-          // Batched shots keep their tensor maps in global memory: fetch the
-          // next item's into the descriptor cache an item ahead.
-          if constexpr (BATCH) prefetch_maps<EXT>(maps_of(decode_hitem<BATCH>(next).shot));
+      int4 w = seg[0], next = nitems > 1 ? seg[1] : w;
+      HItem it = decode_hitem<BATCH>(w);
+      int k = it.z0 - kRadius, i = 0, issued = 0;
+      unsigned sv = 0u;
+      if constexpr (OWN_SCALES) sv = load_scales(it, k);
+      if (lx == 0) prefetch_maps<EXT>(maps_of(it.shot));
+      bool ok = true;
+      while (i < nitems) {
+        // The step's scales, then the next step's loads, before the wait: the
+        // issue must follow the stage's release at once.
+        const HItem cit = it;
+        const int4 cw = w;
+        const int ck = k, zc = k - kRadius;
+        const bool upd = zc >= it.z0;
+        int en = 0;
+        float4 scl;
+        if constexpr (OWN_SCALES) {
+          const ShotDesc &sd = P.one;
+          const int zs = sd.src_z >= 0 ? sd.src_z : sd.cor_z;
+          const int ec = (int)__shfl_sync(0xffffffffu, sv, 11), ep = (int)__shfl_sync(0xffffffffu, sv, 10);
+          en = plane_exponent(__reduce_max_sync(0xffffffffu, lx < 9 && sv <= 0x7f800000u ? sv : 0u),
+                              __shfl_sync(0xffffffffu, sv, 9),
+                              abs(zc - zs) <= kRadius ? fabsf(P.src) + fabsf(P.cor) : 0.0f);
+          scl = make_float4(exp2i(-ec), exp2i(-ep), exp2i(en), 0.0f);
         }
-        for (int k = it.z0 - kRadius; k < it.z1 + kRadius; ++k) {
-          // (The first S waits pass at once: the stage was never filled.)
-          unsigned char *st = smem + stage * L::SB;
-          if (!mbar_spin(bar(st, L::OFF_EMPTY), phase ^ 1u)) {
-            ok = false;
-            break;
+        if (++k >= it.z1 + kRadius && ++i < nitems) {
+          w = next;
+          it = decode_hitem<BATCH>(w);
+          k = it.z0 - kRadius;
+          if (i + 1 < nitems) {
+            next = seg[i + 1];
+            // Batched shots keep their tensor maps in global memory: fetch the
+            // next item's into the descriptor cache an item ahead.
+            if constexpr (BATCH) prefetch_maps<EXT>(maps_of(decode_hitem<BATCH>(next).shot));
           }
+        }
+        if constexpr (OWN_SCALES) {
+          if (i < nitems) sv = load_scales(it, k);
+        }
+        unsigned char *st = smem + stage * L::SB;
+        // (The first S waits pass at once: the stage was never filled.)
+        if (!mbar_spin(bar(st, L::OFF_EMPTY), phase ^ 1u)) {
+          ok = false;
+          break;
+        }
+        if (lx == 0) {
           const int2 pl = issued >= S ? *plane_of(st) : make_int2(-1, 0);
-          const float sc = scale_of(st)->y;
+          const float sc = scale_of(st)->z;
           const unsigned v = take_max(st);
           fence_proxy_async_smem();
-          if (k == it.z0 - kRadius) *reinterpret_cast<int4 *>(st + L::OFF_HDR) = w;
-          *plane_of(st) = make_int2(k - kRadius >= it.z0 ? k - kRadius : -1, it.shot);
-          issue_half<TY, EXT>(st, bar(st, L::OFF_FULL), it, k, maps_of(it.shot));
-          ++issued;
-          if (++stage == S) {
-            stage = 0;
-            phase ^= 1u;
-          }
+          if (ck == cit.z0 - kRadius) *reinterpret_cast<int4 *>(st + L::OFF_HDR) = cw;
+          *plane_of(st) = make_int2(upd ? zc : -1, cit.shot);
+          if constexpr (OWN_SCALES) *scale_of(st) = scl;
+          issue_half<TY, EXT>(st, bar(st, L::OFF_FULL), cit, ck, maps_of(cit.shot));
           fold_max(pl, sc, v);
+          if (OWN_SCALES && upd) {
+            // Every CTA of the plane finds and stores the same.
+            H.e_new[zc] = en;
+            H.m_clear[zc] = 0u;
+          }
+        }
+        if constexpr (OWN_SCALES) __syncwarp();
+        ++issued;
+        if (++stage == S) {
+          stage = 0;
+          phase ^= 1u;
         }
       }
+      if (lx != 0) return;
       // The maxima of the last steps, in order.
       for (int a = issued < S ? issued : S; a >= 1 && ok; --a) {
         const int s2 = stage >= a ? stage - a : stage + S - a;
         unsigned char *st = smem + s2 * L::SB;
         if (!mbar_spin(bar(st, L::OFF_EMPTY), stage >= a ? phase : phase ^ 1u)) ok = false;
-        else fold_max(*plane_of(st), scale_of(st)->y, take_max(st));
+        else fold_max(*plane_of(st), scale_of(st)->z, take_max(st));
       }
       if (!ok) {
         // A bounded wait gave up: wait, bounded, for the loads still in
@@ -345,24 +417,21 @@ __global__ void __launch_bounds__(RegsH<TY, EXT>::kThreads, 1)
     for (int i = 0; i < nitems; ++i) {
       const HItem it = decode_hitem<BATCH>(seg[i]);
       const ShotDesc &sd = BATCH ? P.shots[it.shot] : P.one;
-      const int *e_cur, *e_prev, *e_new;
+      const int src_z = sd.src_z;
+      const int kend = it.z1 + kRadius;
+      const int *e_cur = H.e_cur, *e_prev = H.e_prev, *e_new = H.e_new;
       if constexpr (BATCH) {
         const int *E = H.hshots[it.shot].E;
         e_cur = E + (H.ecur % 3) * sd.sz;
         e_new = E + ((H.ecur + 1) % 3) * sd.sz;
         e_prev = E + ((H.ecur + 2) % 3) * sd.sz;
-      } else {
-        e_cur = H.e_cur;
-        e_new = H.e_new;
-        e_prev = H.e_prev;
       }
-      const int src_z = sd.src_z;
-      const int kend = it.z1 + kRadius;
-      int ec = e_cur[it.z0 - kRadius], ep = 0, en = 0;  // exponents of this step's planes, loaded a step ahead
+      // Exponents of this step's planes, loaded a step ahead.
+      int ec = OWN_SCALES ? 0 : e_cur[it.z0 - kRadius], ep = 0, en = 0;
       for (int k = it.z0 - kRadius; k < kend; ++k) {
-        const float inv = exp2i(-ec);
-        const float2 ps = make_float2(exp2i(-ep), exp2i(en));
-        if (k + 1 < kend) {
+        float inv = exp2i(-ec);
+        const float4 ps = make_float4(inv, exp2i(-ep), exp2i(en), 0.0f);
+        if (!OWN_SCALES && k + 1 < kend) {
           ec = e_cur[k + 1];
           if (k + 1 - kRadius >= it.z0) {
             ep = e_prev[k + 1 - kRadius];
@@ -379,6 +448,7 @@ __global__ void __launch_bounds__(RegsH<TY, EXT>::kThreads, 1)
           return;
         }
         f2 *Hs = reinterpret_cast<f2 *>(smem + L::OFF_TILES + ds * L::TILE_B);
+        if constexpr (OWN_SCALES) inv = scale_of(st)->x;
         // Decode once per cell, two cells per thread (one 64-bit load of two
         // half2 cells, one 128-bit store of their FP32 pairs).  The source
         // cell then gains the step's source
@@ -405,7 +475,7 @@ __global__ void __launch_bounds__(RegsH<TY, EXT>::kThreads, 1)
             if (dt == (src_c >> 1) % NDT) Hs[src_c] = add2(Hs[src_c], splat(P.src));
           }
         }
-        if (dt == 0) *scale_of(st) = ps;
+        if (!OWN_SCALES && dt == 0) *scale_of(st) = ps;
         __syncwarp();
         if (lx == 0) mbar_arrive(bar(st, L::OFF_READY));
         if (k >= it.z0 && k < it.z1) {
@@ -554,14 +624,14 @@ __global__ void __launch_bounds__(RegsH<TY, EXT>::kThreads, 1)
           const unsigned phv = reinterpret_cast<const unsigned *>(st + G::OFF_PHI)[ci];
           unsigned short prv = 0;
           if constexpr (EXT) prv = reinterpret_cast<const unsigned short *>(st + G::OFF_PLO)[ly * G::HX + lx + kRadius];
-          const float2 sc = *scale_of(st);  // 2^-e of the previous field, 2^e of the new one
-          f2 old = decode<EXT>(phv, prv, sc.x);
+          const float4 sc = *scale_of(st);
+          f2 old = decode<EXT>(phv, prv, sc.y);
           if (k == cor_k) old = add2(old, splat(P.cor));
           const f2 curv = Pr[cs];
           const f2 nw = fma2(mk2(rhsp, rhsq), splat(P.dt2), sub2(add2(curv, curv), old));
           unsigned ohv;
           unsigned short orv;
-          encode<EXT>(nw, sc.y, ohv, orv);
+          encode<EXT>(nw, sc.z, ohv, orv);
           if (valid) {
             out_hi[o] = ohv;
             if constexpr (EXT) out_lo[o] = orv;
@@ -603,13 +673,10 @@ __global__ void __launch_bounds__(RegsH<TY, EXT>::kThreads, 1)
   }
 }
 
-// Before each step: the exponent of every plane of the new field (its
-// largest possible magnitude: 4 x the current field's largest magnitude
-// within 4 planes, plus the previous field's at that plane, plus the sources
-// near the source plane), and the previous field's maxima, consumed here, are
-// cleared for the new field's.
-__global__ void k_half_scales(const unsigned *__restrict__ m_cur, unsigned *__restrict__ m_prev, int *__restrict__ e_new,
-                              int sz, int src_z, float src_abs) {
+// Before a single-shot step that does not set its own scales: the exponent of
+// every plane of the new field, whose maxima are cleared.
+__global__ void k_half_scales(const unsigned *m_cur, const unsigned *m_prev, unsigned *m_new, int *e_new, int sz,
+                              int src_z, float src_abs) {
   const int z = blockIdx.x * blockDim.x + threadIdx.x;
   allow_next_launch();
   wait_previous_launch();
@@ -617,16 +684,8 @@ __global__ void k_half_scales(const unsigned *__restrict__ m_cur, unsigned *__re
   float b = 0.0f;
   for (int dz = -kRadius; dz <= kRadius; ++dz)
     if (z + dz >= 0 && z + dz < sz) b = fmaxf(b, __uint_as_float(m_cur[z + dz]));
-  b = 4.0f * b + __uint_as_float(m_prev[z]);
-  if (abs(z - src_z) <= kRadius) b += 4.0f * src_abs;
-  int e = 0;
-  if (b > 0.0f) {
-    int ex;
-    frexpf(b, &ex);  // b < 2^ex
-    e = min(max(14 - ex, -100), 100);
-  }
-  e_new[z] = e;
-  m_prev[z] = 0u;
+  e_new[z] = plane_exponent(__float_as_uint(b), m_prev[z], abs(z - src_z) <= kRadius ? src_abs : 0.0f);
+  m_new[z] = 0u;
 }
 
 // Plane z (= blockIdx.x) of float (p, q) volumes -> stored form, the scale
@@ -725,6 +784,13 @@ bool propagate_half_supported(int tile_rows, int stages) {
 }
 
 cudaError_t propagate_half_launch(const HalfLaunch &L, bool ext, cudaStream_t s) {
+  if (!L.batch && !own_scales(ext, false)) {
+    const ShotDesc &d = L.h.p.one;
+    const cudaError_t e =
+        launch_step(k_half_scales, (d.sz + 127) / 128, 128, 0, s, L.h.m_cur, L.h.m_prev, L.h.m_new, L.h.e_new, d.sz,
+                    d.src_z >= 0 ? d.src_z : d.cor_z, fabsf(L.h.p.src) + fabsf(L.h.p.cor));
+    if (e != cudaSuccess) return e;
+  }
   // The work description the chosen kernel reads must be present.
   if (!L.h.p.seg || !L.h.p.cta_first ||
       (L.batch ? (!L.h.p.shots || !L.h.hshots || !L.h.hmaps) : (!L.h.out_hi || !L.h.e_cur)))
@@ -748,13 +814,10 @@ cudaError_t propagate_half_prepare(int tile_rows, int stages, bool ext, bool bat
   return cudaErrorInvalidValue;
 }
 
-cudaError_t half_scales(const unsigned *m_cur, unsigned *m_prev, int *e_new, int sz, int src_z, float src_abs,
-                        cudaStream_t s) {
-  return launch_step(k_half_scales, (sz + 127) / 128, 128, 0, s, m_cur, m_prev, e_new, sz, src_z, src_abs);
-}
-
-// The same for every running shot of a batch (block i: shot order[i]); the
-// current field is in buffer c and uses exponent slot ecur.
+// Before each persistent step of a batch: the exponent of every plane of
+// every running shot's new field (block i: shot order[i]); the previous
+// field's maxima, consumed here, are cleared for the new field's.  The current
+// field is in buffer c and uses exponent slot ecur.
 __global__ void k_half_scales_batch(const HalfShot *__restrict__ hs, const ShotDesc *__restrict__ sd,
                                     const int *__restrict__ order, int c, int ecur, float src_abs) {
   allow_next_launch();
@@ -768,15 +831,7 @@ __global__ void k_half_scales_batch(const HalfShot *__restrict__ hs, const ShotD
     float b = 0.0f;
     for (int dz = -kRadius; dz <= kRadius; ++dz)
       if (z + dz >= 0 && z + dz < sz) b = fmaxf(b, __uint_as_float(m_cur[z + dz]));
-    b = 4.0f * b + __uint_as_float(m_prev[z]);
-    if (abs(z - src_z) <= kRadius) b += 4.0f * src_abs;
-    int e = 0;
-    if (b > 0.0f) {
-      int ex;
-      frexpf(b, &ex);
-      e = min(max(14 - ex, -100), 100);
-    }
-    e_new[z] = e;
+    e_new[z] = plane_exponent(__float_as_uint(b), m_prev[z], abs(z - src_z) <= kRadius ? src_abs : 0.0f);
     m_prev[z] = 0u;
   }
 }

@@ -333,8 +333,8 @@ int FLETCHER_BatchSetTileConfig(int tile_rows, int stages);
  *   each running its shots one after another (one graph when captured).
  *   A launch waits on no other kernel, so kernels of different chains
  *   share the GPU where one leaves SMs idle, and each chain works on one
- *   shot's memory at a time.  In the 16-bit forms each step is the
- *   single-shot pair of launches (the new planes' scales, then the step).
+ *   shot's memory at a time.  In FP16 each step is the single-shot pair of
+ *   launches (the new planes' scales, then the step), in FP16X one launch.
  * Results are bit-identical in every schedule. */
 int FLETCHER_BatchSetChains(int chains);
 /* The schedule of the last FLETCHER_BatchRun: 0 (persistent launch) or the
