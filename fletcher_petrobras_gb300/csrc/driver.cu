@@ -1900,18 +1900,27 @@ int batch_single_plans(int ctas) {
   return FLETCHER_OK;
 }
 
-// The schedule of an FP32 batch left to the library: one chain when most of
-// its work (updated cells x steps) is in shots that fill the GPU on their
-// own, else the persistent multi-shot launch.
+// The schedule of a batch left to the library: chains when most of its work
+// (updated cells x steps) is in shots that fill the GPU on their own, else the
+// persistent multi-shot launch.  Two chains where there are two such shots or
+// more, of at most kTwoChainCells on average: one shot's launches fill the SMs
+// that the other's last CTAs leave idle.  The launches of larger ones have
+// little to fill, and two at a time only divide the memory's bandwidth.
 int batch_auto_chains(int steps) {
-  double fill = 0.0, total = 0.0;
+  double fill = 0.0, total = 0.0, fill_cells = 0.0;
+  int nfill = 0;
   for (const BatchShot &s : B.shots) {
     const double cells = (double)(s.sx - 2 * B.bord) * (s.sy - 2 * B.bord) * (s.sz - 2 * B.bord);
     const double work = cells * std::min(s.nsteps, steps);
     total += work;
-    if (cells >= kChainFillCells) fill += work;
+    if (cells >= kChainFillCells) {
+      fill += work;
+      fill_cells += cells;
+      ++nfill;
+    }
   }
-  return 2.0 * fill >= total ? 1 : 0;
+  if (2.0 * fill < total) return 0;
+  return nfill > 1 && fill_cells <= kTwoChainCells * nfill ? 2 : 1;
 }
 
 int batch_max_steps() {

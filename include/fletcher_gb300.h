@@ -319,14 +319,14 @@ int FLETCHER_BatchAddShot(int sx, int sy, int sz, const float *model, long iSour
 /* Tile shape for the next FLETCHER_BatchRun (0 = default). */
 int FLETCHER_BatchSetTileConfig(int tile_rows, int stages);
 /* Schedule of a batch's run, after FLETCHER_BatchCreate.
- * chains = -1 (default): one chain when most of the batch's work (updated
- *   cells x steps) is in shots of at least 2.1 M updated cells, which fill
- *   the GPU on their own, else the persistent launch (measured on GB300: 48
- *   shots of 168^3-392^3 ran 7% faster on one chain than on the persistent
- *   launch; 48 shots of 56^3 and 32 of 80^3 ran 6-7% slower).
+ * chains = -1 (default): chains when most of the batch's work (updated cells
+ *   x steps) is in shots of at least 2.1 M updated cells, which fill the GPU
+ *   on their own (two chains where there are two such shots or more, of at
+ *   most 20 M updated cells on average, else one), and the persistent launch
+ *   otherwise.
  * chains = 0: one persistent launch per time step advances every running
- *   shot (FP32: the shots' single-shot plans stacked per CTA; 16-bit forms:
- *   the plane-scale launch of every running shot first).
+ *   shot (large shots' single-shot plans stacked per CTA, small shots pooled;
+ *   16-bit forms: the plane-scale launch of every running shot first).
  * chains = 1 .. 8: every step of a shot is its own single-shot launch; the
  *   shots are dealt, longest run first, each to the stream with the least
  *   work so far, over `chains` concurrent streams,
