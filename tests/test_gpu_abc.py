@@ -78,6 +78,28 @@ def test_inference_path_vs_cpu_oracle():
     assert rel(y, oy) < 1e-2
 
 
+@pytest.mark.parametrize("n", [1, 15, 16, 17, 63, 64, 65, 129])
+def test_network_batch_edges_vs_cpu_oracle(n):
+    """Loss, gradient and outputs where a training block of 64 samples and an
+    inference tile of 16 rows begin and end.  In so few samples an FP16
+    rounding that falls the other way is not averaged out: it changes one of
+    a sample's 32 activations by 2^-11 of itself, so loss and gradient are
+    held to 2^-10."""
+    from oracle import abc_mlp
+
+    learned.init(6)
+    P = learned.get_weights()
+    X = random_features(n, 11 + n)
+    T = np.random.default_rng(12 + n).normal(0, 1, (n, 4)).astype(np.float32)
+    loss, g = learned.gradient(X, T)
+    oloss, og = abc_mlp.loss_and_grad(P, X, T)
+    assert abs(loss - oloss) <= 2.0 ** -10 * oloss
+    assert rel(g, og) < 2.0 ** -10
+    y = learned.forward(X)
+    oy, _ = abc_mlp.forward(P, X)
+    assert np.max(np.abs(y - oy)) < 3e-2 * np.sqrt(np.mean(oy ** 2))
+
+
 def test_collected_samples_vs_cpu_restatement():
     from oracle import abc_mlp
 
