@@ -205,6 +205,79 @@ def test_resident_oneway_steps_vs_cpu_oracle():
     assert np.array_equal(got[:, ~mask], plain.reshape((2,) + shape)[:, ~mask])
 
 
+def _ghost_update(cur, prev, base, c4, prob, weights):
+    """The oracle's features, network and box-scheme update (the medium's
+    coefficients where weights is None), a slab of one distance at a time."""
+    from oracle import abc_mlp
+
+    b, L = prob.bord, learned.LAYER
+    dims = (prob.sx, prob.sy, prob.sz)
+    h = (prob.dx, prob.dy, prob.dz)
+    nxt = base.astype(np.float64)
+    vpz = np.sqrt(c4[7])
+    eps, delta = (np.float32(0.5) * (c4[k] / c4[7] - np.float32(1)) for k in (6, 9))
+    for f in range(6):
+        a, sgn = abc_mlp.face_axis(f), abc_mlp.face_sign(f)
+
+        def slab(F, d):  # the kept box's cells at distance d outward
+            n = b + L - d if sgn < 0 else dims[a] - b - L - 1 + d
+            ix = [slice(b, dims[t] - b) for t in (2, 1, 0)]
+            ix[2 - a] = n
+            return F[(Ellipsis, *ix)]
+
+        for d in range(L - 3, L + 1):
+            g = slab(cur, d)
+            if weights is None:
+                c = slab(vpz, d) if a == 2 else slab(vpz, d) * np.sqrt(np.float32(1) + np.float32(2) * slab(eps, d))
+                r = c * np.float32(prob.dt) / np.float32(h[a])
+                k = np.broadcast_to((1 - r) / (1 + r), g.shape)
+            else:
+                st = [slab(F, d + o)[c] if d + o <= L else np.zeros(g.shape[1:])
+                      for F in (cur, prev) for c in (0, 1) for o in range(-4, 5)]
+                st = np.stack(st, -1).reshape(-1, 36)
+                s = np.abs(st).max(1, keepdims=True)
+                X = np.concatenate([st / s] + [np.reshape(np.broadcast_to(m, g.shape[1:]), (-1, 1)) for m in (
+                    slab(vpz, d) / 4000.0, slab(eps, d), slab(delta, d), d / L)], 1)
+                y, _ = abc_mlp.forward(weights, X)
+                k = abc_mlp.sigmoid(y).T.reshape(g.shape)
+            slab(nxt, d)[...] = slab(cur, d - 1) + k * (g - slab(nxt, d - 1))
+    return nxt
+
+
+@pytest.mark.parametrize("n", [(1, 1, 1), (3, 30, 7), (95, 91, 2), (2, 290, 281)])
+def test_ghost_update_on_ragged_boxes(n):
+    """The boundary kernels where a face's rays are no multiple of a warp's
+    group and where a pass takes one round of the grid or several (16 200
+    rays for the network kernel, 150 000 for the other), against the oracle's
+    update of the plain step; the network's bound as in the test above."""
+    b, L = 4, learned.LAYER
+    prob = learned.Problem("ghost", *n, absorb=L, bord=b, dt=0.0006, steps=1, kind="layered", layers=3, seed=5)
+    shape = (prob.sz, prob.sy, prob.sx)
+    g = np.random.default_rng(sum(n))
+    f = []
+    for _ in range(4):  # pp pc qp qc
+        v = np.zeros(shape, np.float32)
+        v[b:-b, b:-b, b:-b] = g.uniform(-1, 1, tuple(s - 2 * b for s in shape))
+        f.append(v.ravel())
+    model = prob.raw_model()
+    learned.init(6)
+    plain, _ = _one_step(prob, model, f, learned.BOUNDARY_PLAIN)
+    prop = Propagator()
+    prop.initialize(prob.sx, prob.sy, prob.sz, b, prob.dx, prob.dy, prob.dz, prob.dt, model)
+    c4 = prop.coefficients().reshape((10,) + shape)
+    prop.finalize()
+    cur = np.stack([f[1], f[3]]).reshape((2,) + shape).astype(np.float64)
+    prev = np.stack([f[0], f[2]]).reshape((2,) + shape).astype(np.float64)
+    base = plain.reshape((2,) + shape)
+    for mode, weights in ((learned.BOUNDARY_ONEWAY, None), (learned.BOUNDARY_LEARNED, learned.get_weights())):
+        got, _ = _one_step(prob, model, f, mode)
+        want = _ghost_update(cur, prev, base, c4, prob, weights)
+        size = np.max(np.abs(want - base))
+        # Fixed: four cells' FP32 rounding and that of k, 3 ulp of up to 5 / 4 of size each.
+        tol = (2e-6 if weights is None else 1e-2) * size
+        assert np.max(np.abs(got.reshape(want.shape) - want)) < tol
+
+
 def test_training_and_reflected_energy_small():
     """What the trained network gains over the method without it.  Training on
     32 padded models (the library's kernels, reproducible), then the
