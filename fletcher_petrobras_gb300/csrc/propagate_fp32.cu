@@ -16,30 +16,33 @@
 //  * the halo warps (three helper warps) evaluate D1y in the tile's 8 halo
 //    columns, ahead of the compute warps, and add the step's source to the
 //    tile of the plane that holds it;
-//  * TY compute warps: each thread owns one (x, y) column.  When plane k
-//    arrives it reads its 9-point x and y neighbourhoods from shared memory
-//    and forms Der2x, Der2y and the first derivatives D1x, D1y; DerCross xy
-//    is D1x applied to D1y, whose row of the tile only this warp and the
+//  * TY / 2 compute warps, each two rows: a thread owns the columns of two
+//    cells that lie side by side in x.  When plane k arrives it reads its 9-point
+//    x and y neighbourhoods from shared memory, 16 bytes at a time, and forms
+//    Der2x, Der2y and the first derivatives D1x, D1y; DerCross xy
+//    is D1x applied to D1y, whose rows of the tile only this warp and the
 //    halo columns write (so compute warps never wait for one another);
 //    DerCross xz and yz are the z first derivative of the D1x / D1y values,
 //    which each thread keeps for 9 planes in registers, as it keeps p and q
 //    for Der2z; the in-plane terms A and B wait in shared memory;
 //  * both fields travel as one 64-bit (p, q) pair and are updated with the
 //    packed .f32x2 add/mul/fma instructions;
-//  * plane k-4 is completed at step k and written with coalesced 64-bit
+//  * plane k-4 is completed at step k and written with coalesced 128-bit
 //    stores into the previous-field buffer (in place).
 //
-// What bounds it: HBM and the shared-memory pipe, about equally.  At 504^3
-// (183 M updated cells, 64 B each) a step takes 1.79 to 1.81 ms, 96% of the
-// measured copy bandwidth; a plane of a tile costs an SM about 1500 cycles of
-// shared-memory wavefronts (38 loads and stores a warp, the TMA writes), 0.73
-// us, which is what it takes there.  Before the warps were specialised, 16
-// warps that exchanged D1y, and refilled the stages, in one CTA-wide exchange
-// a plane took 2.22 ms.  What made the difference:
+// What bounds it: HBM where the grid is large, elsewhere the latency of a warp's
+// plane (two or three warps a scheduler: half of its issue slots and 45 to 70%
+// of the shared-memory pipe are used).  At 504^3 (183 M updated cells, 64 B each)
+// a step takes 1.76 to 1.79 ms, 97 to 98% of the measured copy bandwidth; a
+// plane of a tile alone on the GPU takes an SM 0.60 us.  Before the warps were
+// specialised, 16 warps that exchanged D1y, and refilled the stages, in one
+// CTA-wide exchange a plane took 2.22 ms.  What made the difference:
 //  * the loop is unrolled over the 9 ring slots, and with the producer, the
 //    source and the timed waits in it the code was 102 KB (the instruction
 //    fetch was the stall of 1.1 of 8.4 cycles an issue); moved to the helper
-//    warps and counted waits, it is 34 KB;
+//    warps and counted waits, it is 50 KB.  (One loop body with a switch over
+//    the slots, 24 KB, is slower: the loads of a plane no longer overlap its
+//    arithmetic; 272^3 updated cells 199 -> 215 us.);
 //  * a stage is refilled the moment its last reader releases it, whichever
 //    warp that is, and the warps may run up to S planes apart.  (Groups of 4
 //    warps that exchange among themselves, with the refill still issued by
@@ -47,10 +50,18 @@
 //    warp find their loads not yet issued.)
 //  * one wait a step (for the halo warps, which wait for the loads) and one
 //    base address for all that a stage holds: 14% fewer instructions, 272^3
-//    updated cells 205.1 -> 203.5 us.
-// 16 rows: 16 compute warps at 112 registers hold the 27 ring values and a
-// plane's neighbourhood without a spill; 12 rows take 225 and 8 rows (two
-// CTAs an SM) 214 us where 16 rows take 203.5 (272^3 updated cells).
+//    updated cells 205.1 -> 203.5 us;
+//  * two cells a thread share a window of 10 cells instead of two of 9, read
+//    as five 16-byte words: 72 instead of 88 shared-memory wavefronts a row
+//    and 26% fewer instructions than one cell a thread.  In us a step: media
+//    table 192^3 updated cells 69.7 -> 63.3, 150 x 97 x 260 49.5 -> 45.2, 88^3
+//    12.4 -> 11.7, 312^3 302.2 -> 298.7, 272^3 200.2 -> 199.4; 504^3 1760 -> 1765 and
+//    a 36 x 32 x 28 grid 5.5 -> 5.65 (fewer warps for one plane's latency).  With
+//    A and B in registers too the loads lose their overlap (272^3 212 us, with
+//    A alone 206).
+// 16 rows: 8 compute warps at 232 registers hold the 54 ring values and a
+// plane's neighbourhood without a spill; 12 rows take 81 and 8 rows (two
+// CTAs an SM) 76 us where 16 rows take 73.3 (192^3 updated cells).
 //
 // Media-table layout (template parameter MT): instead of the ten coefficient
 // planes a stage holds the one-byte medium ids of planes k and k-4 and the
@@ -101,22 +112,24 @@ struct Layout {
 };
 
 // Register split (setmaxnreg): the compute warps take what the helper warps
-// give back.  Per SM sub-partition, TY/4 compute warps and one helper warp
-// share (TY/4 + 1) x the launch's registers a thread (96 at 16 rows, 128 at
-// 12, 80 at 8): 4 x 112 + 32 = 5 x 96, 3 x 160 + 32 = 4 x 128, 2 x 104 + 32 = 3 x 80.
+// give back.  Per SM sub-partition, two compute warps (8 rows: one) and one
+// helper warp share the launch's registers, 168 a thread (8 rows: 128):
+// 2 x 232 + 32 <= 3 x 168, 224 + 32 = 2 x 128.
 constexpr int kHelperRegs = 32;
 template <int TY>
 struct Regs {
-  static constexpr int kCompute = TY == 16 ? 112 : TY == 12 ? 160 : 104;
-  static constexpr int kLaunch = TY == 16 ? 96 : TY == 12 ? 128 : 80;
-  static_assert((TY / 4) * kCompute + kHelperRegs <= (TY / 4 + 1) * kLaunch, "the split exceeds the launch's registers");
+  static constexpr int kWarps = (TY / 2 + 3) / 4 * 4;  // compute warps, whole warpgroups (12 rows leave two idle)
+  static constexpr int kCompute = TY == 8 ? 224 : 232;
+  static constexpr int kLaunch = TY == 8 ? 128 : 168;
+  static_assert((kWarps / 4) * kCompute + kHelperRegs <= (kWarps / 4 + 1) * kLaunch,
+                "the split exceeds the launch's registers");
 };
 
 // HOOK: the fault-injection variant (waits limited to P.wait_ns, CTA 0
 // skipping the loads of step P.stall_step), launched only when a test
 // injects a stall.  MT: the media-table layout of the coefficients.
 template <int TY, int S, bool ISO, bool BATCH, int MINB, bool HOOK = false, bool MT = false>
-__global__ void __launch_bounds__(kTileX *(TY + kHelperWarps), MINB)
+__global__ void __launch_bounds__(kTileX *(Regs<TY>::kWarps + kHelperWarps), MINB)
     k_propagate_fp32(const __grid_constant__ SingleMaps SM, const __grid_constant__ PropParams P) {
   static_assert(!MT || (!BATCH && !HOOK), "the media-table layout runs single-shot plain steps");
   using G = Geo<TY, false, MT>;
@@ -131,6 +144,7 @@ __global__ void __launch_bounds__(kTileX *(TY + kHelperWarps), MINB)
   const int tid = threadIdx.x;
   const int lx = tid & 31;
   const int wid = uniform(tid >> 5);
+  constexpr int CW = Regs<TY>::kWarps;
   const int first = P.cta_first[blockIdx.x], nitems = P.cta_first[blockIdx.x + 1] - first;
   if (nitems <= 0) return;
   constexpr int kHalo = TY / 4 < kHaloWarps ? TY / 4 : kHaloWarps;  // halo warps with work
@@ -139,12 +153,12 @@ __global__ void __launch_bounds__(kTileX *(TY + kHelperWarps), MINB)
       unsigned char *st = smem + s * L::SB;
       mbar_init(bar(st, L::OFF_FULL), 1);
       mbar_init(bar(st, L::OFF_READY), kHalo);
-      mbar_init(bar(st, L::OFF_EMPTY), TY + kHalo);
+      mbar_init(bar(st, L::OFF_EMPTY), TY / 2 + kHalo);
     }
     mbar_fence_init();
   }
   if constexpr (MT) {
-    for (int i = tid; i < kAngleCoef * kMediaMax; i += kTileX * (TY + kHelperWarps)) s_med[i] = P.media[i];
+    for (int i = tid; i < kAngleCoef * kMediaMax; i += kTileX * (CW + kHelperWarps)) s_med[i] = P.media[i];
   }
   __syncthreads();
   allow_next_launch();
@@ -155,12 +169,12 @@ __global__ void __launch_bounds__(kTileX *(TY + kHelperWarps), MINB)
     else return mbar_spin(b, parity);
   };
 
-  if (wid >= TY) {
+  if (wid >= CW) {
     setmaxnreg_dec<kHelperRegs>();
     const int4 *seg = P.seg + first;
     int stage = 0;
     uint32_t phase = 0;
-    if (wid == TY) {
+    if (wid == CW) {
       // ---- producer ----
       if (lx != 0) return;
       auto maps_of = [&](int shot) {
@@ -235,7 +249,7 @@ __global__ void __launch_bounds__(kTileX *(TY + kHelperWarps), MINB)
       return;
     }
     // ---- halo warps ----
-    const int hw = wid - TY - 1;
+    const int hw = wid - CW - 1;
     if (hw >= kHalo) return;
     const int hxc = (lx & 7) < 4 ? (lx & 7) : G::TX + (lx & 7);  // lane -> halo column, row lane / 8 of a group of 4
     int rb = 0;
@@ -295,12 +309,15 @@ __global__ void __launch_bounds__(kTileX *(TY + kHelperWarps), MINB)
 
   // ---- compute warps ----
   setmaxnreg_inc<Regs<TY>::kCompute>();
-  const int ly = wid;
+  if (wid >= TY / 2) return;
+  // Lane 16 r + i: cells 2 i and 2 i + 1 of row 2 wid + r.
+  const int cx = 2 * (lx & 15);
+  const int ly = 2 * wid + (lx >> 4);
   // Spacing factors (unused on isotropic grids).
   const float sxy = P.inv_dxy, sxz = P.inv_dxz, syz = P.inv_dyz;
   const float sxx = P.inv_dxx, syy = P.inv_dyy, szz = P.inv_dzz;
-  const int ci = ly * G::TX + lx;
-  const int hc = (ly + kRadius) * G::HX + (lx + kRadius);
+  const int ci = ly * G::TX + cx;
+  const int hc = (ly + kRadius) * G::HX + (cx + kRadius);
   int stage = 0;
   uint32_t phase = 0;
   int rb = 0;   // exchange buffer (when not in the stages)
@@ -314,18 +331,22 @@ __global__ void __launch_bounds__(kTileX *(TY + kHelperWarps), MINB)
     const Item it = decode_item<BATCH>(uniform4(*reinterpret_cast<const int4 *>(st + L::OFF_HDR)));
     const ShotDesc &sd = BATCH ? P.shots[it.shot] : P.one;
     const int depth = it.z1 - it.z0;
-    const int gx = it.x0 + lx;
+    const int gx = it.x0 + cx;  // even: a TMA tile starts on 16 bytes
     const int gy = it.y0 + ly;
     const int bord = sd.bord, sxs = sd.sx, sys = sd.sy;
-    const bool valid = (gx >= bord) && (gx < sxs - bord) && (gy >= bord) && (gy < sys - bord);
+    const bool row = (gy >= bord) && (gy < sys - bord);
+    const bool va = row && (gx >= bord) && (gx < sxs - bord);
+    const bool vb = row && (gx + 1 >= bord) && (gx + 1 < sxs - bord);
     const long plane = (long)sd.pitch * sys;
     unsigned long long *out =
         reinterpret_cast<unsigned long long *>(sd.F[P.parity ^ 1]) + (it.z0 * plane + (long)gy * sd.pitch + gx);
-    // The cell that lacks the last step's source, if it is this thread's.
-    const int cor_k = (gx == sd.cor_x && gy == sd.cor_y) ? sd.cor_z + kLag - it.z0 : -1000;
+    // The cell that lacks the last step's source, if it is one of this thread's.
+    const int cor_c = sd.cor_x - gx;
+    const int cor_k = ((unsigned)cor_c < 2u && gy == sd.cor_y) ? sd.cor_z + kLag - it.z0 : -1000;
 
-    if (P.skip_rows && (gy < bord || gy >= sys - bord)) {
-      // A row outside the updated region: nothing to compute, only the
+    const int y0w = it.y0 + 2 * wid;
+    if (P.skip_rows && (y0w + 1 < bord || y0w >= sys - bord)) {
+      // Two rows outside the updated region: nothing to compute, only the
       // stages to release in step.  (Not where the plan deals every tile
       // alike: tiles that run ahead of their neighbours share fewer halo
       // rows; 312^3 updated cells 304.7 -> 308.5 us.)
@@ -347,7 +368,7 @@ __global__ void __launch_bounds__(kTileX *(TY + kHelperWarps), MINB)
       continue;
     }
 
-    f2 Pr[kRing], Dx[kRing], Dy[kRing];
+    f2 Pr[2][kRing], Dx[2][kRing], Dy[2][kRing];
 
     for (int kb = -kRadius; kb < depth + kLag; kb += kRing) {
 #pragma unroll
@@ -362,99 +383,145 @@ __global__ void __launch_bounds__(kTileX *(TY + kHelperWarps), MINB)
         const bool center = (unsigned)k < (unsigned)depth;
         const bool upd = k >= kLag;
         const f2 *H = reinterpret_cast<const f2 *>(st) + hc;
-        const f2 c = H[0];
-        f2 xa[4], xb[4], ya[4], yb[4];
+        f2 X[10];           // cells -4 .. +5 of the row
+        f2x2 ya[4], yb[4];  // rows +o and -o
+#pragma unroll
+        for (int o = 0; o < 5; ++o) {
+          const f2x2 v = load2(H + 2 * o - 4);
+          X[2 * o] = v.a;
+          X[2 * o + 1] = v.b;
+        }
 #pragma unroll
         for (int o = 1; o <= 4; ++o) {
-          xa[o - 1] = H[o];
-          xb[o - 1] = H[-o];
-          ya[o - 1] = H[o * G::HX];
-          yb[o - 1] = H[-o * G::HX];
+          ya[o - 1] = load2(H + o * G::HX);
+          yb[o - 1] = load2(H - o * G::HX);
         }
-        const f2 d1x = d1(xa[0], xb[0], xa[1], xb[1], xa[2], xb[2], xa[3], xb[3]);
-        const f2 d1y = d1(ya[0], yb[0], ya[1], yb[1], ya[2], yb[2], ya[3], yb[3]);
-        Pr[j] = c;
-        Dx[j] = d1x;
-        Dy[j] = d1y;
-        f2 d2x, d2y;
+        f2 d2x[2], d2y[2];
         f2 *dr = reinterpret_cast<f2 *>(L::ROWS_IN ? st + L::OFF_SROWS : smem + L::OFF_ROWS + rb * G::ROW_B) +
-                 (ly * G::HX + lx + kRadius);
+                 (ly * G::HX + cx + kRadius);
+#pragma unroll
+        for (int c = 0; c < 2; ++c) {
+          const f2 *x = X + 4 + c;
+          Pr[c][j] = x[0];
+          Dx[c][j] = d1(x[1], x[-1], x[2], x[-2], x[3], x[-3], x[4], x[-4]);
+        }
+        Dy[0][j] = d1(ya[0].a, yb[0].a, ya[1].a, yb[1].a, ya[2].a, yb[2].a, ya[3].a, yb[3].a);
+        Dy[1][j] = d1(ya[0].b, yb[0].b, ya[1].b, yb[1].b, ya[2].b, yb[2].b, ya[3].b, yb[3].b);
         if (center) {
-          d2x = scale<ISO>(d2(c, xa[0], xb[0], xa[1], xb[1], xa[2], xb[2], xa[3], xb[3]), sxx);
-          d2y = scale<ISO>(d2(c, ya[0], yb[0], ya[1], yb[1], ya[2], yb[2], ya[3], yb[3]), syy);
-          dr[0] = d1y;
+#pragma unroll
+          for (int c = 0; c < 2; ++c) {
+            const f2 *x = X + 4 + c;
+            d2x[c] = scale<ISO>(d2(x[0], x[1], x[-1], x[2], x[-2], x[3], x[-3], x[4], x[-4]), sxx);
+          }
+          d2y[0] = scale<ISO>(d2(X[4], ya[0].a, yb[0].a, ya[1].a, yb[1].a, ya[2].a, yb[2].a, ya[3].a, yb[3].a), syy);
+          d2y[1] = scale<ISO>(d2(X[5], ya[0].b, yb[0].b, ya[1].b, yb[1].b, ya[2].b, yb[2].b, ya[3].b, yb[3].b), syy);
+          store2(dr, Dy[0][j], Dy[1][j]);
         }
         __syncwarp();
         if (upd) {
           const int cs = (j + kRing - kLag) % kRing;  // ring slot of plane k-kLag
-          // RP(o): plane k-kLag+o for o = 0..4, k-kLag-(kRing-o) for o > 4.
-#define RP(o) Pr[(cs + (o)) % kRing]
-#define RX(o) Dx[(cs + (o)) % kRing]
-#define RY(o) Dy[(cs + (o)) % kRing]
           constexpr int M1 = kRing - 1, M2 = kRing - 2, M3 = kRing - 3, M4 = kRing - 4;
-          const f2 d2z = scale<ISO>(d2(RP(0), RP(1), RP(M1), RP(2), RP(M2), RP(3), RP(M3), RP(4), RP(M4)), szz);
-          const f2 dxz = scale<ISO>(d1(RX(1), RX(M1), RX(2), RX(M2), RX(3), RX(M3), RX(4), RX(M4)), sxz);
-          const f2 dyz = scale<ISO>(d1(RY(1), RY(M1), RY(2), RY(M2), RY(3), RY(M3), RY(4), RY(M4)), syz);
+          const float *cu =
+              reinterpret_cast<const float *>(st + G::OFF_UPD) + (ly * ((MT ? kVelCoef : kUpdateCoef) * G::TX) + cx);
+          float2 czz, cxz, cyz, v2px, v2pz, v2sz, v2pn;
+          auto pair = [](const float *p) { return *reinterpret_cast<const float2 *>(p); };
+          if constexpr (MT) {
+            const uchar2 md = *reinterpret_cast<const uchar2 *>(st + G::OFF_IDU + ci);
+            auto term = [&](int t) { return make_float2(s_med[t * kMediaMax + md.x], s_med[t * kMediaMax + md.y]); };
+            czz = term(DC_ZZ);
+            cxz = term(DC_XZ);
+            cyz = term(DC_YZ);
+            v2px = pair(cu);
+            v2pz = pair(cu + G::TX);
+            v2sz = pair(cu + 2 * G::TX);
+            v2pn = pair(cu + 3 * G::TX);
+          } else {
+            czz = pair(cu);
+            cxz = pair(cu + G::TX);
+            cyz = pair(cu + 2 * G::TX);
+            v2px = pair(cu + 3 * G::TX);
+            v2pz = pair(cu + 4 * G::TX);
+            v2sz = pair(cu + 5 * G::TX);
+            v2pn = pair(cu + 6 * G::TX);
+          }
+          // (With five slots the plane kLag back is the next one round.)
+          const f2 *ab = reinterpret_cast<const f2 *>(
+              L::AB_IN ? st_next + L::OFF_SAB : smem + L::OFF_AB + (abw == kLag ? 0 : abw + 1) * L::AB_SLOT);
+          const f2x2 A = load2(ab + ci), Bv = load2(ab + G::NT + ci);
+          f2x2 old = load2(reinterpret_cast<const f2 *>(st + G::OFF_PP) + ci);
+          if (k == cor_k) {
+            if (cor_c == 0) old.a = add2(old.a, splat(P.cor));
+            else old.b = add2(old.b, splat(P.cor));
+          }
+          f2 nw[2];
+#pragma unroll
+          for (int c = 0; c < 2; ++c) {
+            auto of = [&](float2 v) { return c ? v.y : v.x; };
+            // RP(o): plane k-kLag+o for o = 0..4, k-kLag-(kRing-o) for o > 4.
+#define RP(o) Pr[c][(cs + (o)) % kRing]
+#define RX(o) Dx[c][(cs + (o)) % kRing]
+#define RY(o) Dy[c][(cs + (o)) % kRing]
+            const f2 d2z = scale<ISO>(d2(RP(0), RP(1), RP(M1), RP(2), RP(M2), RP(3), RP(M3), RP(4), RP(M4)), szz);
+            const f2 dxz = scale<ISO>(d1(RX(1), RX(M1), RX(2), RX(M2), RX(3), RX(M3), RX(4), RX(M4)), sxz);
+            const f2 dyz = scale<ISO>(d1(RY(1), RY(M1), RY(2), RY(M2), RY(3), RY(M3), RY(4), RY(M4)), syz);
 #undef RP
 #undef RX
 #undef RY
-          const float *cu =
-              reinterpret_cast<const float *>(st + G::OFF_UPD) + (ly * ((MT ? kVelCoef : kUpdateCoef) * G::TX) + lx);
-          float czz, cxz, cyz, v2px, v2pz, v2sz, v2pn;
-          if constexpr (MT) {
-            const int md = st[G::OFF_IDU + ci];
-            czz = s_med[(DC_ZZ * kMediaMax) + md];
-            cxz = s_med[(DC_XZ * kMediaMax) + md];
-            cyz = s_med[(DC_YZ * kMediaMax) + md];
-            v2px = cu[0];
-            v2pz = cu[G::TX];
-            v2sz = cu[2 * G::TX];
-            v2pn = cu[3 * G::TX];
-          } else {
-            czz = cu[0];
-            cxz = cu[G::TX];
-            cyz = cu[2 * G::TX];
-            v2px = cu[3 * G::TX];
-            v2pz = cu[4 * G::TX];
-            v2sz = cu[5 * G::TX];
-            v2pn = cu[6 * G::TX];
+            const f2 h1 = fma2(splat(of(cyz)), dyz,
+                               fma2(splat(of(cxz)), dxz, fma2(splat(of(czz)), d2z, c ? A.b : A.a)));
+            const f2 h2 = sub2(add2(c ? Bv.b : Bv.a, d2z), h1);
+            const float h1p = lo(h1), h1q = hi(h1), h2p = lo(h2), h2q = hi(h2);
+            // Explicit roundings: every unrolled copy computes identical floats.
+            const float t = __fmul_rn(of(v2pz), h1q);
+            const float rhsp = __fmaf_rn(of(v2sz), __fsub_rn(h1p, h1q), __fmaf_rn(of(v2px), h2p, t));
+            const float rhsq = __fmaf_rn(-of(v2sz), __fsub_rn(h2p, h2q), __fmaf_rn(of(v2pn), h2p, t));
+            const f2 cur = Pr[c][cs];
+            nw[c] = fma2(mk2(rhsp, rhsq), splat(P.dt2), sub2(add2(cur, cur), c ? old.b : old.a));
           }
-          // (With five slots the plane kLag back is the next one round.)
-          const float4 ab = reinterpret_cast<const float4 *>(
-              L::AB_IN ? st_next + L::OFF_SAB : smem + L::OFF_AB + (abw == kLag ? 0 : abw + 1) * L::AB_SLOT)[ci];
-          const f2 Ak = mk2(ab.x, ab.y), Bk = mk2(ab.z, ab.w);
-          const f2 h1 = fma2(splat(cyz), dyz, fma2(splat(cxz), dxz, fma2(splat(czz), d2z, Ak)));
-          const f2 h2 = sub2(add2(Bk, d2z), h1);
-          const float h1p = lo(h1), h1q = hi(h1), h2p = lo(h2), h2q = hi(h2);
-          // Explicit roundings: every unrolled copy computes identical floats.
-          const float t = __fmul_rn(v2pz, h1q);
-          const float rhsp = __fmaf_rn(v2sz, __fsub_rn(h1p, h1q), __fmaf_rn(v2px, h2p, t));
-          const float rhsq = __fmaf_rn(-v2sz, __fsub_rn(h2p, h2q), __fmaf_rn(v2pn, h2p, t));
-          f2 old = reinterpret_cast<const f2 *>(st + G::OFF_PP)[ci];
-          if (k == cor_k) old = add2(old, splat(P.cor));
-          const f2 cur = Pr[cs];
-          const f2 nw = fma2(mk2(rhsp, rhsq), splat(P.dt2), sub2(add2(cur, cur), old));
-          if (valid) *out = nw.v;
+          if (va && vb) {
+            *reinterpret_cast<ulonglong2 *>(out) = make_ulonglong2(nw[0].v, nw[1].v);
+          } else {
+            if (va) out[0] = nw[0].v;
+            if (vb) out[1] = nw[1].v;
+          }
           out += plane;
         }
         if (center) {
-          const f2 dxy = scale<ISO>(d1(dr[1], dr[-1], dr[2], dr[-2], dr[3], dr[-3], dr[4], dr[-4]), sxy);
-          float cxx, cyy, cxy;
-          if constexpr (MT) {
-            const int md = st[G::OFF_IDC + ci];
-            cxx = s_med[(DC_XX * kMediaMax) + md];
-            cyy = s_med[(DC_YY * kMediaMax) + md];
-            cxy = s_med[(DC_XY * kMediaMax) + md];
-          } else {
-            const float *ca = reinterpret_cast<const float *>(st + G::OFF_ARR) + (ly * (kArrivalCoef * G::TX) + lx);
-            cxx = ca[0];
-            cyy = ca[G::TX];
-            cxy = ca[2 * G::TX];
+          f2 Y[10];  // D1y of cells -4 .. +5 of the row
+#pragma unroll
+          for (int o = 0; o < 5; ++o) {
+            if (o == 2) continue;
+            const f2x2 v = load2(dr + 2 * o - 4);
+            Y[2 * o] = v.a;
+            Y[2 * o + 1] = v.b;
           }
-          const f2 av = fma2(splat(cxy), dxy, fma2(splat(cyy), d2y, mul2(splat(cxx), d2x)));
-          const f2 bv = add2(d2x, d2y);
-          reinterpret_cast<float4 *>(L::AB_IN ? st + L::OFF_SAB : smem + L::OFF_AB + abw * L::AB_SLOT)[ci] =
-              make_float4(lo(av), hi(av), lo(bv), hi(bv));
+          Y[4] = Dy[0][j];
+          Y[5] = Dy[1][j];
+          float2 cxx, cyy, cxy;
+          if constexpr (MT) {
+            const uchar2 md = *reinterpret_cast<const uchar2 *>(st + G::OFF_IDC + ci);
+            auto term = [&](int t) { return make_float2(s_med[t * kMediaMax + md.x], s_med[t * kMediaMax + md.y]); };
+            cxx = term(DC_XX);
+            cyy = term(DC_YY);
+            cxy = term(DC_XY);
+          } else {
+            const float *ca = reinterpret_cast<const float *>(st + G::OFF_ARR) + (ly * (kArrivalCoef * G::TX) + cx);
+            cxx = *reinterpret_cast<const float2 *>(ca);
+            cyy = *reinterpret_cast<const float2 *>(ca + G::TX);
+            cxy = *reinterpret_cast<const float2 *>(ca + 2 * G::TX);
+          }
+          f2 av[2], bv[2];
+#pragma unroll
+          for (int c = 0; c < 2; ++c) {
+            auto of = [&](float2 v) { return c ? v.y : v.x; };
+            const f2 *y = Y + 4 + c;
+            const f2 dxy = scale<ISO>(d1(y[1], y[-1], y[2], y[-2], y[3], y[-3], y[4], y[-4]), sxy);
+            av[c] = fma2(splat(of(cxy)), dxy, fma2(splat(of(cyy)), d2y[c], mul2(splat(of(cxx)), d2x[c])));
+            bv[c] = add2(d2x[c], d2y[c]);
+          }
+          f2 *ab = reinterpret_cast<f2 *>(L::AB_IN ? st + L::OFF_SAB : smem + L::OFF_AB + abw * L::AB_SLOT);
+          store2(ab + ci, av[0], av[1]);
+          store2(ab + G::NT + ci, bv[0], bv[1]);
         }
         // This warp is done with the stage.
         __syncwarp();
@@ -521,7 +588,7 @@ size_t propagate_fp32_smem_bytes(int ty, int st) {
   return 0;
 }
 bool propagate_fp32_supported(int ty, int st) { return propagate_fp32_smem_bytes(ty, st) != 0; }
-int propagate_fp32_threads(int ty) { return kTileX * (ty + kHelperWarps); }
+int propagate_fp32_threads(int ty) { return kTileX * ((ty / 2 + 3) / 4 * 4 + kHelperWarps); }
 int propagate_fp32_ctas_per_sm(int ty) { return ty == 8 ? 2 : 1; }
 
 cudaError_t propagate_fp32_prepare(int ty, int st) {

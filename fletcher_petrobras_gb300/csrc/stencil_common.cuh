@@ -54,6 +54,21 @@ __device__ __forceinline__ f2 d2_ref(f2 c, f2 a1, f2 b1, f2 a2, f2 b2, f2 a3, f2
   return mul_rn(d2inv, r);
 }
 
+// Two neighbouring cells' pairs, one 16-byte access.
+struct f2x2 {
+  f2 a, b;
+};
+__device__ __forceinline__ f2x2 load2(const f2 *p) {
+  const ulonglong2 v = *reinterpret_cast<const ulonglong2 *>(p);
+  f2x2 r;
+  r.a.v = v.x;
+  r.b.v = v.y;
+  return r;
+}
+__device__ __forceinline__ void store2(f2 *p, f2 a, f2 b) {
+  *reinterpret_cast<ulonglong2 *>(p) = make_ulonglong2(a.v, b.v);
+}
+
 // Applies a spacing factor unless the grid is isotropic (then every factor
 // is folded into one dt^2/h^2 at the end).
 template <bool ISO>
