@@ -13,10 +13,11 @@
 // exchange it every plane: a warp announces its row, updates plane k-4, which
 // needs no exchanged data, and only then waits for the other rows.
 //
-// What bounds it: issue (scalar p and q, no fused multiply-adds: about 400
-// instructions a warp and plane).  Against the kernel whose compute warps
-// issued the loads and added the source themselves: 128 x 112 x 104 updated
-// cells 30.6 -> 26.3 us a step, 280 x 200 x 150 170 -> 128, 272^3 327 -> 283.
+// What bounds it: the shared-memory pipe and issue.  Against the kernel whose
+// compute warps issued the loads and added the source themselves, with p and q
+// in scalar instructions: 128 x 112 x 104 updated cells 30.6 -> 26.3 us a step,
+// 280 x 200 x 150 170 -> 128, 272^3 327 -> 283; with packed (p, q) instructions
+// (mul_rn) 23.9, 118 and 253.
 #include "device_util.cuh"
 #include "fletcher_internal.h"
 #include "propagate_fp32_pipe.cuh"
@@ -42,6 +43,7 @@ constexpr int OFF_FULL = OFF_HDR + 16;        // barriers: loads landed,
 constexpr int OFF_READY = OFF_HDR + 24;       //   source and pDx halo rows written,
 constexpr int OFF_XCHG = OFF_HDR + 32;        //   pDx rows of the compute warps written,
 constexpr int OFF_EMPTY = OFF_HDR + 40;       //   released by every reader
+constexpr int OFF_NZ = OFF_HDR + 64;          // stage 0: -0.0f (mul_rn)
 constexpr int SB = OFF_HDR + 128;
 constexpr int OFF_AB = S * SB;                          // [kABSlots][NT] of 16 bytes
 constexpr int OFF_C = OFF_AB + kABSlots * G::NT * 16;   // [kABSlots][NT] of 8 bytes: ch1dxy * pxy
@@ -69,11 +71,13 @@ __global__ void __launch_bounds__(kThreads, 1)
       mbar_init(bar(st, OFF_EMPTY), TY + kHaloWarps);
     }
     mbar_fence_init();
+    *reinterpret_cast<volatile float *>(smem + OFF_NZ) = -0.0f;
   }
   __syncthreads();
   allow_next_launch();
   wait_previous_launch();
   const ShotDesc &sd = P.one;
+  const f2 nz = splat(*reinterpret_cast<volatile float *>(smem + OFF_NZ));
 
   if (wid >= TY) {
     setmaxnreg_dec<kHelperRegs>();
@@ -156,7 +160,7 @@ __global__ void __launch_bounds__(kThreads, 1)
           for (int r = hw; r < 2 * kRadius; r += kHaloWarps) {
             const int hrow = r < kRadius ? r : TY + r;
             const f2 *h = H + hrow * G::HX + lx + kRadius;
-            db[hrow * G::TX + lx] = d1_ref(h[1], h[-1], h[2], h[-2], h[3], h[-3], h[4], h[-4], P.inv_dx);
+            db[hrow * G::TX + lx] = d1_ref(h[1], h[-1], h[2], h[-2], h[3], h[-3], h[4], h[-4], P.inv_dx, nz);
           }
         }
         __syncwarp();
@@ -224,8 +228,8 @@ __global__ void __launch_bounds__(kThreads, 1)
           yb[o - 1] = H[-o * G::HX];
         }
         // der1der1/sample.h:35-49: pDx = Der1_x(p) / dx and pDy = Der1_y(p) / dy.
-        const f2 d1x = d1_ref(xa[0], xb[0], xa[1], xb[1], xa[2], xb[2], xa[3], xb[3], P.inv_dx);
-        const f2 d1y = d1_ref(ya[0], yb[0], ya[1], yb[1], ya[2], yb[2], ya[3], yb[3], P.inv_dy);
+        const f2 d1x = d1_ref(xa[0], xb[0], xa[1], xb[1], xa[2], xb[2], xa[3], xb[3], P.inv_dx, nz);
+        const f2 d1y = d1_ref(ya[0], yb[0], ya[1], yb[1], ya[2], yb[2], ya[3], yb[3], P.inv_dy, nz);
         Pr[j] = c;
         Dx[j] = d1x;
         Dy[j] = d1y;
@@ -233,8 +237,8 @@ __global__ void __launch_bounds__(kThreads, 1)
         f2 *dc = reinterpret_cast<f2 *>(st + OFF_ROWS) + ((ly + kRadius) * G::TX + lx);
         if (center) {
           dc[0] = d1x;
-          d2x = d2_ref(c, xa[0], xb[0], xa[1], xb[1], xa[2], xb[2], xa[3], xb[3], sxx);
-          d2y = d2_ref(c, ya[0], yb[0], ya[1], yb[1], ya[2], yb[2], ya[3], yb[3], syy);
+          d2x = d2_ref(c, xa[0], xb[0], xa[1], xb[1], xa[2], xb[2], xa[3], xb[3], sxx, nz);
+          d2y = d2_ref(c, ya[0], yb[0], ya[1], yb[1], ya[2], yb[2], ya[3], yb[3], syy, nz);
         }
         // Split-phase exchange: announce this warp's pDx, update plane k-4,
         // then wait for the other rows.
@@ -248,9 +252,9 @@ __global__ void __launch_bounds__(kThreads, 1)
 #define RY(o) Dy[(cs + (o)) % kRing]
           constexpr int M1 = kRing - 1, M2 = kRing - 2, M3 = kRing - 3, M4 = kRing - 4;
           // der1der1/sample.h:58-66: pzz, pxz = Der1_z(pDx) / dz, pyz = Der1_z(pDy) / dz.
-          const f2 d2z = d2_ref(RP(0), RP(1), RP(M1), RP(2), RP(M2), RP(3), RP(M3), RP(4), RP(M4), szz);
-          const f2 dxz = d1_ref(RX(1), RX(M1), RX(2), RX(M2), RX(3), RX(M3), RX(4), RX(M4), P.inv_dz);
-          const f2 dyz = d1_ref(RY(1), RY(M1), RY(2), RY(M2), RY(3), RY(M3), RY(4), RY(M4), P.inv_dz);
+          const f2 d2z = d2_ref(RP(0), RP(1), RP(M1), RP(2), RP(M2), RP(3), RP(M3), RP(4), RP(M4), szz, nz);
+          const f2 dxz = d1_ref(RX(1), RX(M1), RX(2), RX(M2), RX(3), RX(M3), RX(4), RX(M4), P.inv_dz, nz);
+          const f2 dyz = d1_ref(RY(1), RY(M1), RY(2), RY(M2), RY(3), RY(M3), RY(4), RY(M4), P.inv_dz, nz);
 #undef RP
 #undef RX
 #undef RY
@@ -265,8 +269,8 @@ __global__ void __launch_bounds__(kThreads, 1)
           // h1 = cpxx + cpyy + cpzz + cpxy + cpxz + cpyz (A = cpxx + cpyy,
           // C = cpxy from the plane's arrival), h2 = pxx + pyy + pzz - h1.
           const f2 Ck = reinterpret_cast<const f2 *>(smem + OFF_C)[slot * G::NT + ci];
-          const f2 h1 = add_rn(add_rn(add_rn(add_rn(Ak, mul_rn(czz, d2z)), Ck), mul_rn(cxz, dxz)), mul_rn(cyz, dyz));
-          const f2 h2 = sub_rn(add_rn(Bk, d2z), h1);
+          const f2 h1 = add2(add2(add2(add2(Ak, mul_rn(czz, d2z, nz)), Ck), mul_rn(cxz, dxz, nz)), mul_rn(cyz, dyz, nz));
+          const f2 h2 = sub2(add2(Bk, d2z), h1);
           const float h1p = lo(h1), h1q = hi(h1), h2p = lo(h2), h2q = hi(h2);
           const float t = __fmul_rn(v2pz, h1q);
           const float rhsp = __fadd_rn(__fadd_rn(__fmul_rn(v2px, h2p), t), __fmul_rn(v2sz, __fsub_rn(h1p, h1q)));
@@ -275,7 +279,7 @@ __global__ void __launch_bounds__(kThreads, 1)
           if (k == cor_k) old = add2(old, splat(P.cor));
           const f2 now = Pr[cs];
           // pp = 2 pc - pp + rhs * dt * dt (der1der1/sample.h:119-120).
-          const f2 nw = add_rn(sub_rn(add_rn(now, now), old), mul_rn(P.dt, mul_rn(P.dt, mk2(rhsp, rhsq))));
+          const f2 nw = add2(sub2(add2(now, now), old), mul_rn(P.dt, mul_rn(P.dt, mk2(rhsp, rhsq), nz), nz));
           if (valid) *out = nw.v;
           out += plane;
         }
@@ -288,13 +292,13 @@ __global__ void __launch_bounds__(kThreads, 1)
           // B = pxx + pyy, C = cpxy.
           constexpr int W = G::TX;
           const f2 pxy = d1_ref(dc[W], dc[-W], dc[2 * W], dc[-2 * W], dc[3 * W], dc[-3 * W], dc[4 * W], dc[-4 * W],
-                                P.inv_dy);
+                                P.inv_dy, nz);
           const float *ca = reinterpret_cast<const float *>(st + G::OFF_ARR) + (ly * (kArrivalCoef * G::TX) + lx);
           const float cxx = ca[0], cyy = ca[G::TX], cxy = ca[2 * G::TX];
-          const f2 av = add_rn(mul_rn(cxx, d2x), mul_rn(cyy, d2y));
-          const f2 bv = add_rn(d2x, d2y);
+          const f2 av = add2(mul_rn(cxx, d2x, nz), mul_rn(cyy, d2y, nz));
+          const f2 bv = add2(d2x, d2y);
           reinterpret_cast<float4 *>(smem + OFF_AB)[abw * G::NT + ci] = make_float4(lo(av), hi(av), lo(bv), hi(bv));
-          reinterpret_cast<f2 *>(smem + OFF_C)[abw * G::NT + ci] = mul_rn(cxy, pxy);
+          reinterpret_cast<f2 *>(smem + OFF_C)[abw * G::NT + ci] = mul_rn(cxy, pxy, nz);
         }
         // This warp is done with the stage.
         __syncwarp();
