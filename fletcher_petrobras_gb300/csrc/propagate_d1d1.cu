@@ -8,16 +8,17 @@
 //
 // The warps are specialised as in propagate_fp32.cu: a producer thread issues
 // the TMA loads, the halo warps add the step's source and evaluate pDx in the
-// tile's 8 halo rows, and 16 compute warps run a tile row each.  As
+// tile's 8 halo rows, and 8 compute warps run two tile rows each.  As
 // pxy = Der1_y(pDx) needs pDx of the rows above and below, the compute warps
-// exchange it every plane: a warp announces its row, updates plane k-4, which
+// exchange it every plane: a warp announces its rows, updates plane k-4, which
 // needs no exchanged data, and only then waits for the other rows.
 //
 // What bounds it: the shared-memory pipe and issue.  Against the kernel whose
 // compute warps issued the loads and added the source themselves, with p and q
 // in scalar instructions: 128 x 112 x 104 updated cells 30.6 -> 26.3 us a step,
 // 280 x 200 x 150 170 -> 128, 272^3 327 -> 283; with packed (p, q) instructions
-// (mul_rn) 23.9, 118 and 253.
+// (mul_rn) 23.9, 118.2 and 252.5, with two cells a thread, as in
+// propagate_fp32.cu, 23.5, 117.8 and 248.6.
 #include "device_util.cuh"
 #include "fletcher_internal.h"
 #include "propagate_fp32_pipe.cuh"
@@ -30,9 +31,10 @@ namespace {
 constexpr int TY = kD1D1Rows, S = kD1D1Stages;
 using G = Geo<TY, true>;
 constexpr int kHelperWarps = 4, kHaloWarps = kHelperWarps - 1;
-constexpr int kThreads = kTileX * (TY + kHelperWarps);
-// Registers: 4 x 112 + 32 = 5 x 96 a sub-partition, as in propagate_fp32.cu.
-constexpr int kComputeRegs = 112, kHelperRegs = 32;
+constexpr int CW = TY / 2;  // compute warps
+constexpr int kThreads = kTileX * (CW + kHelperWarps);
+// Registers: 2 x 232 + 32 <= 3 x 168 a sub-partition, as in propagate_fp32.cu.
+constexpr int kComputeRegs = 232, kHelperRegs = 32;
 
 // Shared memory: S stages (TMA tiles, pDx of the tile's columns with its
 // 4-row halo, a control block), then the in-plane terms (A, B and C) of the
@@ -45,11 +47,10 @@ constexpr int OFF_XCHG = OFF_HDR + 32;        //   pDx rows of the compute warps
 constexpr int OFF_EMPTY = OFF_HDR + 40;       //   released by every reader
 constexpr int OFF_NZ = OFF_HDR + 64;          // stage 0: -0.0f (mul_rn)
 constexpr int SB = OFF_HDR + 128;
-constexpr int OFF_AB = S * SB;                          // [kABSlots][NT] of 16 bytes
-constexpr int OFF_C = OFF_AB + kABSlots * G::NT * 16;   // [kABSlots][NT] of 8 bytes: ch1dxy * pxy
-constexpr size_t kSmem = size_t(OFF_C) + kABSlots * G::NT * 8 + 128;
+constexpr int OFF_ABC = S * SB;  // [kABSlots][A, B, C = ch1dxy * pxy][NT] of 8 bytes
+constexpr size_t kSmem = size_t(OFF_ABC) + kABSlots * G::NT * 24 + 128;
 static_assert(kSmem <= 227 * 1024, "Der1-Der1 shape exceeds the shared memory of a CTA");
-static_assert(OFF_HDR % 128 == 0 && SB % 128 == 0 && OFF_AB % 128 == 0 && OFF_C % 128 == 0, "shared-memory alignment");
+static_assert(OFF_HDR % 128 == 0 && SB % 128 == 0 && OFF_ABC % 128 == 0, "shared-memory alignment");
 
 __global__ void __launch_bounds__(kThreads, 1)
     k_propagate_d1d1(const __grid_constant__ SingleMaps SM, const __grid_constant__ PropParams P) {
@@ -67,8 +68,8 @@ __global__ void __launch_bounds__(kThreads, 1)
       unsigned char *st = smem + s * SB;
       mbar_init(bar(st, OFF_FULL), 1);
       mbar_init(bar(st, OFF_READY), kHaloWarps);
-      mbar_init(bar(st, OFF_XCHG), TY);
-      mbar_init(bar(st, OFF_EMPTY), TY + kHaloWarps);
+      mbar_init(bar(st, OFF_XCHG), CW);
+      mbar_init(bar(st, OFF_EMPTY), CW + kHaloWarps);
     }
     mbar_fence_init();
     *reinterpret_cast<volatile float *>(smem + OFF_NZ) = -0.0f;
@@ -79,12 +80,12 @@ __global__ void __launch_bounds__(kThreads, 1)
   const ShotDesc &sd = P.one;
   const f2 nz = splat(*reinterpret_cast<volatile float *>(smem + OFF_NZ));
 
-  if (wid >= TY) {
+  if (wid >= CW) {
     setmaxnreg_dec<kHelperRegs>();
     const int4 *seg = P.seg + first;
     int stage = 0;
     uint32_t phase = 0;
-    if (wid == TY) {
+    if (wid == CW) {
       // ---- producer ----
       if (lx != 0) return;
       StepMaps maps;
@@ -132,7 +133,7 @@ __global__ void __launch_bounds__(kThreads, 1)
       return;
     }
     // ---- halo warps ----
-    const int hw = wid - TY - 1;
+    const int hw = wid - CW - 1;
     for (int i = 0; i < nitems; ++i) {
       const Item it = decode_item<false>(seg[i]);
       const int src_z = sd.src_z;
@@ -179,10 +180,12 @@ __global__ void __launch_bounds__(kThreads, 1)
 
   // ---- compute warps ----
   setmaxnreg_inc<kComputeRegs>();
-  const int ly = wid;
+  // Lane 16 r + i: cells 2 i and 2 i + 1 of row 2 wid + r.
+  const int cx = 2 * (lx & 15);
+  const int ly = 2 * wid + (lx >> 4);
   const float sxx = P.inv_dxx, syy = P.inv_dyy, szz = P.inv_dzz;
-  const int ci = ly * G::TX + lx;
-  const int hc = (ly + kRadius) * G::HX + (lx + kRadius);
+  const int ci = ly * G::TX + cx;
+  const int hc = (ly + kRadius) * G::HX + (cx + kRadius);
   int stage = 0;
   uint32_t phase = 0;
   int abw = 0;  // shared A/B/C ring slot of the arriving plane (the plane kLag back is at abw + 1)
@@ -194,17 +197,20 @@ __global__ void __launch_bounds__(kThreads, 1)
     }
     const Item it = decode_item<false>(uniform4(*reinterpret_cast<const int4 *>(st + OFF_HDR)));
     const int depth = it.z1 - it.z0;
-    const int gx = it.x0 + lx;
+    const int gx = it.x0 + cx;  // even: a TMA tile starts on 16 bytes
     const int gy = it.y0 + ly;
     const int bord = sd.bord, sxs = sd.sx, sys = sd.sy;
-    const bool valid = (gx >= bord) && (gx < sxs - bord) && (gy >= bord) && (gy < sys - bord);
+    const bool row = (gy >= bord) && (gy < sys - bord);
+    const bool va = row && (gx >= bord) && (gx < sxs - bord);
+    const bool vb = row && (gx + 1 >= bord) && (gx + 1 < sxs - bord);
     const long plane = (long)sd.pitch * sys;
     unsigned long long *out =
         reinterpret_cast<unsigned long long *>(sd.F[P.parity ^ 1]) + (it.z0 * plane + (long)gy * sd.pitch + gx);
-    // The cell that lacks the last step's source, if it is this thread's.
-    const int cor_k = (gx == sd.cor_x && gy == sd.cor_y) ? sd.cor_z + kLag - it.z0 : -1000;
+    // The cell that lacks the last step's source, if it is one of this thread's.
+    const int cor_c = sd.cor_x - gx;
+    const int cor_k = ((unsigned)cor_c < 2u && gy == sd.cor_y) ? sd.cor_z + kLag - it.z0 : -1000;
 
-    f2 Pr[kRing], Dx[kRing], Dy[kRing];
+    f2 Pr[2][kRing], Dx[2][kRing], Dy[2][kRing];
 
     for (int kb = -kRadius; kb < depth + kLag; kb += kRing) {
 #pragma unroll
@@ -218,27 +224,39 @@ __global__ void __launch_bounds__(kThreads, 1)
         const bool center = (unsigned)k < (unsigned)depth;
         const bool upd = k >= kLag;
         const f2 *H = reinterpret_cast<const f2 *>(st) + hc;
-        const f2 c = H[0];
-        f2 xa[4], xb[4], ya[4], yb[4];
+        f2 X[10];           // cells -4 .. +5 of the row
+        f2x2 ya[4], yb[4];  // rows +o and -o
+#pragma unroll
+        for (int o = 0; o < 5; ++o) {
+          const f2x2 v = load2(H + 2 * o - 4);
+          X[2 * o] = v.a;
+          X[2 * o + 1] = v.b;
+        }
 #pragma unroll
         for (int o = 1; o <= 4; ++o) {
-          xa[o - 1] = H[o];
-          xb[o - 1] = H[-o];
-          ya[o - 1] = H[o * G::HX];
-          yb[o - 1] = H[-o * G::HX];
+          ya[o - 1] = load2(H + o * G::HX);
+          yb[o - 1] = load2(H - o * G::HX);
         }
         // der1der1/sample.h:35-49: pDx = Der1_x(p) / dx and pDy = Der1_y(p) / dy.
-        const f2 d1x = d1_ref(xa[0], xb[0], xa[1], xb[1], xa[2], xb[2], xa[3], xb[3], P.inv_dx, nz);
-        const f2 d1y = d1_ref(ya[0], yb[0], ya[1], yb[1], ya[2], yb[2], ya[3], yb[3], P.inv_dy, nz);
-        Pr[j] = c;
-        Dx[j] = d1x;
-        Dy[j] = d1y;
-        f2 d2x, d2y;
-        f2 *dc = reinterpret_cast<f2 *>(st + OFF_ROWS) + ((ly + kRadius) * G::TX + lx);
+#pragma unroll
+        for (int c = 0; c < 2; ++c) {
+          const f2 *x = X + 4 + c;
+          Pr[c][j] = x[0];
+          Dx[c][j] = d1_ref(x[1], x[-1], x[2], x[-2], x[3], x[-3], x[4], x[-4], P.inv_dx, nz);
+        }
+        Dy[0][j] = d1_ref(ya[0].a, yb[0].a, ya[1].a, yb[1].a, ya[2].a, yb[2].a, ya[3].a, yb[3].a, P.inv_dy, nz);
+        Dy[1][j] = d1_ref(ya[0].b, yb[0].b, ya[1].b, yb[1].b, ya[2].b, yb[2].b, ya[3].b, yb[3].b, P.inv_dy, nz);
+        f2 d2x[2], d2y[2];
+        f2 *dc = reinterpret_cast<f2 *>(st + OFF_ROWS) + ((ly + kRadius) * G::TX + cx);
         if (center) {
-          dc[0] = d1x;
-          d2x = d2_ref(c, xa[0], xb[0], xa[1], xb[1], xa[2], xb[2], xa[3], xb[3], sxx, nz);
-          d2y = d2_ref(c, ya[0], yb[0], ya[1], yb[1], ya[2], yb[2], ya[3], yb[3], syy, nz);
+          store2(dc, Dx[0][j], Dx[1][j]);
+#pragma unroll
+          for (int c = 0; c < 2; ++c) {
+            const f2 *x = X + 4 + c;
+            d2x[c] = d2_ref(x[0], x[1], x[-1], x[2], x[-2], x[3], x[-3], x[4], x[-4], sxx, nz);
+          }
+          d2y[0] = d2_ref(X[4], ya[0].a, yb[0].a, ya[1].a, yb[1].a, ya[2].a, yb[2].a, ya[3].a, yb[3].a, syy, nz);
+          d2y[1] = d2_ref(X[5], ya[0].b, yb[0].b, ya[1].b, yb[1].b, ya[2].b, yb[2].b, ya[3].b, yb[3].b, syy, nz);
         }
         // Split-phase exchange: announce this warp's pDx, update plane k-4,
         // then wait for the other rows.
@@ -246,41 +264,55 @@ __global__ void __launch_bounds__(kThreads, 1)
         if (lx == 0) mbar_arrive(bar(st, OFF_XCHG));
         if (upd) {
           const int cs = (j + kRing - kLag) % kRing;  // ring slot of plane k-kLag
-          // RP(o): plane k-kLag+o for o = 0..4, k-kLag-(kRing-o) for o > 4.
-#define RP(o) Pr[(cs + (o)) % kRing]
-#define RX(o) Dx[(cs + (o)) % kRing]
-#define RY(o) Dy[(cs + (o)) % kRing]
           constexpr int M1 = kRing - 1, M2 = kRing - 2, M3 = kRing - 3, M4 = kRing - 4;
-          // der1der1/sample.h:58-66: pzz, pxz = Der1_z(pDx) / dz, pyz = Der1_z(pDy) / dz.
-          const f2 d2z = d2_ref(RP(0), RP(1), RP(M1), RP(2), RP(M2), RP(3), RP(M3), RP(4), RP(M4), szz, nz);
-          const f2 dxz = d1_ref(RX(1), RX(M1), RX(2), RX(M2), RX(3), RX(M3), RX(4), RX(M4), P.inv_dz, nz);
-          const f2 dyz = d1_ref(RY(1), RY(M1), RY(2), RY(M2), RY(3), RY(M3), RY(4), RY(M4), P.inv_dz, nz);
+          const float *cu = reinterpret_cast<const float *>(st + G::OFF_UPD) + (ly * (kUpdateCoef * G::TX) + cx);
+          auto pair = [&](int t) { return *reinterpret_cast<const float2 *>(cu + t * G::TX); };
+          const float2 czz = pair(0), cxz = pair(1), cyz = pair(2);
+          const float2 v2px = pair(3), v2pz = pair(4), v2sz = pair(5), v2pn = pair(6);
+          const f2 *ab = reinterpret_cast<const f2 *>(smem + OFF_ABC) + (abw == kLag ? 0 : abw + 1) * (3 * G::NT) + ci;
+          const f2x2 A = load2(ab), Bv = load2(ab + G::NT), C = load2(ab + 2 * G::NT);
+          f2x2 old = load2(reinterpret_cast<const f2 *>(st + G::OFF_PP) + ci);
+          if (k == cor_k) {
+            if (cor_c == 0) old.a = add2(old.a, splat(P.cor));
+            else old.b = add2(old.b, splat(P.cor));
+          }
+          f2 nw[2];
+#pragma unroll
+          for (int c = 0; c < 2; ++c) {
+            auto of = [&](float2 v) { return c ? v.y : v.x; };
+            // RP(o): plane k-kLag+o for o = 0..4, k-kLag-(kRing-o) for o > 4.
+#define RP(o) Pr[c][(cs + (o)) % kRing]
+#define RX(o) Dx[c][(cs + (o)) % kRing]
+#define RY(o) Dy[c][(cs + (o)) % kRing]
+            // der1der1/sample.h:58-66: pzz, pxz = Der1_z(pDx) / dz, pyz = Der1_z(pDy) / dz.
+            const f2 d2z = d2_ref(RP(0), RP(1), RP(M1), RP(2), RP(M2), RP(3), RP(M3), RP(4), RP(M4), szz, nz);
+            const f2 dxz = d1_ref(RX(1), RX(M1), RX(2), RX(M2), RX(3), RX(M3), RX(4), RX(M4), P.inv_dz, nz);
+            const f2 dyz = d1_ref(RY(1), RY(M1), RY(2), RY(M2), RY(3), RY(M3), RY(4), RY(M4), P.inv_dz, nz);
 #undef RP
 #undef RX
 #undef RY
-          const float *cu = reinterpret_cast<const float *>(st + G::OFF_UPD) + (ly * (kUpdateCoef * G::TX) + lx);
-          const float czz = cu[0], cxz = cu[G::TX], cyz = cu[2 * G::TX];
-          const float v2px = cu[3 * G::TX], v2pz = cu[4 * G::TX];
-          const float v2sz = cu[5 * G::TX], v2pn = cu[6 * G::TX];
-          const int slot = abw == kLag ? 0 : abw + 1;
-          const float4 ab = reinterpret_cast<const float4 *>(smem + OFF_AB)[slot * G::NT + ci];
-          const f2 Ak = mk2(ab.x, ab.y), Bk = mk2(ab.z, ab.w);
-          // der1der1/sample.h:70-117 in its order, each operation rounded:
-          // h1 = cpxx + cpyy + cpzz + cpxy + cpxz + cpyz (A = cpxx + cpyy,
-          // C = cpxy from the plane's arrival), h2 = pxx + pyy + pzz - h1.
-          const f2 Ck = reinterpret_cast<const f2 *>(smem + OFF_C)[slot * G::NT + ci];
-          const f2 h1 = add2(add2(add2(add2(Ak, mul_rn(czz, d2z, nz)), Ck), mul_rn(cxz, dxz, nz)), mul_rn(cyz, dyz, nz));
-          const f2 h2 = sub2(add2(Bk, d2z), h1);
-          const float h1p = lo(h1), h1q = hi(h1), h2p = lo(h2), h2q = hi(h2);
-          const float t = __fmul_rn(v2pz, h1q);
-          const float rhsp = __fadd_rn(__fadd_rn(__fmul_rn(v2px, h2p), t), __fmul_rn(v2sz, __fsub_rn(h1p, h1q)));
-          const float rhsq = __fsub_rn(__fadd_rn(__fmul_rn(v2pn, h2p), t), __fmul_rn(v2sz, __fsub_rn(h2p, h2q)));
-          f2 old = reinterpret_cast<const f2 *>(st + G::OFF_PP)[ci];
-          if (k == cor_k) old = add2(old, splat(P.cor));
-          const f2 now = Pr[cs];
-          // pp = 2 pc - pp + rhs * dt * dt (der1der1/sample.h:119-120).
-          const f2 nw = add2(sub2(add2(now, now), old), mul_rn(P.dt, mul_rn(P.dt, mk2(rhsp, rhsq), nz), nz));
-          if (valid) *out = nw.v;
+            // der1der1/sample.h:70-117 in its order, each operation rounded:
+            // h1 = cpxx + cpyy + cpzz + cpxy + cpxz + cpyz (A = cpxx + cpyy,
+            // C = cpxy from the plane's arrival), h2 = pxx + pyy + pzz - h1.
+            const f2 h1 = add2(add2(add2(add2(c ? A.b : A.a, mul_rn(of(czz), d2z, nz)), c ? C.b : C.a),
+                                    mul_rn(of(cxz), dxz, nz)),
+                               mul_rn(of(cyz), dyz, nz));
+            const f2 h2 = sub2(add2(c ? Bv.b : Bv.a, d2z), h1);
+            const float h1p = lo(h1), h1q = hi(h1), h2p = lo(h2), h2q = hi(h2);
+            const float t = __fmul_rn(of(v2pz), h1q);
+            const float rhsp = __fadd_rn(__fadd_rn(__fmul_rn(of(v2px), h2p), t), __fmul_rn(of(v2sz), __fsub_rn(h1p, h1q)));
+            const float rhsq = __fsub_rn(__fadd_rn(__fmul_rn(of(v2pn), h2p), t), __fmul_rn(of(v2sz), __fsub_rn(h2p, h2q)));
+            const f2 now = Pr[c][cs];
+            // pp = 2 pc - pp + rhs * dt * dt (der1der1/sample.h:119-120).
+            nw[c] = add2(sub2(add2(now, now), c ? old.b : old.a),
+                         mul_rn(P.dt, mul_rn(P.dt, mk2(rhsp, rhsq), nz), nz));
+          }
+          if (va && vb) {
+            *reinterpret_cast<ulonglong2 *>(out) = make_ulonglong2(nw[0].v, nw[1].v);
+          } else {
+            if (va) out[0] = nw[0].v;
+            if (vb) out[1] = nw[1].v;
+          }
           out += plane;
         }
         if (center) {
@@ -290,15 +322,23 @@ __global__ void __launch_bounds__(kThreads, 1)
           }
           // pxy = Der1_y(pDx) / dy (der1der1/sample.h:55); A = cpxx + cpyy,
           // B = pxx + pyy, C = cpxy.
-          constexpr int W = G::TX;
-          const f2 pxy = d1_ref(dc[W], dc[-W], dc[2 * W], dc[-2 * W], dc[3 * W], dc[-3 * W], dc[4 * W], dc[-4 * W],
-                                P.inv_dy, nz);
-          const float *ca = reinterpret_cast<const float *>(st + G::OFF_ARR) + (ly * (kArrivalCoef * G::TX) + lx);
-          const float cxx = ca[0], cyy = ca[G::TX], cxy = ca[2 * G::TX];
-          const f2 av = add2(mul_rn(cxx, d2x, nz), mul_rn(cyy, d2y, nz));
-          const f2 bv = add2(d2x, d2y);
-          reinterpret_cast<float4 *>(smem + OFF_AB)[abw * G::NT + ci] = make_float4(lo(av), hi(av), lo(bv), hi(bv));
-          reinterpret_cast<f2 *>(smem + OFF_C)[abw * G::NT + ci] = mul_rn(cxy, pxy, nz);
+          f2x2 ra[4], rb[4];
+#pragma unroll
+          for (int o = 1; o <= 4; ++o) {
+            ra[o - 1] = load2(dc + o * G::TX);
+            rb[o - 1] = load2(dc - o * G::TX);
+          }
+          const f2 pxy[2] = {
+              d1_ref(ra[0].a, rb[0].a, ra[1].a, rb[1].a, ra[2].a, rb[2].a, ra[3].a, rb[3].a, P.inv_dy, nz),
+              d1_ref(ra[0].b, rb[0].b, ra[1].b, rb[1].b, ra[2].b, rb[2].b, ra[3].b, rb[3].b, P.inv_dy, nz)};
+          const float *ca = reinterpret_cast<const float *>(st + G::OFF_ARR) + (ly * (kArrivalCoef * G::TX) + cx);
+          auto pair = [&](int t) { return *reinterpret_cast<const float2 *>(ca + t * G::TX); };
+          const float2 cxx = pair(0), cyy = pair(1), cxy = pair(2);
+          f2 *ab = reinterpret_cast<f2 *>(smem + OFF_ABC) + abw * (3 * G::NT) + ci;
+          store2(ab, add2(mul_rn(cxx.x, d2x[0], nz), mul_rn(cyy.x, d2y[0], nz)),
+                 add2(mul_rn(cxx.y, d2x[1], nz), mul_rn(cyy.y, d2y[1], nz)));
+          store2(ab + G::NT, add2(d2x[0], d2y[0]), add2(d2x[1], d2y[1]));
+          store2(ab + 2 * G::NT, mul_rn(cxy.x, pxy[0], nz), mul_rn(cxy.y, pxy[1], nz));
         }
         // This warp is done with the stage.
         __syncwarp();
