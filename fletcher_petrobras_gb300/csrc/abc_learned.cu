@@ -1108,6 +1108,11 @@ __global__ void k_abc_fill(const __grid_constant__ Ghost G, const float *coef, i
 // 8192 samples 128 blocks (of 152 SMs).
 constexpr int kTB = 64, kTG = 4, kTT = kTB * kTG;
 constexpr int kTO = kHid / kTG;  // a thread's outputs of a hidden layer
+// More samples than kTrainOnce blocks take (their sums fit the 2 MB that the
+// allocator hands out at once: 14 394 samples 515 -> 470 us a gradient and
+// outputs, of which most is copies) run on a block an SM, several chunks of
+// kTB each.  Fewer take a chunk a block: 8192 samples 306 us, 316 in the loop.
+constexpr int kTrainOnce = 208, kTrainLoop = 152;
 static_assert(kTO % 4 == 0 && kTG >= kOut && kTB % 32 == 0, "float4 stores; an output layer's row per group of warps");
 constexpr int sX = 44, sH = 36;  // row strides in floats: rows 16-byte aligned, float4 reads of 8 rows conflict-free
 
@@ -1164,6 +1169,7 @@ __device__ __forceinline__ void load_row(const float *row, float (&x)[K]) {
 // and of the sums; with one scalar read an operand and one thread a
 // sample it took 41 us for 8192 samples; float4 reads and 4 x 4 register tiles
 // of the sums brought 26 us, four threads a sample 15.5 us.
+template <bool LOOP>
 __global__ void __launch_bounds__(kTT) k_abc_train(const float *feat, const float *tgt, long nsamp, int B,
                                                     uint32_t seed, const float *P, float noise, float *partial,
                                                     float *lpartial) {
@@ -1184,117 +1190,162 @@ __global__ void __launch_bounds__(kTT) k_abc_train(const float *feat, const floa
     else b3[i - oB3] = v;
   }
   const int smp = tid % kTB, grp = tid / kTB, o0 = grp * kTO;
-  const int b = blockIdx.x * kTB + smp;
-  const bool live = b < B;
-  long si = 0;
-  if (live)
-    si = seed ? (long)((((uint64_t)mix32(seed, (uint32_t)b) << 16) ^ mix32(seed + 1u, (uint32_t)b)) % (uint64_t)nsamp)
-              : b;
-  if (tid < kTB) srow[tid] = live ? si : -1;
-  __syncthreads();
-  for (int e = tid; e < kTB * (kIn / 4); e += kTT) {
-    const int q = e / (kIn / 4), k = 4 * (e % (kIn / 4));
-    const long row = srow[q];
-    float f[4] = {0.f, 0.f, 0.f, 0.f};
-    if (row >= 0) {
-      const float4 v = *reinterpret_cast<const float4 *>(feat + row * kIn + k);
-      f[0] = v.x; f[1] = v.y; f[2] = v.z; f[3] = v.w;
-      if (noise > 0.f && k < kSt) {
-        // Input noise (approximately normal, from four uniforms).
-        for (int w = 0; w < 4; ++w) {
-          float u = 0.f;
-          for (int r = 0; r < 4; ++r)
-            u += (float)(mix32(seed ^ (0x51ED27u * (r + 1)), (uint32_t)((blockIdx.x * kTB + q) * kIn + k + w)) >> 8);
-          f[w] += noise * 1.7320508f * (u * (1.0f / 16777216.0f) - 2.0f);
+  constexpr int kT1 = kHid / 4 * (kIn / 4), kT2 = kHid / 4 * (kHid / 4);  // 4 x 4 tiles of the W1 and W2 sums
+  constexpr int kSums = 2 * kHid + kOut * kHid + kOut, kTS = kTT - kT1 - kT2;  // the other sums and their threads
+  static_assert(kTS > 0 && kSums <= 2 * kTS, "a thread takes at most one tile or two other sums");
+  const bool first = tid < kT1;
+  const int nk = first ? kIn : kHid, tile = first ? tid : tid - kT1;
+  const int to = 4 * (tile / (nk / 4)), tk = 4 * (tile % (nk / 4));
+  float l = 0.f, gs[4][4] = {};  // sums over the block's chunks
+  int chunk = blockIdx.x;
+  do {
+    const int b = chunk * kTB + smp;
+    const bool live = b < B;
+    long si = 0;
+    if (live)
+      si = seed ? (long)((((uint64_t)mix32(seed, (uint32_t)b) << 16) ^ mix32(seed + 1u, (uint32_t)b)) % (uint64_t)nsamp)
+                : b;
+    if (LOOP) __syncthreads();  // the last chunk's rows have been read
+    if (tid < kTB) srow[tid] = live ? si : -1;
+    __syncthreads();
+    for (int e = tid; e < kTB * (kIn / 4); e += kTT) {
+      const int q = e / (kIn / 4), k = 4 * (e % (kIn / 4));
+      const long row = srow[q];
+      float f[4] = {0.f, 0.f, 0.f, 0.f};
+      if (row >= 0) {
+        const float4 v = *reinterpret_cast<const float4 *>(feat + row * kIn + k);
+        f[0] = v.x; f[1] = v.y; f[2] = v.z; f[3] = v.w;
+        if (noise > 0.f && k < kSt) {
+          // Input noise (approximately normal, from four uniforms).
+          for (int w = 0; w < 4; ++w) {
+            float u = 0.f;
+            for (int r = 0; r < 4; ++r)
+              u += (float)(mix32(seed ^ (0x51ED27u * (r + 1)), (uint32_t)((chunk * kTB + q) * kIn + k + w)) >> 8);
+            f[w] += noise * 1.7320508f * (u * (1.0f / 16777216.0f) - 2.0f);
+          }
         }
       }
+      *reinterpret_cast<float4 *>(X + q * sX + k) = make_float4(h16(f[0]), h16(f[1]), h16(f[2]), h16(f[3]));
     }
-    *reinterpret_cast<float4 *>(X + q * sX + k) = make_float4(h16(f[0]), h16(f[1]), h16(f[2]), h16(f[3]));
-  }
-  __syncthreads();
-  // D1 and D2 hold the activations' derivatives until the backward pass.
-  float *h1 = H1 + smp * sH, *d1v = D1 + smp * sH, *h2 = H2 + smp * sH, *d2v = D2 + smp * sH;
-  {
-    float x[kIn];
-    load_row(X + smp * sX, x);
-    layer<kIn>(W1, b1, x, o0, h1, d1v);
-  }
-  __syncthreads();
-  {
-    float x[kHid];
-    load_row(h1, x);
-    layer<kHid>(W2, b2, x, o0, h2, d2v);
-  }
-  __syncthreads();
-  if (grp < kOut) {
-    const int o = grp;
-    float x[kHid];
-    load_row(h2, x);
-    float y = b3[o];
+    __syncthreads();
+    // D1 and D2 hold the activations' derivatives until the backward pass.
+    float *h1 = H1 + smp * sH, *d1v = D1 + smp * sH, *h2 = H2 + smp * sH, *d2v = D2 + smp * sH;
+    {
+      float x[kIn];
+      load_row(X + smp * sX, x);
+      layer<kIn>(W1, b1, x, o0, h1, d1v);
+    }
+    __syncthreads();
+    {
+      float x[kHid];
+      load_row(h1, x);
+      layer<kHid>(W2, b2, x, o0, h2, d2v);
+    }
+    __syncthreads();
+    if (grp < kOut) {
+      const int o = grp;
+      float x[kHid];
+      load_row(h2, x);
+      float y = b3[o];
 #pragma unroll
-    for (int k = 0; k < kHid; k += 4) {
-      const float4 w = *reinterpret_cast<const float4 *>(W3 + o * kHid + k);
-      y = fmaf(w.x, x[k], y);
-      y = fmaf(w.y, x[k + 1], y);
-      y = fmaf(w.z, x[k + 2], y);
-      y = fmaf(w.w, x[k + 3], y);
+      for (int k = 0; k < kHid; k += 4) {
+        const float4 w = *reinterpret_cast<const float4 *>(W3 + o * kHid + k);
+        y = fmaf(w.x, x[k], y);
+        y = fmaf(w.y, x[k + 1], y);
+        y = fmaf(w.z, x[k + 2], y);
+        y = fmaf(w.w, x[k + 3], y);
+      }
+      float g = 0.f;
+      if (live) {
+        const float kk = 1.0f / (1.0f + expf(-y));
+        const float ta = tgt[si * kTgt + o], tb = tgt[si * kTgt + 2 + o];
+        const float e = fmaf(kk, ta, -tb);
+        l += e * e;
+        g = e * ta * kk * (1.0f - kk);
+      }
+      DY[smp * 2 + o] = g / (float)B;
     }
-    float g = 0.f, l = 0.f;
-    if (live) {
-      const float kk = 1.0f / (1.0f + expf(-y));
-      const float ta = tgt[si * kTgt + o], tb = tgt[si * kTgt + 2 + o];
-      const float e = fmaf(kk, ta, -tb);
-      l = e * e;
-      g = e * ta * kk * (1.0f - kk);
+    __syncthreads();
+    const float dy0 = DY[smp * 2], dy1 = DY[smp * 2 + 1];
+#pragma unroll
+    for (int o = o0; o < o0 + kTO; o += 4) {
+      float4 d = *reinterpret_cast<float4 *>(d2v + o);
+      const float4 wa = *reinterpret_cast<const float4 *>(W3 + o), wb = *reinterpret_cast<const float4 *>(W3 + kHid + o);
+      d.x *= fmaf(wb.x, dy1, wa.x * dy0);
+      d.y *= fmaf(wb.y, dy1, wa.y * dy0);
+      d.z *= fmaf(wb.z, dy1, wa.z * dy0);
+      d.w *= fmaf(wb.w, dy1, wa.w * dy0);
+      *reinterpret_cast<float4 *>(d2v + o) = d;
     }
-    DY[smp * 2 + o] = g / (float)B;
+    __syncthreads();
+    {
+      float g1[kTO];
+#pragma unroll
+      for (int k = 0; k < kTO; ++k) g1[k] = 0.f;
+#pragma unroll 4
+      for (int o = 0; o < kHid; o += 4) {
+        const float4 d = *reinterpret_cast<const float4 *>(d2v + o);
+        const float dd[4] = {d.x, d.y, d.z, d.w};
+#pragma unroll
+        for (int u = 0; u < 4; ++u)
+#pragma unroll
+          for (int k = 0; k < kTO; k += 4) {
+            const float4 w = *reinterpret_cast<const float4 *>(W2 + (o + u) * kHid + o0 + k);
+            g1[k] = fmaf(w.x, dd[u], g1[k]);
+            g1[k + 1] = fmaf(w.y, dd[u], g1[k + 1]);
+            g1[k + 2] = fmaf(w.z, dd[u], g1[k + 2]);
+            g1[k + 3] = fmaf(w.w, dd[u], g1[k + 3]);
+          }
+      }
+#pragma unroll
+      for (int k = 0; k < kTO; k += 4) {
+        float4 d = *reinterpret_cast<float4 *>(d1v + o0 + k);
+        d.x *= g1[k];
+        d.y *= g1[k + 1];
+        d.z *= g1[k + 2];
+        d.w *= g1[k + 3];
+        *reinterpret_cast<float4 *>(d1v + o0 + k) = d;
+      }
+    }
+    __syncthreads();
+    if (tid < kT1 + kT2) {
+      const float *D = (first ? D1 : D2) + to, *A = (first ? X : H1) + tk;
+      const int sA = first ? sX : sH;
+#pragma unroll 4
+      for (int q = 0; q < kTB; ++q) {
+        const float4 d = *reinterpret_cast<const float4 *>(D + q * sH), a = *reinterpret_cast<const float4 *>(A + q * sA);
+        const float dv[4] = {d.x, d.y, d.z, d.w}, av[4] = {a.x, a.y, a.z, a.w};
+#pragma unroll
+        for (int u = 0; u < 4; ++u)
+#pragma unroll
+          for (int w = 0; w < 4; ++w) gs[u][w] = fmaf(dv[u], av[w], gs[u][w]);
+      }
+    } else {
+      // The biases' and W3's sums.
+#pragma unroll
+      for (int v = 0; v < 2; ++v) {
+        const int e = tid - kT1 - kT2 + v * kTS;
+        float s = gs[0][v];
+        if (e < kHid) {
+          for (int q = 0; q < kTB; ++q) s += D1[q * sH + e];
+        } else if (e < 2 * kHid) {
+          for (int q = 0; q < kTB; ++q) s += D2[q * sH + e - kHid];
+        } else if (e < 2 * kHid + kOut * kHid) {
+          const int o = (e - 2 * kHid) / kHid, k = e % kHid;
+          for (int q = 0; q < kTB; ++q) s = fmaf(DY[q * 2 + o], H2[q * sH + k], s);
+        } else if (e < kSums) {
+          for (int q = 0; q < kTB; ++q) s += DY[q * 2 + e - 2 * kHid - kOut * kHid];
+        }
+        gs[0][v] = s;
+      }
+    }
+  } while (LOOP && (long)(chunk += gridDim.x) * kTB < B);
+  // The block's loss and gradient sums go to its own slots (summed over the
+  // blocks in order by k_abc_reduce: the result does not depend on timing).
+  if (grp < kOut) {
     for (int m = 16; m > 0; m >>= 1) l += __shfl_xor_sync(0xffffffffu, l, m);
     if ((tid & 31) == 0) wl[tid >> 5] = l;
   }
-  __syncthreads();
-  const float dy0 = DY[smp * 2], dy1 = DY[smp * 2 + 1];
-#pragma unroll
-  for (int o = o0; o < o0 + kTO; o += 4) {
-    float4 d = *reinterpret_cast<float4 *>(d2v + o);
-    const float4 wa = *reinterpret_cast<const float4 *>(W3 + o), wb = *reinterpret_cast<const float4 *>(W3 + kHid + o);
-    d.x *= fmaf(wb.x, dy1, wa.x * dy0);
-    d.y *= fmaf(wb.y, dy1, wa.y * dy0);
-    d.z *= fmaf(wb.z, dy1, wa.z * dy0);
-    d.w *= fmaf(wb.w, dy1, wa.w * dy0);
-    *reinterpret_cast<float4 *>(d2v + o) = d;
-  }
-  __syncthreads();
-  {
-    float g1[kTO];
-#pragma unroll
-    for (int k = 0; k < kTO; ++k) g1[k] = 0.f;
-#pragma unroll 4
-    for (int o = 0; o < kHid; o += 4) {
-      const float4 d = *reinterpret_cast<const float4 *>(d2v + o);
-      const float dd[4] = {d.x, d.y, d.z, d.w};
-#pragma unroll
-      for (int u = 0; u < 4; ++u)
-#pragma unroll
-        for (int k = 0; k < kTO; k += 4) {
-          const float4 w = *reinterpret_cast<const float4 *>(W2 + (o + u) * kHid + o0 + k);
-          g1[k] = fmaf(w.x, dd[u], g1[k]);
-          g1[k + 1] = fmaf(w.y, dd[u], g1[k + 1]);
-          g1[k + 2] = fmaf(w.z, dd[u], g1[k + 2]);
-          g1[k + 3] = fmaf(w.w, dd[u], g1[k + 3]);
-        }
-    }
-#pragma unroll
-    for (int k = 0; k < kTO; k += 4) {
-      float4 d = *reinterpret_cast<float4 *>(d1v + o0 + k);
-      d.x *= g1[k];
-      d.y *= g1[k + 1];
-      d.z *= g1[k + 2];
-      d.w *= g1[k + 3];
-      *reinterpret_cast<float4 *>(d1v + o0 + k) = d;
-    }
-  }
-  // The block's loss and gradient sums go to its own slots (summed over the
-  // blocks in order by k_abc_reduce: the result does not depend on timing).
   __syncthreads();
   if (tid == 0) {
     float bl = 0.f;
@@ -1302,48 +1353,19 @@ __global__ void __launch_bounds__(kTT) k_abc_train(const float *feat, const floa
     lpartial[blockIdx.x] = bl / (2.0f * (float)B);
   }
   float *out = partial + (size_t)blockIdx.x * kNP;
-  constexpr int kT1 = kHid / 4 * (kIn / 4), kT2 = kHid / 4 * (kHid / 4);  // 4 x 4 tiles of the W1 and W2 sums
-  static_assert(kT1 + kT2 <= kTT, "a thread takes at most one tile");
   if (tid < kT1 + kT2) {
-    const bool first = tid < kT1;
-    const int nk = first ? kIn : kHid, t = first ? tid : tid - kT1;
-    const int o = 4 * (t / (nk / 4)), k = 4 * (t % (nk / 4));
-    const float *D = (first ? D1 : D2) + o, *A = (first ? X : H1) + k;
-    const int sA = first ? sX : sH;
-    float g[4][4] = {};
-#pragma unroll 4
-    for (int q = 0; q < kTB; ++q) {
-      const float4 d = *reinterpret_cast<const float4 *>(D + q * sH), a = *reinterpret_cast<const float4 *>(A + q * sA);
-      const float dv[4] = {d.x, d.y, d.z, d.w}, av[4] = {a.x, a.y, a.z, a.w};
-#pragma unroll
-      for (int u = 0; u < 4; ++u)
-#pragma unroll
-        for (int w = 0; w < 4; ++w) g[u][w] = fmaf(dv[u], av[w], g[u][w]);
-    }
-    float *dst = out + (first ? oW1 : oW2) + o * nk + k;
+    float *dst = out + (first ? oW1 : oW2) + to * nk + tk;
 #pragma unroll
     for (int u = 0; u < 4; ++u)
 #pragma unroll
-      for (int w = 0; w < 4; ++w) dst[u * nk + w] = g[u][w];
+      for (int w = 0; w < 4; ++w) dst[u * nk + w] = gs[u][w];
   } else {
-    // The biases' and W3's sums.
-    for (int e = tid - kT1 - kT2; e < 2 * kHid + kOut * kHid + kOut; e += kTT - kT1 - kT2) {
-      float s = 0.f;
-      if (e < kHid) {
-        for (int q = 0; q < kTB; ++q) s += D1[q * sH + e];
-        out[oB1 + e] = s;
-      } else if (e < 2 * kHid) {
-        for (int q = 0; q < kTB; ++q) s += D2[q * sH + e - kHid];
-        out[oB2 + e - kHid] = s;
-      } else if (e < 2 * kHid + kOut * kHid) {
-        const int o = (e - 2 * kHid) / kHid, k = e % kHid;
-        for (int q = 0; q < kTB; ++q) s = fmaf(DY[q * 2 + o], H2[q * sH + k], s);
-        out[oW3 + o * kHid + k] = s;
-      } else {
-        const int o = e - 2 * kHid - kOut * kHid;
-        for (int q = 0; q < kTB; ++q) s += DY[q * 2 + o];
-        out[oB3 + o] = s;
-      }
+#pragma unroll
+    for (int v = 0; v < 2; ++v) {
+      const int e = tid - kT1 - kT2 + v * kTS;
+      const int at = e < kHid ? oB1 + e : e < 2 * kHid ? oB2 + e - kHid : e < 2 * kHid + kOut * kHid
+                         ? oW3 + e - 2 * kHid : oB3 + e - 2 * kHid - kOut * kHid;
+      if (e < kSums) out[at] = gs[0][v];
     }
   }
 }
@@ -1489,10 +1511,23 @@ int grid_of(long n, int block) {
   return (int)(b < 1 ? 1 : (b > 4096 ? 4096 : b));
 }
 
+int train_blocks(int n) {
+  const int chunks = (n - 1) / kTB + 1;
+  return chunks <= kTrainOnce ? chunks : kTrainLoop;
+}
+
+void launch_train(const float *feat, const float *tgt, long nsamp, int B, uint32_t seed, float noise, float *partial,
+                  float *lpartial, cudaStream_t s) {
+  const int blocks = train_blocks(B);
+  const auto kern = blocks * kTB < B ? k_abc_train<true> : k_abc_train<false>;
+  kern<<<blocks, kTT, kTrainSmem, s>>>(feat, tgt, nsamp, B, seed, T.P, noise, partial, lpartial);
+}
+
 int train_attr() {
   static bool done = false;
   if (!done) {
-    CKA(cudaFuncSetAttribute(k_abc_train, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTrainSmem));
+    for (auto kern : {k_abc_train<false>, k_abc_train<true>})
+      CKA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTrainSmem));
     done = true;
   }
   return FLETCHER_OK;
@@ -1681,7 +1716,7 @@ extern "C" int FLETCHER_AbcTrain(int iters, int batch, float lr, unsigned seed, 
     return err(FLETCHER_ERR_ARGS, "AbcTrain: bad arguments");
   cudaStream_t s = stream_of();
   if (train_attr()) return FLETCHER_GetLastError();
-  const int blocks = (batch + kTB - 1) / kTB;
+  const int blocks = train_blocks(batch);
   float *loss = nullptr, *partial = nullptr, *lpartial = nullptr;
   CKA(cudaMalloc(&loss, iters * sizeof(float)));
   CKA(cudaMalloc(&partial, (size_t)blocks * kNP * sizeof(float)));
@@ -1690,7 +1725,7 @@ extern "C" int FLETCHER_AbcTrain(int iters, int batch, float lr, unsigned seed, 
   for (int it = 0; it < iters; ++it) {
     uint64_t st = (uint64_t)seed * 1000003ull + (uint64_t)it;
     const uint32_t sd = (uint32_t)splitmix(st) | 1u;
-    k_abc_train<<<blocks, kTT, kTrainSmem, s>>>(T.feat, T.tgt, ns, batch, sd, T.P, noise, partial, lpartial);
+    launch_train(T.feat, T.tgt, ns, batch, sd, noise, partial, lpartial, s);
     k_abc_reduce<<<kReduceBlocks, 32 * kReduceWarps, 0, s>>>(partial, lpartial, blocks, T.grad, loss + it);
     ++T.adam_t;
     const float lr_t = lr * 0.5f * (1.0f + cosf(3.14159265f * (float)it / (float)iters));
@@ -1711,7 +1746,7 @@ extern "C" int FLETCHER_AbcGradient(const float *feat, const float *tgt, int n, 
   if (!T.weights) return err(FLETCHER_ERR_ARGS, "AbcGradient: no network");
   if (!feat || !tgt || !grad || n < 1) return err(FLETCHER_ERR_ARGS, "AbcGradient: bad arguments");
   if (train_attr()) return FLETCHER_GetLastError();
-  const int blocks = (n + kTB - 1) / kTB;
+  const int blocks = train_blocks(n);
   float *df = nullptr, *dt = nullptr, *dl = nullptr, *dg = nullptr, *partial = nullptr, *lpartial = nullptr;
   CKA(cudaMalloc(&df, (size_t)n * kIn * sizeof(float)));
   CKA(cudaMalloc(&dt, (size_t)n * kTgt * sizeof(float)));
@@ -1721,7 +1756,7 @@ extern "C" int FLETCHER_AbcGradient(const float *feat, const float *tgt, int n, 
   CKA(cudaMalloc(&lpartial, blocks * sizeof(float)));
   CKA(cudaMemcpy(df, feat, (size_t)n * kIn * sizeof(float), cudaMemcpyHostToDevice));
   CKA(cudaMemcpy(dt, tgt, (size_t)n * kTgt * sizeof(float), cudaMemcpyHostToDevice));
-  k_abc_train<<<blocks, kTT, kTrainSmem>>>(df, dt, n, n, 0u, T.P, 0.f, partial, lpartial);
+  launch_train(df, dt, n, n, 0u, 0.f, partial, lpartial, 0);
   k_abc_reduce<<<kReduceBlocks, 32 * kReduceWarps>>>(partial, lpartial, blocks, dg, dl);
   CKA(cudaGetLastError());
   CKA(cudaMemcpy(grad, dg, kNP * sizeof(float), cudaMemcpyDeviceToHost));

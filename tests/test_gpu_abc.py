@@ -78,10 +78,11 @@ def test_inference_path_vs_cpu_oracle():
     assert rel(y, oy) < 1e-2
 
 
-@pytest.mark.parametrize("n", [1, 15, 16, 17, 63, 64, 65, 129])
+@pytest.mark.parametrize("n", [1, 15, 16, 17, 63, 64, 65, 129, 13312, 13313, 19521])
 def test_network_batch_edges_vs_cpu_oracle(n):
     """Loss, gradient and outputs where a training block of 64 samples and an
-    inference tile of 16 rows begin and end.  In so few samples an FP16
+    inference tile of 16 rows begin and end, and where a block begins to take
+    several chunks of 64 (from 13 313 samples).  In few samples an FP16
     rounding that falls the other way is not averaged out: it changes one of
     a sample's 32 activations by 2^-11 of itself, so loss and gradient are
     held to 2^-10."""
