@@ -1782,7 +1782,11 @@ int batch_seal(int rows, int stages) {
 // 108^3 (20) FP32 211 -> 235, 16-bit 314 -> 265.  So the line lies at 14 planes
 // a CTA for FP32, which streams from DRAM (pool pieces share no halos), and
 // at 64 for the 16-bit forms (6 shots of 158^3, 52 planes: FP16X 429 -> 404).
-constexpr double kPooledPlanes = 64.0, kPooledPlanesHbm = 14.0;
+// In the pool a tile with few rows counts at least kPooledRowShare of a full
+// one, more than in a large grid's plan: its pieces are short, their time the
+// latency of their planes.  At 0.8, 0.9 and 1: 24 shots of 48^3 64.3, 60.4 and
+// 60.8 us a step, 24 of 64^3 156, 148 and 147, FP16X 24 of 48^3 83.4, 79.2 and 81.2.
+constexpr double kPooledPlanes = 64.0, kPooledPlanesHbm = 14.0, kPooledRowShare = 0.9;
 int batch_plan(int ctas) {
   if (B.d_plan && B.plan_ctas == ctas) return FLETCHER_OK;
   if (B.d_plan) cudaFree(B.d_plan);
@@ -1815,7 +1819,8 @@ int batch_plan(int ctas) {
       const int shot = B.order[oi];
       const BatchShot &s = B.shots[shot];
       if (pooled[oi]) {
-        const int last = last_tile_rows(s.sy, B.bord, s.nty, TY);
+        const int last =
+            std::max(last_tile_rows(s.sy, B.bord, s.nty, TY), (int)ceil(kPooledRowShare * TY));
         for (int t = 0; t < s.ntx * s.nty; ++t)
           pool.push_back(Column{t % s.ntx, kRadius + t / s.ntx * TY, B.bord, s.sz - B.bord,
                                 t / s.ntx == s.nty - 1 ? last : TY, shot});
