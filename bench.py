@@ -425,7 +425,7 @@ def run_gb300(args, ws, rank, local, group):
 def run_batch_form(args, ws, rank, local, group, shots=None):
     """C3: 48 independent shots of uneven size run as one batch, the whole
     time loop one CUDA graph, tile shape from the autotuner, schedule chosen
-    by the library (FLETCHER_BatchSetChains default: one chain of
+    by the library (FLETCHER_BatchSetChains default: one or two chains of
     single-shot launches when the shots fill the GPU on their own, else one
     persistent launch per step for all running shots); against the same
     shots run one after another through the single-shot path (one launch

@@ -40,7 +40,7 @@ class Batch:
 
     def __init__(self, bord=4, dx=12.5, dy=12.5, dz=12.5, dt=0.0006, form: str = "fp32", chains: int | None = None):
         """form: storage form of every shot's fields ("fp32", "fp16", "fp16x").
-        chains: schedule of an FP32 batch (FLETCHER_BatchSetChains; None keeps
+        chains: schedule of the batch (FLETCHER_BatchSetChains; None keeps
         the library's default)."""
         self.lib = _lib.load()
         self.lib.FLETCHER_ClearError()

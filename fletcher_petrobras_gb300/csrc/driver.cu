@@ -117,10 +117,9 @@ double g_init_mark[6];
 double now_s() {
   return std::chrono::duration<double>(std::chrono::steady_clock::now().time_since_epoch()).count();
 }
-// Coefficient layout of the FP32 form (FLETCHER_SetCoefLayout).  The plane
-// layout is the default: at 504^3 the media table, with 36% fewer bytes per
-// step, ran 3-5% slower (2.30-2.48 against 2.22 ms per step; the step is
-// bound by its per-plane chain of shared-memory reads, not by DRAM).
+// Coefficient layout of the FP32 form (FLETCHER_SetCoefLayout).  The planes,
+// which hold any model, are the default; the media table streams 36% fewer
+// bytes per step (504^3: 1.49 against 1.79 ms) for models of at most 256 media.
 int g_coef_layout = FLETCHER_COEF_PLANES;
 // Fault injection for the failure-path tests (FLETCHER_InjectFault): the
 // device allocation that fails (counted down, -1: none), and the stall of
@@ -819,9 +818,10 @@ int initialize(int sx, int sy, int sz, int bord, float dx, float dy, float dz, f
     return fail(FLETCHER_ERR_ARGS, "unknown storage form %d", g_form);
   const bool half = g_form != FLETCHER_FORM_FP32;
   const bool ext = g_form == FLETCHER_FORM_FP16X;
-  // Default shapes (measured at 504^3): 16 rows; 5 stages for FP32 (2.20 ms
-  // per step against 2.40 for 12 x 5) and FP16X (3.45 against 3.68 for 16 x 4),
-  // 4 for FP16 (3.02 against 3.18 for 16 x 5).
+  // Default shapes: 16 rows; 5 stages for FP32 (504^3 1.765 ms per step, 1.79
+  // with 4; 192^3 updated cells 73.3 us, 81 for 12 x 5 and 76 for 8 x 4) and
+  // FP16X (272^3 updated cells 274 us, 279 with 4), 4 for FP16 (298 x 249 x 215
+  // 189 us, 202 with 5).
   if (g_numerics == FLETCHER_NUMERICS_D1D1 && g_form != FLETCHER_FORM_FP32)
     return fail(FLETCHER_ERR_ARGS, "the Der1-Der1 numerics need the FP32 form");
   const bool d1d1 = g_numerics == FLETCHER_NUMERICS_D1D1;

@@ -48,7 +48,11 @@ constexpr int kMediaMax = 256;
 constexpr int kAngleCoef = 6;
 constexpr int kVelCoef = 4;
 constexpr int kIdShift = 12;
-constexpr int kMediaStages = 7;  // default pipeline depth of the media-table layout (fastest at 504^3)
+// Default pipeline depth of the media-table layout.  5, 6 and 7 stages, us a
+// step: 504^3 1487, 1573 and 1571, 272^3 updated cells 176, 193 and 189, 192^3
+// 63.7, 63.1 and 63.5 (with more stages the CTAs run further apart and share
+// less in L2).
+constexpr int kMediaStages = 5;
 static_assert((kRadius + kIdShift) % 16 == 0 && kTileX % 16 == 0, "id tiles must start on 16-byte boundaries");
 static_assert(DC_V2PX == kAngleCoef && DC_V2PN == kNumCoef - 1, "velocity terms follow the angle terms");
 

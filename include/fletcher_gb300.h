@@ -138,11 +138,9 @@ int FLETCHER_SetNumerics(int mode);
  *   pairs keeps them in a table, one byte per cell names the pair, and a
  *   step streams 41 bytes per cell (the four velocity coefficients stay per
  *   cell).  The floats used are the same, so results are bit-identical to
- *   FLETCHER_COEF_PLANES.  16-row tiles of 5, 6 or 7 stages (default 7).
- *   On GB300 at 504^3 it streams 36% fewer bytes but runs 3-5% slower than
- *   the planes (the step's limit is its per-plane chain of shared-memory
- *   reads, which the table lengthens, not DRAM); it leaves more HBM
- *   bandwidth to other work on the GPU.
+ *   FLETCHER_COEF_PLANES.  16-row tiles of 5, 6 or 7 stages (default 5).
+ *   On GB300 it streams 36% fewer bytes and a step takes 0.83 of the
+ *   planes' time at 504^3 (1.49 against 1.79 ms).
  *   DRIVER_Initialize fails with FLETCHER_ERR_ARGS when the model has more
  *   pairs, or with a 16-bit form or the Der1-Der1 numerics.
  * FLETCHER_COEF_AUTO: FLETCHER_COEF_MEDIA where the form, the numerics,
