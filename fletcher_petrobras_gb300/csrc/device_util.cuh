@@ -72,13 +72,12 @@ __device__ __forceinline__ bool mbar_wait(uint64_t *bar, uint32_t parity, uint64
   }
 }
 // The same with the limit counted in tries (a few instructions, where the
-// timed loop would bloat an unrolled caller): each try suspends the thread
-// for at most about kSpinHintNs, so the limit is about 2 s.
+// timed loop would bloat an unrolled caller).  A try suspends the thread for
+// at most about kSpinHintNs.
 constexpr uint32_t kSpinTries = 1u << 20, kSpinHintNs = 2000;
-__device__ __forceinline__ bool mbar_spin(uint64_t *bar, uint32_t parity) {
-  uint32_t n = kSpinTries;
+__device__ __forceinline__ bool mbar_spin(uint64_t *bar, uint32_t parity, uint32_t tries = kSpinTries) {
   while (!mbar_try_wait_hint(bar, parity, kSpinHintNs))
-    if (--n == 0) return false;
+    if (--tries == 0) return false;
   return true;
 }
 // Moves registers between the warpgroups of a CTA (warpgroup-uniform).

@@ -31,6 +31,7 @@
 #include <vector>
 
 #include "../../include/fletcher_gb300.h"
+#include "device_util.cuh"
 #include "fletcher_internal.h"
 
 using namespace flt;
@@ -122,11 +123,12 @@ double now_s() {
 // bytes per step (504^3: 1.49 against 1.79 ms) for models of at most 256 media.
 int g_coef_layout = FLETCHER_COEF_PLANES;
 // Fault injection for the failure-path tests (FLETCHER_InjectFault): the
-// device allocation that fails (counted down, -1: none), and the stall of
-// the next propagate launch (CTA 0's step to skip, -1: none; its wait limit).
+// device allocation that fails (counted down, -1: none), and the faults of the
+// next propagate launch (the step of CTA 0 whose loads are skipped, the one at
+// which a helper warp gives up, -1: none; the tries of its waits).
 int g_fault_alloc = -1;
-int g_fault_stall = -1;
-unsigned long long g_fault_wait_ns = 0;
+int g_fault_stall = -1, g_fault_quit = -1;
+unsigned g_fault_tries = kSpinTries;
 int g_last_err = FLETCHER_OK;
 char g_errmsg[512] = "";
 
@@ -1108,11 +1110,11 @@ int step() {
   P.dt2 = P.iso ? (g.dt * g.dt) * P.inv_dxx : g.dt * g.dt;
   P.dt = g.dt;
   P.err = g.err_dev;
-  // Every wait is bounded (2 s); an injected stall (tests) uses its own limit
-  // and applies to this one launch.
-  P.wait_ns = g_fault_stall >= 0 && g_fault_wait_ns ? g_fault_wait_ns : kWaitLimitNs;
+  // An injected fault (tests) applies to this one launch.
   P.stall_step = g_fault_stall;
-  g_fault_stall = -1;
+  P.quit_step = g_fault_quit;
+  P.wait_tries = g_fault_tries;
+  g_fault_stall = g_fault_quit = -1;
   ShotDesc &want = P.one;
   want = g.desc;
   want.src_x = want.src_y = want.src_z = -1000;
@@ -1388,18 +1390,18 @@ extern "C" int FLETCHER_InjectFault(int kind, int arg, int wait_us) {
   switch (kind) {
     case FLETCHER_FAULT_NONE:
       g_fault_alloc = -1;
-      g_fault_stall = -1;
-      g_fault_wait_ns = 0;
+      g_fault_stall = g_fault_quit = -1;
       return FLETCHER_OK;
     case FLETCHER_FAULT_ALLOC:
       if (arg < 0) return fail(FLETCHER_ERR_ARGS, "FLETCHER_InjectFault: allocation index must be >= 0");
       g_fault_alloc = arg;
       return FLETCHER_OK;
     case FLETCHER_FAULT_STALL:
+    case FLETCHER_FAULT_QUIT:
       if (arg < 0 || wait_us < 1000 || wait_us > 2000000)
-        return fail(FLETCHER_ERR_ARGS, "FLETCHER_InjectFault: stall step must be >= 0 and the wait 1 ms .. 2 s");
-      g_fault_stall = arg;
-      g_fault_wait_ns = (unsigned long long)wait_us * 1000ull;
+        return fail(FLETCHER_ERR_ARGS, "FLETCHER_InjectFault: step must be >= 0 and the wait 1 ms .. 2 s");
+      (kind == FLETCHER_FAULT_STALL ? g_fault_stall : g_fault_quit) = arg;
+      g_fault_tries = (unsigned)((unsigned long long)wait_us * 1000ull / kSpinHintNs);
       return FLETCHER_OK;
     default:
       return fail(FLETCHER_ERR_ARGS, "FLETCHER_InjectFault: unknown kind %d", kind);
@@ -1940,8 +1942,7 @@ int batch_issue(int it0, int it1, const float *src) {
   PropLaunch L;
   memset(&L, 0, sizeof(L));
   L.batch = true;
-  L.p.wait_ns = kWaitLimitNs;
-  L.p.stall_step = -1;
+  L.p.stall_step = L.p.quit_step = -1;
   L.tile_rows = B.sealed_rows;
   L.stages = B.stages;
   PropParams &P = L.p;
@@ -2028,8 +2029,7 @@ int batch_issue_chains(int chains, int steps, const float *src) {
   L.tile_rows = B.sealed_rows;
   L.stages = B.stages;
   PropParams &P = L.p;
-  P.wait_ns = kWaitLimitNs;
-  P.stall_step = -1;
+  P.stall_step = P.quit_step = -1;
   P.inv_dx = 1.0f / B.dx;
   P.inv_dy = 1.0f / B.dy;
   P.inv_dz = 1.0f / B.dz;

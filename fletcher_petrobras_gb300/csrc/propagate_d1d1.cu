@@ -52,6 +52,8 @@ constexpr size_t kSmem = size_t(OFF_ABC) + kABSlots * G::NT * 24 + 128;
 static_assert(kSmem <= 227 * 1024, "Der1-Der1 shape exceeds the shared memory of a CTA");
 static_assert(OFF_HDR % 128 == 0 && SB % 128 == 0 && OFF_ABC % 128 == 0, "shared-memory alignment");
 
+// HOOK: the fault-injection variant, as in propagate_fp32.cu.
+template <bool HOOK>
 __global__ void __launch_bounds__(kThreads, 1)
     k_propagate_d1d1(const __grid_constant__ SingleMaps SM, const __grid_constant__ PropParams P) {
   extern __shared__ unsigned char smem_dyn[];
@@ -77,6 +79,8 @@ __global__ void __launch_bounds__(kThreads, 1)
   __syncthreads();
   allow_next_launch();
   wait_previous_launch();
+  // Every wait is bounded.
+  auto wait = [&](uint64_t *b, uint32_t parity) { return mbar_spin(b, parity, HOOK ? P.wait_tries : kSpinTries); };
   const ShotDesc &sd = P.one;
   const f2 nz = splat(*reinterpret_cast<volatile float *>(smem + OFF_NZ));
 
@@ -107,13 +111,13 @@ __global__ void __launch_bounds__(kThreads, 1)
         for (int k = it.z0 - kRadius; k < it.z1 + kLag; ++k) {
           unsigned char *st = smem + stage * SB;
           // (The first S waits pass at once: the stage was never filled.)
-          if (!mbar_spin(bar(st, OFF_EMPTY), phase ^ 1u)) {
+          if (!wait(bar(st, OFF_EMPTY), phase ^ 1u)) {
             ok = false;
             break;
           }
           fence_proxy_async_smem();
           if (k == it.z0 - kRadius) *reinterpret_cast<int4 *>(st + OFF_HDR) = w;
-          issue_step<TY>(st, bar(st, OFF_FULL), it, k, maps);
+          if (!HOOK || issued != P.stall_step || blockIdx.x != 0) issue_step<TY>(st, bar(st, OFF_FULL), it, k, maps);
           ++issued;
           if (++stage == S) {
             stage = 0;
@@ -134,13 +138,23 @@ __global__ void __launch_bounds__(kThreads, 1)
     }
     // ---- halo warps ----
     const int hw = wid - CW - 1;
+    const int src_z = sd.src_z;
+    auto halo_barrier = [] { asm volatile("bar.sync 1, %0;" ::"n"(32 * kHaloWarps) : "memory"); };
+    [[maybe_unused]] int step = 0;
     for (int i = 0; i < nitems; ++i) {
       const Item it = decode_item<false>(seg[i]);
-      const int src_z = sd.src_z;
       for (int k = it.z0 - kRadius; k < it.z1 + kLag; ++k) {
         unsigned char *st = smem + stage * SB;
-        if (!mbar_spin(bar(st, OFF_FULL), phase)) {
-          atomicOr(P.err, 1u);
+        bool ok = wait(bar(st, OFF_FULL), phase);
+        if constexpr (HOOK) ok = ok && !(hw == 1 && blockIdx.x == 0 && step++ == P.quit_step);
+        if (!__all_sync(0xffffffffu, ok)) {
+          // Another halo warp's wait may have succeeded: this one meets the
+          // others at every barrier (below) still to come before it leaves.
+          if (lx == 0) atomicOr(P.err, 1u);
+          for (int a = i; a < nitems; ++a) {
+            const Item w = decode_item<false>(seg[a]);
+            if (src_z >= (a == i ? k : w.z0 - kRadius) && src_z < w.z1 + kLag) halo_barrier();
+          }
           return;
         }
         f2 *H = reinterpret_cast<f2 *>(st);
@@ -153,7 +167,7 @@ __global__ void __launch_bounds__(kThreads, 1)
             H[ry * G::HX + rx] = add2(H[ry * G::HX + rx], splat(P.src));
             fence_proxy_async_smem();
           }
-          asm volatile("bar.sync 1, %0;" ::"n"(32 * kHaloWarps) : "memory");
+          halo_barrier();
         }
         if (k >= it.z0 && k < it.z1) {
           // pDx of the tile's 4-row y halo (halo-tile rows 0..3 and TY+4..TY+7).
@@ -191,8 +205,8 @@ __global__ void __launch_bounds__(kThreads, 1)
   int abw = 0;  // shared A/B/C ring slot of the arriving plane (the plane kLag back is at abw + 1)
   unsigned char *st = smem;
   for (int item = 0; item < nitems; ++item) {
-    if (!mbar_spin(bar(st, OFF_READY), phase)) {
-      if (lx == 0) atomicOr(P.err, 1u);
+    if (!wait(bar(st, OFF_READY), phase)) {
+      atomicOr(P.err, 1u);
       return;
     }
     const Item it = decode_item<false>(uniform4(*reinterpret_cast<const int4 *>(st + OFF_HDR)));
@@ -217,8 +231,8 @@ __global__ void __launch_bounds__(kThreads, 1)
       for (int j = 0; j < kRing; ++j) {
         const int k = kb + j;  // plane, counted from the item's first
         if (k >= depth + kLag) break;
-        if (!mbar_spin(bar(st, OFF_READY), phase)) {
-          if (lx == 0) atomicOr(P.err, 1u);
+        if (!wait(bar(st, OFF_READY), phase)) {
+          atomicOr(P.err, 1u);
           return;
         }
         const bool center = (unsigned)k < (unsigned)depth;
@@ -316,8 +330,8 @@ __global__ void __launch_bounds__(kThreads, 1)
           out += plane;
         }
         if (center) {
-          if (!mbar_spin(bar(st, OFF_XCHG), phase)) {
-            if (lx == 0) atomicOr(P.err, 2u);
+          if (!wait(bar(st, OFF_XCHG), phase)) {
+            atomicOr(P.err, 2u);
             return;
           }
           // pxy = Der1_y(pDx) / dy (der1der1/sample.h:55); A = cpxx + cpyy,
@@ -356,16 +370,22 @@ __global__ void __launch_bounds__(kThreads, 1)
 
 }  // namespace
 
-// One shape (kD1D1Rows x kD1D1Stages), single shot.
-cudaError_t propagate_d1d1_launch(const PropLaunch &L, cudaStream_t s) {
+template <bool HOOK>
+static cudaError_t launch_d1d1(const PropLaunch &L, cudaStream_t s) {
   static bool ready = false;
   if (!ready) {
-    const cudaError_t e = cudaFuncSetAttribute(k_propagate_d1d1, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmem);
+    const cudaError_t e =
+        cudaFuncSetAttribute(k_propagate_d1d1<HOOK>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmem);
     if (e != cudaSuccess) return e;
     ready = true;
   }
+  return launch_step(k_propagate_d1d1<HOOK>, L.grid, kThreads, kSmem, s, L.m, L.p);
+}
+
+// One shape (kD1D1Rows x kD1D1Stages), single shot.
+cudaError_t propagate_d1d1_launch(const PropLaunch &L, cudaStream_t s) {
   if (L.batch || L.tile_rows != TY || L.stages != S) return cudaErrorInvalidValue;
-  return launch_step(k_propagate_d1d1, L.grid, kThreads, kSmem, s, L.m, L.p);
+  return fault_injected(L.p) ? launch_d1d1<true>(L, s) : launch_d1d1<false>(L, s);
 }
 
 }  // namespace flt

@@ -125,9 +125,9 @@ struct Regs {
                 "the split exceeds the launch's registers");
 };
 
-// HOOK: the fault-injection variant (waits limited to P.wait_ns, CTA 0
-// skipping the loads of step P.stall_step), launched only when a test
-// injects a stall.  MT: the media-table layout of the coefficients.
+// HOOK: the fault-injection variant (waits limited to P.wait_tries tries, CTA 0
+// skipping the loads of its P.stall_step-th step, or one of its halo warps
+// giving up at its P.quit_step-th), launched only when a test injects a fault.  MT: the media-table layout of the coefficients.
 template <int TY, int S, bool ISO, bool BATCH, int MINB, bool HOOK = false, bool MT = false>
 __global__ void __launch_bounds__(kTileX *(Regs<TY>::kWarps + kHelperWarps), MINB)
     k_propagate_fp32(const __grid_constant__ SingleMaps SM, const __grid_constant__ PropParams P) {
@@ -163,11 +163,8 @@ __global__ void __launch_bounds__(kTileX *(Regs<TY>::kWarps + kHelperWarps), MIN
   __syncthreads();
   allow_next_launch();
   wait_previous_launch();
-  // Every wait is bounded; the fault-injection variant's by P.wait_ns.
-  auto wait = [&](uint64_t *b, uint32_t parity) {
-    if constexpr (HOOK) return mbar_wait(b, parity, P.wait_ns);
-    else return mbar_spin(b, parity);
-  };
+  // Every wait is bounded.
+  auto wait = [&](uint64_t *b, uint32_t parity) { return mbar_spin(b, parity, HOOK ? P.wait_tries : kSpinTries); };
 
   if (wid >= CW) {
     setmaxnreg_dec<kHelperRegs>();
@@ -252,6 +249,8 @@ __global__ void __launch_bounds__(kTileX *(Regs<TY>::kWarps + kHelperWarps), MIN
     const int hw = wid - CW - 1;
     if (hw >= kHalo) return;
     const int hxc = (lx & 7) < 4 ? (lx & 7) : G::TX + (lx & 7);  // lane -> halo column, row lane / 8 of a group of 4
+    [[maybe_unused]] int step = 0;
+    auto halo_barrier = [] { asm volatile("bar.sync 1, %0;" ::"n"(32 * kHalo) : "memory"); };
     int rb = 0;
     for (int i = 0; i < nitems; ++i) {
       const Item it = decode_item<BATCH>(seg[i]);
@@ -265,8 +264,18 @@ __global__ void __launch_bounds__(kTileX *(Regs<TY>::kWarps + kHelperWarps), MIN
           const int es = stage >= L::NB ? stage - L::NB : stage + S - L::NB;
           ok = ok && wait(bar(smem + es * L::SB, L::OFF_EMPTY), stage >= L::NB ? phase : phase ^ 1u);
         }
-        if (!ok) {
-          atomicOr(P.err, 1u);
+        // Test hook: a halo warp of CTA 0 gives up at its P.quit_step-th step.
+        if constexpr (HOOK) ok = ok && !(hw == 1 && blockIdx.x == 0 && step++ == P.quit_step);
+        if (!__all_sync(0xffffffffu, ok)) {
+          // Another halo warp's wait may have succeeded: this one meets the
+          // others at every barrier (below) still to come before it leaves, so
+          // that none waits there for a warp that has left.
+          if (lx == 0) atomicOr(P.err, 1u);
+          for (int a = i; a < nitems; ++a) {
+            const Item w = decode_item<BATCH>(seg[a]);
+            const int zs = (BATCH ? P.shots[w.shot] : P.one).src_z;
+            if (zs >= (a == i ? k : w.z0 - kRadius) && zs < w.z1 + kLag) halo_barrier();
+          }
           return;
         }
         f2 *H = reinterpret_cast<f2 *>(st);
@@ -279,7 +288,7 @@ __global__ void __launch_bounds__(kTileX *(Regs<TY>::kWarps + kHelperWarps), MIN
             H[ry * G::HX + rx] = add2(H[ry * G::HX + rx], splat(P.src));
             fence_proxy_async_smem();
           }
-          asm volatile("bar.sync 1, %0;" ::"n"(32 * kHalo) : "memory");
+          halo_barrier();
         }
         if (k >= it.z0 && k < it.z1) {
           f2 *db = reinterpret_cast<f2 *>(L::ROWS_IN ? st + L::OFF_SROWS : smem + L::OFF_ROWS + rb * G::ROW_B);
@@ -325,7 +334,7 @@ __global__ void __launch_bounds__(kTileX *(Regs<TY>::kWarps + kHelperWarps), MIN
   unsigned char *st = smem;
   for (int item = 0; item < nitems; ++item) {
     if (!wait(bar(st, L::OFF_READY), phase)) {
-      if (lx == 0) atomicOr(P.err, 1u);
+      atomicOr(P.err, 1u);
       return;
     }
     const Item it = decode_item<BATCH>(uniform4(*reinterpret_cast<const int4 *>(st + L::OFF_HDR)));
@@ -352,7 +361,7 @@ __global__ void __launch_bounds__(kTileX *(Regs<TY>::kWarps + kHelperWarps), MIN
       // rows; 312^3 updated cells 304.7 -> 308.5 us.)
       for (int k = -kRadius; k < depth + kLag; ++k) {
         if (!wait(bar(st, L::OFF_READY), phase)) {
-          if (lx == 0) atomicOr(P.err, 1u);
+          atomicOr(P.err, 1u);
           return;
         }
         __syncwarp();
@@ -376,7 +385,7 @@ __global__ void __launch_bounds__(kTileX *(Regs<TY>::kWarps + kHelperWarps), MIN
         const int k = kb + j;  // plane, counted from the item's first
         if (k >= depth + kLag) break;
         if (!wait(bar(st, L::OFF_READY), phase)) {
-          if (lx == 0) atomicOr(P.err, 1u);
+          atomicOr(P.err, 1u);
           return;
         }
         unsigned char *const st_next = stage == S - 1 ? smem : st + L::SB;
@@ -605,7 +614,7 @@ static cudaError_t launch_hook(const PropLaunch &L, cudaStream_t s) {
   constexpr size_t smem = smem_bytes<TY, S>();
   // Any pipeline depth of the step's own shape: the plan depends on the rows
   // only.  (The coefficient planes are present in either layout.)
-  if (L.batch || L.d1d1 || L.tile_rows != TY) return cudaErrorInvalidValue;
+  if (L.batch || L.tile_rows != TY) return cudaErrorInvalidValue;
   auto kern = L.p.iso ? k_propagate_fp32<TY, S, true, false, 1, true> : k_propagate_fp32<TY, S, false, false, 1, true>;
   const cudaError_t e = set_smem(kern, smem);
   if (e != cudaSuccess) return e;
@@ -641,8 +650,8 @@ bool propagate_fp32_media_supported(int ty, int st) {
 }
 
 cudaError_t propagate_fp32_launch(const PropLaunch &L, cudaStream_t s) {
-  if (L.p.stall_step >= 0) return launch_hook(L, s);
   if (L.d1d1) return propagate_d1d1_launch(L, s);
+  if (fault_injected(L.p)) return launch_hook(L, s);
   if (L.media) {
     if (L.batch || !L.p.media) return cudaErrorInvalidValue;
 #define X(a, b) \

@@ -245,8 +245,9 @@ __device__ __forceinline__ void issue_half(unsigned char *stage, uint64_t *bar, 
 __host__ __device__ constexpr bool own_scales(bool ext, bool batch) { return ext && !batch; }
 
 // BATCH: the items belong to the shots of a batch (P.shots, H.hshots,
-// H.hmaps: buffers, exponents and tensor maps by shot).
-template <int TY, int S, bool ISO, bool EXT, bool BATCH>
+// H.hmaps: buffers, exponents and tensor maps by shot).  HOOK: the
+// fault-injection variant, as in propagate_fp32.cu.
+template <int TY, int S, bool ISO, bool EXT, bool BATCH, bool HOOK = false>
 __global__ void __launch_bounds__(RegsH<TY, EXT>::kThreads, 1)
     k_propagate_half(const __grid_constant__ HalfMaps M, const __grid_constant__ HalfParams H) {
   using G = GeoH<TY, EXT>;
@@ -280,6 +281,8 @@ __global__ void __launch_bounds__(RegsH<TY, EXT>::kThreads, 1)
   __syncthreads();
   allow_next_launch();
   wait_previous_launch();
+  // Every wait is bounded.
+  auto wait = [&](uint64_t *b, uint32_t parity) { return mbar_spin(b, parity, HOOK ? P.wait_tries : kSpinTries); };
 
   if (wid >= TY) {
     setmaxnreg_dec<RegsH<TY, EXT>::kHelper>();
@@ -361,7 +364,7 @@ __global__ void __launch_bounds__(RegsH<TY, EXT>::kThreads, 1)
         }
         unsigned char *st = smem + stage * L::SB;
         // (The first S waits pass at once: the stage was never filled.)
-        if (!mbar_spin(bar(st, L::OFF_EMPTY), phase ^ 1u)) {
+        if (!wait(bar(st, L::OFF_EMPTY), phase ^ 1u)) {
           ok = false;
           break;
         }
@@ -373,7 +376,8 @@ __global__ void __launch_bounds__(RegsH<TY, EXT>::kThreads, 1)
           if (ck == cit.z0 - kRadius) *reinterpret_cast<int4 *>(st + L::OFF_HDR) = cw;
           *plane_of(st) = make_int2(upd ? zc : -1, cit.shot);
           if constexpr (OWN_SCALES) *scale_of(st) = scl;
-          issue_half<TY, EXT>(st, bar(st, L::OFF_FULL), cit, ck, maps_of(cit.shot));
+          if (!HOOK || issued != P.stall_step || blockIdx.x != 0)
+            issue_half<TY, EXT>(st, bar(st, L::OFF_FULL), cit, ck, maps_of(cit.shot));
           fold_max(pl, sc, v);
           if (OWN_SCALES && upd) {
             // Every CTA of the plane finds and stores the same.
@@ -388,12 +392,15 @@ __global__ void __launch_bounds__(RegsH<TY, EXT>::kThreads, 1)
           phase ^= 1u;
         }
       }
-      if (lx != 0) return;
+      if (lx != 0) {
+        if (!ok) atomicOr(P.err, 2u);
+        return;
+      }
       // The maxima of the last steps, in order.
       for (int a = issued < S ? issued : S; a >= 1 && ok; --a) {
         const int s2 = stage >= a ? stage - a : stage + S - a;
         unsigned char *st = smem + s2 * L::SB;
-        if (!mbar_spin(bar(st, L::OFF_EMPTY), stage >= a ? phase : phase ^ 1u)) ok = false;
+        if (!wait(bar(st, L::OFF_EMPTY), stage >= a ? phase : phase ^ 1u)) ok = false;
         else fold_max(*plane_of(st), scale_of(st)->z, take_max(st));
       }
       if (!ok) {
@@ -413,6 +420,8 @@ __global__ void __launch_bounds__(RegsH<TY, EXT>::kThreads, 1)
     const int dt = hw * 32 + lx;  // thread among the decode warps
     constexpr int NDT = 32 * kDecodeWarps;
     const int hxc = (lx & 7) < 4 ? (lx & 7) : G::TX + (lx & 7);  // lane -> halo column, row lane / 8 of a group of 4
+    auto decode_barrier = [] { asm volatile("bar.sync 1, %0;" ::"n"(NDT) : "memory"); };
+    [[maybe_unused]] int step = 0;
     int ds = 0;
     for (int i = 0; i < nitems; ++i) {
       const HItem it = decode_hitem<BATCH>(seg[i]);
@@ -442,9 +451,18 @@ __global__ void __launch_bounds__(RegsH<TY, EXT>::kThreads, 1)
         // (With ND = S that is the step whose stage was refilled.)
         const int es = stage >= L::ND ? stage - L::ND : stage + S - L::ND;
         unsigned char *st = smem + stage * L::SB;
-        if ((L::ND < S && !mbar_spin(bar(smem + es * L::SB, L::OFF_EMPTY), stage >= L::ND ? phase : phase ^ 1u)) ||
-            !mbar_spin(bar(st, L::OFF_FULL), phase)) {
-          atomicOr(P.err, 1u);
+        bool ok = (L::ND == S || wait(bar(smem + es * L::SB, L::OFF_EMPTY), stage >= L::ND ? phase : phase ^ 1u)) &&
+                  wait(bar(st, L::OFF_FULL), phase);
+        if constexpr (HOOK) ok = ok && !(hw == 1 && blockIdx.x == 0 && step++ == P.quit_step);
+        if (!__all_sync(0xffffffffu, ok)) {
+          // Another decode warp's wait may have succeeded: this one meets the
+          // others at every barrier (below) still to come before it leaves, so
+          // that none waits there for a warp that has left.
+          if (lx == 0) atomicOr(P.err, 1u);
+          for (int a = i; a < nitems; ++a) {
+            const HItem w = decode_hitem<BATCH>(seg[a]);
+            for (int z = a == i ? max(k, w.z0) : w.z0; z < w.z1; ++z) decode_barrier();
+          }
           return;
         }
         f2 *Hs = reinterpret_cast<f2 *>(smem + L::OFF_TILES + ds * L::TILE_B);
@@ -481,7 +499,7 @@ __global__ void __launch_bounds__(RegsH<TY, EXT>::kThreads, 1)
         if (k >= it.z0 && k < it.z1) {
           // D1y in the halo columns, from rows that the other decode warps
           // wrote too.
-          asm volatile("bar.sync 1, %0;" ::"n"(NDT) : "memory");
+          decode_barrier();
           f2 *db = Hs + G::HXY;
           for (int r = hw * 4 + (lx >> 3); r < TY; r += 4 * kDecodeWarps) {
             const f2 *h = Hs + (r + kRadius) * G::HX + hxc;
@@ -520,8 +538,8 @@ __global__ void __launch_bounds__(RegsH<TY, EXT>::kThreads, 1)
   int abw = 0;  // shared A/B ring slot of the arriving plane (the plane 4 back is at abw + 1)
   unsigned char *st = smem;
   for (int item = 0; item < nitems; ++item) {
-    if (!mbar_spin(bar(st, L::OFF_READY), phase)) {
-      if (lx == 0) atomicOr(P.err, 1u);
+    if (!wait(bar(st, L::OFF_READY), phase)) {
+      atomicOr(P.err, 1u);
       return;
     }
     const HItem it = decode_hitem<BATCH>(uniform4(*reinterpret_cast<const int4 *>(st + L::OFF_HDR)));
@@ -541,8 +559,8 @@ __global__ void __launch_bounds__(RegsH<TY, EXT>::kThreads, 1)
       // A row outside the updated region: nothing to compute, only the
       // stages to release in step.
       for (int k = -kRadius; k < depth + kRadius; ++k) {
-        if (!mbar_spin(bar(st, L::OFF_READY), phase)) {
-          if (lx == 0) atomicOr(P.err, 1u);
+        if (!wait(bar(st, L::OFF_READY), phase)) {
+          atomicOr(P.err, 1u);
           return;
         }
         __syncwarp();
@@ -565,8 +583,8 @@ __global__ void __launch_bounds__(RegsH<TY, EXT>::kThreads, 1)
       for (int j = 0; j < 9; ++j) {
         const int k = kb + j;  // plane, counted from the item's first
         if (k >= depth + kRadius) break;
-        if (!mbar_spin(bar(st, L::OFF_READY), phase)) {
-          if (lx == 0) atomicOr(P.err, 1u);
+        if (!wait(bar(st, L::OFF_READY), phase)) {
+          atomicOr(P.err, 1u);
           return;
         }
         unsigned char *const st_next = stage == S - 1 ? smem : st + L::SB;
@@ -646,8 +664,8 @@ __global__ void __launch_bounds__(RegsH<TY, EXT>::kThreads, 1)
           if (lx == 0 && mb) atomicMax(max_of(st), mb);
         }
         if (center) {
-          if (!mbar_spin(bar(st, L::OFF_HALO), phase)) {
-            if (lx == 0) atomicOr(P.err, 2u);
+          if (!wait(bar(st, L::OFF_HALO), phase)) {
+            atomicOr(P.err, 2u);
             return;
           }
           const f2 dxy = scale<ISO>(d1(dr[1], dr[-1], dr[2], dr[-2], dr[3], dr[-3], dr[4], dr[-4]), sxy);
@@ -775,6 +793,20 @@ static cudaError_t launch_half_t(const HalfLaunch &L, cudaStream_t s) {
   return launch_step(kern, L.grid, RegsH<TY, EXT>::kThreads, LayoutH<TY, S, EXT>::BYTES, s, L.m, L.h);
 }
 
+// The fault-injection variant: the form's default shape, single shot,
+// isotropic grid.  (Any pipeline depth of the step's own shape: the plan and
+// the maps depend on the rows only.)
+template <bool EXT>
+static cudaError_t launch_half_hook(const HalfLaunch &L, cudaStream_t s) {
+  constexpr int TY = 16, S = EXT ? 5 : 4;
+  if (L.batch || L.tile_rows != TY || !L.h.p.iso) return cudaErrorInvalidValue;
+  auto kern = k_propagate_half<TY, S, true, EXT, false, true>;
+  const cudaError_t e =
+      cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)LayoutH<TY, S, EXT>::BYTES);
+  if (e != cudaSuccess) return e;
+  return launch_step(kern, L.grid, RegsH<TY, EXT>::kThreads, LayoutH<TY, S, EXT>::BYTES, s, L.m, L.h);
+}
+
 bool propagate_half_supported(int tile_rows, int stages) {
 #define X(a, b) \
   if (tile_rows == a && stages == b) return true;
@@ -795,6 +827,7 @@ cudaError_t propagate_half_launch(const HalfLaunch &L, bool ext, cudaStream_t s)
   if (!L.h.p.seg || !L.h.p.cta_first ||
       (L.batch ? (!L.h.p.shots || !L.h.hshots || !L.h.hmaps) : (!L.h.out_hi || !L.h.e_cur)))
     return cudaErrorInvalidValue;
+  if (fault_injected(L.h.p)) return ext ? launch_half_hook<true>(L, s) : launch_half_hook<false>(L, s);
 #define X(a, b)                                                                                             \
   if (L.tile_rows == a && L.stages == b)                                                                    \
     return ext ? (L.batch ? launch_half_t<a, b, true, true>(L, s) : launch_half_t<a, b, true, false>(L, s)) \

@@ -163,18 +163,21 @@ int FLETCHER_CoefLayout(void);
  * FLETCHER_FAULT_ALLOC: the device allocation `arg` allocations from now
  *   (0 = the next one) fails as if memory were exhausted; the call that
  *   makes it reports FLETCHER_ERR_NOMEM and releases what it allocated.
- * FLETCHER_FAULT_STALL: in the next propagate launch (FP32 form, default
- *   16 x 5 tiles and numerics; that launch uses a variant of the kernel
- *   built with the hook, the regular kernels carry none), CTA 0
- *   skips the loads of its step `arg` (counted from 0), and every wait of
- *   that launch gives up after wait_us microseconds (1000 .. 2000000); the
- *   CTA's waits for that stage run out, it drains the loads in flight and
- *   leaves, and the step reports FLETCHER_ERR_TIMEOUT.  The fields of that
- *   step are then undefined; the state stays usable (re-initialise it).
+ * FLETCHER_FAULT_STALL: in the next propagate launch (single shot, the
+ *   form's default tile rows, 16-bit forms on isotropic grids; that launch uses
+ *   a variant of the kernel built with the hook, the regular kernels carry
+ *   none), CTA 0 skips the loads of its step `arg` (counted from 0), and every
+ *   wait of that launch gives up after wait_us microseconds (1000 .. 2000000)
+ *   at most; the CTA's waits for that stage run out, it drains the loads in
+ *   flight and leaves, and the step reports FLETCHER_ERR_TIMEOUT.  The fields of
+ *   that step are then undefined; the state stays usable (re-initialise it).
+ * FLETCHER_FAULT_QUIT: the same, but instead of skipping loads one of CTA 0's
+ *   helper warps gives up at its step `arg` as if its wait had run out.
  * FLETCHER_FAULT_NONE: cancels pending injections. */
 #define FLETCHER_FAULT_NONE 0
 #define FLETCHER_FAULT_ALLOC 1
 #define FLETCHER_FAULT_STALL 2
+#define FLETCHER_FAULT_QUIT 3
 int FLETCHER_InjectFault(int kind, int arg, int wait_us);
 
 /* Kernel shape override for tuning (0 keeps the default): rows per tile,

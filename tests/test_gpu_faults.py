@@ -12,6 +12,8 @@
   FLETCHER_ERR_NOMEM, releases the rest, and the next set-up succeeds.
 * Non-finite model values are rejected at set-up, naming array and cell.
 """
+import time
+
 import numpy as np
 import pytest
 
@@ -20,7 +22,7 @@ from fletcher_petrobras_gb300 import FletcherError, Problem, Propagator
 
 pytestmark = pytest.mark.gpu
 
-FAULT_NONE, FAULT_ALLOC, FAULT_STALL = 0, 1, 2
+FAULT_NONE, FAULT_ALLOC, FAULT_STALL, FAULT_QUIT = 0, 1, 2, 3
 ERR_TIMEOUT, ERR_NOMEM, ERR_ARGS = 3, 4, 1
 
 PROB = Problem("faults", 36, 30, 28, absorb=5, dt=0.0006, steps=12, fcut=45.0, kind="layered", layers=3, seed=6)
@@ -64,6 +66,43 @@ def test_stalled_pipeline_reports_timeout_then_recovers(stall_step, orc):
     # The injection applied to that one launch only.
     lib.FLETCHER_ClearError()
     prop.finalize()
+    clean_run(orc)
+
+
+def failing_step(prob, kind, arg, wait_us, zchunks, **kw):
+    """A step with a source in which the fault is injected, after a normal
+    one; returns the seconds it took to report the give-up."""
+    prop = Propagator(zchunks=zchunks, **kw)
+    prop.initialize(prob.sx, prob.sy, prob.sz, prob.bord, prob.dx, prob.dy, prob.dz, prob.dt, prob.model())
+    prop.insert_source(1, prob.i_source, 1.0)
+    prop.propagate(1)
+    prop.insert_source(2, prob.i_source, 1.0)
+    assert prop.lib.FLETCHER_InjectFault(kind, arg, wait_us) == 0
+    t = time.perf_counter()
+    with pytest.raises(FletcherError, match=r"gave up waiting.*\(code 3\)"):
+        prop.propagate(2)
+    t = time.perf_counter() - t
+    prop.lib.FLETCHER_ClearError()
+    prop.finalize()
+    Propagator()  # the default form, numerics and shape again
+    return t
+
+
+FORMS = [dict(), dict(form="fp16"), dict(form="fp16x"), dict(numerics="d1d1")]
+# The source's plane is step 16 of CTA 0's column; in the second problem every
+# CTA has several items, the source's plane in one of the later ones.
+DEEP = PROB.with_(source=(20, 20, 16))
+SHORT = Problem("short", 170, 130, 30, absorb=5, dt=0.0006, steps=9, fcut=45.0, kind="layered", layers=4, seed=12,
+                source=(68, 52, 30))
+
+
+@pytest.mark.parametrize("prob,zchunks,step", [(DEEP, -1, 0), (DEEP, -1, 16), (DEEP, -1, 20), (SHORT, -16, 1)])
+@pytest.mark.parametrize("kw", FORMS, ids=lambda k: next(iter(k.values()), "fp32"))
+def test_helper_warp_that_gives_up_leaves_no_other_waiting(kw, prob, zchunks, step, orc):
+    """A helper warp whose wait runs out while its sisters' waits succeed: they
+    meet at a barrier once a plane (16-bit forms) or on the source's plane, and
+    every warp leaves."""
+    failing_step(prob, FAULT_QUIT, step, 20000, zchunks, **kw)
     clean_run(orc)
 
 
