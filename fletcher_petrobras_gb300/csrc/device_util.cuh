@@ -72,8 +72,9 @@ __device__ __forceinline__ bool mbar_wait(uint64_t *bar, uint32_t parity, uint64
   }
 }
 // The same with the limit counted in tries (a few instructions, where the
-// timed loop would bloat an unrolled caller).  A try suspends the thread for
-// at most about kSpinHintNs.
+// timed loop would bloat an unrolled caller).  A try that fails suspends the
+// thread for up to kSpinHintNs: 200 000 of them took 0.37 s, so the default
+// limit is 1.9 s.
 constexpr uint32_t kSpinTries = 1u << 20, kSpinHintNs = 2000;
 __device__ __forceinline__ bool mbar_spin(uint64_t *bar, uint32_t parity, uint32_t tries = kSpinTries) {
   while (!mbar_try_wait_hint(bar, parity, kSpinHintNs))

@@ -262,9 +262,10 @@ bool resident_dims(int *sx, int *sy, int *sz);  // grid of the resident state (a
 cudaStream_t resident_stream();      // the library's stream
 void snapshot_release();             // driver.cu calls it when the state goes away
 
-// Time limit of every device-side wait (ns).
+// Time limit of the learned layer's grid barriers (ns); the step kernels count
+// their tries instead (mbar_spin).
 constexpr uint64_t kWaitLimitNs = 2000000000ull;
-// Limit of an aborting producer's wait for each stage's loads.
+// Limit of an aborting producer's wait for each stage's loads (ns).
 constexpr uint64_t kDrainNs = 200000000ull;
 
 }  // namespace flt

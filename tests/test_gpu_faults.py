@@ -106,6 +106,19 @@ def test_helper_warp_that_gives_up_leaves_no_other_waiting(kw, prob, zchunks, st
     clean_run(orc)
 
 
+@pytest.mark.parametrize("kw", FORMS, ids=lambda k: next(iter(k.values()), "fp32"))
+def test_counted_waits_end_in_time(kw, orc):
+    """Waits limited by a count of tries end within the limit they stand for:
+    the stalled stage's readers after one, the producer, which waits for them,
+    after another, then its drain of the missing loads (200 ms), and a second
+    for the rest."""
+    wait_s = 0.4
+    t = failing_step(DEEP, FAULT_STALL, 3, int(wait_s * 1e6), -1, **kw)
+    print(f"gave up after {t:.3f} s")
+    assert t < 2 * wait_s + 0.2 + 1.0
+    clean_run(orc)
+
+
 def test_stall_argument_checks():
     lib = Propagator().lib
     lib.FLETCHER_ClearError()
