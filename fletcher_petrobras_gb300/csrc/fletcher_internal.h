@@ -143,6 +143,18 @@ inline cudaError_t launch_step(void (*kern)(K...), int grid, int block, size_t s
   return cudaLaunchKernelEx(&cfg, kern, args...);
 }
 
+// Before a step kernel's first launch: its dynamic shared-memory limit, and a
+// check of its register split.  setmaxnreg moves registers between the warps of
+// a CTA within what the launch gives them; a kernel compiled to fewer than
+// `launch_regs` a thread would leave setmaxnreg.inc waiting without limit.
+inline cudaError_t prepare_step_kernel(const void *kern, size_t smem, int launch_regs) {
+  cudaFuncAttributes a;
+  const cudaError_t e = cudaFuncGetAttributes(&a, kern);
+  if (e != cudaSuccess) return e;
+  if (a.numRegs < launch_regs) return cudaErrorInvalidKernelImage;
+  return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+}
+
 inline bool fault_injected(const PropParams &P) { return P.stall_step >= 0 || P.quit_step >= 0; }
 
 size_t propagate_fp32_smem_bytes(int tile_rows, int stages);

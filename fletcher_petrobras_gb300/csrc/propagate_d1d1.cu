@@ -34,7 +34,9 @@ constexpr int kHelperWarps = 4, kHaloWarps = kHelperWarps - 1;
 constexpr int CW = TY / 2;  // compute warps
 constexpr int kThreads = kTileX * (CW + kHelperWarps);
 // Registers: 2 x 232 + 32 <= 3 x 168 a sub-partition, as in propagate_fp32.cu.
-constexpr int kComputeRegs = 232, kHelperRegs = 32;
+constexpr int kComputeRegs = 232, kHelperRegs = 32, kLaunchRegs = 168;
+static_assert(CW / 4 * kComputeRegs + kHelperWarps / 4 * kHelperRegs <= (CW + kHelperWarps) / 4 * kLaunchRegs,
+              "the split exceeds the launch's registers");
 
 // Shared memory: S stages (TMA tiles, pDx of the tile's columns with its
 // 4-row halo, a control block), then the in-plane terms (A, B and C) of the
@@ -374,8 +376,7 @@ template <bool HOOK>
 static cudaError_t launch_d1d1(const PropLaunch &L, cudaStream_t s) {
   static bool ready = false;
   if (!ready) {
-    const cudaError_t e =
-        cudaFuncSetAttribute(k_propagate_d1d1<HOOK>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmem);
+    const cudaError_t e = prepare_step_kernel((const void *)k_propagate_d1d1<HOOK>, kSmem, kLaunchRegs);
     if (e != cudaSuccess) return e;
     ready = true;
   }

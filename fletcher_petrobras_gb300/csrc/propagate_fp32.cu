@@ -554,11 +554,6 @@ constexpr size_t smem_bytes() {
   return Layout<TY, S, MT>::BYTES;
 }
 
-template <class K>
-static cudaError_t set_smem(K kern, size_t smem) {
-  return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-}
-
 template <int TY, int S, int MINB>
 static cudaError_t prepare_t() {
   constexpr size_t smem = smem_bytes<TY, S>();
@@ -566,7 +561,7 @@ static cudaError_t prepare_t() {
   cudaError_t e = cudaSuccess;
   for (auto kern : {k_propagate_fp32<TY, S, true, false, MINB>, k_propagate_fp32<TY, S, false, false, MINB>,
                     k_propagate_fp32<TY, S, true, true, MINB>, k_propagate_fp32<TY, S, false, true, MINB>})
-    if (e == cudaSuccess) e = set_smem(kern, smem);
+    if (e == cudaSuccess) e = prepare_step_kernel((const void *)kern, smem, Regs<TY>::kLaunch);
   return e;
 }
 
@@ -616,7 +611,7 @@ static cudaError_t launch_hook(const PropLaunch &L, cudaStream_t s) {
   // only.  (The coefficient planes are present in either layout.)
   if (L.batch || L.tile_rows != TY) return cudaErrorInvalidValue;
   auto kern = L.p.iso ? k_propagate_fp32<TY, S, true, false, 1, true> : k_propagate_fp32<TY, S, false, false, 1, true>;
-  const cudaError_t e = set_smem(kern, smem);
+  const cudaError_t e = prepare_step_kernel((const void *)kern, smem, Regs<TY>::kLaunch);
   if (e != cudaSuccess) return e;
   return launch_step(kern, L.grid, propagate_fp32_threads(TY), smem, s, L.m, L.p);
 }
@@ -633,7 +628,7 @@ static cudaError_t launch_media_t(const PropLaunch &L, cudaStream_t s) {
   static bool ready = false;
   if (!ready) {
     for (auto kern : {kern_i, kern_a}) {
-      const cudaError_t e = set_smem(kern, smem);
+      const cudaError_t e = prepare_step_kernel((const void *)kern, smem, Regs<TY>::kLaunch);
       if (e != cudaSuccess) return e;
     }
     ready = true;

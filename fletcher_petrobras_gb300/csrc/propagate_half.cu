@@ -776,8 +776,8 @@ static cudaError_t prepare_half_t() {
   static bool ready = false;
   if (!ready) {
     for (auto kern : {k_propagate_half<TY, S, true, EXT, BATCH>, k_propagate_half<TY, S, false, EXT, BATCH>}) {
-      const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                 (int)LayoutH<TY, S, EXT>::BYTES);
+      const cudaError_t e =
+          prepare_step_kernel((const void *)kern, LayoutH<TY, S, EXT>::BYTES, RegsH<TY, EXT>::kLaunch);
       if (e != cudaSuccess) return e;
     }
     ready = true;
@@ -802,7 +802,7 @@ static cudaError_t launch_half_hook(const HalfLaunch &L, cudaStream_t s) {
   if (L.batch || L.tile_rows != TY || !L.h.p.iso) return cudaErrorInvalidValue;
   auto kern = k_propagate_half<TY, S, true, EXT, false, true>;
   const cudaError_t e =
-      cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)LayoutH<TY, S, EXT>::BYTES);
+      prepare_step_kernel((const void *)kern, LayoutH<TY, S, EXT>::BYTES, RegsH<TY, EXT>::kLaunch);
   if (e != cudaSuccess) return e;
   return launch_step(kern, L.grid, RegsH<TY, EXT>::kThreads, LayoutH<TY, S, EXT>::BYTES, s, L.m, L.h);
 }
