@@ -52,3 +52,32 @@ def test_autotune_is_transparent_and_persists(tmp_path, form):
     for a, b in zip(base, again):
         assert np.array_equal(a, b)
     assert len(open(path).read().splitlines()) == 1
+
+
+@pytest.mark.parametrize("kw,built", [
+    (dict(), {(16, 4), (16, 5), (12, 4), (12, 5), (12, 6), (8, 4), (8, 5)}),
+    (dict(form="fp16"), {(16, 4), (16, 5), (12, 4), (12, 5), (12, 6), (8, 6)}),
+    (dict(form="fp16x"), {(16, 4), (16, 5), (12, 4), (12, 5), (12, 6), (8, 6)}),
+    (dict(coef_layout="media"), {(16, 5), (16, 6), (16, 7)}),
+], ids=["fp32", "fp16", "fp16x", "media"])
+def test_autotune_tries_every_built_shape_from_the_present_one(tmp_path, kw, built):
+    p = PROB
+    prop = Propagator(**kw)
+    prop.initialize(p.sx, p.sy, p.sz, p.bord, p.dx, p.dy, p.dz, p.dt, p.model())
+    r, s = C.c_int(0), C.c_int(0)
+
+    def shape():
+        return prop.lib.FLETCHER_GetTileConfig(C.byref(r), C.byref(s)), (r.value, s.value)
+
+    _, start = shape()
+    assert prop.lib.FLETCHER_Autotune(str(tmp_path / "c.txt").encode(), 1) == 0
+    tried = []
+    for it in range(2 * len(built)):
+        prop.propagate(it)
+        active, now = shape()
+        if active:
+            tried.append(now)
+    prop.finalize()
+    Propagator()
+    assert not active
+    assert tried[0] == start and set(tried) == built

@@ -54,6 +54,25 @@ def test_batch_tuner_candidates_are_built_shapes(lib, tmp_path):
             assert (r.value, s.value) == (rows, stages)
 
 
+def test_batch_tuner_tries_every_built_shape(lib, tmp_path):
+    """The shapes the configuration lookup accepts for a form are those built
+    for it: the batch tuner tries each of them."""
+    import ctypes as C
+
+    from fletcher_petrobras_gb300.autotune import CANDIDATES, HALF_CANDIDATES
+
+    r, s = C.c_int(0), C.c_int(0)
+    for form, cands in ((0, CANDIDATES), (1, HALF_CANDIDATES), (2, HALF_CANDIDATES)):
+        built = set()
+        for rows in range(4, 33, 4):
+            for stages in range(2, 9):
+                path = str(tmp_path / f"b{form}_{rows}_{stages}.txt").encode()
+                assert lib.FLETCHER_TuneConfigStore(path, b"G", 100, form, rows, stages) == 0
+                if lib.FLETCHER_TuneConfigLookup(path, b"G", 100, form, C.byref(r), C.byref(s)) == 1:
+                    built.add((rows, stages))
+        assert built == set(cands)
+
+
 def test_batch_form_is_checked_before_any_device_call(lib):
     from fletcher_petrobras_gb300._lib import fptr
     from fletcher_petrobras_gb300.batch import Batch
