@@ -2,14 +2,17 @@
 
 Times each built (tile rows, pipeline stages) shape on the actual problem for
 a few steps and keeps the fastest; results are cached in a JSON file keyed by
-GPU name, form and problem shape class, so later runs skip the search (the
-reference's block-size tuners cached their choice per GPU and size in
+GPU name, form, problem shape class and library build, so later runs skip the
+search until the kernels change (the reference's block-size tuners cached their choice per GPU and size in
 configurations.txt, original_singleGPU_PDP/model.c:51-113).
 """
 from __future__ import annotations
 
+import hashlib
 import json
 import os
+
+from . import _lib
 
 CANDIDATES = [(16, 5), (16, 4), (12, 5), (12, 4), (12, 6), (8, 5), (8, 4)]  # built FP32 shapes
 HALF_CANDIDATES = [(16, 5), (16, 4), (12, 5), (12, 4), (12, 6), (8, 6)]  # built 16-bit shapes
@@ -23,6 +26,13 @@ def gpu_name() -> str:
         return torch.cuda.get_device_name(0)
     except Exception:
         return "unknown-gpu"
+
+
+def library_id() -> str:
+    """Digest of the built library: a winner timed on other kernels is no
+    answer for these."""
+    with open(_lib._LIB_PATH, "rb") as f:
+        return hashlib.sha1(f.read()).hexdigest()[:12]
 
 
 def _load(path):
@@ -49,7 +59,7 @@ def tune_batch(batch, steps: int = 20, cache: str | None = DEFAULT_CACHE, candid
     form = getattr(batch, "form", "fp32")
     if candidates is None:
         candidates = CANDIDATES if form == "fp32" else HALF_CANDIDATES
-    key = f"{gpu_name()}|{form}|{shape_class(batch.probs)}"
+    key = f"{gpu_name()}|{form}|{shape_class(batch.probs)}|{library_id()}"
     data = _load(cache) if cache else {}
     if key in data:
         rec = data[key]

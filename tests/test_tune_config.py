@@ -73,6 +73,39 @@ def test_batch_tuner_tries_every_built_shape(lib, tmp_path):
         assert built == set(cands)
 
 
+def test_batch_tuner_cache_does_not_outlive_the_kernels(tmp_path, monkeypatch):
+    """A cached shape is reused by the library that timed it and timed anew by
+    another build."""
+    from fletcher_petrobras_gb300 import Problem, autotune
+
+    class Timed:
+        form = "fp32"
+        probs = [Problem("t", 40, 40, 40, absorb=4)]
+        tile, runs = None, 0
+
+        def set_tile(self, rows, stages):
+            self.tile = (rows, stages)
+
+        def run(self, max_steps):
+            self.runs += 1
+            return 1.0 if self.tile == fast else 2.0
+
+        def reset(self):
+            pass
+
+    path = str(tmp_path / "autotune.json")
+    fast = (12, 5)
+    assert autotune.tune_batch(Timed(), cache=path)["tile"] == [12, 5]
+    again = Timed()
+    assert autotune.tune_batch(again, cache=path)["cached"] and again.runs == 0 and again.tile == (12, 5)
+    other = tmp_path / "other.so"
+    other.write_bytes(b"another build")
+    monkeypatch.setattr(autotune._lib, "_LIB_PATH", str(other))
+    fast = (16, 4)
+    rec = autotune.tune_batch(Timed(), cache=path)
+    assert not rec["cached"] and rec["tile"] == [16, 4]
+
+
 def test_batch_form_is_checked_before_any_device_call(lib):
     from fletcher_petrobras_gb300._lib import fptr
     from fletcher_petrobras_gb300.batch import Batch
