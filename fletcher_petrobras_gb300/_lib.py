@@ -87,6 +87,8 @@ SIGNATURES = {
     "FLETCHER_AbcGradient": (C.c_int, [FP, FP, C.c_int, FP, FP]),
     "FLETCHER_AbcForward": (C.c_int, [FP, C.c_int, FP]),
     "FLETCHER_SetBoundary": (C.c_int, [C.c_int, C.c_int, C.c_float]),
+    "FLETCHER_PlanShot": (C.c_int, [C.c_int] * 10 + [IP, C.c_int, IP, C.POINTER(C.c_long)]),
+    "FLETCHER_PlanBatch": (C.c_int, [C.c_int, C.c_int, IP] + [C.c_int] * 4 + [IP, C.c_int, IP]),
     "FLETCHER_PlanSegments": (C.c_int, [C.c_int] * 7 + [IP, C.c_int, IP, C.POINTER(C.c_long)]),
     "FLETCHER_AbcLayerCells": (C.c_long, []),
     "FLETCHER_AbcSetInterval": (C.c_int, [C.c_int]),

@@ -60,7 +60,6 @@ struct State {
   ShotDesc desc;                 // the shot (passed by value to every launch)
   ShotMaps maps;                 // its TMA descriptors
   int tile_rows = 12, stages = 5, zchunks = 0;
-  int ntx = 0, nty = 0;      // tiles in x and y
   int4 *seg = nullptr;       // the plan as work segments {x0, y0, z0, z1}
   int *cta_first = nullptr;  // [seg_grid + 1]: first segment of each CTA
   int nseg = 0, grid = 0;
@@ -607,8 +606,19 @@ bool plan_hbm(int form, int numerics, bool media) {
   return form == FLETCHER_FORM_FP32 && numerics == FLETCHER_NUMERICS_FAST && !media;
 }
 
-// Rows of the last of `nty` tile rows that lie in the updated region.
-int last_tile_rows(int sy, int bord, int nty, int TY) { return sy - bord - kRadius - (nty - 1) * TY; }
+// Tiles in x and y, and the rows of the last tile row that lie in the updated
+// region.
+int tiles_x(int sx, int bord) { return (sx - bord - kRadius + kTileX - 1) / kTileX; }
+int tiles_y(int sy, int bord, int TY) { return (sy - bord - kRadius + TY - 1) / TY; }
+int last_tile_rows(int sy, int bord, int TY) { return sy - bord - kRadius - (tiles_y(sy, bord, TY) - 1) * TY; }
+
+// The plan of a shot's own launches.  (The Der1-Der1 kernel's warps exchange
+// rows: all of them compute.)
+Split plan_shot(int ctas, int sx, int sy, int sz, int bord, int TY, int req, int form, int numerics, bool media) {
+  return plan_segments(ctas, tiles_x(sx, bord), tiles_y(sy, bord, TY), TY,
+                       numerics == FLETCHER_NUMERICS_D1D1 ? TY : last_tile_rows(sy, bord, TY), bord, sz - 2 * bord,
+                       req, plan_hbm(form, numerics, media));
+}
 
 int check_dims(int sx, int sy, int sz) {
   if (!g.init) return fail(FLETCHER_ERR_ARGS, "DRIVER_Initialize has not been called");
@@ -785,13 +795,8 @@ int setup_tiles(int rows, int stages) {
   if (half_form() && build_half_maps(g.hm, g.Hh, g.Hl, g.maps, sx, sy, sz, g.pitch, TY)) return g_last_err;
   g.tile_rows = rows;
   g.stages = stages;
-  g.ntx = (sx - bord - kRadius + kTileX - 1) / kTileX;
-  g.nty = (sy - bord - kRadius + TY - 1) / TY;
   const int ctas = g.num_sms * (half_form() ? 1 : propagate_fp32_ctas_per_sm(TY));
-  // (The Der1-Der1 kernel's warps exchange rows: all of them compute.)
-  const int last_rows = g.numerics == FLETCHER_NUMERICS_D1D1 ? TY : last_tile_rows(sy, bord, g.nty, TY);
-  const Split sp = plan_segments(ctas, g.ntx, g.nty, TY, last_rows, bord, sz - 2 * bord, g.zchunks,
-                                 plan_hbm(g.form, g.numerics, g.media));
+  const Split sp = plan_shot(ctas, sx, sy, sz, bord, TY, g.zchunks, g.form, g.numerics, g.media);
   if (g.seg) cudaFree(g.seg);
   if (g.cta_first) cudaFree(g.cta_first);
   g.seg = nullptr;
@@ -1430,6 +1435,19 @@ extern "C" int FLETCHER_PlanSegments(int ctas, int ntx, int nty, int tile_rows, 
   return n;
 }
 
+extern "C" int FLETCHER_PlanShot(int ctas, int sx, int sy, int sz, int bord, int tile_rows, int zchunks, int form,
+                                 int numerics, int media, int *seg_out, int cap, int *first_out, long *max_cost) {
+  if (ctas < 1 || bord < kRadius || sx <= 2 * bord || sy <= 2 * bord || sz <= 2 * bord || tile_rows < 1 || cap < 0 ||
+      !first_out)
+    return -fail(FLETCHER_ERR_ARGS, "FLETCHER_PlanShot: bad arguments");
+  const Split sp = plan_shot(ctas, sx, sy, sz, bord, tile_rows, zchunks, form, numerics, media != 0);
+  const int n = (int)sp.seg.size();
+  if (seg_out && n <= cap) memcpy(seg_out, sp.seg.data(), sizeof(int4) * n);
+  memcpy(first_out, sp.first.data(), sizeof(int) * (ctas + 1));
+  if (max_cost) *max_cost = sp.max_cost;
+  return n;
+}
+
 extern "C" int FLETCHER_SetTileConfig(int rows, int stages, int zchunks) {
   const int r = rows ? rows : 16, s = stages ? stages : 5;
   if (!propagate_fp32_supported(r, s) && !propagate_half_supported(r, s) && !propagate_fp32_media_supported(r, s))
@@ -1614,7 +1632,6 @@ struct BatchShot {
   int *E = nullptr;
   unsigned *Mx = nullptr;
   float *coef = nullptr;
-  int ntx = 0, nty = 0;
 };
 
 struct Batch {
@@ -1723,6 +1740,14 @@ bool batch_shape_built(int rows, int stages) {
   return batch_half() ? propagate_half_supported(rows, stages) : propagate_fp32_supported(rows, stages);
 }
 
+// Shot indices, longest run first.
+std::vector<int> by_steps(const std::vector<BatchShot> &shots) {
+  std::vector<int> order(shots.size());
+  for (size_t i = 0; i < order.size(); ++i) order[i] = (int)i;
+  std::stable_sort(order.begin(), order.end(), [&](int a, int b) { return shots[a].nsteps > shots[b].nsteps; });
+  return order;
+}
+
 int batch_seal(int rows, int stages) {
   if (!batch_shape_built(rows, stages))
     return fail(FLETCHER_ERR_ARGS, "tile shape (%d rows, %d stages) is not built for form %d", rows, stages, B.form);
@@ -1736,15 +1761,10 @@ int batch_seal(int rows, int stages) {
   std::vector<ShotMaps> maps(ns);
   std::vector<HalfShot> hshots(ns);
   std::vector<HalfShotMaps> hmaps(ns);
-  B.order.resize(ns);
-  for (int i = 0; i < ns; ++i) B.order[i] = i;
-  std::stable_sort(B.order.begin(), B.order.end(),
-                   [](int a, int b) { return B.shots[a].nsteps > B.shots[b].nsteps; });
+  B.order = by_steps(B.shots);
   for (int oi = 0; oi < ns; ++oi) {
     const int i = B.order[oi];
     BatchShot &s = B.shots[i];
-    s.ntx = (s.sx - B.bord - kRadius + kTileX - 1) / kTileX;
-    s.nty = (s.sy - B.bord - kRadius + rows - 1) / rows;
     if (build_maps(&maps[i], s.F, s.coef, s.sx, s.sy, s.sz, s.pitch, rows)) return g_last_err;
     if (batch_half()) {
       if (build_half_maps(hmaps[i].m, s.Hh, s.Hl, maps[i], s.sx, s.sy, s.sz, s.pitch, rows)) return g_last_err;
@@ -1804,43 +1824,43 @@ int batch_seal(int rows, int stages) {
 // latency of their planes.  At 0.8, 0.9 and 1: 24 shots of 48^3 64.3, 60.4 and
 // 60.8 us a step, 24 of 64^3 156, 148 and 147, FP16X 24 of 48^3 83.4, 79.2 and 81.2.
 constexpr double kPooledPlanes = 64.0, kPooledPlanesHbm = 14.0, kPooledRowShare = 0.9;
-int batch_plan(int ctas) {
-  if (B.d_plan && B.plan_ctas == ctas) return FLETCHER_OK;
-  if (B.d_plan) cudaFree(B.d_plan);
-  if (B.d_first) cudaFree(B.d_first);
-  B.d_plan = nullptr;
-  B.d_first = nullptr;
-  const int ns = (int)B.shots.size(), TY = B.sealed_rows;
-  if (!batch_half() && ns >= 32768) return fail(FLETCHER_ERR_ARGS, "a batch holds at most 32767 shots");
+struct BatchPlan {
+  std::vector<int4> seg;
+  std::vector<long> off;   // by number of running shots r: offset of its list (r - 1)
+  std::vector<int> first;  //   and each CTA's first segment, at (r - 1) * (ctas + 1)
+  std::vector<int> grid;
+};
+
+// `order`: shot indices, longest run first.
+BatchPlan plan_batch(const std::vector<BatchShot> &shots, const std::vector<int> &order, int bord, int form, int TY,
+                     int ctas) {
+  const int ns = (int)shots.size();
+  const double line = form == FLETCHER_FORM_FP32 ? kPooledPlanesHbm : kPooledPlanes;
   std::vector<Split> own(ns);
   std::vector<char> pooled(ns, 0);
   for (int oi = 0; oi < ns; ++oi) {
-    const BatchShot &s = B.shots[B.order[oi]];
-    if (!batch_half() && s.sx >= 65536) return fail(FLETCHER_ERR_ARGS, "batched shots need sx < 65536");
-    const int depth = s.sz - 2 * B.bord;
-    pooled[oi] = (double)s.ntx * s.nty * depth < (batch_half() ? kPooledPlanes : kPooledPlanesHbm) * ctas;
-    if (!pooled[oi])
-      own[oi] = plan_segments(ctas, s.ntx, s.nty, TY, last_tile_rows(s.sy, B.bord, s.nty, TY), B.bord, depth, 0,
-                              plan_hbm(B.form, FLETCHER_NUMERICS_FAST, false));
+    const BatchShot &s = shots[order[oi]];
+    pooled[oi] = (double)tiles_x(s.sx, bord) * tiles_y(s.sy, bord, TY) * (s.sz - 2 * bord) < line * ctas;
+    if (!pooled[oi]) own[oi] = plan_shot(ctas, s.sx, s.sy, s.sz, bord, TY, 0, form, FLETCHER_NUMERICS_FAST, false);
   }
-  std::vector<int4> plan;
-  std::vector<int> first((size_t)ns * (ctas + 1));
-  B.plan_off.assign(ns, 0);
-  B.plan_grid.assign(ns, 1);
+  BatchPlan bp;
+  bp.first.resize((size_t)ns * (ctas + 1));
+  bp.off.assign(ns, 0);
+  bp.grid.assign(ns, 1);
   for (int r = 1; r <= ns; ++r) {
-    if (r < ns && B.shots[B.order[r - 1]].nsteps == B.shots[B.order[r]].nsteps) continue;  // never r running
+    if (r < ns && shots[order[r - 1]].nsteps == shots[order[r]].nsteps) continue;  // never r running
     std::vector<std::vector<int4>> per(ctas);
     std::vector<long> cost(ctas, 0);
     std::vector<Column> pool;
     for (int oi = 0; oi < r; ++oi) {
-      const int shot = B.order[oi];
-      const BatchShot &s = B.shots[shot];
+      const int shot = order[oi];
+      const BatchShot &s = shots[shot];
       if (pooled[oi]) {
-        const int last =
-            std::max(last_tile_rows(s.sy, B.bord, s.nty, TY), (int)ceil(kPooledRowShare * TY));
-        for (int t = 0; t < s.ntx * s.nty; ++t)
-          pool.push_back(Column{t % s.ntx, kRadius + t / s.ntx * TY, B.bord, s.sz - B.bord,
-                                t / s.ntx == s.nty - 1 ? last : TY, shot});
+        const int ntx = tiles_x(s.sx, bord), nty = tiles_y(s.sy, bord, TY);
+        const int last = std::max(last_tile_rows(s.sy, bord, TY), (int)ceil(kPooledRowShare * TY));
+        for (int t = 0; t < ntx * nty; ++t)
+          pool.push_back(Column{t % ntx, kRadius + t / ntx * TY, bord, s.sz - bord, t / ntx == nty - 1 ? last : TY,
+                                shot});
         continue;
       }
       for (int b = 0; b < ctas; ++b)
@@ -1852,22 +1872,39 @@ int batch_plan(int ctas) {
     }
     const std::vector<long> base(cost);
     deal_pool(pool, TY, base, pool_cap(pool, TY, base), &per, &cost);
-    const size_t at = plan.size();
-    B.plan_off[r - 1] = (long)at;
-    int *f = first.data() + (size_t)(r - 1) * (ctas + 1);
+    const size_t at = bp.seg.size();
+    bp.off[r - 1] = (long)at;
+    int *f = bp.first.data() + (size_t)(r - 1) * (ctas + 1);
     for (int b = 0; b < ctas; ++b) {
-      f[b] = (int)(plan.size() - at);
-      plan.insert(plan.end(), per[b].begin(), per[b].end());
+      f[b] = (int)(bp.seg.size() - at);
+      bp.seg.insert(bp.seg.end(), per[b].begin(), per[b].end());
     }
-    f[ctas] = (int)(plan.size() - at);
+    f[ctas] = (int)(bp.seg.size() - at);
     int grid = ctas;  // CTAs past the last one with work are not launched
     while (grid > 1 && f[grid - 1] == f[grid]) --grid;
-    B.plan_grid[r - 1] = grid;
+    bp.grid[r - 1] = grid;
   }
-  CK(dev_malloc(&B.d_plan, sizeof(int4) * plan.size()));
-  CK(dev_malloc(&B.d_first, sizeof(int) * first.size()));
-  CK(upload(B.d_plan, plan));
-  CK(upload(B.d_first, first));
+  return bp;
+}
+
+int batch_plan(int ctas) {
+  if (B.d_plan && B.plan_ctas == ctas) return FLETCHER_OK;
+  if (B.d_plan) cudaFree(B.d_plan);
+  if (B.d_first) cudaFree(B.d_first);
+  B.d_plan = nullptr;
+  B.d_first = nullptr;
+  if (!batch_half()) {
+    if (B.shots.size() >= 32768) return fail(FLETCHER_ERR_ARGS, "a batch holds at most 32767 shots");
+    for (const BatchShot &s : B.shots)
+      if (s.sx >= 65536) return fail(FLETCHER_ERR_ARGS, "batched shots need sx < 65536");
+  }
+  const BatchPlan bp = plan_batch(B.shots, B.order, B.bord, B.form, B.sealed_rows, ctas);
+  B.plan_off = bp.off;
+  B.plan_grid = bp.grid;
+  CK(dev_malloc(&B.d_plan, sizeof(int4) * bp.seg.size()));
+  CK(dev_malloc(&B.d_first, sizeof(int) * bp.first.size()));
+  CK(upload(B.d_plan, bp.seg));
+  CK(upload(B.d_first, bp.first));
   CK(cudaStreamSynchronize(g_stream));
   B.plan_ctas = ctas;
   return FLETCHER_OK;
@@ -1877,7 +1914,7 @@ int batch_plan(int ctas) {
 // column).
 bool batch_packs() {
   for (const BatchShot &s : B.shots)
-    if (s.ntx > 65535) return false;
+    if (tiles_x(s.sx, B.bord) > 65535) return false;
   return B.shots.size() <= 65536;
 }
 
@@ -1899,10 +1936,8 @@ int batch_single_plans(int ctas) {
   std::vector<int> firsts;
   for (int i = 0; i < ns; ++i) {
     const BatchShot &s = B.shots[i];
-    const int depth = s.sz - 2 * B.bord;
-    const Split sp = plan_segments(ctas, s.ntx, s.nty, B.sealed_rows,
-                                   last_tile_rows(s.sy, B.bord, s.nty, B.sealed_rows), B.bord, depth, 0,
-                                   plan_hbm(B.form, FLETCHER_NUMERICS_FAST, false));
+    const Split sp =
+        plan_shot(ctas, s.sx, s.sy, s.sz, B.bord, B.sealed_rows, 0, B.form, FLETCHER_NUMERICS_FAST, false);
     B.s_seg_off[i] = (long)segs.size();
     B.s_first_off[i] = (long)firsts.size();
     segs.insert(segs.end(), sp.seg.begin(), sp.seg.end());
@@ -2369,6 +2404,32 @@ extern "C" int FLETCHER_BatchSetTileConfig(int rows, int stages) {
   B.rows = r;
   B.stages = s;
   return FLETCHER_OK;
+}
+
+extern "C" int FLETCHER_PlanBatch(int ctas, int nshots, const int *shots, int bord, int tile_rows, int form, int running,
+                                  int *seg_out, int cap, int *first_out) {
+  if (ctas < 1 || nshots < 1 || nshots > 32767 || !shots || bord < kRadius || tile_rows < 1 || running < 1 ||
+      running > nshots || cap < 0 || !first_out)
+    return -fail(FLETCHER_ERR_ARGS, "FLETCHER_PlanBatch: bad arguments");
+  std::vector<BatchShot> v(nshots);
+  for (int i = 0; i < nshots; ++i) {
+    BatchShot &s = v[i];
+    s.sx = shots[4 * i];
+    s.sy = shots[4 * i + 1];
+    s.sz = shots[4 * i + 2];
+    s.nsteps = shots[4 * i + 3];
+    if (s.sx <= 2 * bord || s.sx >= 65536 || s.sy <= 2 * bord || s.sz <= 2 * bord)
+      return -fail(FLETCHER_ERR_ARGS, "FLETCHER_PlanBatch: bad grid of shot %d", i);
+  }
+  const std::vector<int> order = by_steps(v);
+  if (running < nshots && v[order[running - 1]].nsteps == v[order[running]].nsteps)
+    return -fail(FLETCHER_ERR_ARGS, "FLETCHER_PlanBatch: never %d shots running", running);
+  const BatchPlan bp = plan_batch(v, order, bord, form, tile_rows, ctas);
+  const int *f = bp.first.data() + (size_t)(running - 1) * (ctas + 1);
+  const int n = f[ctas];
+  if (seg_out && n <= cap) memcpy(seg_out, bp.seg.data() + bp.off[running - 1], sizeof(int4) * n);
+  memcpy(first_out, f, sizeof(int) * (ctas + 1));
+  return n;
 }
 
 extern "C" int FLETCHER_BatchLastChains(void) { return B.last_chains; }

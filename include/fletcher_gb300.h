@@ -186,16 +186,27 @@ int FLETCHER_InjectFault(int kind, int arg, int wait_us);
  * round-robin). */
 int FLETCHER_SetTileConfig(int tile_rows, int stages, int zchunks);
 
-/* The work split of a single-shot launch (host only): ntx x nty tiles of
- * 32 x tile_rows cells, planes [zlo, zlo + depth), over `ctas` persistent
- * CTAs.  Whole rounds of z-chunks go round-robin (CTAs side by side on
- * neighbouring tiles); the last partial round is cut into contiguous pieces
- * that fill every CTA up to the same cost.  Writes the segments {x0, y0, z0,
- * z1} CTA by CTA into seg_out (when they fit in `cap`), each CTA's first
+/* Work splits (host only).  Whole rounds of z-chunks go round-robin over `ctas`
+ * persistent CTAs (CTAs side by side on neighbouring tiles of 32 x tile_rows
+ * cells); the last partial round, and where the plan counts them apart the
+ * tiles with fewer rows in the updated region, are cut into contiguous pieces
+ * that fill every CTA up to the same cost.  A call writes the segments {x0, y0,
+ * z0, z1} CTA by CTA into seg_out (when they fit in `cap`), each CTA's first
  * segment into first_out [ctas + 1], and the busiest CTA's cost (its planes
- * plus 4 a segment for the halo) into max_cost;
- * returns the segment count (negative on error).  zchunks as in
- * FLETCHER_SetTileConfig (0: the cheapest plan). */
+ * plus 4 a segment for the halo, a tile with fewer rows at its share) into
+ * max_cost; it returns the segment count (negative on error).
+ * FLETCHER_PlanShot: the split of a shot's own launches, as DRIVER_Initialize
+ *   makes it for that grid, form, numerics and coefficient layout (media: the
+ *   media table).  zchunks as in FLETCHER_SetTileConfig (0: the cheapest plan).
+ * FLETCHER_PlanSegments: the same for ntx x nty tiles, all of them whole, and
+ *   planes [zlo, zlo + depth), with the FP32 form's coefficient planes.
+ * FLETCHER_PlanBatch: the split of a batch's persistent launch while the
+ *   `running` shots of the longest runs advance; shots: {sx, sy, sz, steps}
+ *   each.  Segments are {tile x index + (shot << 16), y0, z0, z1}. */
+int FLETCHER_PlanShot(int ctas, int sx, int sy, int sz, int bord, int tile_rows, int zchunks, int form, int numerics,
+                      int media, int *seg_out, int cap, int *first_out, long *max_cost);
+int FLETCHER_PlanBatch(int ctas, int nshots, const int *shots, int bord, int tile_rows, int form, int running,
+                       int *seg_out, int cap, int *first_out);
 int FLETCHER_PlanSegments(int ctas, int ntx, int nty, int tile_rows, int zlo, int depth, int zchunks, int *seg_out,
                           int cap, int *first_out, long *max_cost);
 
