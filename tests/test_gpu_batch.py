@@ -242,3 +242,23 @@ def test_half_chain_schedule_matches_single_shot_runs(form, chains):
             assert np.abs(ref[0]).max() > 0.0
             for k in range(4):
                 assert np.array_equal(got[i][k], ref[k]), (form, chains, use_graph, i, k)
+
+
+@pytest.mark.parametrize("form", ["fp32", "fp16x"])
+@pytest.mark.parametrize("n,shots,chains", [(121, 2, 2), (121, 1, 1), (267, 2, 1)])
+def test_default_schedule_takes_two_chains_for_two_filling_shots(n, shots, chains, form):
+    """Shots of 2.1 M updated cells and more run on two chains where there are
+    two of them, of at most 20 M cells on average, else on one: the fields of
+    their single-shot runs, bit for bit."""
+    probs = [Problem(f"two{i}", n, n - 2 * i, n, absorb=4, dt=0.0006, steps=4 + i, fcut=45.0, kind="layered",
+                     layers=3, seed=31 + i) for i in range(shots)]
+    models = [p.model() for p in probs]
+    batch = Batch(form=form)
+    for p, m in zip(probs, models):
+        batch.add(p, m)
+    batch.run()
+    assert batch.info()["chains"] == chains
+    got = [batch.field(i, 0) for i in range(shots)]
+    batch.close()
+    for p, m, f in zip(probs, models, got):
+        assert np.array_equal(f, single(p, m, form)[0])
