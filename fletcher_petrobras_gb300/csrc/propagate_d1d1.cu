@@ -19,6 +19,8 @@
 // 280 x 200 x 150 170 -> 128, 272^3 327 -> 283; with packed (p, q) instructions
 // (mul_rn) 23.9, 118.2 and 252.5, with two cells a thread, as in
 // propagate_fp32.cu, 23.5, 117.8 and 248.6.
+#include <limits.h>
+
 #include "device_util.cuh"
 #include "fletcher_internal.h"
 #include "propagate_fp32_pipe.cuh"
@@ -143,22 +145,14 @@ __global__ void __launch_bounds__(kThreads, 1)
     const int src_z = sd.src_z;
     auto halo_barrier = [] { asm volatile("bar.sync 1, %0;" ::"n"(32 * kHaloWarps) : "memory"); };
     [[maybe_unused]] int step = 0;
-    for (int i = 0; i < nitems; ++i) {
+    int i, k;
+    for (i = 0; i < nitems; ++i) {
       const Item it = decode_item<false>(seg[i]);
-      for (int k = it.z0 - kRadius; k < it.z1 + kLag; ++k) {
+      for (k = it.z0 - kRadius; k < it.z1 + kLag; ++k) {
         unsigned char *st = smem + stage * SB;
         bool ok = wait(bar(st, OFF_FULL), phase);
         if constexpr (HOOK) ok = ok && !(hw == 1 && blockIdx.x == 0 && step++ == P.quit_step);
-        if (!__all_sync(0xffffffffu, ok)) {
-          // Another halo warp's wait may have succeeded: this one meets the
-          // others at every barrier (below) still to come before it leaves.
-          if (lx == 0) atomicOr(P.err, 1u);
-          for (int a = i; a < nitems; ++a) {
-            const Item w = decode_item<false>(seg[a]);
-            if (src_z >= (a == i ? k : w.z0 - kRadius) && src_z < w.z1 + kLag) halo_barrier();
-          }
-          return;
-        }
+        if (!__all_sync(0xffffffffu, ok)) goto gave_up;
         f2 *H = reinterpret_cast<f2 *>(st);
         if (k == src_z) {
           // Fused source (original/OpenMP/openmp_insertsource.c:7-13): the
@@ -190,6 +184,14 @@ __global__ void __launch_bounds__(kThreads, 1)
           phase ^= 1u;
         }
       }
+    }
+    return;
+  gave_up:
+    // Meet the other halo warps at every barrier still to come (propagate_fp32.cu).
+    if (lx == 0) atomicOr(P.err, 1u);
+    for (; i < nitems; ++i, k = INT_MIN) {
+      const Item it = decode_item<false>(seg[i]);
+      if (src_z >= max(k, it.z0 - kRadius) && src_z < it.z1 + kLag) halo_barrier();
     }
     return;
   }

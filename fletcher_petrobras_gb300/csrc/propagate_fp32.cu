@@ -74,6 +74,8 @@
 // its weights are the products L_i L_j of the first-derivative weights
 // (original/derivatives.h:13-31); the FP32 rounding differs from the
 // reference's grouped sum, which the parity tolerance covers.
+#include <limits.h>
+
 #include "device_util.cuh"
 #include "fletcher_internal.h"
 #include "propagate_fp32_pipe.cuh"
@@ -252,11 +254,12 @@ __global__ void __launch_bounds__(kTileX *(Regs<TY>::kWarps + kHelperWarps), MIN
     [[maybe_unused]] int step = 0;
     auto halo_barrier = [] { asm volatile("bar.sync 1, %0;" ::"n"(32 * kHalo) : "memory"); };
     int rb = 0;
-    for (int i = 0; i < nitems; ++i) {
+    int i, k;
+    for (i = 0; i < nitems; ++i) {
       const Item it = decode_item<BATCH>(seg[i]);
       const ShotDesc &sd = BATCH ? P.shots[it.shot] : P.one;
       const int src_z = sd.src_z;
-      for (int k = it.z0 - kRadius; k < it.z1 + kLag; ++k) {
+      for (k = it.z0 - kRadius; k < it.z1 + kLag; ++k) {
         unsigned char *st = smem + stage * L::SB;
         bool ok = wait(bar(st, L::OFF_FULL), phase);
         if constexpr (L::NB < S) {
@@ -266,18 +269,7 @@ __global__ void __launch_bounds__(kTileX *(Regs<TY>::kWarps + kHelperWarps), MIN
         }
         // Test hook: a halo warp of CTA 0 gives up at its P.quit_step-th step.
         if constexpr (HOOK) ok = ok && !(hw == 1 && blockIdx.x == 0 && step++ == P.quit_step);
-        if (!__all_sync(0xffffffffu, ok)) {
-          // Another halo warp's wait may have succeeded: this one meets the
-          // others at every barrier (below) still to come before it leaves, so
-          // that none waits there for a warp that has left.
-          if (lx == 0) atomicOr(P.err, 1u);
-          for (int a = i; a < nitems; ++a) {
-            const Item w = decode_item<BATCH>(seg[a]);
-            const int zs = (BATCH ? P.shots[w.shot] : P.one).src_z;
-            if (zs >= (a == i ? k : w.z0 - kRadius) && zs < w.z1 + kLag) halo_barrier();
-          }
-          return;
-        }
+        if (!__all_sync(0xffffffffu, ok)) goto gave_up;
         f2 *H = reinterpret_cast<f2 *>(st);
         if (k == src_z) {
           // Fused source (original/OpenMP/openmp_insertsource.c:7-13): the
@@ -312,6 +304,18 @@ __global__ void __launch_bounds__(kTileX *(Regs<TY>::kWarps + kHelperWarps), MIN
           phase ^= 1u;
         }
       }
+    }
+    return;
+  gave_up:
+    // Another halo warp's wait may have succeeded: this one meets the others at
+    // every barrier still to come before it leaves, so that none waits there for
+    // a warp that has left.  (Inside the loop this code costs the media-table
+    // layout 1%.)
+    if (lx == 0) atomicOr(P.err, 1u);
+    for (; i < nitems; ++i, k = INT_MIN) {
+      const Item it = decode_item<BATCH>(seg[i]);
+      const int src_z = (BATCH ? P.shots[it.shot] : P.one).src_z;
+      if (src_z >= max(k, it.z0 - kRadius) && src_z < it.z1 + kLag) halo_barrier();
     }
     return;
   }
