@@ -197,10 +197,10 @@ __device__ __forceinline__ long ghost_index(const Ghost &G, long i, int sy, int 
 
 // ---- features -------------------------------------------------------------------
 
-// vpz, epsilon, delta of a cell from its coefficients (v2pz = vpz^2,
+// vpz, epsilon, delta of a cell of the updated region from its coefficients (v2pz = vpz^2,
 // v2px = vpz^2 (1 + 2 eps), v2pn = vpz^2 (1 + 2 delta): original/precomp.h).
 __device__ __forceinline__ float4 medium_of(const float *coef, int x, int y, int z, int sy, int pitch) {
-  const float *c = coef + coef_index(x, y, z, sy, pitch);
+  const float *c = coef + coef_index(x - kRadius, y, z, sy, pitch);
   const float v2px = c[DC_V2PX * kTileX], v2pz = c[DC_V2PZ * kTileX], v2pn = c[DC_V2PN * kTileX];
   float4 m;
   m.x = sqrtf(v2pz);
@@ -290,7 +290,7 @@ __device__ float2 outer_update(const float2 *F, const float *coef, int x, int y,
   const float qxx = d2[0].y * sx2, qyy = d2[1].y * sy2, qzz = d2[2].y * sz2;
   const float pxy = dc[0].x * sxy, pyz = dc[1].x * syz, pxz = dc[2].x * sxz;
   const float qxy = dc[0].y * sxy, qyz = dc[1].y * syz, qxz = dc[2].y * sxz;
-  const float *c0 = coef + coef_index(x, y, z, sy, pitch);
+  const float *c0 = coef + coef_index(x - kRadius, y, z, sy, pitch);
   auto C = [&](int k) { return c0[k * kTileX]; };
   const float cxx = C(DC_XX), cyy = C(DC_YY), czz = C(DC_ZZ), cxy = C(DC_XY), cyz = C(DC_YZ), cxz = C(DC_XZ);
   const float h1p = cxx * pxx + cyy * pyy + czz * pzz + cxy * pxy + cyz * pyz + cxz * pxz;

@@ -11,26 +11,26 @@ constexpr int kTileX = 32;   // tile width in x: one warp per tile row
 constexpr int kNumCoef = 10;
 
 // Device coefficient block layout: [z][y][t][c][32], c in this order and t the
-// tile column of cell x (32 cells, the tiles of the step kernels: t =
-// (x + kCoefShift) / 32), so that the coefficients a tile row needs together
-// are contiguous: 384 bytes of the first three, read when a plane arrives
-// (in-plane terms), and 896 of the other seven, read when the plane is updated
-// four planes later.  Against ten separate planes ([z][c][y][x], 128 bytes at
-// a time): 504^3 1.865 -> 1.792 ms a step (and up to 2.03 ms before on other
-// boxes), 128^3 + shell 82.0 -> 76.4 us.
+// tile column of the step kernels (32 cells, from x = kRadius + 32 t; the
+// kRadius columns before the first tile, which no step reads, follow the row's
+// last cell), so that the coefficients a tile row needs together are
+// contiguous: 384 bytes of the first three, read when a plane arrives (in-plane
+// terms), and 896 of the other seven, read when the plane is updated four planes
+// later.  Against ten separate planes ([z][c][y][x], 128 bytes at a time), of
+// the same size: 504^3 1.865 -> 1.792 ms a step (and up to 2.03 ms before on
+// other boxes), 128^3 + shell 82.0 -> 76.4 us.
 enum DevCoef {
   DC_XX = 0, DC_YY, DC_XY,                    // arrival: ch1dxx ch1dyy ch1dxy
   DC_ZZ, DC_XZ, DC_YZ, DC_V2PX, DC_V2PZ, DC_V2SZ, DC_V2PN  // update
 };
-constexpr int kCoefShift = kTileX - kRadius;  // tiles start at x = kRadius + 32 t
-__host__ __device__ inline int coef_tiles(int pitch) { return pitch / kTileX + 1; }
-// Floats of the block; index of coefficient 0 of cell (x, y, z), that of
-// coefficient c being kTileX * c further.
+__host__ __device__ inline int coef_tiles(int pitch) { return pitch / kTileX; }
+// Floats of the block; column of cell x in its row; index of coefficient 0 of a
+// column of row (y, z), that of coefficient c being kTileX * c further.
 __host__ __device__ inline size_t coef_floats(int sy, int sz, int pitch) {
   return (size_t)sz * sy * coef_tiles(pitch) * (kNumCoef * kTileX);
 }
-__host__ __device__ inline size_t coef_index(int x, int y, int z, int sy, int pitch) {
-  const int xs = x + kCoefShift;
+__host__ __device__ inline int coef_column(int x, int sx) { return x >= kRadius ? x - kRadius : sx - kRadius + x; }
+__host__ __device__ inline size_t coef_index(int xs, int y, int z, int sy, int pitch) {
   return (((size_t)z * sy + y) * coef_tiles(pitch) + xs / kTileX) * (kNumCoef * kTileX) + xs % kTileX;
 }
 constexpr int kArrivalCoef = 3;

@@ -77,7 +77,7 @@ __device__ __forceinline__ void issue_step(unsigned char *stage, uint64_t *bar, 
   const bool upd = (k - kLag >= it.z0);
   const uint32_t bytes =
       G::HALO_B + (center ? G::ARR_B + G::ID_B : 0) + (upd ? G::UPD_B + G::PP_B + G::ID_B : 0);
-  const int ct = (it.x0 + kCoefShift) / kTileX;  // tile column in the coefficient block
+  const int ct = (it.x0 - kRadius) / kTileX;  // tile column in the coefficient block
   mbar_arrive_expect_tx(bar, bytes);
   tma_load_3d(stage, m.cur, bar, it.x0 - kRadius, it.y0 - kRadius, k);
   if constexpr (MT) {

@@ -226,7 +226,7 @@ __device__ __forceinline__ void issue_half(unsigned char *stage, uint64_t *bar, 
   mbar_arrive_expect_tx(bar, bytes);
   tma_load_3d(stage, &M.cur_hi, bar, it.x0 - kRadius, it.y0 - kRadius, k);
   if constexpr (EXT) tma_load_3d(stage + G::OFF_LO, &M.cur_lo, bar, it.x0 - kRadius, it.y0 - kRadius, k);
-  const int ct = (it.x0 + kCoefShift) / kTileX;  // tile column in the coefficient block
+  const int ct = (it.x0 - kRadius) / kTileX;  // tile column in the coefficient block
   if (center) tma_load_4d(stage + G::OFF_ARR, &M.arr, bar, 0, ct, it.y0, k);
   if (upd) {
     tma_load_4d(stage + G::OFF_UPD, &M.upd, bar, kArrivalCoef * kTileX, ct, it.y0, k - kRadius);

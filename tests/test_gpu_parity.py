@@ -389,3 +389,39 @@ def test_last_tile_row_with_few_rows(ny, orc):
     ref = orc.run_f32(prob, m)
     for a, b in zip(got, ref):
         assert rel_l2(a, b) < TOL_SHORT
+
+
+@pytest.mark.parametrize("sx", [9, 28, 32, 33, 36, 37, 64, 65, 96, 97, 100])
+def test_coefficient_block_holds_each_row_in_its_pitch(sx, orc):
+    """The coefficient block takes ten floats per cell of the pitched grid, no
+    more, and holds every cell's terms, those of the four columns before the
+    first tile too (angles that differ by column, so the media table's entries
+    come from every column)."""
+    sy, sz, bord = 23, 18, 4
+    n, pitched = sx * sy * sz, (sx + 31) // 32 * 32 * sy * sz
+    g = np.random.default_rng(sx)
+    m = np.empty((6, n), np.float32)
+    m[0] = g.uniform(1500, 4000, n)
+    m[1] = m[0] * 0.5
+    m[2] = g.uniform(0, 0.3, n)
+    m[3] = m[2] * g.uniform(0, 1, n).astype(np.float32)
+    m[4] = np.tile(g.uniform(-np.pi, np.pi, sx), sy * sz)
+    m[5] = np.tile(g.uniform(-np.pi / 2, np.pi / 2, sx), sy * sz)
+    fields = [(1e-3 * g.standard_normal(n)).astype(np.float32) for _ in range(4)]
+    ref = orc.precompute(m)
+    out = []
+    for layout in ("planes", "media"):
+        prop = Propagator(coef_layout=layout)
+        prop.initialize(sx, sy, sz, bord, 12.5, 12.5, 12.5, 0.0006, m, *fields)
+        if layout == "planes":
+            assert prop.device_bytes() == 2 * 8 * pitched + 40 * pitched + 4 * n
+        got = prop.coefficients()
+        ulp = np.abs(got.view(np.int32).astype(np.int64) - ref.view(np.int32).astype(np.int64))
+        assert ulp.max() <= 1 and np.count_nonzero(ulp) <= 1e-4 * ulp.size + 2
+        prop.run(5)
+        prop.synchronize()
+        out.append([prop.field(k) for k in range(4)])
+        prop.finalize()
+    Propagator()
+    for a, b in zip(*out):
+        assert np.isfinite(a).all() and np.array_equal(a, b)
