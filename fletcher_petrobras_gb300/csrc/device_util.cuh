@@ -90,25 +90,6 @@ template <int N>
 __device__ __forceinline__ void setmaxnreg_dec() {
   asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(N));
 }
-// Orders: the values in `v` have been produced (their loads have returned)
-// before any later volatile asm executes.
-__device__ __forceinline__ void consumed(unsigned long long v) { asm volatile("" ::"l"(v)); }
-__device__ __forceinline__ void consumed(float v) { asm volatile("" ::"f"(v)); }
-__device__ __forceinline__ unsigned atom_add_relaxed_cta(unsigned *p, unsigned v) {
-  unsigned old;
-  asm volatile("atom.relaxed.cta.shared::cta.add.u32 %0, [%1], %2;" : "=r"(old) : "r"(smem_addr(p)), "r"(v) : "memory");
-  return old;
-}
-
-// Shared-memory atomic add with acquire-release semantics at CTA scope:
-// orders this thread's earlier shared-memory reads before the increment and
-// makes the other threads' released reads visible to the one that sees the
-// final count.
-__device__ __forceinline__ unsigned atom_add_acq_rel_cta(unsigned *p, unsigned v) {
-  unsigned old;
-  asm volatile("atom.acq_rel.cta.shared::cta.add.u32 %0, [%1], %2;" : "=r"(old) : "r"(smem_addr(p)), "r"(v) : "memory");
-  return old;
-}
 
 // ---- dependent launches ----------------------------------------------------
 // A step's launch may start while the launch before it still runs
@@ -176,6 +157,5 @@ __device__ __forceinline__ f2 fma2(f2 a, f2 b, f2 c) {
   asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r.v) : "l"(a.v), "l"(b.v), "l"(c.v));
   return r;
 }
-__device__ __forceinline__ f2 ld_shared2(const f2 *p) { return *p; }
 
 }  // namespace flt
