@@ -294,9 +294,9 @@ __global__ void __launch_bounds__(RegsH<TY, EXT>::kThreads, 1)
       // ---- producer ----
       // (One thread, or with OWN_SCALES its warp: lane 0 issues and stores.)
       if (!OWN_SCALES && lx != 0) return;
-      auto maps_of = [&](int shot) -> const HalfMaps & {
-        if constexpr (BATCH) return H.hmaps[shot].m[P.parity];
-        else return M;
+      auto maps_of = [&](int shot) -> const HalfMaps * {
+        if constexpr (BATCH) return &H.hmaps[shot].m[P.parity];
+        else return &M;
       };
       // What the scales of step k of an item need, by lane, loaded a step ahead:
       // lanes 0..8 the current field's maxima within 4 planes of the plane
@@ -329,7 +329,7 @@ __global__ void __launch_bounds__(RegsH<TY, EXT>::kThreads, 1)
       int k = it.z0 - kRadius, i = 0, issued = 0;
       unsigned sv = 0u;
       if constexpr (OWN_SCALES) sv = load_scales(it, k);
-      if (lx == 0) prefetch_maps<EXT>(maps_of(it.shot));
+      if (lx == 0) prefetch_maps<EXT>(*maps_of(it.shot));
       bool ok = true;
       while (i < nitems) {
         // The step's scales, then the next step's loads, before the wait: the
@@ -357,7 +357,7 @@ __global__ void __launch_bounds__(RegsH<TY, EXT>::kThreads, 1)
             next = seg[i + 1];
             // Batched shots keep their tensor maps in global memory: fetch the
             // next item's into the descriptor cache an item ahead.
-            if constexpr (BATCH) prefetch_maps<EXT>(maps_of(decode_hitem<BATCH>(next).shot));
+            if constexpr (BATCH) prefetch_maps<EXT>(*maps_of(decode_hitem<BATCH>(next).shot));
           }
         }
         if constexpr (OWN_SCALES) {
@@ -378,7 +378,7 @@ __global__ void __launch_bounds__(RegsH<TY, EXT>::kThreads, 1)
           *plane_of(st) = make_int2(upd ? zc : -1, cit.shot);
           if constexpr (OWN_SCALES) *scale_of(st) = scl;
           if (!HOOK || issued != P.stall_step || blockIdx.x != 0)
-            issue_half<TY, EXT>(st, bar(st, L::OFF_FULL), cit, ck, maps_of(cit.shot));
+            issue_half<TY, EXT>(st, bar(st, L::OFF_FULL), cit, ck, *maps_of(cit.shot));
           fold_max(pl, sc, v);
           if (OWN_SCALES && upd) {
             // Every CTA of the plane finds and stores the same.
@@ -550,7 +550,7 @@ __global__ void __launch_bounds__(RegsH<TY, EXT>::kThreads, 1)
     const int gy = it.y0 + ly;
     const bool valid = (gx >= sd.bord) && (gx < sd.sx - sd.bord) && (gy >= sd.bord) && (gy < sd.sy - sd.bord);
     const long plane = (long)sd.pitch * sd.sy;
-    long o = it.z0 * plane + (long)gy * sd.pitch + gx;
+    long at = it.z0 * plane + (long)gy * sd.pitch + gx;
     unsigned *const out_hi = BATCH ? H.hshots[it.shot].hi[1 - P.parity] : H.out_hi;
     unsigned short *const out_lo = BATCH ? H.hshots[it.shot].lo[1 - P.parity] : H.out_lo;
     // The cell that lacks the last step's source, if it is this thread's.
@@ -652,10 +652,10 @@ __global__ void __launch_bounds__(RegsH<TY, EXT>::kThreads, 1)
           unsigned short orv;
           encode<EXT>(nw, sc.z, ohv, orv);
           if (valid) {
-            out_hi[o] = ohv;
-            if constexpr (EXT) out_lo[o] = orv;
+            out_hi[at] = ohv;
+            if constexpr (EXT) out_lo[at] = orv;
           }
-          o += plane;
+          at += plane;
           // The warp's largest magnitude: the bits of non-negative floats
           // order like the floats, so one integer warp reduction finds it
           // (a NaN, above every finite value, reaches the range check).
