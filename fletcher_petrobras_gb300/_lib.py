@@ -85,6 +85,7 @@ SIGNATURES = {
     "FLETCHER_AbcGetSamples": (C.c_int, [C.c_long, C.c_long, FP, FP, IP]),
     "FLETCHER_AbcTrain": (C.c_int, [C.c_int, C.c_int, C.c_float, C.c_uint, C.c_float, FP]),
     "FLETCHER_AbcGradient": (C.c_int, [FP, FP, C.c_int, FP, FP]),
+    "FLETCHER_AbcGradientBytes": (C.c_size_t, [C.c_int]),
     "FLETCHER_AbcForward": (C.c_int, [FP, C.c_int, FP]),
     "FLETCHER_SetBoundary": (C.c_int, [C.c_int, C.c_int, C.c_float]),
     "FLETCHER_PlanShot": (C.c_int, [C.c_int] * 10 + [IP, C.c_int, IP, C.POINTER(C.c_long)]),

@@ -1105,14 +1105,17 @@ __global__ void k_abc_fill(const __grid_constant__ Ghost G, const float *coef, i
 
 // A training block: kTB samples with kTG threads each, which take the outputs
 // of a layer in kTG equal parts.  64 samples a block rather than 128 give
-// 8192 samples 128 blocks (of 152 SMs).
+// 8192 samples 128 blocks (of 152 SMs).  Two blocks, a cluster, write one set of
+// sums: the allocator hands out 2 MB at a time, and a call whose memory crosses
+// that takes 0.1 ms more (with a set a block, 6528 to 8100 samples took 220
+// instead of 112 us).
 constexpr int kTB = 64, kTG = 4, kTT = kTB * kTG;
 constexpr int kTO = kHid / kTG;  // a thread's outputs of a hidden layer
-// More samples than kTrainOnce blocks take (their sums fit the 2 MB that the
-// allocator hands out at once: 14 394 samples 515 -> 470 us a gradient and
-// outputs, of which most is copies) run on a block an SM, several chunks of
-// kTB each.  Fewer take a chunk a block: 8192 samples 306 us, 316 in the loop.
-constexpr int kTrainOnce = 208, kTrainLoop = 152;
+// More samples than kTrainOnce blocks take run on kTrainLoop blocks, several
+// chunks of kTB each; fewer take a chunk a block.  (152: the GB300's SMs, and
+// fixed, so that the sums and their order are the same everywhere.)
+constexpr int kCluster = 2, kTrainOnce = 208, kTrainLoop = 152;
+static_assert(kTrainOnce % kCluster == 0 && kTrainLoop % kCluster == 0, "whole clusters");
 static_assert(kTO % 4 == 0 && kTG >= kOut && kTB % 32 == 0, "float4 stores; an output layer's row per group of warps");
 constexpr int sX = 44, sH = 36;  // row strides in floats: rows 16-byte aligned, float4 reads of 8 rows conflict-free
 
@@ -1161,18 +1164,18 @@ __device__ __forceinline__ void load_row(const float *row, float (&x)[K]) {
 
 // Forward and backward of B samples (index b of the batch: a random sample,
 // or b itself when seed is 0): each block writes its part of the loss
-// sum_c (sigmoid(y_c) a_c - b_c)^2 / (2 B) and of the gradient to its own
-// slots of lpartial and partial.  Weights are used FP16-rounded, hidden
+// sum_c (sigmoid(y_c) a_c - b_c)^2 / (2 B) and of the gradient to its cluster's
+// row of partial (the gradient, then the loss).  Weights are used FP16-rounded, hidden
 // pre-activations and activations are rounded to FP16 (as inference does),
 // the derivatives treat the roundings as the identity.  noise > 0 perturbs the
 // stencil inputs.  What bounds it: the shared-memory reads of a sample's chain
 // and of the sums; with one scalar read an operand and one thread a
 // sample it took 41 us for 8192 samples; float4 reads and 4 x 4 register tiles
-// of the sums brought 26 us, four threads a sample 15.5 us.
+// of the sums brought 26 us, four threads a sample 15.7 us, 16.4 with the
+// cluster's exchange.
 template <bool LOOP>
-__global__ void __launch_bounds__(kTT) k_abc_train(const float *feat, const float *tgt, long nsamp, int B,
-                                                    uint32_t seed, const float *P, float noise, float *partial,
-                                                    float *lpartial) {
+__global__ void __cluster_dims__(kCluster, 1, 1) __launch_bounds__(kTT) k_abc_train(const float *feat, const float *tgt, long nsamp, int B,
+                                                    uint32_t seed, const float *P, float noise, float *partial) {
   extern __shared__ __align__(16) float sm[];
   float *X = sm, *H1 = X + kTB * sX, *D1 = H1 + kTB * sH, *H2 = D1 + kTB * sH, *D2 = H2 + kTB * sH;
   float *W1 = D2 + kTB * sH, *W2 = W1 + kHid * kIn, *W3 = W2 + kHid * kHid;
@@ -1340,19 +1343,32 @@ __global__ void __launch_bounds__(kTT) k_abc_train(const float *feat, const floa
       }
     }
   } while (LOOP && (long)(chunk += gridDim.x) * kTB < B);
-  // The block's loss and gradient sums go to its own slots (summed over the
-  // blocks in order by k_abc_reduce: the result does not depend on timing).
+  // The cluster's loss and gradient sums go to its own row (summed over the
+  // clusters in order by k_abc_reduce: the result does not depend on timing).
+  // The second block hands its sums to the first through that one's shared
+  // memory, thread by thread, where X and H1 have been read.
+  static_assert(16 * kTT + 1 <= kTB * (sX + sH), "the handed sums fit X and H1");
   if (grp < kOut) {
     for (int m = 16; m > 0; m >>= 1) l += __shfl_xor_sync(0xffffffffu, l, m);
     if ((tid & 31) == 0) wl[tid >> 5] = l;
   }
-  __syncthreads();
-  if (tid == 0) {
-    float bl = 0.f;
+  cluster_barrier();
+  float bl = 0.f;
+  if (tid == 0)
     for (int w = 0; w < kOut * kTB / 32; ++w) bl += wl[w];
-    lpartial[blockIdx.x] = bl / (2.0f * (float)B);
+  const bool second = blockIdx.x & 1;
+  if (second) {
+    const uint32_t to0 = peer_smem_addr(sm, 0);
+#pragma unroll
+    for (int v = 0; v < 16; ++v) st_cluster(to0 + 4u * (v * kTT + tid), gs[v / 4][v % 4]);
+    if (tid == 0) st_cluster(to0 + 4u * 16 * kTT, bl);
   }
-  float *out = partial + (size_t)blockIdx.x * kNP;
+  cluster_barrier();
+  if (second) return;
+#pragma unroll
+  for (int v = 0; v < 16; ++v) gs[v / 4][v % 4] += sm[v * kTT + tid];
+  float *out = partial + (size_t)(blockIdx.x / kCluster) * (kNP + 1);
+  if (tid == 0) out[kNP] = (bl + sm[16 * kTT]) / (2.0f * (float)B);
   if (tid < kT1 + kT2) {
     float *dst = out + (first ? oW1 : oW2) + to * nk + tk;
 #pragma unroll
@@ -1370,20 +1386,20 @@ __global__ void __launch_bounds__(kTT) k_abc_train(const float *feat, const floa
   }
 }
 
-// Sums of the training blocks' partial gradients and losses, in block order:
+// Sums of the training clusters' partial gradients and losses, in order:
 // a block takes 32 parameters, its 8 warps a contiguous eighth of the
-// training blocks each, added up in order (5.9 us with one thread a
-// parameter, 3.7 us so).
+// clusters each, added up in order (5.9 us with one thread a
+// parameter, 3.7 us so, 3.0 with half as many rows).
 constexpr int kReduceWarps = 8;
-__global__ void __launch_bounds__(32 * kReduceWarps) k_abc_reduce(const float *partial, const float *lpartial,
-                                                                   int nblocks, float *grad, float *loss) {
+__global__ void __launch_bounds__(32 * kReduceWarps) k_abc_reduce(const float *partial, int nparts, float *grad,
+                                                                   float *loss) {
   __shared__ float part[kReduceWarps][33];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   const int e = blockIdx.x * 32 + lane;  // kNP is the loss
-  const int b0 = (int)((long)nblocks * w / kReduceWarps), b1 = (int)((long)nblocks * (w + 1) / kReduceWarps);
+  const int b0 = (int)((long)nparts * w / kReduceWarps), b1 = (int)((long)nparts * (w + 1) / kReduceWarps);
   float g = 0.f;
   if (e <= kNP)
-    for (int b = b0; b < b1; ++b) g += e < kNP ? partial[(size_t)b * kNP + e] : lpartial[b];
+    for (int b = b0; b < b1; ++b) g += partial[(size_t)b * (kNP + 1) + e];
   part[w][lane] = g;
   __syncthreads();
   if (w == 0 && e <= kNP) {
@@ -1511,16 +1527,17 @@ int grid_of(long n, int block) {
   return (int)(b < 1 ? 1 : (b > 4096 ? 4096 : b));
 }
 
-int train_blocks(int n) {
+// Clusters that n samples take, a set of sums each.
+int train_parts(int n) {
   const int chunks = (n - 1) / kTB + 1;
-  return chunks <= kTrainOnce ? chunks : kTrainLoop;
+  return (chunks <= kTrainOnce ? chunks + kCluster - 1 : kTrainLoop) / kCluster;
 }
 
 void launch_train(const float *feat, const float *tgt, long nsamp, int B, uint32_t seed, float noise, float *partial,
-                  float *lpartial, cudaStream_t s) {
-  const int blocks = train_blocks(B);
-  const auto kern = blocks * kTB < B ? k_abc_train<true> : k_abc_train<false>;
-  kern<<<blocks, kTT, kTrainSmem, s>>>(feat, tgt, nsamp, B, seed, T.P, noise, partial, lpartial);
+                  cudaStream_t s) {
+  const int blocks = train_parts(B) * kCluster;
+  const auto kern = (long)blocks * kTB < B ? k_abc_train<true> : k_abc_train<false>;
+  kern<<<blocks, kTT, kTrainSmem, s>>>(feat, tgt, nsamp, B, seed, T.P, noise, partial);
 }
 
 int train_attr() {
@@ -1716,17 +1733,16 @@ extern "C" int FLETCHER_AbcTrain(int iters, int batch, float lr, unsigned seed, 
     return err(FLETCHER_ERR_ARGS, "AbcTrain: bad arguments");
   cudaStream_t s = stream_of();
   if (train_attr()) return FLETCHER_GetLastError();
-  const int blocks = train_blocks(batch);
-  float *loss = nullptr, *partial = nullptr, *lpartial = nullptr;
+  const int parts = train_parts(batch);
+  float *loss = nullptr, *partial = nullptr;
   CKA(cudaMalloc(&loss, iters * sizeof(float)));
-  CKA(cudaMalloc(&partial, (size_t)blocks * kNP * sizeof(float)));
-  CKA(cudaMalloc(&lpartial, blocks * sizeof(float)));
+  CKA(cudaMalloc(&partial, (size_t)parts * (kNP + 1) * sizeof(float)));
   const float b1 = 0.9f, b2 = 0.999f;
   for (int it = 0; it < iters; ++it) {
     uint64_t st = (uint64_t)seed * 1000003ull + (uint64_t)it;
     const uint32_t sd = (uint32_t)splitmix(st) | 1u;
-    launch_train(T.feat, T.tgt, ns, batch, sd, noise, partial, lpartial, s);
-    k_abc_reduce<<<kReduceBlocks, 32 * kReduceWarps, 0, s>>>(partial, lpartial, blocks, T.grad, loss + it);
+    launch_train(T.feat, T.tgt, ns, batch, sd, noise, partial, s);
+    k_abc_reduce<<<kReduceBlocks, 32 * kReduceWarps, 0, s>>>(partial, parts, T.grad, loss + it);
     ++T.adam_t;
     const float lr_t = lr * 0.5f * (1.0f + cosf(3.14159265f * (float)it / (float)iters));
     k_abc_adam<<<(kNP + 255) / 256, 256, 0, s>>>(T.P, T.grad, T.m, T.v, kNP, lr_t, b1, b2, 1e-8f,
@@ -1738,7 +1754,6 @@ extern "C" int FLETCHER_AbcTrain(int iters, int batch, float lr, unsigned seed, 
   CKA(cudaStreamSynchronize(s));
   cudaFree(loss);
   cudaFree(partial);
-  cudaFree(lpartial);
   return FLETCHER_OK;
 }
 
@@ -1746,28 +1761,29 @@ extern "C" int FLETCHER_AbcGradient(const float *feat, const float *tgt, int n, 
   if (!T.weights) return err(FLETCHER_ERR_ARGS, "AbcGradient: no network");
   if (!feat || !tgt || !grad || n < 1) return err(FLETCHER_ERR_ARGS, "AbcGradient: bad arguments");
   if (train_attr()) return FLETCHER_GetLastError();
-  const int blocks = train_blocks(n);
-  float *df = nullptr, *dt = nullptr, *dl = nullptr, *dg = nullptr, *partial = nullptr, *lpartial = nullptr;
+  const int parts = train_parts(n);
+  // The sums, then one more row: the gradient and the loss.
+  float *df = nullptr, *dt = nullptr, *partial = nullptr;
   CKA(cudaMalloc(&df, (size_t)n * kIn * sizeof(float)));
   CKA(cudaMalloc(&dt, (size_t)n * kTgt * sizeof(float)));
-  CKA(cudaMalloc(&dl, sizeof(float)));
-  CKA(cudaMalloc(&dg, kNP * sizeof(float)));
-  CKA(cudaMalloc(&partial, (size_t)blocks * kNP * sizeof(float)));
-  CKA(cudaMalloc(&lpartial, blocks * sizeof(float)));
+  CKA(cudaMalloc(&partial, (size_t)(parts + 1) * (kNP + 1) * sizeof(float)));
+  float *dg = partial + (size_t)parts * (kNP + 1);
   CKA(cudaMemcpy(df, feat, (size_t)n * kIn * sizeof(float), cudaMemcpyHostToDevice));
   CKA(cudaMemcpy(dt, tgt, (size_t)n * kTgt * sizeof(float), cudaMemcpyHostToDevice));
-  launch_train(df, dt, n, n, 0u, 0.f, partial, lpartial, 0);
-  k_abc_reduce<<<kReduceBlocks, 32 * kReduceWarps>>>(partial, lpartial, blocks, dg, dl);
+  launch_train(df, dt, n, n, 0u, 0.f, partial, 0);
+  k_abc_reduce<<<kReduceBlocks, 32 * kReduceWarps>>>(partial, parts, dg, dg + kNP);
   CKA(cudaGetLastError());
   CKA(cudaMemcpy(grad, dg, kNP * sizeof(float), cudaMemcpyDeviceToHost));
-  if (loss) CKA(cudaMemcpy(loss, dl, sizeof(float), cudaMemcpyDeviceToHost));
+  if (loss) CKA(cudaMemcpy(loss, dg + kNP, sizeof(float), cudaMemcpyDeviceToHost));
   cudaFree(df);
   cudaFree(dt);
-  cudaFree(dl);
-  cudaFree(dg);
   cudaFree(partial);
-  cudaFree(lpartial);
   return FLETCHER_OK;
+}
+
+extern "C" size_t FLETCHER_AbcGradientBytes(int n) {
+  if (n < 1) return 0;
+  return sizeof(float) * ((size_t)n * (kIn + kTgt) + (size_t)(train_parts(n) + 1) * (kNP + 1));
 }
 
 extern "C" int FLETCHER_AbcForward(const float *feat, int n, float *out) {

@@ -509,6 +509,8 @@ int FLETCHER_AbcTrain(int iters, int batch, float lr, unsigned seed, float noise
  * targets [n][4]): loss = sum_c (sigmoid(y_c) a_c - b_c)^2 / (2 n) and its
  * gradient with respect to the master weights. */
 int FLETCHER_AbcGradient(const float *features, const float *targets, int n, float *grad, float *loss);
+/* Device memory that such a call on n samples takes (and gives back). */
+size_t FLETCHER_AbcGradientBytes(int n);
 
 /* The inference path (tensor cores) on n given feature rows: raw outputs
  * y [n][2] (k = sigmoid(y)). */

@@ -121,3 +121,13 @@ def test_boundary_arguments_are_checked_on_the_host(lib):
     assert lib.FLETCHER_SetBoundary(7, 8, 0.0) != 0
     lib.FLETCHER_ClearError()
     assert lib.FLETCHER_AbcLayerCells() == 0
+
+
+def test_gradient_scratch_is_one_set_of_sums_per_128_samples(lib):
+    """What a gradient of n samples takes besides its inputs and outputs: a set
+    of 2434 sums and a loss for every 128 samples, at most (the allocator hands
+    out 2 MB at a time; a call that crosses that takes twice as long)."""
+    for n in (1, 63, 64, 65, 128, 129, 6528, 8192, 13312, 13313, 60000, 2 ** 31 - 1):
+        scratch = lib.FLETCHER_AbcGradientBytes(n) - 4 * (44 * n + 2434 + 1)
+        assert 0 < scratch <= 4 * 2435 * (-(-n // 128))
+    assert lib.FLETCHER_AbcGradientBytes(0) == 0
