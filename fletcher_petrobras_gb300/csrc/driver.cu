@@ -1634,6 +1634,7 @@ struct BatchShot {
   unsigned short *Hl[2] = {nullptr, nullptr};
   int *E = nullptr;
   unsigned *Mx = nullptr;
+  int mslot[2] = {-1, -1};  // Mx slot of the maxima of the field in buffer b (-1: zero everywhere)
   float *coef = nullptr;
 };
 
@@ -1985,6 +1986,38 @@ int batch_auto_chains(int steps) {
   return nfill > 1 && fill_cells <= kTwoChainCells * nfill ? 2 : 1;
 }
 
+// The maxima of the 16-bit fields, to where the schedule looks for them at its
+// first step: slots 0 and 1, by buffer (persistent launch), or 0 and 3, the
+// other two cleared (chains).  A batch that has run before may have left them
+// elsewhere.
+int place_maxima(bool chains) {
+  for (BatchShot &s : B.shots) {
+    const int want[2] = {0, chains ? 3 : 1};
+    if (s.mslot[0] >= 0 && (chains || s.mslot[0] != want[0] || s.mslot[1] != want[1])) {
+      unsigned *tmp = reinterpret_cast<unsigned *>(B.scratch);  // a shot's cells
+      const size_t bytes = s.sz * sizeof(unsigned);
+      for (int b = 0; b < 2; ++b)
+        CK(cudaMemcpyAsync(tmp + b * s.sz, s.Mx + s.mslot[b] * s.sz, bytes, cudaMemcpyDeviceToDevice, g_stream));
+      CK(cudaMemsetAsync(s.Mx, 0, 4 * bytes, g_stream));
+      for (int b = 0; b < 2; ++b)
+        CK(cudaMemcpyAsync(s.Mx + want[b] * s.sz, tmp + b * s.sz, bytes, cudaMemcpyDeviceToDevice, g_stream));
+    }
+    s.mslot[0] = want[0];
+    s.mslot[1] = want[1];
+  }
+  return FLETCHER_OK;
+}
+
+// Where a run of `steps` steps on chains leaves them: the field of step it in
+// slot it % 4.
+void chained_maxima(int steps) {
+  for (BatchShot &s : B.shots) {
+    const int n = std::min(s.nsteps, steps);
+    s.mslot[n & 1] = n % 4;
+    s.mslot[1 - (n & 1)] = (n + 3) % 4;
+  }
+}
+
 int batch_max_steps() {
   int m = 0;
   for (auto &s : B.shots) m = std::max(m, s.nsteps);
@@ -2307,6 +2340,7 @@ extern "C" int FLETCHER_BatchReset(void) {
     }
     if (s.E) CK(cudaMemsetAsync(s.E, 0, 3 * s.sz * sizeof(int), g_stream));
     if (s.Mx) CK(cudaMemsetAsync(s.Mx, 0, 4 * s.sz * sizeof(unsigned), g_stream));
+    s.mslot[0] = s.mslot[1] = -1;
   }
   CK(cudaStreamSynchronize(g_stream));
   return FLETCHER_OK;
@@ -2336,6 +2370,7 @@ extern "C" int FLETCHER_BatchRun(const float *src, int max_steps, int use_graph,
       propagate_half_prepare(B.sealed_rows, B.stages, B.form == FLETCHER_FORM_FP16X, false) != cudaSuccess)
     return fail(FLETCHER_ERR_CUDA, "kernel attribute set-up failed");
   if (chains ? batch_single_plans(B.ctas) : batch_plan(B.ctas)) return g_last_err;
+  if (batch_half() && place_maxima(chains)) return g_last_err;
   auto issue = [&]() { return chains ? batch_issue_chains(nchains, steps, src) : batch_issue(0, steps, src); };
   cudaEvent_t e0, e1;
   CK(cudaEventCreate(&e0));
@@ -2359,6 +2394,7 @@ extern "C" int FLETCHER_BatchRun(const float *src, int max_steps, int use_graph,
     return g_last_err;
   }
   CK(cudaEventRecord(e1, g_stream));
+  if (batch_half() && chains) chained_maxima(steps);
   CK(cudaStreamSynchronize(g_stream));
   float ms = 0.f;
   CK(cudaEventElapsedTime(&ms, e0, e1));

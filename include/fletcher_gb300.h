@@ -357,7 +357,9 @@ int FLETCHER_BatchLastChains(void);
  * assumes a full run): step it adds src[it] at each running shot's source
  * cell (the reference's InsertSource) then advances.  use_graph != 0
  * captures the loop in a CUDA graph first.  *elapsed_ms (may be NULL) =
- * device time of the loop. */
+ * device time of the loop.  FLETCHER_BatchReset comes before another run from
+ * zero; without it a run finds the last one's fields where step 0 looks for
+ * them only after an even number of steps (16-bit forms: a multiple of 6). */
 int FLETCHER_BatchRun(const float *src, int max_steps, int use_graph, float *elapsed_ms);
 /* Zeroes every shot's fields (the coefficients stay). */
 int FLETCHER_BatchReset(void);

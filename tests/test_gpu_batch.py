@@ -262,3 +262,27 @@ def test_default_schedule_takes_two_chains_for_two_filling_shots(n, shots, chain
     batch.close()
     for p, m, f in zip(probs, models, got):
         assert np.array_equal(f, single(p, m, form)[0])
+
+
+@pytest.mark.parametrize("form", ["fp16", "fp16x"])
+@pytest.mark.parametrize("steps", [6, 12, 18])
+def test_second_run_is_the_same_in_every_schedule(steps, form):
+    """A run from the state that another run left, in the same schedule or not:
+    the planes' largest magnitudes are found where that run put them, so the
+    fields are those of two persistent runs, bit for bit."""
+    shots = [p.with_(steps=steps) for p in SHOTS[:2]]
+    models = [p.model() for p in shots]
+    out = []
+    for first, second in ((0, 0), (1, 1), (2, 2), (0, 1), (1, 0)):
+        batch = Batch(form=form, chains=first)
+        for p, m in zip(shots, models):
+            batch.add(p, m)
+        batch.run()
+        assert batch.lib.FLETCHER_BatchSetChains(second) == 0
+        batch.run()
+        out.append([batch.field(i, k) for i in range(len(shots)) for k in range(4)])
+        batch.close()
+    assert np.abs(out[0][0]).max() > 0
+    for got in out[1:]:
+        for a, b in zip(got, out[0]):
+            assert np.array_equal(a, b)
