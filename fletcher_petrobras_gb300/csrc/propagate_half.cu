@@ -14,8 +14,8 @@
 // significand for every value (3 bytes per value).
 //
 // The CTA is warp-specialised as in propagate_fp32.cu: a producer thread
-// issues the TMA loads, the decode warps (three helper warps) turn the (p, q)
-// halo tile of the arriving plane into an FP32 shared-memory tile, once per
+// issues the TMA loads, the decode warps (three or seven helper warps, RegsH)
+// turn the (p, q) halo tile of the arriving plane into an FP32 shared-memory tile, once per
 // cell, and evaluate D1y in its halo columns, and TY compute warps run the
 // FP32 stencil on it.  The updated plane is encoded with its new scale, and
 // the CTA's largest magnitude on it is folded (atomicMax) into the per-plane
@@ -24,7 +24,7 @@
 //
 // What bounds it: FP16 the shared-memory pipe (80% busy) and issue (68%),
 // with the FP32 stencil's reads plus the decode; FP16X issue (its decode and
-// encode).  272^3 updated cells: FP16 230 us a step, FP16X 280, against 337
+// encode).  272^3 updated cells: FP16 229 us a step, FP16X 275, against 337
 // and 377 us when all 16 warps decoded each plane between two CTA-wide
 // barriers.  The residual bytes take no conversion instruction (decode,
 // encode): 12 of 310 us.  Four decoded tiles instead of three: FP16 244 ->
