@@ -107,7 +107,7 @@ struct LayoutH {
 // sub-partition share what the launch gives them.
 // FP16X at 16 rows decodes with seven warps (272^3 updated cells: 311 us a
 // step with three of 32 registers, 287 with three of 64, which keep more cells
-// in flight, 280 with seven of 32; its compute warps then spill 32 bytes); FP16
+// in flight, 280 with seven of 32; its compute warps then spill 40 bytes); FP16
 // with three (230 us; 246 with 64 registers, its compute warps at 104).
 template <int TY, bool EXT>
 struct RegsH {
