@@ -17,7 +17,7 @@ LAUNCH = {("fp32", 16): 168, ("fp32", 12): 168, ("fp32", 8): 128, ("d1d1", 16): 
 
 
 @pytest.mark.parametrize("source", ["propagate_fp32", "propagate_d1d1", "propagate_half"])
-def test_launch_registers(source):
+def test_launch_registers(source, lib):
     kind = source.split("_")[1]
     log = open(os.path.join(OUT, source + ".cu.o.log")).read()
     found = re.findall(r"Compiling entry function '\S*k_propagate_%s(\S*)'.*?Used (\d+) registers" % kind, log, re.S)
